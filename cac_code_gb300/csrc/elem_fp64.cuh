@@ -1,0 +1,373 @@
+// FP64 element passes (sm_103a): one block per element, positions of only the
+// sites a row interacts with.
+//
+// Included by two translation units, like force_fp64.cuh: k_force_exact.cu
+// (-fmad=false, FP64_EXACT_TU) keeps the reference's sequence of IEEE
+// operations per pair and its order of summation, so its results are bit for
+// bit the reference's; k_force_fma.cu contracts and uses the refined
+// reciprocals.  The arithmetic follows PairLJCut::ecompute
+// (pair_lj_cut.cpp:295-442), PairEAM::ecompute (pair_eam.cpp:761-1141) and the
+// gather of pair_lj_cut.cpp:424-428.
+//
+// What bounds it: the FP64 unit (a warp instruction holds it for 16 cycles).
+// An interpolated position costs 45 FP64 instructions, and of the 1,331 sites
+// of an 11 x 11 x 11 element the rows of 2 x 2 x 2 Gauss points and 8 nodes
+// reach about 500.  So each row's list is tested in FP32 first, on coordinates
+// relative to the element's node 0 with a bound derived from their size
+// (pass_limit), and only the entries that pass get an FP64 position, formed
+// where the pair is evaluated: no site array, no list of the step in memory,
+// no F'(rho) of sites that nothing reaches.
+//
+// A block takes RB rows at a time.  Its warps scan the rows' lists 32 entries
+// at a time and append what passes, in list order, to the rows' buffers in
+// shared memory; all threads then evaluate the buffered pairs of all rows
+// (full warps whatever a row holds), leave each pair's terms in shared memory,
+// and one thread per row and component adds them in list order.  Rows whose
+// buffer fills up go on where they stopped in a further round.
+#pragma once
+#include "internal.h"
+
+namespace cacg {
+namespace FP64NS {
+
+namespace {
+
+constexpr int RB = 8;           // rows of an element per round
+constexpr int ROW_CAP = 128;    // buffered entries per row
+constexpr int ELEM_NT = 128;    // threads per block
+
+// m = min((int) q, n1) and p = min(q - m, 1): for 1 <= q < 2^20 from the bits
+// of q, without conversions (they issue at the FP64 rate): the integer part is
+// q with the mantissa bits below the point cleared.  low: m is at least that.
+__device__ __forceinline__ int split_index(double q, int n1, int low, double &p) {
+  const int hi = __double2hiint(q);
+  const unsigned e = (unsigned) (hi >> 20) - 1023u;
+  if (e < 20u) {
+    const int sh = 20 - (int) e;
+    const int m = ((hi & 0xFFFFF) | 0x100000) >> sh;
+    if (m <= n1 && m >= low) {
+      p = q - __hiloint2double(hi & (int) (0xFFFFFFFFu << sh), 0);
+      return m;
+    }
+  }
+  int m = (int) q;
+  m = m < n1 ? m : n1;
+  m = low > m ? low : m;
+  p = q - m;
+  p = p < 1.0 ? p : 1.0;
+  return m;
+}
+
+// FP32 limit of the squared distance of two points of an element (coordinates
+// relative to node 0, at most R; absolute coordinates at most X) that FP64
+// arithmetic may place within the cutoff.  With u = 2^-24 a relative node is
+// within u R of its value, an interpolated coordinate within 10 u R (weights
+// >= 0 of sum 1, rounded once, eight products and sums), a difference within
+// 22 u R; FP64 positions are within 12 * 2^-53 X each.  Both bounds are taken
+// with slack, and the sum of squares and the limit itself within 1e-5.
+__device__ __forceinline__ float pass_limit(float cutsq, float R, float X) {
+  const float u = 5.9604645e-8f, v = 1.110223e-16f;
+  const float r = sqrtf(cutsq) * 1.000001f + 1.7320509f * (24.f * u * R + 32.f * v * X);
+  return r * r * 1.00001f;
+}
+
+// w0 x0 + w1 x1 + ... over an element's 8 nodes without contraction in either
+// mode, as the reference interpolates (its first addition, to 0, changes
+// nothing but the sign of a zero).  Coordinates reach 1e3 and more: a fused
+// rounding would move a site by ~1e-13, which the stiff pair forces amplify.
+__device__ __forceinline__ double node_sum(const double (&w)[NPE], const double *__restrict__ x,
+                                           int stride) {
+  double a = __dmul_rn(w[0], x[0]);
+#pragma unroll
+  for (int k = 1; k < NPE; k++) a = __dadd_rn(a, __dmul_rn(w[k], x[stride * k]));
+  return a;
+}
+
+__device__ __forceinline__ void load8(const double *__restrict__ p, double (&w)[NPE]) {
+#pragma unroll
+  for (int k = 0; k < NPE / 2; k++) {
+    const double2 d = __ldg(reinterpret_cast<const double2 *>(p) + k);
+    w[2 * k] = d.x;
+    w[2 * k + 1] = d.y;
+  }
+}
+
+__device__ __forceinline__ double eam_slope(const EamTables &e, double rho) {
+  double p;
+  const int m = split_index(rho * e.rdrho + 1.0, e.nrho - 1, 1, p);
+  const double *c = e.frho + 7 * (size_t) m;
+  return (c[0] * p + c[1]) * p + c[2];
+}
+
+// DENSITY: the 8 node rows of each element -> erho; otherwise the force rows
+// (row list fjj of the type; all rows when it is null) -> nodef.
+// SELF: every list entry is a site of the row's own element.
+template <bool EAM, bool DENSITY, bool SELF>
+__global__ void __launch_bounds__(ELEM_NT)
+k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
+         double *__restrict__ out) {
+  constexpr int NC = DENSITY ? 1 : 3;
+  __shared__ double s_nx[24], s_er[NPE], s_p[RB][3], s_N[RB][NPE], s_fpi[RB], s_f[RB][3];
+  __shared__ double s_t[RB][NC][ROW_CAP + 1];
+  __shared__ int s_ent[RB][ROW_CAP];
+  __shared__ int s_cnt[RB], s_at[RB], s_len[RB], s_start[RB], s_jj[RB];
+  __shared__ float4 s_nf4[6];
+  __shared__ float s_pf[RB][3];
+  __shared__ float s_lim;
+  float *s_nf = reinterpret_cast<float *>(s_nf4);
+  const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ty = a.etype[e], ioff = a.int_off[ty];
+  const int naz = a.nae[3 * ty + 2];
+  const double *__restrict__ S0 = a.spa_inter + (size_t) a.inter_off[ty] * NPE;
+  const float4 *__restrict__ F0 = a.spa_inter_f + (size_t) a.inter_off[ty] * 2;
+  const int kb = a.kb, kmask = (1 << kb) - 1;
+  if (warp == 0) {
+    float r = 0.f, x = 0.f;
+    if (lane < 24) {
+      const double v = a.nodex[24 * (size_t) e + lane];
+      s_nx[lane] = v;
+      const double v0 = __shfl_sync(0x00FFFFFFu, v, lane % 3);
+      const float f = SELF ? (float) (v - v0) : (float) v;
+      s_nf[lane] = f;
+      r = fabsf(f);
+      x = fabsf((float) v);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      r = fmaxf(r, __shfl_xor_sync(0xffffffffu, r, o));
+      x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
+    }
+    if (lane == 0) s_lim = SELF ? pass_limit((float) cutsq, r, x) : a.cut_pass;
+  } else if (warp == 1 && EAM && !DENSITY) {
+    if (lane < NPE) s_er[lane] = a.erho[NPE * (size_t) e + lane];
+  }
+  const int nr_rows = DENSITY ? NPE : (a.fjj ? a.fjj_off[ty + 1] - a.fjj_off[ty] : a.numint[ty]);
+  double nf = 0.0;  // threads 0..23: the nodal force component
+  for (int rb = 0; rb < nr_rows; rb += RB) {
+    const int nb = min(RB, nr_rows - rb);
+    __syncthreads();
+    if (tid < nb) {
+      const int q = rb + tid;
+      const int jj = DENSITY ? a.node_list[ty * NPE + q] : (a.fjj ? a.fjj[a.fjj_off[ty] + q] : q);
+      const int r = a.row_first[e] + jj;
+      s_jj[tid] = jj;
+      s_start[tid] = a.row_start[r];
+      s_len[tid] = a.row_start[r + 1] - a.row_start[r];
+      s_at[tid] = 0;
+    }
+    __syncthreads();
+    // the rows' points: FP64 (a row's node itself in the density pass) and FP32
+    for (int t = tid; t < nb * 3; t += ELEM_NT) {
+      const int r = t / 3, d = t % 3, jj = s_jj[r];
+      const double *N = a.spa_int + ((size_t) ioff + jj) * NPE;
+      double w[NPE];
+      load8(N, w);
+      if (DENSITY) s_p[r][d] = s_nx[3 * (rb + r) + d];
+      else s_p[r][d] = node_sum(w, s_nx + d, 3);
+      float pf = 0.f;
+#pragma unroll
+      for (int k = 0; k < NPE; k++) {
+        if (d == 0) s_N[r][k] = w[k];
+        pf += (float) w[k] * s_nf[3 * k + d];
+      }
+      s_pf[r][d] = pf;
+      if (EAM && !DENSITY && d == 0) {
+        double rho = 0.0;
+#pragma unroll
+        for (int k = 0; k < NPE; k++) rho += w[k] * s_er[k];
+        s_fpi[r] = eam_slope(eam, rho);
+      }
+    }
+    double acc = 0.0;  // threads below NC * nb: row tid / NC, component tid % NC
+    __syncthreads();
+    const float lim = s_lim;
+    while (true) {
+      // scan: what passes the FP32 test, in list order
+      for (int r = warp; r < nb; r += ELEM_NT / 32) {
+        const int n = s_len[r];
+        const int *__restrict__ ent = a.ent + s_start[r];
+        const float px = s_pf[r][0], py = s_pf[r][1], pz = s_pf[r][2];
+        int at = s_at[r], cnt = 0;
+        for (; at < n && cnt + 32 <= ROW_CAP; at += 32) {
+          const bool live = at + lane < n;
+          const int code = live ? __ldg(ent + at + lane) : 0;
+          bool pass = false;
+          if (live) {
+            int line = code >> kb;
+            const float4 *x4 = s_nf4;
+            if (SELF) {
+              line -= e * a.maxlines;
+            } else {
+              const int j = line / a.maxlines;
+              line -= j * a.maxlines;
+              if (j != e) x4 = a.node_f + 6 * (size_t) j;
+            }
+            float x[24];
+#pragma unroll
+            for (int k = 0; k < 6; k++) {
+              const float4 v = x4[k];
+              x[4 * k] = v.x;
+              x[4 * k + 1] = v.y;
+              x[4 * k + 2] = v.z;
+              x[4 * k + 3] = v.w;
+            }
+            const int nj = line * naz + (code & kmask);
+            const float4 w0 = __ldg(F0 + 2 * (size_t) nj), w1 = __ldg(F0 + 2 * (size_t) nj + 1);
+            const float w[NPE] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+            float sx = 0.f, sy = 0.f, sz = 0.f;
+#pragma unroll
+            for (int k = 0; k < NPE; k++) {
+              sx = __fmaf_rn(w[k], x[3 * k], sx);
+              sy = __fmaf_rn(w[k], x[3 * k + 1], sy);
+              sz = __fmaf_rn(w[k], x[3 * k + 2], sz);
+            }
+            const float dx = px - sx, dy = py - sy, dz = pz - sz;
+            pass = dx * dx + dy * dy + dz * dz <= lim;
+          }
+          const unsigned b = __ballot_sync(0xffffffffu, pass);
+          if (pass) s_ent[r][cnt + __popc(b & ((1u << lane) - 1u))] = code;
+          cnt += __popc(b);
+        }
+        if (lane == 0) {
+          s_cnt[r] = cnt;
+          s_at[r] = at;
+        }
+      }
+      __syncthreads();
+      int total = 0;
+      bool more = false;
+      for (int r = 0; r < nb; r++) {
+        total += s_cnt[r];
+        more = more || s_at[r] < s_len[r];
+      }
+      // the buffered pairs of all rows, one after another
+      for (int idx = tid; idx < total; idx += ELEM_NT) {
+        int r = 0, k = idx;
+        while (k >= s_cnt[r]) k -= s_cnt[r++];
+        const int code = s_ent[r][k];
+        int line = code >> kb, j = e;
+        if (SELF) {
+          line -= e * a.maxlines;
+        } else {
+          j = line / a.maxlines;
+          line -= j * a.maxlines;
+        }
+        const int nj = line * naz + (code & kmask);
+        double S[NPE];
+        load8(S0 + (size_t) nj * NPE, S);
+        const double *x = SELF || j == e ? s_nx : a.nodex + 24 * (size_t) j;
+        const double dx = s_p[r][0] - node_sum(S, x, 3);
+        const double dy = s_p[r][1] - node_sum(S, x + 1, 3);
+        const double dz = s_p[r][2] - node_sum(S, x + 2, 3);
+        const double rsq = dx * dx + dy * dy + dz * dz;
+        double t0 = 0.0, t1 = 0.0, t2 = 0.0;
+        if (rsq < cutsq) {
+          if (EAM) {
+#ifdef FP64_EXACT_TU
+            const double rr = sqrt(rsq);
+#else
+            const double recip = rsqrt_nr(rsq);
+            const double rr = rsq * recip;
+#endif
+            double p;
+            const int m = split_index(rr * eam.rdr + 1.0, eam.nr - 1, -0x7fffffff, p);
+            const double *c = eam.rhor + 7 * (size_t) m;
+            if (DENSITY) {
+              t0 = ((c[3] * p + c[4]) * p + c[5]) * p + c[6];
+            } else {
+              const double *er = SELF || j == e ? s_er : a.erho + NPE * (size_t) j;
+              double rho = 0.0;
+#pragma unroll
+              for (int q = 0; q < NPE; q++) rho += S[q] * er[q];
+              const double fpj = eam_slope(eam, rho);
+              const double rhoip = (c[0] * p + c[1]) * p + c[2];
+              const double *z = eam.z2r + 7 * (size_t) m;
+              const double z2p = (z[0] * p + z[1]) * p + z[2];
+              const double z2 = ((z[3] * p + z[4]) * p + z[5]) * p + z[6];
+#ifdef FP64_EXACT_TU
+              const double recip = 1.0 / rr;
+#endif
+              const double phi = z2 * recip;
+              const double phip = z2p * recip - phi * recip;
+              const double psip = (s_fpi[r] + fpj) * rhoip + phip;
+              const double fpair = -psip * recip;
+              t0 = dx * fpair;
+              t1 = dy * fpair;
+              t2 = dz * fpair;
+            }
+          } else {
+#ifdef FP64_EXACT_TU
+            const double r2inv = 1.0 / rsq;
+#else
+            const double r2inv = rcp_nr(rsq);
+#endif
+            const double r6inv = r2inv * r2inv * r2inv;
+            const double forcelj = r6inv * (lj1 * r6inv - lj2);
+            const double fpair = forcelj * r2inv;
+            t0 = dx * fpair;
+            t1 = dy * fpair;
+            t2 = dz * fpair;
+          }
+        }
+        // a pair beyond the cutoff leaves 0, which changes no sum
+        s_t[r][0][k] = t0;
+        if (!DENSITY) {
+          s_t[r][1 % NC][k] = t1;
+          s_t[r][2 % NC][k] = t2;
+        }
+      }
+      __syncthreads();
+      if (tid < NC * nb) {
+        const double *t = s_t[tid / NC][tid % NC];
+        const int n = s_cnt[tid / NC];
+#pragma unroll 8
+        for (int k = 0; k < n; k++) acc += t[k];
+      }
+      if (!more) break;
+      __syncthreads();
+    }
+    if (DENSITY) {
+      if (tid < nb) out[NPE * (size_t) e + rb + tid] = acc;
+    } else {
+      if (tid < 3 * nb) s_f[tid / 3][tid % 3] = acc;
+      __syncthreads();
+      // the nodal gather in row order (rows of weight 0 add nothing)
+      if (tid < 24)
+        for (int r = 0; r < nb; r++)
+          nf += a.weight[ioff + s_jj[r]] * s_N[r][tid / 3] * s_f[r][tid % 3];
+    }
+  }
+  if (!DENSITY && tid < 24) out[24 * (size_t) e + tid] = nf;
+}
+
+}  // namespace
+
+#ifndef FP64_EXACT_TU
+namespace {
+__global__ void k_node_f(const double *__restrict__ nodex, long long n, float *__restrict__ out) {
+  const long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x;
+  if (t < n) out[t] = (float) nodex[t];
+}
+}  // namespace
+
+// float copies of all nodes, for lists that reach other elements
+void node_floats(const double *nodex, int nelem, float4 *out, cudaStream_t s) {
+  if (nelem <= 0) return;
+  const long long n = 24LL * nelem;
+  k_node_f<<<(int) ((n + 255) / 256), 256, 0, s>>>(nodex, n, reinterpret_cast<float *>(out));
+  check(cudaGetLastError(), "node_floats");
+}
+#endif
+
+void elem_pass(const Elem64Args &a, int pass, bool self, const EamTables &e, double lj1, double lj2,
+               double cutsq, double *out, cudaStream_t s) {
+  if (a.nlocal_e <= 0) return;
+  auto k = pass == 0 ? (self ? k_elem64<false, false, true> : k_elem64<false, false, false>)
+           : pass == 1 ? (self ? k_elem64<true, true, true> : k_elem64<true, true, false>)
+                       : (self ? k_elem64<true, false, true> : k_elem64<true, false, false>);
+  k<<<a.nlocal_e, ELEM_NT, 0, s>>>(a, e, lj1, lj2, cutsq, out);
+  check(cudaGetLastError(), "elem_pass");
+}
+
+}  // namespace FP64NS (per translation unit)
+}  // namespace cacg

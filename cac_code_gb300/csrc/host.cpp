@@ -200,6 +200,7 @@ struct cacg_context {
 
   // device arrays: atoms
   DBuf<double4> d_x;
+  DBuf<float4> d_spa_inter_f, d_node_f;  // FP32 site shape functions; float nodes (FP64 modes)
   DBuf<float4> d_xh, d_site_h;  // float copies for the FP32 cutoff pre-tests
   // mixed precision: FP32 spline tables, double-single element nodes and
   // integration-point shape functions, packed site positions and site F'(rho),
@@ -526,14 +527,17 @@ struct cacg_context {
   // are bounded by the box plus the ghost margin plus a motion allowance; each
   // float coordinate is within u|x| (u = 2^-24) of the double, the float
   // difference within a further u|dx|, and the float sum of squares within 3u.
-  float cut_pass(double cutsq) const {
+  // nu: a float coordinate is within nu u|x| of the double (1: rounded; an
+  // FP32 interpolation of rounded nodes by rounded weights, 8 products and
+  // sums: 10)
+  float cut_pass(double cutsq, double nu = 1.0) const {
     double X = 0.0;
     for (int d = 0; d < 3; d++)
       X = std::max(X, std::max(std::fabs(lo[d]), std::fabs(hi[d])) + cutghost[d] + max_size +
                           10.0 * skin + 1.0);
     const double u = std::ldexp(1.0, -24);
     const double rn = std::max(cutneighmax, std::sqrt(cutsq));
-    const double delta = 2.0 * u * X * 1.001 + u * (rn + 1.0);
+    const double delta = 2.0 * nu * u * X * 1.001 + u * (rn + 1.0);
     const double guard = 4.0 * u * cutsq + (1.0 + 4.0 * u) * (2.0 * std::sqrt(3.0) * rn * delta +
                                                               3.0 * delta * delta);
     float c = (float) (cutsq + guard);
@@ -632,6 +636,8 @@ cacg_context::~cacg_context() {
   for (auto *b : b4) b->release();
   d_xh.release();
   d_site_h.release();
+  d_spa_inter_f.release();
+  d_node_f.release();
   d_xl.release();
   d_rhor_val4.release();
   d_ftab.release();
@@ -1706,6 +1712,11 @@ void cacg_context::element_tables() {
   upload(d_spa_int, spa_int, s);
   upload(d_weight, w_all, s);
   upload(d_spa_inter, spa_inter, s);
+  std::vector<float4> sif(spa_inter.size() / 4);
+  for (size_t k = 0; k < sif.size(); k++)
+    sif[k] = make_float4((float) spa_inter[4 * k], (float) spa_inter[4 * k + 1],
+                         (float) spa_inter[4 * k + 2], (float) spa_inter[4 * k + 3]);
+  upload(d_spa_inter_f, sif, s);
   upload(d_spa_csub, spa_csub, s);
   upload(d_spa_isub, spa_isub, s);
   upload(d_int_off, int_off, s);
@@ -3130,6 +3141,68 @@ void cacg_context::pair_ecompute() {
   bool exact = !fast();
   int nall = enlocal + enghost;
   ElemTables t = etab();
+  if (codes_ok) {
+    // one block per element (elem_fp64.cuh): positions of the sites in reach only
+    Elem64Args q{};
+    q.nodex = d_nodex.p;
+    q.etype = d_etype.p;
+    q.row_first = d_row_first.p;
+    q.node_list = d_node_list.p;
+    q.numint = d_numint.p;
+    q.int_off = d_int_off.p;
+    q.inter_off = d_inter_off.p;
+    q.row_start = d_row_start.p;
+    q.ent = d_ent.p;
+    if (!exact) {
+      q.fjj = d_fjj.p;
+      q.fjj_off = d_fjj_off.p;
+    }
+    q.spa_int = d_spa_int.p;
+    q.spa_inter = d_spa_inter.p;
+    q.spa_inter_f = d_spa_inter_f.p;
+    q.weight = d_weight.p;
+    q.maxlines = maxlines;
+    q.nlocal_e = enlocal;
+    q.nae = d_nae.p;
+    q.kb = code_kb;
+    const double csq = pair_style == 1 ? ljtab.cutsq[1 * (MAXT + 1) + 1] : cutforcesq;
+    q.cut_pass = cut_pass(csq, 12.0);
+    if (!self_contained) {
+      d_node_f.ensure(6 * (size_t) nall, s);
+      kmark(KT_SITES, 0);
+      fp64_fma::node_floats(d_nodex.p, nall, d_node_f.p, s);
+      kmark(KT_SITES, 1);
+      launches++;
+      q.node_f = d_node_f.p;
+    }
+    auto pass = exact ? fp64_exact::elem_pass : fp64_fma::elem_pass;
+    if (pair_style == 1) {
+      const int a = 1 * (MAXT + 1) + 1;
+      kmark(KT_ELEM_FORCE, 0);
+      pass(q, 0, self_contained, EamTables{}, ljtab.lj1[a], ljtab.lj2[a], csq, d_nodef.p, s);
+      kmark(KT_ELEM_FORCE, 1);
+      launches++;
+      return;
+    }
+    const EamTables e = eamtab();
+    d_erho.ensure((size_t) NPE * nall, s);
+    kmark(KT_ELEM_RHO, 0);
+    pass(q, 1, self_contained, e, 0.0, 0.0, csq, d_erho.p, s);
+    kmark(KT_ELEM_RHO, 1);
+    launches += 2;
+    if (!self_contained) {
+      // eforward_comm_pair: ghost nodal densities from their owners (comm_brick.cpp:978-1010)
+      launch_copy_root(d_erho.p, NPE, d_eroot.p, enlocal, enghost, s);
+      launches++;
+    }
+    q.erho = d_erho.p;
+    kmark(KT_ELEM_FORCE, 0);
+    pass(q, 2, self_contained, e, 0.0, 0.0, csq, d_nodef.p, s);
+    kmark(KT_ELEM_FORCE, 1);
+    return;
+  }
+  // lists that the line codes do not hold (more than 64 sites a line, or too
+  // many lines): site arrays of the step.
   // sites of every local and ghost element at the current node positions,
   // with their float copies, then this step's short lists of the rows
   d_site_h.ensure(std::max(nsites, 1), s);

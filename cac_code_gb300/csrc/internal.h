@@ -201,9 +201,26 @@ void launch_ip_list(const double *nodex, const double *ex, const int *etype,
                     double cutsq, int maxip, int rowstride, int *ipnum, int *ipent,
                     int *overflow, cudaStream_t s);
 
+// ---- FP64 element passes (elem_fp64.cuh) ----
+struct Elem64Args {
+  const double *nodex, *erho;   // all elements (erho: EAM force pass)
+  const float4 *node_f;         // float nodes of all elements (lists that reach other elements)
+  const int *etype, *row_first, *node_list, *numint, *int_off, *inter_off;
+  const int *row_start, *ent;   // integration-point lists, row-major line codes
+  const int *fjj, *fjj_off;     // rows of nonzero weight per type (null: all rows)
+  const double *spa_int, *spa_inter, *weight;
+  const float4 *spa_inter_f;    // site shape functions, FP32 (8 per site)
+  int maxlines, nlocal_e;
+  const int *nae;               // lattice sizes per type
+  int kb;                       // bits of the site index in a line code
+  float cut_pass;               // FP32 limit for absolute coordinates
+};
+
 // ---- forces: same kernels in two translation units (force_fp64.cuh) ----
 // fp64_exact (k_force_exact.cu, -fmad=false) and fp64_fma (k_force_fma.cu).
 #define CACG_FORCE_DECLS                                                                   \
+  void elem_pass(const Elem64Args &a, int pass, bool self, const EamTables &e, double lj1,   \
+                 double lj2, double cutsq, double *out, cudaStream_t s);                    \
   void lj_atoms(const double4 *x, const int *type, const int *num, const int *list,         \
                 int stride, int nlocal, const void *tab, double *f, cudaStream_t s);        \
   void eam_rho_atoms(const double4 *x, const int *num, const int *list, int stride,         \
@@ -234,6 +251,9 @@ CACG_FORCE_DECLS
 // fp64_fma (k_force_fma.cu): FP32 pre-test against cut_pass on the float
 // copies (xh, site_h), Newton-refined reciprocals, weight-0 rows skipped.
 namespace fp64_fma {
+void elem_pass(const Elem64Args &a, int pass, bool self, const EamTables &e, double lj1,
+               double lj2, double cutsq, double *out, cudaStream_t s);
+void node_floats(const double *nodex, int nelem, float4 *out, cudaStream_t s);
 void lj_atoms(const double4 *x, const float4 *xh, const int *type, const int *num,
               const int *list, int stride, int nlocal, const void *tab, float cut_pass,
               double *f, cudaStream_t s);

@@ -1,7 +1,9 @@
 // FP64 pair kernels, reference operation order without contraction (bit-identical to the CPU reference).
 // Build flag: -fmad=false.  Kernel bodies live in force_fp64.cuh.
 #define FP64NS fp64_exact
+#define FP64_EXACT_TU
 #include "force_fp64.cuh"
+#include "elem_fp64.cuh"
 
 namespace cacg {
 namespace fp64_exact {

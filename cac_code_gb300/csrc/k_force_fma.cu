@@ -636,3 +636,6 @@ void gather_nodef(const double *fip, const int *etype, const int *row_first, int
 
 }  // namespace fp64_fma
 }  // namespace cacg
+
+#define FP64NS fp64_fma
+#include "elem_fp64.cuh"
