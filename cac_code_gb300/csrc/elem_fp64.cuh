@@ -33,26 +33,33 @@ namespace FP64NS {
 namespace {
 
 constexpr int RB = 8;           // rows of an element per round
-constexpr int ROW_CAP = 128;    // buffered entries per row
+constexpr int ROW_CAP = 96;     // buffered entries per row
 constexpr int ELEM_NT = 128;    // threads per block
+
+#ifdef FP64_EXACT_TU
+constexpr int NT3 = 3;          // buffered per pair: the three terms
+#else
+constexpr int NT3 = 4;          // the vector and the pair factor (summed with one FMA)
+#endif
 
 // m = min((int) q, n1) and p = min(q - m, 1): for 1 <= q < 2^20 from the bits
 // of q, without conversions (they issue at the FP64 rate): the integer part is
-// q with the mantissa bits below the point cleared.  low: m is at least that.
-__device__ __forceinline__ int split_index(double q, int n1, int low, double &p) {
+// q with the mantissa bits below the point cleared.  m is at least 1, as it is
+// for every r >= 0 and as rho's index is clamped.
+__device__ __forceinline__ int split_index(double q, int n1, double &p) {
   const int hi = __double2hiint(q);
   const unsigned e = (unsigned) (hi >> 20) - 1023u;
   if (e < 20u) {
     const int sh = 20 - (int) e;
     const int m = ((hi & 0xFFFFF) | 0x100000) >> sh;
-    if (m <= n1 && m >= low) {
+    if (m <= n1) {
       p = q - __hiloint2double(hi & (int) (0xFFFFFFFFu << sh), 0);
       return m;
     }
   }
   int m = (int) q;
   m = m < n1 ? m : n1;
-  m = low > m ? low : m;
+  m = m > 1 ? m : 1;
   p = q - m;
   p = p < 1.0 ? p : 1.0;
   return m;
@@ -94,7 +101,7 @@ __device__ __forceinline__ void load8(const double *__restrict__ p, double (&w)[
 
 __device__ __forceinline__ double eam_slope(const EamTables &e, double rho) {
   double p;
-  const int m = split_index(rho * e.rdrho + 1.0, e.nrho - 1, 1, p);
+  const int m = split_index(rho * e.rdrho + 1.0, e.nrho - 1, p);
   const double *c = e.frho + 7 * (size_t) m;
   return (c[0] * p + c[1]) * p + c[2];
 }
@@ -106,7 +113,7 @@ template <bool EAM, bool DENSITY, bool SELF>
 __global__ void __launch_bounds__(ELEM_NT)
 k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
          double *__restrict__ out) {
-  constexpr int NC = DENSITY ? 1 : 3;
+  constexpr int NC = DENSITY ? 1 : NT3, NS = DENSITY ? 1 : 3;  // buffered values, sums
   __shared__ double s_nx[24], s_er[NPE], s_p[RB][3], s_N[RB][NPE], s_fpi[RB], s_f[RB][3];
   __shared__ double s_t[RB][NC][ROW_CAP + 1];
   __shared__ int s_ent[RB][ROW_CAP];
@@ -158,12 +165,15 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
     __syncthreads();
     // the rows' points: FP64 (a row's node itself in the density pass) and FP32
     for (int t = tid; t < nb * 3; t += ELEM_NT) {
-      const int r = t / 3, d = t % 3, jj = s_jj[r];
-      const double *N = a.spa_int + ((size_t) ioff + jj) * NPE;
+      const int r = t / 3, d = t % 3;
+      if (DENSITY) {
+        s_p[r][d] = s_nx[3 * (rb + r) + d];
+        s_pf[r][d] = s_nf[3 * (rb + r) + d];
+        continue;
+      }
       double w[NPE];
-      load8(N, w);
-      if (DENSITY) s_p[r][d] = s_nx[3 * (rb + r) + d];
-      else s_p[r][d] = node_sum(w, s_nx + d, 3);
+      load8(a.spa_int + ((size_t) ioff + s_jj[r]) * NPE, w);
+      s_p[r][d] = node_sum(w, s_nx + d, 3);
       float pf = 0.f;
 #pragma unroll
       for (int k = 0; k < NPE; k++) {
@@ -171,14 +181,14 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
         pf += (float) w[k] * s_nf[3 * k + d];
       }
       s_pf[r][d] = pf;
-      if (EAM && !DENSITY && d == 0) {
+      if (EAM && d == 0) {
         double rho = 0.0;
 #pragma unroll
         for (int k = 0; k < NPE; k++) rho += w[k] * s_er[k];
         s_fpi[r] = eam_slope(eam, rho);
       }
     }
-    double acc = 0.0;  // threads below NC * nb: row tid / NC, component tid % NC
+    double acc = 0.0;  // threads below NS * nb: row tid / NS, component tid % NS
     __syncthreads();
     const float lim = s_lim;
     while (true) {
@@ -260,8 +270,9 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
         const double dy = s_p[r][1] - node_sum(S, x + 1, 3);
         const double dz = s_p[r][2] - node_sum(S, x + 2, 3);
         const double rsq = dx * dx + dy * dy + dz * dz;
-        double t0 = 0.0, t1 = 0.0, t2 = 0.0;
-        if (rsq < cutsq) {
+        double t0 = 0.0, fpair = 0.0;
+        const bool in = rsq < cutsq;
+        if (in) {
           if (EAM) {
 #ifdef FP64_EXACT_TU
             const double rr = sqrt(rsq);
@@ -270,7 +281,7 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
             const double rr = rsq * recip;
 #endif
             double p;
-            const int m = split_index(rr * eam.rdr + 1.0, eam.nr - 1, -0x7fffffff, p);
+            const int m = split_index(rr * eam.rdr + 1.0, eam.nr - 1, p);
             const double *c = eam.rhor + 7 * (size_t) m;
             if (DENSITY) {
               t0 = ((c[3] * p + c[4]) * p + c[5]) * p + c[6];
@@ -290,10 +301,7 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
               const double phi = z2 * recip;
               const double phip = z2p * recip - phi * recip;
               const double psip = (s_fpi[r] + fpj) * rhoip + phip;
-              const double fpair = -psip * recip;
-              t0 = dx * fpair;
-              t1 = dy * fpair;
-              t2 = dz * fpair;
+              fpair = -psip * recip;
             }
           } else {
 #ifdef FP64_EXACT_TU
@@ -303,25 +311,37 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
 #endif
             const double r6inv = r2inv * r2inv * r2inv;
             const double forcelj = r6inv * (lj1 * r6inv - lj2);
-            const double fpair = forcelj * r2inv;
-            t0 = dx * fpair;
-            t1 = dy * fpair;
-            t2 = dz * fpair;
+            fpair = forcelj * r2inv;
           }
         }
-        // a pair beyond the cutoff leaves 0, which changes no sum
-        s_t[r][0][k] = t0;
-        if (!DENSITY) {
-          s_t[r][1 % NC][k] = t1;
-          s_t[r][2 % NC][k] = t2;
+        // a pair beyond the cutoff leaves zeros, which change no sum
+        if (DENSITY) {
+          s_t[r][0][k] = t0;
+        } else {
+#ifdef FP64_EXACT_TU
+          s_t[r][0][k] = in ? dx * fpair : 0.0;
+          s_t[r][1 % NC][k] = in ? dy * fpair : 0.0;
+          s_t[r][2 % NC][k] = in ? dz * fpair : 0.0;
+#else
+          s_t[r][0][k] = in ? dx : 0.0;
+          s_t[r][1 % NC][k] = in ? dy : 0.0;
+          s_t[r][2 % NC][k] = in ? dz : 0.0;
+          s_t[r][3 % NC][k] = fpair;
+#endif
         }
       }
       __syncthreads();
-      if (tid < NC * nb) {
-        const double *t = s_t[tid / NC][tid % NC];
-        const int n = s_cnt[tid / NC];
+      if (tid < NS * nb) {
+        const int r = tid / NS, n = s_cnt[r];
+        const double *t = s_t[r][tid % NS];
+#ifdef FP64_EXACT_TU
 #pragma unroll 8
         for (int k = 0; k < n; k++) acc += t[k];
+#else
+        const double *g = s_t[r][NC - 1];
+#pragma unroll 8
+        for (int k = 0; k < n; k++) acc = DENSITY ? acc + t[k] : fma(t[k], g[k], acc);
+#endif
       }
       if (!more) break;
       __syncthreads();

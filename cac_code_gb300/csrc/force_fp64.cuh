@@ -24,38 +24,6 @@ struct LJTab {
   double cutsq[(MAXT + 1) * (MAXT + 1)];
 };
 
-__global__ void __launch_bounds__(128)
-k_lj_atoms(const double4 *__restrict__ x, const int *__restrict__ type,
-           const int *__restrict__ num, const int *__restrict__ list, int stride, int nlocal,
-           const LJTab *__restrict__ tab, double *__restrict__ f) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nlocal) return;
-  const double4 xi = x[i];
-  const int it = type[i];
-  const int n = num[i];
-  double fx = 0.0, fy = 0.0, fz = 0.0;
-  for (int k = 0; k < n; k++) {
-    int j = __ldg(list + (size_t) k * stride + i);
-    double4 xj = x[j];
-    double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-    double rsq = dx * dx + dy * dy + dz * dz;
-    int jt = type[j];
-    int ij = it * (MAXT + 1) + jt;
-    if (rsq < tab->cutsq[ij]) {
-      double r2inv = 1.0 / rsq;
-      double r6inv = r2inv * r2inv * r2inv;
-      double forcelj = r6inv * (tab->lj1[ij] * r6inv - tab->lj2[ij]);
-      double fpair = forcelj * r2inv;
-      fx += dx * fpair;
-      fy += dy * fpair;
-      fz += dz * fpair;
-    }
-  }
-  f[3 * i] = fx;
-  f[3 * i + 1] = fy;
-  f[3 * i + 2] = fz;
-}
-
 __device__ __forceinline__ double spline_value(const double *__restrict__ c, double p) {
   return ((c[3] * p + c[4]) * p + c[5]) * p + c[6];
 }
@@ -109,45 +77,6 @@ k_eam_rho_atoms(const double4 *__restrict__ x, const int *__restrict__ num,
   double p;
   int m = rhoindex(r, e, p);
   fp[i] = spline_deriv(e.frho + 7 * m, p);
-}
-
-__global__ void __launch_bounds__(128)
-k_eam_force_atoms(const double4 *__restrict__ x, const int *__restrict__ num,
-                  const int *__restrict__ list, int stride, int nlocal, EamTables e,
-                  const double *__restrict__ fp, double *__restrict__ f) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nlocal) return;
-  const double4 xi = x[i];
-  const double fpi = fp[i];
-  const int n = num[i];
-  double fx = 0.0, fy = 0.0, fz = 0.0;
-  for (int k = 0; k < n; k++) {
-    int j = __ldg(list + (size_t) k * stride + i);
-    double4 xj = x[j];
-    double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-    double rsq = dx * dx + dy * dy + dz * dz;
-    if (rsq < e.cutforcesq) {
-      double r = sqrt(rsq);
-      double p;
-      int m = rindex(r, e, p);
-      double rhoip = spline_deriv(e.rhor + 7 * m, p);
-      double rhojp = rhoip;  // same table for every type pair (single funcfl file)
-      const double *z = e.z2r + 7 * m;
-      double z2p = spline_deriv(z, p);
-      double z2 = spline_value(z, p);
-      double recip = 1.0 / r;
-      double phi = z2 * recip;
-      double phip = z2p * recip - phi * recip;
-      double psip = fpi * rhojp + __ldg(fp + j) * rhoip + phip;
-      double fpair = -psip * recip;
-      fx += dx * fpair;
-      fy += dy * fpair;
-      fz += dz * fpair;
-    }
-  }
-  f[3 * i] = fx;
-  f[3 * i + 1] = fy;
-  f[3 * i + 2] = fz;
 }
 
 // integration-point position: sum_k N_k x_k (pair_lj_cut.cpp:363-367)

@@ -327,6 +327,7 @@ struct cacg_context {
   DBuf<double4> d_bx;
   DBuf<int> d_num, d_list;
   DBuf<int> d_snum, d_slist;  // per-step short lists (FP32 guarded cutoff test)
+  DBuf<unsigned char> d_sr;   // and their distances (FP64 modes)
   int maxneigh = 64, stride = 0;
   // elements
   DBuf<double> d_ex, d_nodex, d_nodev, d_nodef, d_nodexhold, d_erho, d_emass, d_diag, d_fip,
@@ -638,6 +639,7 @@ cacg_context::~cacg_context() {
   d_site_h.release();
   d_spa_inter_f.release();
   d_node_f.release();
+  d_sr.release();
   d_xl.release();
   d_rhor_val4.release();
   d_ftab.release();
@@ -2497,42 +2499,52 @@ void cacg_context::pair_compute_pass(int pass) {
     pair_compute_mixed(pass);
     return;
   }
-  const float cp = atom_cut_pass();
+  if (pair_style == 1 && pass != 1) return;
+  auto atom_pass = exact ? fp64_exact::atom_pass : fp64_fma::atom_pass;
+  d_snum.ensure(nlocal, s);
+  Atoms64Args q{};
+  q.x = d_x.p;
+  q.type = d_type.p;
+  q.num = d_num.p;
+  q.list = d_list.p;
+  q.stride = stride;
+  q.nlocal = nlocal;
+  q.cut_pass = atom_cut_pass();
+  q.f = d_f.p;
   if (pass == 1) {
-    // float copies and the short list of this step (both FP64 modes)
     d_xh.ensure(nall, s);
     launch_split_hi(d_x.p, d_xh.p, nall, s);
-    d_snum.ensure(nlocal, s);
-    d_slist.ensure((size_t) maxneigh * stride, s);
-    fp64_fma::filter_atoms(d_xh.p, d_num.p, d_list.p, stride, nlocal, cp, d_snum.p, d_slist.p, s);
-    launches += 2;
+    launches++;
   }
-  const int *num = d_snum.p, *lst = d_slist.p;
+  q.xh = d_xh.p;
+  q.snum = d_snum.p;
   if (pair_style == 1) {
-    if (pass != 1) return;
     kmark(KT_ATOM1, 0);
-    if (exact) fp64_exact::lj_atoms(d_x.p, d_type.p, num, lst, stride, nlocal, d_ljtab.p, d_f.p, s);
-    else fp64_fma::lj_atoms(d_x.p, d_xh.p, d_type.p, num, lst, stride, nlocal, d_ljtab.p, cp, d_f.p, s);
+    atom_pass(q, 0, EamTables{}, d_ljtab.p, s);
     kmark(KT_ATOM1, 1);
     launches++;
     return;
   }
-  EamTables e = eamtab();
+  const EamTables e = eamtab();
   if (pass == 1) {
+    d_slist.ensure((size_t) maxneigh * stride, s);
+    d_sr.ensure((size_t) maxneigh * stride * (exact ? fp64_exact::pair_bytes() : fp64_fma::pair_bytes()),
+                s);
     d_rho.ensure(nall, s);
     d_fp.ensure(nall, s);
-    kmark(KT_ATOM1, 0);
-    if (exact) fp64_exact::eam_rho_atoms(d_x.p, num, lst, stride, nlocal, e, d_rho.p, d_fp.p, s);
-    else fp64_fma::eam_rho_atoms(d_x.p, d_xh.p, num, lst, stride, nlocal, e, cp, d_rho.p, d_fp.p, s);
-    kmark(KT_ATOM1, 1);
+  }
+  q.slist = d_slist.p;
+  q.sr = d_sr.p;
+  q.rho = d_rho.p;
+  q.fp = d_fp.p;
+  const int k = pass == 1 ? KT_ATOM1 : KT_ATOM2;
+  kmark(k, 0);
+  atom_pass(q, pass, e, nullptr, s);
+  kmark(k, 1);
+  launches++;
+  if (pass == 1) {
     // forward_comm_pair: ghost fp = owner fp (comm_brick.cpp:941-971)
     launch_copy_root(d_fp.p, 1, d_root.p, nlocal, nghost, s);
-    launches += 2;
-  } else {
-    kmark(KT_ATOM2, 0);
-    if (exact) fp64_exact::eam_force_atoms(d_x.p, num, lst, stride, nlocal, e, d_fp.p, d_f.p, s);
-    else fp64_fma::eam_force_atoms(d_x.p, d_xh.p, num, lst, stride, nlocal, e, cp, d_fp.p, d_f.p, s);
-    kmark(KT_ATOM2, 1);
     launches++;
   }
 }

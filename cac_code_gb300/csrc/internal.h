@@ -201,6 +201,19 @@ void launch_ip_list(const double *nodex, const double *ex, const int *etype,
                     double cutsq, int maxip, int rowstride, int *ipnum, int *ipent,
                     int *overflow, cudaStream_t s);
 
+// ---- FP64 atom passes (atoms_fp64.cuh) ----
+struct Atoms64Args {
+  const double4 *x;
+  const float4 *xh;            // float copies for the FP32 cutoff test
+  const int *type;             // LJ
+  const int *num, *list;       // atom list, column-major
+  int stride, nlocal;
+  float cut_pass;
+  int *snum, *slist;           // short lists: written by pass 1, read by pass 2
+  void *sr;                    // their distances (pair_bytes() each)
+  double *rho, *fp, *f;
+};
+
 // ---- FP64 element passes (elem_fp64.cuh) ----
 struct Elem64Args {
   const double *nodex, *erho;   // all elements (erho: EAM force pass)
@@ -219,15 +232,13 @@ struct Elem64Args {
 // ---- forces: same kernels in two translation units (force_fp64.cuh) ----
 // fp64_exact (k_force_exact.cu, -fmad=false) and fp64_fma (k_force_fma.cu).
 #define CACG_FORCE_DECLS                                                                   \
+  void atom_pass(const Atoms64Args &a, int pass, const EamTables &e, const void *ljtab,     \
+                 cudaStream_t s);                                                           \
+  size_t pair_bytes();                                                                      \
   void elem_pass(const Elem64Args &a, int pass, bool self, const EamTables &e, double lj1,   \
                  double lj2, double cutsq, double *out, cudaStream_t s);                    \
-  void lj_atoms(const double4 *x, const int *type, const int *num, const int *list,         \
-                int stride, int nlocal, const void *tab, double *f, cudaStream_t s);        \
   void eam_rho_atoms(const double4 *x, const int *num, const int *list, int stride,         \
                      int nlocal, EamTables e, double *rho, double *fp, cudaStream_t s);     \
-  void eam_force_atoms(const double4 *x, const int *num, const int *list, int stride,       \
-                       int nlocal, EamTables e, const double *fp, double *f,                \
-                       cudaStream_t s);                                                     \
   void lj_ip(const double *nodex, const int *etype, const int *row_elem, const int *row_jj, \
              int nrows, const int *ipnum, const int *ipent, int rowstride,                  \
              const double4 *site_x, ElemTables t, double lj1, double lj2, double cutsq,      \
@@ -254,15 +265,9 @@ namespace fp64_fma {
 void elem_pass(const Elem64Args &a, int pass, bool self, const EamTables &e, double lj1,
                double lj2, double cutsq, double *out, cudaStream_t s);
 void node_floats(const double *nodex, int nelem, float4 *out, cudaStream_t s);
-void lj_atoms(const double4 *x, const float4 *xh, const int *type, const int *num,
-              const int *list, int stride, int nlocal, const void *tab, float cut_pass,
-              double *f, cudaStream_t s);
-void eam_rho_atoms(const double4 *x, const float4 *xh, const int *num, const int *list,
-                   int stride, int nlocal, EamTables e, float cut_pass, double *rho,
-                   double *fp, cudaStream_t s);
-void eam_force_atoms(const double4 *x, const float4 *xh, const int *num, const int *list,
-                     int stride, int nlocal, EamTables e, float cut_pass, const double *fp,
-                     double *f, cudaStream_t s);
+void atom_pass(const Atoms64Args &a, int pass, const EamTables &e, const void *ljtab,
+               cudaStream_t s);
+size_t pair_bytes();
 void lj_ip(const double *nodex, const int *etype, const int *row_elem, const int *row_jj,
            int nrows, const int *ipnum, const int *ipent, int rowstride, const double4 *site_x,
            const float4 *site_h, ElemTables t, double lj1, double lj2, double cutsq,
@@ -293,8 +298,6 @@ void site_fp_needed(const double *erho, const int *etype, const int *site_base, 
                     const int *need_elem, int nneed, ElemTables t, EamTables e, double *site_fp,
                     cudaStream_t s);
 // per-step short lists (FP32 guarded cutoff test), used by both FP64 modes
-void filter_atoms(const float4 *xh, const int *num, const int *list, int stride, int nlocal,
-                  float cut_pass, int *snum, int *slist, cudaStream_t s);
 void filter_rows(const double *nodex, const int *etype, const int *row_elem, const int *row_jj,
                  int nrows, const int *ipnum, const int *ipent, int rowstride,
                  const float4 *site_h, ElemTables t, float cut_pass, int only_needed, int *snum,

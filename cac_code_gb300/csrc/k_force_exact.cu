@@ -4,6 +4,7 @@
 #define FP64_EXACT_TU
 #include "force_fp64.cuh"
 #include "elem_fp64.cuh"
+#include "atoms_fp64.cuh"
 
 namespace cacg {
 namespace fp64_exact {
@@ -12,26 +13,11 @@ namespace {
 inline int nblk(long long n, int t) { return (int) ((n + t - 1) / t); }
 }
 
-void lj_atoms(const double4 *x, const int *type, const int *num, const int *list, int stride,
-              int nlocal, const void *tab, double *f, cudaStream_t s) {
-  if (nlocal <= 0) return;
-  k_lj_atoms<<<nblk(nlocal, 128), 128, 0, s>>>(x, type, num, list, stride, nlocal,
-                                              (const LJTab *) tab, f);
-  check(cudaGetLastError(), "lj_atoms");
-}
-
 void eam_rho_atoms(const double4 *x, const int *num, const int *list, int stride, int nlocal,
                    EamTables e, double *rho, double *fp, cudaStream_t s) {
   if (nlocal <= 0) return;
   k_eam_rho_atoms<<<nblk(nlocal, 128), 128, 0, s>>>(x, num, list, stride, nlocal, e, rho, fp);
   check(cudaGetLastError(), "eam_rho_atoms");
-}
-
-void eam_force_atoms(const double4 *x, const int *num, const int *list, int stride, int nlocal,
-                     EamTables e, const double *fp, double *f, cudaStream_t s) {
-  if (nlocal <= 0) return;
-  k_eam_force_atoms<<<nblk(nlocal, 128), 128, 0, s>>>(x, num, list, stride, nlocal, e, fp, f);
-  check(cudaGetLastError(), "eam_force_atoms");
 }
 
 void lj_ip(const double *nodex, const int *etype, const int *row_elem, const int *row_jj,

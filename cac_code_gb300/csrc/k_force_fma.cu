@@ -75,107 +75,6 @@ __device__ __forceinline__ float rsq_f(float4 a, float4 b) {
   return dx * dx + dy * dy + dz * dz;
 }
 
-__global__ void __launch_bounds__(128)
-k_lj_atoms(const double4 *__restrict__ x, const float4 *__restrict__ xh,
-           const int *__restrict__ type, const int *__restrict__ num,
-           const int *__restrict__ list, int stride, int nlocal, const LJTab *__restrict__ tab,
-           float cut_pass, double *__restrict__ f) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nlocal) return;
-  const double4 xi = x[i];
-  const float4 hi = xh[i];
-  const int it = type[i];
-  const int n = num[i];
-  double fx = 0.0, fy = 0.0, fz = 0.0;
-  for (int k = 0; k < n; k++) {
-    int j = __ldg(list + (size_t) k * stride + i);
-    double4 xj = x[j];
-    double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-    double rsq = dx * dx + dy * dy + dz * dz;
-    int ij = it * (MAXT + 1) + type[j];
-    if (rsq < tab->cutsq[ij]) {
-      double r2inv = rcp_nr(rsq);
-      double r6inv = r2inv * r2inv * r2inv;
-      double forcelj = r6inv * (tab->lj1[ij] * r6inv - tab->lj2[ij]);
-      double fpair = forcelj * r2inv;
-      fx += dx * fpair;
-      fy += dy * fpair;
-      fz += dz * fpair;
-    }
-  }
-  f[3 * i] = fx;
-  f[3 * i + 1] = fy;
-  f[3 * i + 2] = fz;
-}
-
-__global__ void __launch_bounds__(128)
-k_eam_rho_atoms(const double4 *__restrict__ x, const float4 *__restrict__ xh,
-                const int *__restrict__ num, const int *__restrict__ list, int stride,
-                int nlocal, EamTables e, float cut_pass, double *__restrict__ rho,
-                double *__restrict__ fp) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nlocal) return;
-  const double4 xi = x[i];
-  const float4 hi = xh[i];
-  const int n = num[i];
-  double r = 0.0;
-  for (int k = 0; k < n; k++) {
-    int j = __ldg(list + (size_t) k * stride + i);
-    double4 xj = x[j];
-    double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-    double rsq = dx * dx + dy * dy + dz * dz;
-    if (rsq < e.cutforcesq) {
-      double p;
-      int m = rindex(rsq * rsqrt_nr(rsq), e, p);
-      r += spline_value(e.rhor + 7 * m, p);
-    }
-  }
-  rho[i] = r;
-  double p;
-  int m = rhoindex(r, e, p);
-  fp[i] = spline_deriv(e.frho + 7 * m, p);
-}
-
-__global__ void __launch_bounds__(128)
-k_eam_force_atoms(const double4 *__restrict__ x, const float4 *__restrict__ xh,
-                  const int *__restrict__ num, const int *__restrict__ list, int stride,
-                  int nlocal, EamTables e, float cut_pass, const double *__restrict__ fp,
-                  double *__restrict__ f) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nlocal) return;
-  const double4 xi = x[i];
-  const float4 hi = xh[i];
-  const double fpi = fp[i];
-  const int n = num[i];
-  double fx = 0.0, fy = 0.0, fz = 0.0;
-  for (int k = 0; k < n; k++) {
-    int j = __ldg(list + (size_t) k * stride + i);
-    double4 xj = x[j];
-    double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-    double rsq = dx * dx + dy * dy + dz * dz;
-    if (rsq < e.cutforcesq) {
-      double recip = rsqrt_nr(rsq);
-      double r = rsq * recip;
-      double p;
-      int m = rindex(r, e, p);
-      double rhoip = spline_deriv(e.rhor + 7 * m, p);
-      const double *z = e.z2r + 7 * m;
-      double z2p = spline_deriv(z, p);
-      double z2 = spline_value(z, p);
-      double phi = z2 * recip;
-      double phip = z2p * recip - phi * recip;
-      double psip = fpi * rhoip + __ldg(fp + j) * rhoip + phip;
-      double fpair = -psip * recip;
-      fx += dx * fpair;
-      fy += dy * fpair;
-      fz += dz * fpair;
-    }
-  }
-  f[3 * i] = fx;
-  f[3 * i + 1] = fy;
-  f[3 * i + 2] = fz;
-}
-
 // Positions are interpolated without contraction (explicit round-to-nearest
 // multiply and add), exactly as the exact mode: element coordinates reach
 // |x| ~ 1e3, and a fused rounding there would move a site by ~1e-13, which the
@@ -356,26 +255,9 @@ __global__ void k_gather_nodef(const double *__restrict__ fip, const int *__rest
   nodef[tid] = acc;
 }
 
-// Per-step short lists: the entries of a row whose FP32 distance passes the
+// Per-step short lists of the rows: the entries whose FP32 distance passes the
 // guarded cutoff test (any entry inside the cutoff in exact arithmetic passes),
-// in list order.  Both EAM passes and the element passes then iterate mostly
-// interacting pairs, so the FP64 branch seldom diverges inside a warp.
-__global__ void __launch_bounds__(128)
-k_filter_atoms(const float4 *__restrict__ xh, const int *__restrict__ num,
-               const int *__restrict__ list, int stride, int nlocal, float cut_pass,
-               int *__restrict__ snum, int *__restrict__ slist) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nlocal) return;
-  const float4 hi = xh[i];
-  const int n = num[i];
-  int m = 0;
-  for (int k = 0; k < n; k++) {
-    int j = __ldg(list + (size_t) k * stride + i);
-    if (rsq_f(hi, __ldg(xh + j)) <= cut_pass) slist[(size_t) m++ * stride + i] = j;
-  }
-  snum[i] = m;
-}
-
+// in list order.
 // rows: all rows (mode 0), rows of nonzero weight or node rows (mode 1)
 __global__ void __launch_bounds__(128)
 k_filter_rows(const double *__restrict__ nodex, const int *__restrict__ etype,
@@ -500,14 +382,6 @@ __global__ void k_sites_fma(const double *__restrict__ nodex, const int *__restr
 
 }  // namespace
 
-void filter_atoms(const float4 *xh, const int *num, const int *list, int stride, int nlocal,
-                  float cut_pass, int *snum, int *slist, cudaStream_t s) {
-  if (nlocal <= 0) return;
-  k_filter_atoms<<<nblk(nlocal, 128), 128, 0, s>>>(xh, num, list, stride, nlocal, cut_pass,
-                                                  snum, slist);
-  check(cudaGetLastError(), "filter_atoms");
-}
-
 void filter_rows(const double *nodex, const int *etype, const int *row_elem, const int *row_jj,
                  int nrows, const int *ipnum, const int *ipent, int rowstride,
                  const float4 *site_h, ElemTables t, float cut_pass, int only_needed, int *snum,
@@ -557,33 +431,6 @@ void sites(const double *nodex, const int *etype, const int *site_base, int nele
   if (nelem <= 0) return;
   k_sites_fma<<<nelem, 128, 0, s>>>(nodex, etype, site_base, t, site_x, site_h);
   check(cudaGetLastError(), "sites_fma");
-}
-
-void lj_atoms(const double4 *x, const float4 *xh, const int *type, const int *num,
-              const int *list, int stride, int nlocal, const void *tab, float cut_pass,
-              double *f, cudaStream_t s) {
-  if (nlocal <= 0) return;
-  k_lj_atoms<<<nblk(nlocal, 128), 128, 0, s>>>(x, xh, type, num, list, stride, nlocal,
-                                              (const LJTab *) tab, cut_pass, f);
-  check(cudaGetLastError(), "lj_atoms_fma");
-}
-
-void eam_rho_atoms(const double4 *x, const float4 *xh, const int *num, const int *list,
-                   int stride, int nlocal, EamTables e, float cut_pass, double *rho,
-                   double *fp, cudaStream_t s) {
-  if (nlocal <= 0) return;
-  k_eam_rho_atoms<<<nblk(nlocal, 128), 128, 0, s>>>(x, xh, num, list, stride, nlocal, e,
-                                                   cut_pass, rho, fp);
-  check(cudaGetLastError(), "eam_rho_atoms_fma");
-}
-
-void eam_force_atoms(const double4 *x, const float4 *xh, const int *num, const int *list,
-                     int stride, int nlocal, EamTables e, float cut_pass, const double *fp,
-                     double *f, cudaStream_t s) {
-  if (nlocal <= 0) return;
-  k_eam_force_atoms<<<nblk(nlocal, 128), 128, 0, s>>>(x, xh, num, list, stride, nlocal, e,
-                                                     cut_pass, fp, f);
-  check(cudaGetLastError(), "eam_force_atoms_fma");
 }
 
 void lj_ip(const double *nodex, const int *etype, const int *row_elem, const int *row_jj,
@@ -639,3 +486,4 @@ void gather_nodef(const double *fip, const int *etype, const int *row_first, int
 
 #define FP64NS fp64_fma
 #include "elem_fp64.cuh"
+#include "atoms_fp64.cuh"
