@@ -324,7 +324,9 @@ struct cacg_context {
   DBuf<double> d_v, d_f, d_xhold, d_rho, d_fp, d_mass;
   DBuf<int> d_type, d_tag, d_root, d_send;
   DBuf<int> d_abin, d_bcount, d_bstart, d_bmem, d_stencil;
-  DBuf<double4> d_bx;
+  DBuf<float4> d_bxf;   // members in bin order: float coordinates and the index
+  DBuf<int2> d_runs;    // the stencil's bins that follow each other
+  int nruns = 0;
   DBuf<int> d_num, d_list;
   DBuf<int> d_snum, d_slist;  // per-step short lists (FP32 guarded cutoff test)
   DBuf<unsigned char> d_sr;   // and their distances (FP64 modes)
@@ -341,6 +343,7 @@ struct cacg_context {
   DBuf<int> d_sipnum, d_sipent;
   DBuf<int> d_force_rows, d_need, d_need_elem, d_site_flag, d_site_pos;
   int nforce = 0, nneed = 0;
+  long long need_of = -1;  // the element list build that d_need belongs to
   int maxip = 128, rowstride = 0;
   // tables
   DBuf<double> d_spa_int, d_weight, d_spa_inter, d_spa_csub, d_spa_isub, d_frho, d_rhor, d_z2r;
@@ -532,6 +535,16 @@ struct cacg_context {
   // FP32 interpolation of rounded nodes by rounded weights, 8 products and
   // sums: 10)
   float cut_pass(double cutsq, double nu = 1.0) const {
+    float c = (float) (cutsq + cut_guard(cutsq, nu));
+    return std::nextafter(std::nextafter(c, 3.0e38f), 3.0e38f);
+  }
+  // and the other way: a pair whose float rsq is below the returned value has
+  // an exact rsq below cutsq
+  float cut_surely(double cutsq) const {
+    float c = (float) (cutsq - cut_guard(cutsq, 1.0));
+    return std::nextafter(std::nextafter(c, -3.0e38f), -3.0e38f);
+  }
+  double cut_guard(double cutsq, double nu) const {
     double X = 0.0;
     for (int d = 0; d < 3; d++)
       X = std::max(X, std::max(std::fabs(lo[d]), std::fabs(hi[d])) + cutghost[d] + max_size +
@@ -539,10 +552,8 @@ struct cacg_context {
     const double u = std::ldexp(1.0, -24);
     const double rn = std::max(cutneighmax, std::sqrt(cutsq));
     const double delta = 2.0 * nu * u * X * 1.001 + u * (rn + 1.0);
-    const double guard = 4.0 * u * cutsq + (1.0 + 4.0 * u) * (2.0 * std::sqrt(3.0) * rn * delta +
-                                                              3.0 * delta * delta);
-    float c = (float) (cutsq + guard);
-    return std::nextafter(std::nextafter(c, 3.0e38f), 3.0e38f);
+    return 4.0 * u * cutsq + (1.0 + 4.0 * u) * (2.0 * std::sqrt(3.0) * rn * delta +
+                                                3.0 * delta * delta);
   }
   float atom_cut_pass() const {
     if (pair_style == 2) return cut_pass(cutforcesq);
@@ -574,6 +585,7 @@ struct cacg_context {
   void neighbor_build();
   void neighbor_ebuild();
   void neighbor_nbuild();
+  void ensure_need();
   void pair_compute();
   void pair_compute_pass(int pass);
   void pair_compute_mixed(int pass);
@@ -633,13 +645,15 @@ struct cacg_context {
 };
 
 cacg_context::~cacg_context() {
-  DBuf<double4> *b4[] = {&d_x, &d_bx, &d_ebx, &d_site_x, &d_subc};
+  DBuf<double4> *b4[] = {&d_x, &d_ebx, &d_site_x, &d_subc};
   for (auto *b : b4) b->release();
   d_xh.release();
   d_site_h.release();
   d_spa_inter_f.release();
   d_node_f.release();
   d_sr.release();
+  d_bxf.release();
+  d_runs.release();
   d_xl.release();
   d_rhor_val4.release();
   d_ftab.release();
@@ -1985,6 +1999,13 @@ void cacg_context::setup_bins() {
         if (bin_distance(i, j, k) < cutneighmaxsq)
           stencil.push_back(k * bins.mbin[1] * bins.mbin[0] + j * bins.mbin[0] + i);
   upload(d_stencil, stencil, stream);
+  std::vector<int2> runs;
+  for (int b : stencil) {
+    if (!runs.empty() && runs.back().x + runs.back().y == b) runs.back().y++;
+    else runs.push_back(make_int2(b, 1));
+  }
+  nruns = (int) runs.size();
+  upload(d_runs, runs, stream);
 }
 
 void cacg_context::init() {
@@ -2337,17 +2358,19 @@ void cacg_context::neighbor_build() {
   check(cudaMemsetAsync(d_misc.p + 1, 0, sizeof(int) * 2, s), "memset");
   launch_coord2bin_atoms(d_x.p, nall, bins, d_abin.p, d_misc.p + 1, s);
   build_bins(d_abin.p, nall, bins.mbins, d_bcount, d_bstart, d_bmem, d_scan, s);
-  d_bx.ensure(nall, s);
-  launch_gather_bin_x_atoms(d_bmem.p, d_x.p, d_bx.p, nall, s);
+  d_bxf.ensure(nall, s);
+  launch_gather_bin_x_atoms(d_bmem.p, d_x.p, d_bxf.p, nall, s);
+  const float band_hi = cut_pass(cutneighmaxsq);
+  const float band_lo = cut_surely(cutneighmaxsq);
   launches += 7;
   stride = (nlocal + 31) / 32 * 32;
   d_num.ensure(nlocal, s);
   for (int attempt = 0; attempt < 3; attempt++) {
     d_list.ensure((size_t) maxneigh * stride, s);
     check(cudaMemsetAsync(d_misc.p + 2, 0, sizeof(int), s), "memset");
-    launch_atom_list(d_x.p, d_abin.p, d_bstart.p, d_bmem.p, d_bx.p, d_stencil.p,
-                     (int) stencil.size(), bins.mbins, nlocal, cutneighmaxsq, maxneigh, stride,
-                     d_num.p, d_list.p, d_misc.p + 2, s);
+    launch_atom_list(d_x.p, d_abin.p, d_bstart.p, d_bxf.p, d_runs.p, nruns, bins.mbins, nlocal,
+                     cutneighmaxsq, band_lo, band_hi, maxneigh, stride, d_num.p, d_list.p,
+                     d_misc.p + 2, s);
     launches++;
     check(cudaMemcpyAsync(h_pin + 1, d_misc.p + 1, sizeof(int) * 2, cudaMemcpyDeviceToHost, s), "ovf");
     sync();
@@ -2407,18 +2430,16 @@ void cacg_context::neighbor_nbuild() {
   }
   int nall = enlocal + enghost;
   ElemTables t = etab();
-  d_site_x.ensure(std::max(nsites, 1), s);
-  launch_sites(d_nodex.p, d_etype.p, d_site_base.p, nall, t, d_site_x.p, nullptr, s);
   d_subc.ensure((size_t) nall * nsub, s);
   launch_sub_centres(d_nodex.p, nall, t, d_subc.p, s);
-  launches += 2;
+  launches++;
   rowstride = (nrows + 31) / 32 * 32;
   d_ipnum.ensure(std::max(nrows, 1), s);
   for (int attempt = 0; attempt < 3; attempt++) {
     d_ipent.ensure((size_t) maxip * rowstride, s);
     check(cudaMemsetAsync(d_misc.p + 5, 0, sizeof(int), s), "memset");
     launch_ip_list(d_nodex.p, d_ex.p, d_etype.p, d_row_elem.p, d_row_jj.p, nrows, d_enum.p,
-                   d_elist.p, estride, d_subc.p, d_site_x.p, d_site_base.p, t, cut_elesq,
+                   d_elist.p, estride, d_subc.p, d_spa_inter_f.p, d_site_base.p, t, cut_elesq,
                    cut_subelesq, cutneighmaxsq, maxip, rowstride, d_ipnum.p, d_ipent.p,
                    d_misc.p + 5, s);
     launches++;
@@ -2433,27 +2454,16 @@ void cacg_context::neighbor_nbuild() {
   check(cudaMemsetAsync(d_fip.p, 0, sizeof(double) * 3 * std::max(nrows, 1), s), "fip");
   d_fipf.ensure(3 * (size_t) std::max(nrows, 1), s);
   check(cudaMemsetAsync(d_fipf.p, 0, sizeof(float2) * 3 * std::max(nrows, 1), s), "fipf");
-  // the sites any list references: the per-step site kernels compute only these
-  d_site_flag.ensure(std::max(nsites, 1), s);
-  d_site_pos.ensure(std::max(nsites, 1), s);
-  check(cudaMemsetAsync(d_site_flag.p, 0, sizeof(int) * std::max(nsites, 1), s), "flag");
-  fp64_fma::mark_sites(d_ipnum.p, d_ipent.p, nrows, rowstride, d_site_flag.p, s);
-  scan_exclusive(d_site_flag.p, d_site_pos.p, nsites, d_misc.p + 7, d_scan, s);
-  check(cudaMemcpyAsync(h_pin + 7, d_misc.p + 7, sizeof(int), cudaMemcpyDeviceToHost, s), "nneed");
+  need_of = -1;
   // the lists row-major for the mixed passes: row_start[nrows] = all entries
   d_row_start.ensure((size_t) nrows + 1, s);
   scan_exclusive(d_ipnum.p, d_row_start.p, nrows, d_row_start.p + nrows, d_scan, s);
   check(cudaMemcpyAsync(h_pin + 10, d_row_start.p + nrows, sizeof(int), cudaMemcpyDeviceToHost, s),
         "entries");
   sync();
-  nneed = h_pin[7];
   d_ent.ensure(std::max(h_pin[10], 1), s);
   mixed::ip_csr(d_ipnum.p, d_ipent.p, nrows, rowstride, d_row_start.p, d_ent.p, s);
-  d_need.ensure(std::max(nneed, 1), s);
-  d_need_elem.ensure(std::max(nneed, 1), s);
-  fp64_fma::need_compact(d_site_flag.p, d_site_pos.p, nsites, d_site_base.p, nall, d_need.p,
-                         d_need_elem.p, s);
-  launches += 4;
+  launches += 2;
   // for the mixed passes: the row-major lists as line codes
   // (element * maxlines + line) << 6 | kk, and the lines every row's entries
   // (every force row's) reference, a bit per site
@@ -2479,6 +2489,29 @@ void cacg_context::neighbor_nbuild() {
   }
   elist_builds++;
   elists_built = true;
+}
+
+// The sites that any integration-point list references, for the passes over
+// site arrays (thermo, lists that the line codes do not hold, the site count):
+// once per list build, when one of them asks.
+void cacg_context::ensure_need() {
+  if (need_of == elist_builds || enlocal == 0) return;
+  cudaStream_t s = stream;
+  d_misc.ensure(32, s);
+  d_site_flag.ensure(std::max(nsites, 1), s);
+  d_site_pos.ensure(std::max(nsites, 1), s);
+  check(cudaMemsetAsync(d_site_flag.p, 0, sizeof(int) * std::max(nsites, 1), s), "flag");
+  fp64_fma::mark_sites(d_ipnum.p, d_ipent.p, nrows, rowstride, d_site_flag.p, s);
+  scan_exclusive(d_site_flag.p, d_site_pos.p, nsites, d_misc.p + 7, d_scan, s);
+  check(cudaMemcpyAsync(h_pin + 7, d_misc.p + 7, sizeof(int), cudaMemcpyDeviceToHost, s), "nneed");
+  sync();
+  nneed = h_pin[7];
+  d_need.ensure(std::max(nneed, 1), s);
+  d_need_elem.ensure(std::max(nneed, 1), s);
+  fp64_fma::need_compact(d_site_flag.p, d_site_pos.p, nsites, d_site_base.p, enlocal + enghost,
+                         d_need.p, d_need_elem.p, s);
+  launches += 4;
+  need_of = elist_builds;
 }
 
 // ------------------------------------------------------------------ forces
@@ -3218,7 +3251,9 @@ void cacg_context::pair_ecompute() {
   // sites of every local and ghost element at the current node positions,
   // with their float copies, then this step's short lists of the rows
   d_site_h.ensure(std::max(nsites, 1), s);
-  // contraction-free in both modes: bit-identical to the all-sites kernel
+  ensure_need();
+  d_site_x.ensure(std::max(nsites, 1), s);
+  // contraction-free in both modes
   kmark(KT_SITES, 0);
   fp64_fma::sites_needed(d_nodex.p, d_etype.p, d_site_base.p, d_need.p, d_need_elem.p, nneed, t,
                          d_site_x.p, d_site_h.p, s);
@@ -3327,6 +3362,7 @@ void cacg_context::compute_thermo(double *out) {
     int nall = enlocal + enghost;
     ElemTables t = etab();
     EamTables e = eamtab();
+    ensure_need();
     d_site_x.ensure(std::max(nsites, 1), s);
     d_site_h.ensure(std::max(nsites, 1), s);
     fp64_fma::sites_needed(d_nodex.p, d_etype.p, d_site_base.p, d_need.p, d_need_elem.p, nneed, t,
@@ -4795,6 +4831,7 @@ int cacg_run_host(cacg_handle h, int nsteps, double *x, double *v, double *nodex
 
 int cacg_get_counts(cacg_handle h, long long *c, int n) {
   API_BEGIN
+  if (h->elists_built && n > 13) h->ensure_need();
   long long v[31] = {h->nlocal, h->nghost, 0, h->enlocal, h->enghost, 0, h->nrows, 0,
                      h->nrebuild, (long long) h->stencil.size(), h->ntimestep, h->nsites,
                      h->launches, h->nneed, h->nforce, 0, h->sur ? h->nfar : 0, 0, 0,

@@ -174,30 +174,30 @@ void launch_coord2bin_elems(const double *ex, int n, const BinGeom &g, int *bin,
 // counting sort by bin, members of a bin in ascending index order
 void build_bins(const int *bin, int n, int mbins, DBuf<int> &count, DBuf<int> &start,
                 DBuf<int> &members, DBuf<int> &scratch, cudaStream_t s);
-void launch_gather_bin_x_atoms(const int *members, const double4 *x, double4 *bx, int n,
+void launch_gather_bin_x_atoms(const int *members, const double4 *x, float4 *bxf, int n,
                                cudaStream_t s);
 void launch_gather_bin_x_elems(const int *members, const double *ex, double4 *bx, int n,
                                cudaStream_t s);
 
 // ---- neighbor lists (k_neigh.cu) ----
-void launch_atom_list(const double4 *x, const int *bin, const int *bstart, const int *bmem,
-                      const double4 *bx, const int *stencil, int nstencil, int mbins, int nlocal,
-                      double cutsq, int maxneigh, int stride, int *num, int *list,
-                      int *overflow, cudaStream_t s);
+// bxf: members in bin order (float xyz, index); runs: first offset and length of
+// the stencil's bins that follow each other; [lo, hi]: decided in FP64
+void launch_atom_list(const double4 *x, const int *bin, const int *bstart, const float4 *bxf,
+                      const int2 *runs, int nruns, int mbins, int nlocal, double cutsq, float lo,
+                      float hi, int maxneigh, int stride, int *num, int *list, int *overflow,
+                      cudaStream_t s);
 void launch_elem_list(const double *ex, const int *bin, const int *bstart, const int *bmem,
                       const double4 *bx, const int *stencil, int nstencil, int mbins, int nlocal,
                       double cutsq, int maxneigh, int stride, int *num, int *list,
                       int *overflow, cudaStream_t s);
 // site_h (may be null): float copy of each site for the FP32 pre-tests
-void launch_sites(const double *nodex, const int *etype, const int *site_base, int nelem,
-                  ElemTables t, double4 *site_x, float4 *site_h, cudaStream_t s);
 void launch_split_hi(const double4 *x, float4 *xh, int n, cudaStream_t s);
 void launch_sub_centres(const double *nodex, int nelem, ElemTables t, double4 *subc,
                         cudaStream_t s);
 void launch_ip_list(const double *nodex, const double *ex, const int *etype,
                     const int *row_elem, const int *row_jj, int nrows, const int *enum_,
-                    const int *elist, int estride, const double4 *subc, const double4 *site_x,
-                    const int *site_base, ElemTables t, double cut_elesq, double cut_subelesq,
+                    const int *elist, int estride, const double4 *subc,
+                    const float4 *spa_inter_f, const int *site_base, ElemTables t, double cut_elesq, double cut_subelesq,
                     double cutsq, int maxip, int rowstride, int *ipnum, int *ipent,
                     int *overflow, cudaStream_t s);
 
@@ -284,8 +284,6 @@ void eam_ip(const double *nodex, const double *erho, const int *etype, const int
             EamTables e, float cut_pass, const int *rows, double *fip, cudaStream_t s);
 void gather_nodef(const double *fip, const int *etype, const int *row_first, int nlocal_e,
                   ElemTables t, double *nodef, cudaStream_t s);
-void sites(const double *nodex, const int *etype, const int *site_base, int nelem, ElemTables t,
-           double4 *site_x, float4 *site_h, cudaStream_t s);
 // the sites any integration-point list references (computed per rebuild)
 void mark_sites(const int *ipnum, const int *ipent, int nrows, int rowstride, int *flag,
                 cudaStream_t s);

@@ -368,10 +368,14 @@ __global__ void k_bin_sort(const int *__restrict__ bin, int n, const int *__rest
   members_out[s0 + rank] = i;
 }
 
+// members in bin order: float coordinates and the index
 __global__ void k_gather_bx_atoms(const int *__restrict__ mem, const double4 *__restrict__ x,
-                                  double4 *__restrict__ bx, int n) {
+                                  float4 *__restrict__ bxf, int n) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < n) bx[p] = x[mem[p]];
+  if (p >= n) return;
+  const int i = mem[p];
+  const double4 c = x[i];
+  bxf[p] = make_float4((float) c.x, (float) c.y, (float) c.z, __int_as_float(i));
 }
 
 __global__ void k_gather_bx_elems(const int *__restrict__ mem, const double *__restrict__ ex,
@@ -534,10 +538,10 @@ void build_bins(const int *bin, int n, int mbins, DBuf<int> &count, DBuf<int> &s
   check(cudaGetLastError(), "build_bins");
 }
 
-void launch_gather_bin_x_atoms(const int *members, const double4 *x, double4 *bx, int n,
+void launch_gather_bin_x_atoms(const int *members, const double4 *x, float4 *bxf, int n,
                                cudaStream_t s) {
   if (n <= 0) return;
-  k_gather_bx_atoms<<<nblk(n, 256), 256, 0, s>>>(members, x, bx, n);
+  k_gather_bx_atoms<<<nblk(n, 256), 256, 0, s>>>(members, x, bxf, n);
   check(cudaGetLastError(), "gather_bx_atoms");
 }
 

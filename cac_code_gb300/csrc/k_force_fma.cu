@@ -358,28 +358,6 @@ __global__ void k_site_fp_needed(const double *__restrict__ erho, const int *__r
   site_fp[sid] = spline_deriv(eam.frho + 7 * m, p);
 }
 
-// site positions with fused multiply-adds (the exact mode uses k_sites in
-// k_neigh.cu, built without contraction); also writes the float copy
-__global__ void k_sites_fma(const double *__restrict__ nodex, const int *__restrict__ etype,
-                            const int *__restrict__ site_base, ElemTables t,
-                            double4 *__restrict__ site_x, float4 *__restrict__ site_h) {
-  __shared__ double nx[24];
-  const int e = blockIdx.x;
-  if (threadIdx.x < 24) nx[threadIdx.x] = nodex[24 * (size_t) e + threadIdx.x];
-  __syncthreads();
-  const int ty = etype[e];
-  const int nint = t.inter_num[ty];
-  const double *S0 = t.spa_inter + (size_t) t.inter_off[ty] * NPE;
-  const int base = site_base[e];
-  for (int nj = threadIdx.x; nj < nint; nj += blockDim.x) {
-    const double *S = S0 + (size_t) nj * NPE;
-    double a, b, c;
-    ip_position(S, nx, a, b, c);
-    site_x[base + nj] = make_double4(a, b, c, 0.0);
-    site_h[base + nj] = make_float4((float) a, (float) b, (float) c, 0.f);
-  }
-}
-
 }  // namespace
 
 void filter_rows(const double *nodex, const int *etype, const int *row_elem, const int *row_jj,
@@ -424,13 +402,6 @@ void site_fp_needed(const double *erho, const int *etype, const int *site_base, 
   k_site_fp_needed<<<nblk(nneed, 128), 128, 0, s>>>(erho, etype, site_base, need, need_elem,
                                                    nneed, t, e, site_fp);
   check(cudaGetLastError(), "site_fp_needed");
-}
-
-void sites(const double *nodex, const int *etype, const int *site_base, int nelem, ElemTables t,
-           double4 *site_x, float4 *site_h, cudaStream_t s) {
-  if (nelem <= 0) return;
-  k_sites_fma<<<nelem, 128, 0, s>>>(nodex, etype, site_base, t, site_x, site_h);
-  check(cudaGetLastError(), "sites_fma");
 }
 
 void lj_ip(const double *nodex, const int *etype, const int *row_elem, const int *row_jj,

@@ -18,35 +18,72 @@ namespace {
 
 inline int nblk(long long n, int t) { return (int) ((n + t - 1) / t); }
 
-__global__ void __launch_bounds__(128)
+// Atom list, one warp per atom.  The stencil's bins that follow each other in
+// x are one run of the bin-ordered members, so the warp walks the runs 32
+// members at a time and a ballot appends the hits in the reference's order
+// (stencil order, members in index order).  A distance is decided in FP32 on
+// the float copies outside [lo, hi] (no float rounding moves a pair across the
+// cutoff there) and in the reference's FP64 arithmetic inside: of ~560
+// candidates a pair of FP64 units need not see more than the few in the band.
+// One thread per atom with FP64 throughout took 1,133 us for 72,600 atoms.
+constexpr int AL_BLOCK = 256;
+
+__global__ void __launch_bounds__(AL_BLOCK)
 k_atom_list(const double4 *__restrict__ x, const int *__restrict__ bin,
-            const int *__restrict__ bstart, const int *__restrict__ bmem,
-            const double4 *__restrict__ bx, const int *__restrict__ stencil, int nstencil,
-            int mbins, int nlocal, double cutsq, int maxneigh, int stride,
-            int *__restrict__ num, int *__restrict__ list, int *__restrict__ overflow) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+            const int *__restrict__ bstart, const float4 *__restrict__ bxf,
+            const int2 *__restrict__ runs, int nruns, int mbins, int nlocal, double cutsq, float lo,
+            float hi, int maxneigh, int stride, int *__restrict__ num, int *__restrict__ list,
+            int *__restrict__ overflow) {
+  const int i = (int) ((blockIdx.x * (long long) AL_BLOCK + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
   if (i >= nlocal) return;
   const double4 xi = x[i];
+  const float fx = (float) xi.x, fy = (float) xi.y, fz = (float) xi.z;
   const int ib = bin[i];
   int n = 0;
-  for (int k = 0; k < nstencil; k++) {
-    int b = ib + __ldg(stencil + k);
-    if (b < 0 || b >= mbins) continue;
-    int p1 = __ldg(bstart + b + 1);
-    for (int p = __ldg(bstart + b); p < p1; p++) {
-      int j = __ldg(bmem + p);
-      if (j == i) continue;
-      double4 xj = bx[p];
-      double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-      double rsq = dx * dx + dy * dy + dz * dz;
-      if (rsq <= cutsq) {
-        if (n < maxneigh) list[(size_t) n * stride + i] = j;
-        n++;
+  for (int r0 = 0; r0 < nruns; r0 += 32) {
+    // this lane's run: its members' range
+    int p0 = 0, p1 = 0;
+    if (r0 + lane < nruns) {
+      const int2 run = __ldg(runs + r0 + lane);
+      const int b0 = max(ib + run.x, 0), b1 = min(ib + run.x + run.y, mbins);
+      if (b0 < b1) {
+        p0 = __ldg(bstart + b0);
+        p1 = __ldg(bstart + b1);
+      }
+    }
+    const int nr = min(32, nruns - r0);
+    for (int r = 0; r < nr; r++) {
+      const int q1 = __shfl_sync(0xffffffffu, p1, r);
+      for (int q = __shfl_sync(0xffffffffu, p0, r); q < q1; q += 32) {
+        bool hit = false;
+        int j = i;
+        if (q + lane < q1) {
+          const float4 c = __ldg(bxf + q + lane);
+          j = __float_as_int(c.w);
+          const float gx = fx - c.x, gy = fy - c.y, gz = fz - c.z;
+          const float g = gx * gx + gy * gy + gz * gz;
+          hit = g < lo;
+          if (!hit && !(g > hi)) {
+            const double4 xj = x[j];
+            const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+            hit = dx * dx + dy * dy + dz * dz <= cutsq;
+          }
+          hit = hit && j != i;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (hit) {
+          const int slot = n + __popc(m & ((1u << lane) - 1u));
+          if (slot < maxneigh) list[(size_t) slot * stride + i] = j;
+        }
+        n += __popc(m);
       }
     }
   }
-  num[i] = n;
-  if (n > maxneigh) atomicMax(overflow, n);
+  if (lane == 0) {
+    num[i] = n;
+    if (n > maxneigh) atomicMax(overflow, n);
+  }
 }
 
 __global__ void __launch_bounds__(128)
@@ -80,34 +117,6 @@ k_elem_list(const double *__restrict__ ex, const int *__restrict__ bin,
   if (n > maxneigh) atomicMax(overflow, n);
 }
 
-// Interpolated lattice sites of every element (Element::interpolate_atom_vec,
-// element.cpp:1226-1272): x = sum_k N_k x_k in node order.  One block per element.
-__global__ void k_sites(const double *__restrict__ nodex, const int *__restrict__ etype,
-                        const int *__restrict__ site_base, ElemTables t,
-                        double4 *__restrict__ site_x, float4 *__restrict__ site_h) {
-  __shared__ double nx[24];
-  const int e = blockIdx.x;
-  if (threadIdx.x < 24) nx[threadIdx.x] = nodex[24 * (size_t) e + threadIdx.x];
-  __syncthreads();
-  const int ty = etype[e];
-  const int nint = t.inter_num[ty];
-  const double *S0 = t.spa_inter + (size_t) t.inter_off[ty] * NPE;
-  const int base = site_base[e];
-  for (int nj = threadIdx.x; nj < nint; nj += blockDim.x) {
-    const double *S = S0 + (size_t) nj * NPE;
-    double a = 0, b = 0, c = 0;
-#pragma unroll
-    for (int k = 0; k < NPE; k++) {
-      double s = S[k];
-      a += s * nx[3 * k];
-      b += s * nx[3 * k + 1];
-      c += s * nx[3 * k + 2];
-    }
-    site_x[base + nj] = make_double4(a, b, c, 0.0);
-    if (site_h) site_h[base + nj] = make_float4((float) a, (float) b, (float) c, 0.f);
-  }
-}
-
 __global__ void k_split_hi(const double4 *__restrict__ x, float4 *__restrict__ xh, int n) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -133,29 +142,50 @@ __global__ void k_sub_centres(const double *__restrict__ nodex, int nelem, ElemT
   subc[tid] = make_double4(a, b, c, 0.0);
 }
 
-// One warp per integration point row.
+// Integration-point lists, one warp per row.  Sites are tested in FP32 on
+// coordinates relative to node 0 of the row's element, interpolated from float
+// nodes and weights: with R the largest such coordinate a difference is within
+// 22 u R (u = 2^-24), and FP64 arithmetic on absolute coordinates up to X
+// places the pair within 24 * 2^-53 X of that.  Only a distance that these
+// bounds leave open (near the cutoff, or near the 1e-2 that excludes the row's
+// own site) is formed in FP64, as the reference does (Interpolate_to_atom_vec,
+// element.cpp:1226-1272, then full_node_neighbor.cpp:150-190).  The FP64
+// positions of all sites, local and ghost, took 579 us and the FP64 tests
+// 636 us for 1,024 elements of 1,331 sites.
+__device__ __forceinline__ double node_interp(const double *__restrict__ N,
+                                              const double *__restrict__ x, int d) {
+  double a = 0;
+#pragma unroll
+  for (int k = 0; k < NPE; k++) a += N[k] * x[3 * k + d];
+  return a;
+}
+
 __global__ void __launch_bounds__(128)
 k_ip_list(const double *__restrict__ nodex, const double *__restrict__ ex,
           const int *__restrict__ etype, const int *__restrict__ row_elem,
           const int *__restrict__ row_jj, int nrows, const int *__restrict__ enum_,
           const int *__restrict__ elist, int estride, const double4 *__restrict__ subc,
-          const double4 *__restrict__ site_x, const int *__restrict__ site_base, ElemTables t,
+          const float4 *__restrict__ spa_inter_f, const int *__restrict__ site_base, ElemTables t,
           double cut_elesq, double cut_subelesq, double cutsq, int maxip, int rowstride,
           int *__restrict__ ipnum, int *__restrict__ ipent, int *__restrict__ overflow) {
+  __shared__ float s_nodes[4][24];
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (r >= nrows) return;
+  float *s_x = s_nodes[threadIdx.x >> 5];
   const unsigned lt_mask = (1u << lane) - 1u;
   const int e = row_elem[r], jj = row_jj[r], ty = etype[e];
   const double *N = t.spa_int + ((size_t) t.int_off[ty] + jj) * NPE;
   const double *nxe = nodex + 24 * (size_t) e;
-  double ix = 0, iy = 0, iz = 0;
-#pragma unroll
-  for (int k = 0; k < NPE; k++) {
-    ix += N[k] * nxe[3 * k];
-    iy += N[k] * nxe[3 * k + 1];
-    iz += N[k] * nxe[3 * k + 2];
-  }
+  // the row's point: lanes 0..2 a component each
+  const double pd = lane < 3 ? node_interp(N, nxe, lane) : 0.0;
+  const double ix = __shfl_sync(0xffffffffu, pd, 0), iy = __shfl_sync(0xffffffffu, pd, 1),
+               iz = __shfl_sync(0xffffffffu, pd, 2);
+  const double x0 = nxe[lane % 3];  // node 0, this lane's component
+  const float pf = lane < 3 ? (float) (pd - x0) : 0.f;
+  const float px = __shfl_sync(0xffffffffu, pf, 0), py = __shfl_sync(0xffffffffu, pf, 1),
+              pz = __shfl_sync(0xffffffffu, pf, 2);
+  const float rc = sqrtf((float) cutsq);
   int n = 0;
   const int nsub = t.nsub;
   const int ne = enum_[e];
@@ -168,8 +198,24 @@ k_ip_list(const double *__restrict__ nodex, const double *__restrict__ ex,
       double npdis = (ix - cx) * (ix - cx) + (iy - cy) * (iy - cy) + (iz - cz) * (iz - cz);
       if (!(npdis <= cut_elesq)) continue;
     }
+    // the element's nodes relative to node 0 of the row's element
+    float R = 0.f, X = 0.f;
+    __syncwarp();
+    if (lane < 24) {
+      const double v = nodex[24 * (size_t) j + lane];
+      const float f = (float) (v - x0);
+      s_x[lane] = f;
+      R = fmaxf(fabsf(f), fabsf(pf));
+      X = fabsf((float) v);
+    }
+    __syncwarp();
+    R = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(R)));
+    X = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(X)));
+    const float delta = 1.7320509f * (24.f * 5.9604645e-8f * R + 32.f * 1.110223e-16f * X);
+    const float a0 = rc * 0.999999f - delta, a1 = rc * 1.000001f + delta, a2 = 0.01f * 1.000001f + delta;
+    const float lo = a0 > 0.f ? a0 * a0 * 0.99999f : -1.f, hi = a1 * a1 * 1.00001f;
+    const float near0 = self ? a2 * a2 * 1.00001f : -1.f;
     // sub-element centre test, lanes over sub-elements
-    unsigned submask = 0;
     for (int s0 = 0; s0 < nsub; s0 += 32) {
       int isub = s0 + lane;
       bool pass = false;
@@ -187,6 +233,7 @@ k_ip_list(const double *__restrict__ nodex, const double *__restrict__ ex,
         int isub2 = s0 + bit;
         int first = t.sub_first[isub2], cnt = t.sub_first[isub2 + 1] - first;
         const int sb = site_base[j];
+        const size_t at0 = (size_t) t.inter_off[etype[j]];
         for (int m0 = 0; m0 < cnt; m0 += 32) {
           int mm = m0 + lane;
           bool hit = false;
@@ -194,10 +241,27 @@ k_ip_list(const double *__restrict__ nodex, const double *__restrict__ ex,
           if (mm < cnt) {
             int nj = t.list_inter_sub[first + mm];
             sid = sb + nj;
-            double4 sx = site_x[sid];
-            double dx = sx.x - ix, dy = sx.y - iy, dz = sx.z - iz;
-            double rsq = dx * dx + dy * dy + dz * dz;
-            hit = self ? (rsq <= cutsq && rsq > 1.0e-4) : (rsq <= cutsq);
+            const float4 w0 = __ldg(spa_inter_f + 2 * (at0 + nj));
+            const float4 w1 = __ldg(spa_inter_f + 2 * (at0 + nj) + 1);
+            const float w[NPE] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+            float sx = 0.f, sy = 0.f, sz = 0.f;
+#pragma unroll
+            for (int k = 0; k < NPE; k++) {
+              sx = __fmaf_rn(w[k], s_x[3 * k], sx);
+              sy = __fmaf_rn(w[k], s_x[3 * k + 1], sy);
+              sz = __fmaf_rn(w[k], s_x[3 * k + 2], sz);
+            }
+            const float gx = sx - px, gy = sy - py, gz = sz - pz;
+            const float g = gx * gx + gy * gy + gz * gz;
+            hit = g < lo && g > near0;
+            if (!hit && !(g > hi)) {
+              const double *S = t.spa_inter + (at0 + nj) * NPE;
+              const double *xj = nodex + 24 * (size_t) j;
+              const double dx = node_interp(S, xj, 0) - ix, dy = node_interp(S, xj, 1) - iy,
+                           dz = node_interp(S, xj, 2) - iz;
+              const double rsq = dx * dx + dy * dy + dz * dz;
+              hit = self ? (rsq <= cutsq && rsq > 1.0e-4) : (rsq <= cutsq);
+            }
           }
           unsigned hb = __ballot_sync(0xffffffffu, hit);
           if (hit) {
@@ -207,7 +271,6 @@ k_ip_list(const double *__restrict__ nodex, const double *__restrict__ ex,
           n += __popc(hb);
         }
       }
-      (void) submask;
     }
   }
   if (lane == 0) {
@@ -218,14 +281,14 @@ k_ip_list(const double *__restrict__ nodex, const double *__restrict__ ex,
 
 }  // namespace
 
-void launch_atom_list(const double4 *x, const int *bin, const int *bstart, const int *bmem,
-                      const double4 *bx, const int *stencil, int nstencil, int mbins,
-                      int nlocal, double cutsq, int maxneigh, int stride, int *num, int *list,
-                      int *overflow, cudaStream_t s) {
+void launch_atom_list(const double4 *x, const int *bin, const int *bstart, const float4 *bxf,
+                      const int2 *runs, int nruns, int mbins, int nlocal, double cutsq, float lo,
+                      float hi, int maxneigh, int stride, int *num, int *list, int *overflow,
+                      cudaStream_t s) {
   if (nlocal <= 0) return;
-  k_atom_list<<<nblk(nlocal, 128), 128, 0, s>>>(x, bin, bstart, bmem, bx, stencil, nstencil,
-                                                 mbins, nlocal, cutsq, maxneigh, stride, num,
-                                                 list, overflow);
+  k_atom_list<<<nblk((long long) nlocal * 32, AL_BLOCK), AL_BLOCK, 0, s>>>(
+      x, bin, bstart, bxf, runs, nruns, mbins, nlocal, cutsq, lo, hi, maxneigh, stride, num, list,
+      overflow);
   check(cudaGetLastError(), "atom_list");
 }
 
@@ -238,13 +301,6 @@ void launch_elem_list(const double *ex, const int *bin, const int *bstart, const
                                                  mbins, nlocal, cutsq, maxneigh, stride, num,
                                                  list, overflow);
   check(cudaGetLastError(), "elem_list");
-}
-
-void launch_sites(const double *nodex, const int *etype, const int *site_base, int nelem,
-                  ElemTables t, double4 *site_x, float4 *site_h, cudaStream_t s) {
-  if (nelem <= 0) return;
-  k_sites<<<nelem, 128, 0, s>>>(nodex, etype, site_base, t, site_x, site_h);
-  check(cudaGetLastError(), "sites");
 }
 
 void launch_split_hi(const double4 *x, float4 *xh, int n, cudaStream_t s) {
@@ -262,13 +318,13 @@ void launch_sub_centres(const double *nodex, int nelem, ElemTables t, double4 *s
 
 void launch_ip_list(const double *nodex, const double *ex, const int *etype,
                     const int *row_elem, const int *row_jj, int nrows, const int *enum_,
-                    const int *elist, int estride, const double4 *subc, const double4 *site_x,
-                    const int *site_base, ElemTables t, double cut_elesq, double cut_subelesq,
+                    const int *elist, int estride, const double4 *subc,
+                    const float4 *spa_inter_f, const int *site_base, ElemTables t, double cut_elesq, double cut_subelesq,
                     double cutsq, int maxip, int rowstride, int *ipnum, int *ipent,
                     int *overflow, cudaStream_t s) {
   if (nrows <= 0) return;
   k_ip_list<<<nblk((long long) nrows * 32, 128), 128, 0, s>>>(
-      nodex, ex, etype, row_elem, row_jj, nrows, enum_, elist, estride, subc, site_x,
+      nodex, ex, etype, row_elem, row_jj, nrows, enum_, elist, estride, subc, spa_inter_f,
       site_base, t, cut_elesq, cut_subelesq, cutsq, maxip, rowstride, ipnum, ipent, overflow);
   check(cudaGetLastError(), "ip_list");
 }

@@ -84,3 +84,32 @@ def test_forces_match_the_oracle(cacg_lib, oracle_lib, name, mode):
             assert np.array_equal(got.view(np.int64), np.ascontiguousarray(ref).view(np.int64))
         else:
             assert np.abs(got - ref).max() <= FP64_TOL * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("nae,skin", [(8, 2.0 * C.A_LJ), (6, 1.5 ** 0.5 * 2.0 * C.A_LJ), (4, 2.8)])
+def test_lists_on_a_perfect_lattice(cacg_lib, oracle_lib, nae, skin):
+    """List radii at (and off) a shell of the undisplaced lattice: pairs whose
+    FP32 distance cannot tell on which side of the radius they lie, own and
+    other elements' sites among them, entry for entry."""
+    m = _slab("lj/cut", (3, 2 * nae, 2 * nae), nae, 2, L.gauss_intp(nae, False), 5, 0.0)
+    o = oracle_lib.Oracle(m, units="lj", pair="lj/cut", skin=skin, lj=(1.0, 1.0, 2.5), dt=0.005)
+    o.setup()
+    want = tuple(o.atom_list()) + tuple(o.elem_lists())
+    s = cacg_lib.System(0)
+    try:
+        s.command("units lj")
+        s.command("boundary f p p")
+        s.load_model(m)
+        s.command("pair_style lj/cut 2.5")
+        s.command("pair_coeff 1 1 1.0 1.0")
+        s.command(f"neighbor {skin!r} bin")
+        s.init()
+        s.setup()
+        s.neighbor_build()
+        s.neighbor_ebuild()
+        s.neighbor_nbuild()
+        got = tuple(s.atom_list()) + tuple(s.elem_lists())
+    finally:
+        s.close()
+    for g, w in zip(got, want):
+        assert np.array_equal(g, w)
