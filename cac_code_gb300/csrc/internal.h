@@ -530,11 +530,29 @@ void centro(const double4 *x, const int *num, const int *list, int stride, int i
 
 // ---- tensor-core GEMM (k_gemm.cu) and the surrogate MLP (mlp.cu) ----
 namespace gemm {
-// C = A B^T, bf16 operands (K-major), fp32 accumulation; kind: 0 store C,
-// 1 C = acc + bias, 2 Z = acc + bias and H = silu(Z), 3 H = acc * silu'(Z),
-// 4 H = silu(acc + bias)
-void gemm_tn(const void *A, int lda, const void *B, int ldb, int M, int N, int K, int kind,
-             const float *bias, float *c, int ldc, void *h, int ldh, int *err, cudaStream_t s);
+// C = A B^T, bf16 operands (K-major), fp32 accumulation
+void gemm_tn(const void *A, int lda, const void *B, int ldb, int M, int N, int K, float *c, int ldc,
+             int *err, cudaStream_t s);
+// One training step's passes for the members stacked in these arrays (layers
+// 0..3; B rows per member, a multiple of 128)
+struct TrainArgs {
+  int members, B, n_valid;       // n_valid rows of each member count
+  int splits, tps;               // the batch in `splits` parts of `tps` 64-row tiles
+  const float *p;                // parameters [members][pstride]
+  long pstride, ow[4], ob[4];    // offsets of weights and biases
+  const float *tb;               // targets [members * B][24]
+  void *h[4], *ht[4];            // bf16 inputs of the layers [members * B][64 | 256], transposed
+  float *z[3];                   // pre-activations [members * B][256], tile-transposed
+  void *g[4], *gt[4];            // bf16 gradients [members * B][256 | 64], transposed
+  void *w[4], *wt[4];            // bf16 weights [members * 256 | 24][64 | 256]; transposed (1..3)
+  float *part;                   // weight-gradient partial sums [splits][members][pstride]
+  int *err;
+};
+struct TrainPlan;  // the arrays' tensor maps, made once per call
+TrainPlan *train_plan(const TrainArgs &t);
+void train_plan_free(TrainPlan *p);
+// loss: [members][B / 128] sums of squared errors
+void train_passes(const TrainPlan &p, double *loss, cudaStream_t s);
 // all members and layers of the surrogate in one launch (k_mlp_ensemble)
 void mlp_ensemble(const void *xf, int n, const void *w1s, const void *w2s, const void *w3s,
                   const void *w4s, const float *bias, int members, const float *norm, float *mean,

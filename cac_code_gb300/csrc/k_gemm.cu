@@ -8,17 +8,13 @@
 // accumulator, and releases each stage with tcgen05.commit on the stage's
 // "empty" mbarrier.  After the last commit the four warps read the
 // accumulator back with tcgen05.ld (warp w owns TMEM lanes 32w..32w+31, i.e.
-// rows 32w..32w+31 of the tile) and apply one of the epilogues below.
+// rows 32w..32w+31 of the tile).
 //
 // Every mbarrier wait is bounded; a wait that runs out sets *err, the CTA
 // waits (bounded) for the copies it issued, frees its TMEM and returns.
 //
-// Epilogues (the surrogate MLP's forward and backward passes):
-//   STORE_F32    C = acc                          (fp32, ldc)
-//   BIAS_F32     C = acc + bias[n]                (fp32, ldc)
-//   BIAS_SILU    Z = acc + bias[n] (fp32, ldc);  H = silu(Z) (bf16, ldh)
-//   DSILU        H = acc * silu'(Z[m, n])         (bf16, ldh; Z read, ldc)
-//   SILU_ONLY    H = silu(acc + bias[n])          (bf16, ldh; inference)
+// k_gemm_tn is the plain product; the surrogate's training passes (k_train_*)
+// and its inference (k_mlp_ensemble) build on the same pieces.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -137,12 +133,8 @@ __device__ __forceinline__ float siluf_(float z) {
 }
 
 struct Epi {
-  int kind;
-  const float *bias;
-  float *c;  // fp32 out (STORE_F32, BIAS_F32, BIAS_SILU: Z) or Z in (DSILU)
+  float *c;
   int ldc;
-  __nv_bfloat16 *h;  // bf16 out (BIAS_SILU, DSILU)
-  int ldh;
 };
 
 template <int BN, int STAGES>
@@ -261,54 +253,15 @@ k_gemm_tn(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUt
       if (row >= M) continue;
       const int col = n0 + c;
       const bool full = col + 16 <= N;
-      if (ep.kind == 0 || ep.kind == 1) {
-        float *dst = ep.c + (size_t) row * ep.ldc + col;
-        if (ep.kind == 1)
+      float *dst = ep.c + (size_t) row * ep.ldc + col;
+      if (full && (ep.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
 #pragma unroll
-          for (int i = 0; i < 16; i++) v[i] += col + i < N ? ep.bias[col + i] : 0.f;
-        if (full && (ep.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-#pragma unroll
-          for (int i = 0; i < 4; i++)
-            reinterpret_cast<float4 *>(dst)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 16; i++)
-            if (col + i < N) dst[i] = v[i];
-        }
-        continue;
-      }
-      // bf16 outputs: 16 values as two 16-byte stores where the row allows it
-      float hv[16];
-      if (ep.kind == 2 || ep.kind == 4) {
-        float *z = ep.c ? ep.c + (size_t) row * ep.ldc + col : nullptr;
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-          const float zz = v[i] + (col + i < N ? ep.bias[col + i] : 0.f);
-          if (ep.kind == 2 && col + i < N) z[i] = zz;
-          hv[i] = zz * sigmoidf_(zz);
-        }
-      } else {
-        const float *z = ep.c + (size_t) row * ep.ldc + col;
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-          const float zz = col + i < N ? z[i] : 0.f, sg = sigmoidf_(zz);
-          hv[i] = v[i] * sg * (1.f + zz * (1.f - sg));
-        }
-      }
-      __nv_bfloat16 *h = ep.h + (size_t) row * ep.ldh + col;
-      if (full && (ep.ldh & 7) == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0) {
-        unsigned w[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          __nv_bfloat162 p2 = __floats2bfloat162_rn(hv[2 * i], hv[2 * i + 1]);
-          w[i] = *reinterpret_cast<unsigned *>(&p2);
-        }
-        reinterpret_cast<uint4 *>(h)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-        reinterpret_cast<uint4 *>(h)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+        for (int i = 0; i < 4; i++)
+          reinterpret_cast<float4 *>(dst)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
       } else {
 #pragma unroll
         for (int i = 0; i < 16; i++)
-          if (col + i < N) h[i] = __float2bfloat16(hv[i]);
+          if (col + i < N) dst[i] = v[i];
       }
     }
   }
@@ -544,6 +497,294 @@ k_mlp_ensemble(const __grid_constant__ CUtensorMap tma_x, const __grid_constant_
   }
 }
 
+// ---------------------------------------------------------------- training
+//
+// One Adam step of every member at once: grid.y (or .x) runs over the members,
+// whose activations, weights and gradients are stacked.  A layer kernel forms a
+// 128-row tile of one layer (forward or backward) and writes what the next
+// kernels read, as they read it: the activation (or gradient) row-major, K-major
+// for the next layer, and transposed, K-major for the weight gradients, so that
+// no transpose runs by itself; Z transposed within the tile, so that a warp's
+// loads and stores are whole lines.  The weight gradients of all layers are one
+// launch, the batch split over blocks that leave partial sums, which the
+// update kernel adds in order (no atomics: the same result at every run), with
+// the bias gradients, Adam and the new BF16 weights.
+//
+// What bounded it: launches and idle SMs.  One member's 2,048-row step was 45
+// launches, GEMMs on 2 to 16 blocks whose epilogues stored one float a line,
+// and took 508 us; the step of four members now takes 10 launches.
+constexpr int TR_NT = 512, TR_STAGES = 4, TR_A = BM * BK * 2, TR_B = 256 * BK * 2;
+constexpr int TR_H = 256, TR_IN = 64, TR_OUT = 24, TR_OUTP = 64;
+
+size_t train_smem() { return 1024 + (size_t) TR_STAGES * (TR_A + TR_B) + (2 * TR_STAGES + 1) * 8 + 16; }
+
+struct TrainSmem {
+  unsigned char *sa, *sb;
+  unsigned long long *bars;  // full, empty, done
+  unsigned *tmem_slot;
+};
+
+__device__ __forceinline__ TrainSmem train_smem_of(unsigned char *raw) {
+  TrainSmem m;
+  m.sa = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(raw) + 1023) &
+                                           ~static_cast<uintptr_t>(1023));
+  m.sb = m.sa + TR_STAGES * TR_A;
+  m.bars = reinterpret_cast<unsigned long long *>(m.sb + TR_STAGES * TR_B);
+  m.tmem_slot = reinterpret_cast<unsigned *>(m.bars + 2 * TR_STAGES + 1);
+  return m;
+}
+
+// barriers and a 256-column TMEM accumulator; all threads
+__device__ __forceinline__ unsigned train_begin(const TrainSmem &m, int *s_fail) {
+  if (threadIdx.x == 0) {
+    *s_fail = 0;
+    for (int i = 0; i < 2 * TR_STAGES + 1; i++) mbar_init(smem_u32(m.bars + i), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(m.tmem_slot)),
+                 "r"(256)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  return *m.tmem_slot;
+}
+
+__device__ __forceinline__ void train_end(unsigned tmem) {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256) : "memory");
+  }
+}
+
+// D[128][bn] = sum over nk k-tiles (from tile k0) of A rows ya.. and B rows yb..;
+// thread 0 streams and issues, all threads wait: true when D is complete
+__device__ __forceinline__ bool train_mma(const TrainSmem &m, unsigned tmem, const CUtensorMap *ta,
+                                          const CUtensorMap *tb, int k0, int nk, int ya, int yb,
+                                          int bn, int *err, int *s_fail) {
+  if (threadIdx.x == 0) {
+    const unsigned idesc = idesc_bf16(bn), bytes = TR_A + (unsigned) bn * BK * 2;
+    int issued = 0, consumed = 0;
+    bool ok = true;
+    auto load = [&](int kt) {
+      const int st = kt % TR_STAGES;
+      const unsigned fb = smem_u32(m.bars + st);
+      mbar_expect_tx(fb, bytes);
+      tma_load_2d(smem_u32(m.sa + st * TR_A), ta, (k0 + kt) * BK, ya, fb);
+      tma_load_2d(smem_u32(m.sb + st * TR_B), tb, (k0 + kt) * BK, yb, fb);
+      issued++;
+    };
+    for (int kt = 0; kt < TR_STAGES && kt < nk; kt++) load(kt);
+    for (int kt = 0; kt < nk && ok; kt++) {
+      const int st = kt % TR_STAGES;
+      if (!mbar_wait(smem_u32(m.bars + st), (kt / TR_STAGES) & 1)) {
+        ok = false;
+        break;
+      }
+      consumed++;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const unsigned a_addr = smem_u32(m.sa + st * TR_A), b_addr = smem_u32(m.sb + st * TR_B);
+#pragma unroll
+      for (int kk = 0; kk < BK / 16; kk++)
+        mma_bf16(tmem, sw128_desc(a_addr + kk * 32), sw128_desc(b_addr + kk * 32), idesc,
+                 (kt | kk) != 0);
+      mma_commit(smem_u32(m.bars + TR_STAGES + st));
+      // refill the stage the previous k-tile used, once its MMAs are done
+      if (kt >= 1 && kt - 1 + TR_STAGES < nk) {
+        const int pk = kt - 1, ps = pk % TR_STAGES;
+        if (!mbar_wait(smem_u32(m.bars + TR_STAGES + ps), (pk / TR_STAGES) & 1)) {
+          ok = false;
+          break;
+        }
+        load(pk + TR_STAGES);
+      }
+    }
+    mma_commit(smem_u32(m.bars + 2 * TR_STAGES));
+    if (!ok) {
+      atomicExch(err, 1);
+      // let the copies and MMAs already issued finish before the block's shared
+      // memory and TMEM go away
+      for (int k = consumed; k < issued; k++)
+        mbar_wait(smem_u32(m.bars + k % TR_STAGES), (k / TR_STAGES) & 1);
+      mbar_wait(smem_u32(m.bars + 2 * TR_STAGES), 0);
+      *s_fail = 1;
+    }
+  }
+  __syncwarp();
+  const bool ready = mbar_wait(smem_u32(m.bars + 2 * TR_STAGES), 0);
+  if (!ready && (threadIdx.x & 31) == 0) atomicExch(err, 2);
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  return __syncthreads_and(ready && *((volatile int *) s_fail) == 0) != 0;
+}
+
+struct TrainLayer {
+  int B, nk, bn, brows;        // rows per member, k-tiles, tile width, weight rows per member
+  const float *bias;           // member m's at bias + m * pstride
+  long pstride;
+  float *z;                    // [tile][256][128]
+  __nv_bfloat16 *h, *ht;       // [members * B][ldh], [members * cols][B]
+  int ldh;
+  const float *t;              // OUT: targets [members * B][24]
+  int n_valid;
+  double *part;                // OUT: [members][tiles] sums of squared errors
+  int *err;
+};
+
+// KIND 0: Z = acc + bias, H = silu(Z); 1: the output layer, G = 2 (Y - T) / (24 n)
+// and the squared errors; 2: G = acc * silu'(Z)
+template <int KIND>
+__global__ void __launch_bounds__(TR_NT, 1)
+k_train_layer(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb,
+              TrainLayer L) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  __shared__ int s_fail;
+  __shared__ double s_red[4];
+  const TrainSmem sm = train_smem_of(smem_raw);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = warp & 3, cg = warp >> 2;
+  const int member = blockIdx.y, r = blockIdx.x * BM + q * 32 + lane;  // row within the member
+  const size_t grow = (size_t) member * L.B + r;
+  const unsigned tmem = train_begin(sm, &s_fail);
+  const bool ok = train_mma(sm, tmem, &ta, &tb, 0, L.nk, member * L.B + blockIdx.x * BM,
+                            member * L.brows, L.bn, L.err, &s_fail);
+  const unsigned tl = tmem + ((unsigned) (q * 32) << 16);
+  if (ok && KIND != 1) {
+    float *zt = L.z + ((size_t) member * (L.B / BM) + blockIdx.x) * (TR_H * BM) + q * 32 + lane;
+    const float *bias = KIND == 0 ? L.bias + member * L.pstride : nullptr;
+#pragma unroll 1
+    for (int c = cg * 64; c < cg * 64 + 64; c += 16) {
+      float v[16], zz[16];
+      if (KIND == 2) {
+#pragma unroll
+        for (int i = 0; i < 16; i++) zz[i] = zt[(size_t) (c + i) * BM];
+      }
+      tmem_ld16(tl + c, v);
+      float hv[16];
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        if (KIND == 0) {
+          const float z = v[i] + __ldg(bias + c + i);
+          zt[(size_t) (c + i) * BM] = z;
+          hv[i] = z * sigmoidf_(z);
+        } else {
+          const float z = zz[i], sg = sigmoidf_(z);
+          hv[i] = v[i] * sg * (1.f + z * (1.f - sg));
+        }
+      }
+      unsigned w[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const __nv_bfloat162 p2 = __floats2bfloat162_rn(hv[2 * i], hv[2 * i + 1]);
+        w[i] = *reinterpret_cast<const unsigned *>(&p2);
+        __nv_bfloat16 *ht = L.ht + ((size_t) member * TR_H + c + 2 * i) * L.B + r;
+        ht[0] = p2.x;
+        ht[L.B] = p2.y;
+      }
+      uint4 *h = reinterpret_cast<uint4 *>(L.h + grow * L.ldh + c);
+      h[0] = make_uint4(w[0], w[1], w[2], w[3]);
+      h[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+  }
+  if (KIND == 1) {
+    double sq = 0.0;
+    if (ok && cg == 0) {
+      float y[32];
+      tmem_ld16(tl, *reinterpret_cast<float(*)[16]>(y));
+      tmem_ld16(tl + 16, *reinterpret_cast<float(*)[16]>(y + 16));
+      const float *bias = L.bias + member * L.pstride, *t = L.t + grow * TR_OUT;
+#pragma unroll
+      for (int c = 0; c < TR_OUT; c += 2) {
+        float g[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          g[i] = 0.f;
+          if (r < L.n_valid) {
+            const float d = y[c + i] + __ldg(bias + c + i) - t[c + i];
+            sq += (double) d * d;
+            g[i] = 2.f * d / ((float) L.n_valid * TR_OUT);
+          }
+        }
+        const __nv_bfloat162 p2 = __floats2bfloat162_rn(g[0], g[1]);
+        *reinterpret_cast<__nv_bfloat162 *>(L.h + grow * L.ldh + c) = p2;
+        __nv_bfloat16 *ht = L.ht + ((size_t) member * TR_OUT + c) * L.B + r;
+        ht[0] = p2.x;
+        ht[L.B] = p2.y;
+      }
+    }
+    if (cg == 0) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, o);
+      if (lane == 0) s_red[q] = sq;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+      L.part[member * gridDim.x + blockIdx.x] = (s_red[0] + s_red[1]) + (s_red[2] + s_red[3]);
+  }
+  train_end(tmem);
+}
+
+// weight gradients dW_l = G_l^T H_{l-1} of layers 0..3, both operands transposed
+// (K = the batch): blocks of a layer's 128-row tiles x `splits` parts of the
+// batch of `tps` k-tiles; partial sums to part[split][member][nparam]
+struct TrainDwMaps {
+  CUtensorMap a[4], b[4];
+};
+struct TrainDw {
+  int B, splits, tps;
+  float *part;
+  long nparam, off[4];
+  int *err;
+};
+
+__global__ void __launch_bounds__(TR_NT, 1)
+k_train_dw(const __grid_constant__ TrainDwMaps maps, TrainDw d) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  __shared__ int s_fail;
+  const TrainSmem sm = train_smem_of(smem_raw);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = warp & 3, cg = warp >> 2;
+  const int member = blockIdx.y, S = d.splits;
+  // layers 1, 2 (256 x 256), 0 (256 x 32), 3 (24 x 256)
+  int b = blockIdx.x, l = 1;
+  if (b >= 6 * S) {
+    l = 3;
+    b -= 6 * S;
+  } else if (b >= 4 * S) {
+    l = 0;
+    b -= 4 * S;
+  } else if (b >= 2 * S) {
+    l = 2;
+    b -= 2 * S;
+  }
+  const int tile = b / S, split = b % S;
+  const int arows = l == 3 ? TR_OUT : TR_H, brows = l == 0 ? TR_IN : TR_H, ldw = l == 0 ? 32 : TR_H;
+  const int k0 = split * d.tps, nk = min(d.tps, d.B / BK - k0);
+  const unsigned tmem = train_begin(sm, &s_fail);
+  const bool ok = train_mma(sm, tmem, &maps.a[l], &maps.b[l], k0, nk, member * arows + tile * BM,
+                            member * brows, brows, d.err, &s_fail);
+  const int row = tile * BM + q * 32 + lane;
+  if (ok) {
+    const unsigned tl = tmem + ((unsigned) (q * 32) << 16);
+    float *out = d.part + ((size_t) split * gridDim.y + member) * d.nparam + d.off[l] + (size_t) row * ldw;
+#pragma unroll 1
+    for (int c = cg * 64; c < min(cg * 64 + 64, ldw); c += 16) {
+      float v[16];
+      tmem_ld16(tl + c, v);
+      if (row < arows)
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          reinterpret_cast<float4 *>(out + c)[i] =
+              make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    }
+  }
+  train_end(tmem);
+}
+
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
   if (!fn) {
@@ -599,14 +840,14 @@ void launch(const CUtensorMap &ta, const CUtensorMap &tb, int M, int N, int K, c
 // C = A * B^T with A [M x K] (lda), B [N x K] (ldb), bf16, K % 64 == 0,
 // lda, ldb multiples of 8, 16-byte aligned bases.  BN = 32, 64, 128 or 256
 // by N (N > 256 is split over grid.y).
-void gemm_tn(const void *A, int lda, const void *B, int ldb, int M, int N, int K, int kind,
-             const float *bias, float *c, int ldc, void *h, int ldh, int *err, cudaStream_t s) {
+void gemm_tn(const void *A, int lda, const void *B, int ldb, int M, int N, int K, float *c, int ldc,
+             int *err, cudaStream_t s) {
   if (M <= 0 || N <= 0) return;
   if (K <= 0 || K % BK || lda % 8 || ldb % 8 || (reinterpret_cast<uintptr_t>(A) & 15) ||
       (reinterpret_cast<uintptr_t>(B) & 15))
     throw CudaError{cudaErrorInvalidValue,
                     "gemm_tn: K must be a multiple of 64, leading dimensions multiples of 8"};
-  Epi ep{kind, bias, c, ldc, static_cast<__nv_bfloat16 *>(h), ldh};
+  Epi ep{c, ldc};
   const int bn = N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : 256;
   CUtensorMap ta = make_map(A, M, K, lda, BM);
   CUtensorMap tb = make_map(B, N, K, ldb, bn);
@@ -616,6 +857,101 @@ void gemm_tn(const void *A, int lda, const void *B, int ldb, int M, int N, int K
     case 128: launch<128, 4>(ta, tb, M, N, K, ep, err, s); break;
     default: launch<256, 3>(ta, tb, M, N, K, ep, err, s); break;
   }
+}
+
+// The tensor maps of a training call (the buffers stay where they are).
+struct TrainPlan {
+  TrainArgs t;
+  CUtensorMap act[7], wts[7];  // forward layers 0..3, backward layers 2, 1, 0
+  TrainDwMaps dw;
+};
+
+TrainPlan *train_plan(const TrainArgs &t) {
+  static const bool attr = [] {
+    for (const void *k : {(const void *) k_train_layer<0>, (const void *) k_train_layer<1>,
+                          (const void *) k_train_layer<2>, (const void *) k_train_dw})
+      check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) train_smem()),
+            "training smem attribute");
+    return true;
+  }();
+  (void) attr;
+  const int M = t.members, B = t.B;
+  auto act = [&](const void *p, int cols) { return make_map(p, M * B, cols, cols, BM); };
+  TrainPlan *pl = new TrainPlan;
+  try {
+    pl->t = t;
+    for (int l = 0; l < 4; l++) {
+      const int kc = l == 0 ? TR_IN : TR_H, rows = l == 3 ? TR_OUT : TR_H;
+      pl->act[l] = act(t.h[l], kc);
+      pl->wts[l] = make_map(t.w[l], M * rows, kc, kc, l == 3 ? 32 : TR_H);
+      pl->dw.a[l] = make_map(t.gt[l], M * rows, B, B, BM);
+      pl->dw.b[l] = make_map(t.ht[l], M * kc, B, B, kc);
+    }
+    for (int l = 2; l >= 0; l--) {
+      const int kc = l == 2 ? TR_OUTP : TR_H;
+      pl->act[6 - l] = act(t.g[l + 1], kc);
+      pl->wts[6 - l] = make_map(t.wt[l + 1], M * TR_H, kc, kc, TR_H);
+    }
+  } catch (...) {
+    delete pl;
+    throw;
+  }
+  return pl;
+}
+
+void train_plan_free(TrainPlan *p) { delete p; }
+
+// One step's forward and backward passes and weight-gradient partial sums; the
+// squared errors go to `loss` ([members][B / 128])
+void train_passes(const TrainPlan &pl, double *loss, cudaStream_t s) {
+  const TrainArgs &t = pl.t;
+  const size_t smem = train_smem();
+  auto bf = [](void *p) { return static_cast<__nv_bfloat16 *>(p); };
+  const dim3 grid(t.B / BM, t.members);
+  TrainLayer L{};
+  L.B = t.B;
+  L.pstride = t.pstride;
+  L.n_valid = t.n_valid;
+  L.t = t.tb;
+  L.part = loss;
+  L.err = t.err;
+  // forward: h_l = silu(h_{l-1} W_l^T + b_l), then the output layer
+  for (int l = 0; l < 3; l++) {
+    L.nk = l == 0 ? 1 : TR_H / BK;
+    L.bn = L.brows = L.ldh = TR_H;
+    L.bias = t.p + t.ob[l];
+    L.z = t.z[l];
+    L.h = bf(t.h[l + 1]);
+    L.ht = bf(t.ht[l + 1]);
+    k_train_layer<0><<<grid, TR_NT, smem, s>>>(pl.act[l], pl.wts[l], L);
+  }
+  L.nk = TR_H / BK;
+  L.bn = 32;
+  L.brows = TR_OUT;
+  L.bias = t.p + t.ob[3];
+  L.h = bf(t.g[3]);
+  L.ldh = TR_OUTP;
+  L.ht = bf(t.gt[3]);
+  k_train_layer<1><<<grid, TR_NT, smem, s>>>(pl.act[3], pl.wts[3], L);
+  // backward: g_l = (g_{l+1} W_{l+1}) silu'(z_l)
+  for (int l = 2; l >= 0; l--) {
+    L.nk = (l == 2 ? TR_OUTP : TR_H) / BK;
+    L.bn = L.brows = L.ldh = TR_H;
+    L.z = t.z[l];
+    L.h = bf(t.g[l]);
+    L.ht = bf(t.gt[l]);
+    k_train_layer<2><<<grid, TR_NT, smem, s>>>(pl.act[6 - l], pl.wts[6 - l], L);
+  }
+  TrainDw d{};
+  d.B = t.B;
+  d.splits = t.splits;
+  d.tps = t.tps;
+  d.part = t.part;
+  d.nparam = t.pstride;
+  d.err = t.err;
+  for (int l = 0; l < 4; l++) d.off[l] = t.ow[l];
+  k_train_dw<<<dim3(7 * t.splits, t.members), TR_NT, smem, s>>>(pl.dw, d);
+  check(cudaGetLastError(), "train_passes");
 }
 
 // The fused ensemble on normalised bf16 features xf[n][64]; weights stacked

@@ -2,20 +2,14 @@
 // (SiLU) that maps an element's 24 nodal displacements (about their mean,
 // relative to the ideal lattice) and 8 nodal densities to its 24 nodal forces.
 //
-// Every matrix product, forward and backward, runs on the tensor cores through
-// gemm::gemm_tn (BF16 operands, FP32 accumulation, k_gemm.cu).  Master weights,
+// Every matrix product, forward and backward, runs on the tensor cores (BF16
+// operands, FP32 accumulation, k_gemm.cu), all members of a step together.  Master weights,
 // Adam moments and gradients are FP32; activations cross layers as BF16 and
 // pre-activations are kept in FP32 for the SiLU derivative.  The reference has
 // no counterpart: it evaluates every element by integration-point quadrature.
 //
-// Layouts (row-major, K-major operands as the GEMM wants them):
-//   parameters per member, flattened: W1[256][32] b1[256] W2[256][256] b2
-//   W3[256][256] b3 W4[24][256] b4[24]
-//   bf16 copies: w1[256][64] (K padded), w2, w3, w4[24][256];
-//   for the backward pass w2t = W2^T, w3t = W3^T, w4t[256][64] = W4^T padded.
-//   activations x0[B][64] (features, zero padded), z_l (FP32) and h_l (BF16)
-//   [B][256], output y[B][24] (FP32), gradients g4[B][64], g_l[B][256] (BF16).
-//   dW_l = g_l^T h_{l-1}: both operands transposed first ([rows][B]).
+// Parameters per member, flattened: W1[256][32] b1[256] W2[256][256] b2
+// W3[256][256] b3 W4[24][256] b4[24]; the step's arrays are gemm::TrainArgs.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -24,6 +18,7 @@
 #include <cstring>
 #include <stdexcept>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "cacg.h"
@@ -44,95 +39,109 @@ constexpr long oW1 = 0, ob1 = oW1 + (long) NH * NIN, oW2 = ob1 + NH, ob2 = oW2 +
 
 inline int nblk(long long n, int t) { return (int) ((n + t - 1) / t); }
 
-__global__ void k_cast_pad(const float *__restrict__ src, int rows, int cols, int lds,
-                           bf16 *__restrict__ dst, int ldd, int rows_out) {
-  long i = blockIdx.x * (long) blockDim.x + threadIdx.x;
-  if (i >= (long) rows_out * ldd) return;
-  int r = (int) (i / ldd), c = (int) (i % ldd);
-  dst[i] = __float2bfloat16(r < rows && c < cols ? src[(long) r * lds + c] : 0.f);
-}
+// The current parameters' BF16 copies, stacked over the members: forward
+// weights w[0..3] ([256][64] K padded, [256][256] twice, [24][256]), transposed
+// wt[1..3] ([256][256] twice, [256][64] padded), biases for inference [792].
+struct Copies {
+  bf16 *w[4], *wt[4];
+  float *bias;
+};
 
-// dst[c][r] = src[r][c] (rows x cols -> cols x ldd, zero beyond rows)
-__global__ void k_cast_transpose(const float *__restrict__ src, int rows, int cols,
-                                 bf16 *__restrict__ dst, int ldd) {
-  long i = blockIdx.x * (long) blockDim.x + threadIdx.x;
-  if (i >= (long) cols * ldd) return;
-  int c = (int) (i / ldd), r = (int) (i % ldd);
-  dst[i] = __float2bfloat16(r < rows ? src[(long) r * cols + c] : 0.f);
-}
+constexpr int BIASES = 3 * NH + NOUT;
+constexpr long WEIGHTS = NPARAM - BIASES;
 
-// out[c][r] = in[r][c] for r < rows, c < cols (32x32 tiles through shared memory)
-__global__ void k_transpose(const bf16 *__restrict__ in, int rows, int cols, int ldi,
-                            bf16 *__restrict__ out, int ldo) {
-  __shared__ bf16 t[32][33];
-  int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    int r = r0 + k, c = c0 + threadIdx.x;
-    t[k][threadIdx.x] = (r < rows && c < cols) ? in[(long) r * ldi + c] : __float2bfloat16(0.f);
-  }
-  __syncthreads();
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    int c = c0 + k, r = r0 + threadIdx.x;
-    if (c < cols && r < rows) out[(long) c * ldo + r] = t[threadIdx.x][k];
+// writes parameter i of a member to its copies
+__device__ __forceinline__ void put_copy(const Copies &c, int member, int layer, int r, int col,
+                                         float v) {
+  const bf16 b = __float2bfloat16(v);
+  if (layer == 0) {
+    c.w[0][((size_t) member * NH + r) * NINP + col] = b;
+  } else if (layer < 3) {
+    c.w[layer][((size_t) member * NH + r) * NH + col] = b;
+    c.wt[layer][((size_t) member * NH + col) * NH + r] = b;
+  } else {
+    c.w[3][((size_t) member * NOUT + r) * NH + col] = b;
+    c.wt[3][((size_t) member * NH + col) * NGP + r] = b;
   }
 }
 
-// column sums of a bf16 [rows][ld] matrix, added into fp32 out[cols] (zeroed
-// by the caller): block (x, y) sums 256 rows of 32 columns
-__global__ void k_colsum(const bf16 *__restrict__ g, int rows, int cols, int ld,
-                         float *__restrict__ out) {
-  __shared__ float red[8][33];
-  const int c = blockIdx.x * 32 + threadIdx.x;
-  const int r0 = blockIdx.y * 256, r1 = min(rows, r0 + 256);
-  float s = 0.f;
-  if (c < cols)
-    for (int r = r0 + threadIdx.y; r < r1; r += blockDim.y) s += __bfloat162float(g[(long) r * ld + c]);
-  red[threadIdx.y][threadIdx.x] = s;
-  __syncthreads();
-  if (threadIdx.y == 0 && c < cols) {
-    float t = 0.f;
-    for (int k = 0; k < (int) blockDim.y; k++) t += red[k][threadIdx.x];
-    atomicAdd(out + c, t);
-  }
-}
+enum { UPDATE_COPY = 0, UPDATE_GRAD = 1, UPDATE_ADAM = 2 };
 
-// g4 = 2 (y - t) / (n_valid * 24) as bf16 [B][64] (zero padding and rows), and
-// per-block partial sums of (y - t)^2
-__global__ void k_loss_grad(const float *__restrict__ y, const float *__restrict__ t, int B,
-                            int n_valid, bf16 *__restrict__ g4, double *__restrict__ part) {
-  __shared__ double red[256];
-  long i = blockIdx.x * (long) blockDim.x + threadIdx.x;
-  double sq = 0.0;
-  if (i < (long) B * NGP) {
-    int r = (int) (i / NGP), c = (int) (i % NGP);
-    float gv = 0.f;
-    if (r < n_valid && c < NOUT) {
-      float d = y[(long) r * NOUT + c] - t[(long) r * NOUT + c];
-      sq = (double) d * d;
-      gv = 2.f * d / ((float) n_valid * NOUT);
+struct UpdateArgs {
+  float *p, *m, *v, *g;   // [members][NPARAM] (GRAD writes g, ADAM p, m, v)
+  const float *part;      // weight-gradient partial sums [splits][members][NPARAM]
+  const bf16 *gt[4];      // gradients at the layers' outputs, transposed [members * rows][B]
+  int splits, B, first;   // first: member of blockIdx.y == 0
+  float lr, b1, b2, eps, bc1, bc2;
+  Copies c;
+};
+
+// blockIdx.y: member; the first WB blocks take the weights (a thread each, the
+// partial sums added in order), the others the biases (a warp each, the column
+// sum of the gradient: rows of the transposed array)
+constexpr int UB = 256;
+constexpr int WB = (int) ((WEIGHTS + UB - 1) / UB), BB = (BIASES + UB / 32 - 1) / (UB / 32);
+
+template <int MODE>
+__global__ void __launch_bounds__(UB) k_update(UpdateArgs a) {
+  const int member = a.first + blockIdx.y;
+  long off;            // in the member's parameters
+  int layer, r, col;   // weight (r, col), or bias r with col < 0
+  float g = 0.f;
+  if ((int) blockIdx.x < WB) {
+    long i = blockIdx.x * (long) UB + threadIdx.x;
+    if (i >= WEIGHTS) return;
+    layer = 0;
+    int cols = NIN;
+    if (i >= (long) NH * NIN) {
+      i -= (long) NH * NIN;
+      layer = i < (long) NH * NH ? 1 : i < 2L * NH * NH ? 2 : 3;
+      i -= (long) (layer - 1) * NH * NH;
+      cols = NH;
     }
-    g4[i] = __float2bfloat16(gv);
+    r = (int) (i / cols);
+    col = (int) (i % cols);
+    off = (layer == 0 ? oW1 : layer == 1 ? oW2 : layer == 2 ? oW3 : oW4) + i;
+    if (MODE != UPDATE_COPY)
+      for (int s = 0; s < a.splits; s++)
+        g += a.part[((size_t) s * gridDim.y + blockIdx.y) * NPARAM + off];
+  } else {
+    const int j = ((int) blockIdx.x - WB) * (UB / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (j >= BIASES) return;
+    layer = j / NH;
+    r = j % NH;
+    col = -1;
+    off = (layer == 0 ? ob1 : layer == 1 ? ob2 : layer == 2 ? ob3 : ob4) + r;
+    if (MODE != UPDATE_COPY) {
+      const int rows = layer == 3 ? NOUT : NH;
+      const uint4 *q = reinterpret_cast<const uint4 *>(a.gt[layer] +
+                                                       ((size_t) blockIdx.y * rows + r) * a.B);
+      for (int k = lane; k < a.B / 8; k += 32) {
+        const uint4 u = __ldg(q + k);
+        for (unsigned w : {u.x, u.y, u.z, u.w})
+          g += __uint_as_float(w << 16) + __uint_as_float(w & 0xFFFF0000u);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
+    }
+    if (lane != 0) return;
   }
-  red[threadIdx.x] = sq;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int) threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
+  const size_t at = (size_t) member * NPARAM + off;
+  if (MODE == UPDATE_GRAD) {
+    a.g[at] = g;
+    return;
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
-}
-
-__global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
-                       float *__restrict__ v, long n, float lr, float b1, float b2, float eps,
-                       float bc1, float bc2) {
-  long i = blockIdx.x * (long) blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float gi = g[i];
-  float mi = b1 * m[i] + (1.f - b1) * gi;
-  float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  p[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+  float p = a.p[at];
+  if (MODE == UPDATE_ADAM) {
+    const float mi = a.b1 * a.m[at] + (1.f - a.b1) * g;
+    const float vi = a.b2 * a.v[at] + (1.f - a.b2) * g * g;
+    a.m[at] = mi;
+    a.v[at] = vi;
+    p -= a.lr * (mi / a.bc1) / (sqrtf(vi / a.bc2) + a.eps);
+    a.p[at] = p;
+  }
+  if (col >= 0) put_copy(a.c, member, layer, r, col, p);
+  else a.c.bias[(size_t) member * BIASES + layer * NH + r] = p;
 }
 
 // normalised features as bf16 [n][64]: (x - mean) * inv_std, zero padded
@@ -156,40 +165,29 @@ __global__ void k_targets(const float *__restrict__ t, long n, const float *__re
   out[i] = (t[i] - norm[2 * NIN + c]) / norm[2 * NIN + NOUT + c];
 }
 
-// rows of a permutation into a contiguous batch (features bf16, targets fp32)
-__global__ void k_gather(const bf16 *__restrict__ xall, const float *__restrict__ tall,
-                         const int *__restrict__ idx, int nb, bf16 *__restrict__ x0,
-                         float *__restrict__ tb) {
-  long i = blockIdx.x * (long) blockDim.x + threadIdx.x;
-  if (i >= (long) nb * NINP) return;
-  int r = (int) (i / NINP), c = (int) (i % NINP);
-  int src = idx[r];
-  x0[i] = src >= 0 ? xall[(long) src * NINP + c] : __float2bfloat16(0.f);
-  if (c < NOUT) tb[(long) r * NOUT + c] = src >= 0 ? tall[(long) src * NOUT + c] : 0.f;
-}
-
-// ensemble mean (denormalised) and spread: max over outputs of the members'
-// standard deviation, in force units
-__global__ void k_ensemble(const float *__restrict__ y, long n, int members, long mstride,
-                           const float *__restrict__ norm, float *__restrict__ mean,
-                           float *__restrict__ spread) {
-  long r = blockIdx.x * (long) blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  float smax = 0.f;
-  for (int c = 0; c < NOUT; c++) {
-    float s1 = 0.f, s2 = 0.f;
-    for (int k = 0; k < members; k++) {
-      float v = y[k * mstride + r * NOUT + c];
-      s1 += v;
-      s2 += v * v;
-    }
-    float mu = s1 / members;
-    float var = fmaxf(s2 / members - mu * mu, 0.f);
-    float sd = norm[2 * NIN + NOUT + c];
-    mean[r * NOUT + c] = mu * sd + norm[2 * NIN + c];
-    smax = fmaxf(smax, sqrtf(var) * sd);
+// The members' batches: features x0 [members * B][64] and their transpose
+// [members * 64][B], targets tb [members * B][24]; row r of member m is sample
+// idx[m * istride + r] (idx null: r), zero for r >= n
+__global__ void __launch_bounds__(256)
+k_gather(const bf16 *__restrict__ xall, const float *__restrict__ tall, const int *__restrict__ idx,
+         long istride, int n, int B, bf16 *__restrict__ x0, bf16 *__restrict__ x0t,
+         float *__restrict__ tb) {
+  __shared__ bf16 t[32][NINP + 2];
+  const int member = blockIdx.y, r0 = blockIdx.x * 32;
+  for (int k = threadIdx.x; k < 32 * NINP; k += 256) {
+    const int r = k / NINP, c = k % NINP;
+    const int src = r0 + r >= n ? -1 : idx ? idx[member * istride + r0 + r] : r0 + r;
+    const bf16 v = src >= 0 ? xall[(long) src * NINP + c] : __float2bfloat16(0.f);
+    const size_t row = (size_t) member * B + r0 + r;
+    x0[row * NINP + c] = v;
+    t[r][c] = v;
+    if (c < NOUT) tb[row * NOUT + c] = src >= 0 ? tall[(long) src * NOUT + c] : 0.f;
   }
-  spread[r] = smax;
+  __syncthreads();
+  for (int k = threadIdx.x; k < 32 * NINP; k += 256) {
+    const int c = k / 32, r = k % 32;
+    x0t[((size_t) member * NINP + c) * B + r0 + r] = t[r][c];
+  }
 }
 
 // splitmix64: seeded, platform-independent initialisation
@@ -201,35 +199,29 @@ struct Rng {
     z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
     return z ^ (z >> 31);
   }
+  void skip(unsigned long long n) { s += n * 0x9E3779B97F4A7C15ull; }
   double uniform() { return (next() >> 11) * (1.0 / 9007199254740992.0); }
 };
 
 }  // namespace
 
-struct Member {
-  DBuf<float> p, m, v, g;
-  DBuf<bf16> w1, w2, w3, w4, w2t, w3t, w4t;
-};
-
 struct Net {
   int device = 0, members = 0;
   cudaStream_t stream = nullptr;
-  std::vector<Member> mem;
   float norm[2 * NIN + 2 * NOUT];  // in_mean, in_inv_std, out_mean, out_std
   double force_scale = 1.0;        // rms nodal-force magnitude of the training targets
   long long adam_steps = 0;
   std::string err;
   DBuf<float> d_norm;
-  int bcap = 0;
-  DBuf<bf16> x0, h1, h2, h3, g4, g3, g2, g1, x0t, h1t, h2t, h3t, g1t, g2t, g3t, g4t;
-  DBuf<float> z1, z2, z3, y, tb, db;
-  DBuf<double> part;
+  // per member, stacked: parameters, Adam moments, gradients, BF16 copies
+  DBuf<float> p, m, v, g, bias;
+  DBuf<bf16> w[4], wt[4];
+  // one step's arrays (see gemm::TrainArgs)
+  DBuf<bf16> h[4], ht[4], gr[4], grt[4];
+  DBuf<float> z[3], tb, part;
+  DBuf<double> loss;
   DBuf<int> errflag;
-  // inference buffers
-  long long icap = 0;
-  DBuf<bf16> ix0, ih1, ih2, ih3;
-  DBuf<float> iy, iw1b;
-  DBuf<bf16> iw1;  // all members' W1 stacked [members*256][64]
+  size_t g4_rows = 0;  // rows of gr[3] whose padding is zero
 
   void sync() { check(cudaStreamSynchronize(stream), "mlp sync"); }
 
@@ -246,184 +238,169 @@ struct Net {
 
   void init_params(unsigned long long seed) {
     Rng rng{seed};
-    std::vector<float> h(NPARAM);
+    std::vector<float> hp((size_t) members * NPARAM, 0.f);
     for (int k = 0; k < members; k++) {
-      Member &M = mem[k];
+      float *q = hp.data() + (size_t) k * NPARAM;
       auto fill = [&](long off, int rows, int cols, double gain) {
         double a = gain * std::sqrt(3.0 / cols);
-        for (long i = 0; i < (long) rows * cols; i++) h[off + i] = (float) ((2 * rng.uniform() - 1) * a);
+        for (long i = 0; i < (long) rows * cols; i++) q[off + i] = (float) ((2 * rng.uniform() - 1) * a);
       };
-      std::fill(h.begin(), h.end(), 0.f);
       fill(oW1, NH, NIN, 1.0);
       fill(oW2, NH, NH, 1.0);
       fill(oW3, NH, NH, 1.0);
       fill(oW4, NOUT, NH, 0.1);
-      M.p.ensure(NPARAM, stream);
-      M.m.ensure(NPARAM, stream);
-      M.v.ensure(NPARAM, stream);
-      M.g.ensure(NPARAM, stream);
-      check(cudaMemcpyAsync(M.p.p, h.data(), sizeof(float) * NPARAM, cudaMemcpyHostToDevice, stream), "params");
-      check(cudaMemsetAsync(M.m.p, 0, sizeof(float) * NPARAM, stream), "adam m");
-      check(cudaMemsetAsync(M.v.p, 0, sizeof(float) * NPARAM, stream), "adam v");
-      refresh(k);
     }
+    const size_t np = hp.size(), mm = (size_t) members;
+    for (DBuf<float> *b : {&p, &m, &v, &g}) b->ensure(np, stream);
+    bias.ensure(mm * BIASES, stream);
+    w[0].ensure(mm * NH * NINP, stream);
+    w[1].ensure(mm * NH * NH, stream);
+    w[2].ensure(mm * NH * NH, stream);
+    w[3].ensure(mm * NOUT * NH, stream);
+    wt[1].ensure(mm * NH * NH, stream);
+    wt[2].ensure(mm * NH * NH, stream);
+    wt[3].ensure(mm * NH * NGP, stream);
+    // the padding of W1 and W4^T stays zero
+    check(cudaMemsetAsync(w[0].p, 0, sizeof(bf16) * mm * NH * NINP, stream), "w1");
+    check(cudaMemsetAsync(wt[3].p, 0, sizeof(bf16) * mm * NH * NGP, stream), "w4t");
+    check(cudaMemcpyAsync(p.p, hp.data(), sizeof(float) * np, cudaMemcpyHostToDevice, stream), "params");
+    check(cudaMemsetAsync(m.p, 0, sizeof(float) * np, stream), "adam m");
+    check(cudaMemsetAsync(v.p, 0, sizeof(float) * np, stream), "adam v");
+    refresh(0, members);
     sync();
   }
 
-  // bf16 copies of member k's weights (forward and transposed)
-  void refresh(int k) {
-    Member &M = mem[k];
-    stacked = false;
-    cudaStream_t s = stream;
-    M.w1.ensure((size_t) NH * NINP, s);
-    M.w2.ensure((size_t) NH * NH, s);
-    M.w3.ensure((size_t) NH * NH, s);
-    M.w4.ensure((size_t) NOUT * NH, s);
-    M.w2t.ensure((size_t) NH * NH, s);
-    M.w3t.ensure((size_t) NH * NH, s);
-    M.w4t.ensure((size_t) NH * NGP, s);
-    k_cast_pad<<<nblk((long) NH * NINP, 256), 256, 0, s>>>(M.p.p + oW1, NH, NIN, NIN, M.w1.p, NINP, NH);
-    k_cast_pad<<<nblk((long) NH * NH, 256), 256, 0, s>>>(M.p.p + oW2, NH, NH, NH, M.w2.p, NH, NH);
-    k_cast_pad<<<nblk((long) NH * NH, 256), 256, 0, s>>>(M.p.p + oW3, NH, NH, NH, M.w3.p, NH, NH);
-    k_cast_pad<<<nblk((long) NOUT * NH, 256), 256, 0, s>>>(M.p.p + oW4, NOUT, NH, NH, M.w4.p, NH, NOUT);
-    k_cast_transpose<<<nblk((long) NH * NH, 256), 256, 0, s>>>(M.p.p + oW2, NH, NH, M.w2t.p, NH);
-    k_cast_transpose<<<nblk((long) NH * NH, 256), 256, 0, s>>>(M.p.p + oW3, NH, NH, M.w3t.p, NH);
-    k_cast_transpose<<<nblk((long) NH * NGP, 256), 256, 0, s>>>(M.p.p + oW4, NOUT, NH, M.w4t.p, NGP);
+  UpdateArgs update_args(int first) {
+    UpdateArgs a{};
+    a.p = p.p;
+    a.m = m.p;
+    a.v = v.p;
+    a.g = g.p;
+    a.first = first;
+    for (int l = 0; l < 4; l++) {
+      a.c.w[l] = w[l].p;
+      a.c.wt[l] = wt[l].p;
+      a.gt[l] = grt[l].p;
+    }
+    a.c.bias = bias.p;
+    return a;
+  }
+
+  // BF16 copies of the members' weights (forward and transposed)
+  void refresh(int first, int count) {
+    k_update<UPDATE_COPY><<<dim3(WB + BB, count), UB, 0, stream>>>(update_args(first));
     check(cudaGetLastError(), "mlp refresh");
   }
 
-  void ensure_batch(int B) {
-    if (B <= bcap) return;
+  // the batch in parts of at least 8 k-tiles (512 rows), at most 16 parts: the
+  // weight-gradient blocks of 4 members x 2,048 rows then fill one wave (112
+  // blocks), and a part's sums cost 0.6 MB a member
+  static void split(int B, int &splits, int &tps) {
+    const int nkt = B / 64;
+    tps = std::max(8, (nkt + 15) / 16);
+    splits = (nkt + tps - 1) / tps;
+  }
+
+  // `count` members from `first` with B rows each
+  gemm::TrainArgs batch(int first, int count, int B, int n_valid) {
     cudaStream_t s = stream;
-    size_t b = (size_t) B;
-    x0.ensure(b * NINP, s);
-    for (DBuf<bf16> *p : {&h1, &h2, &h3, &g3, &g2, &g1}) p->ensure(b * NH, s);
-    g4.ensure(b * NGP, s);
-    x0t.ensure(b * NINP, s);
-    for (DBuf<bf16> *p : {&h1t, &h2t, &h3t, &g1t, &g2t, &g3t}) p->ensure(b * NH, s);
-    g4t.ensure(b * NOUT, s);
-    for (DBuf<float> *p : {&z1, &z2, &z3}) p->ensure(b * NH, s);
-    y.ensure(b * NOUT, s);
+    const size_t b = (size_t) count * B;
+    int splits, tps;
+    split(B, splits, tps);
+    h[0].ensure(b * NINP, s);
+    ht[0].ensure(b * NINP, s);
+    for (int l = 1; l < 4; l++) {
+      h[l].ensure(b * NH, s);
+      ht[l].ensure(b * NH, s);
+      gr[l - 1].ensure(b * NH, s);
+      grt[l - 1].ensure(b * NH, s);
+      z[l - 1].ensure(b * NH, s);
+    }
+    if (gr[3].cap < b * NGP) g4_rows = 0;
+    gr[3].ensure(b * NGP, s);
+    if (g4_rows < b) {  // columns 24..63 stay zero
+      check(cudaMemsetAsync(gr[3].p, 0, sizeof(bf16) * b * NGP, s), "g4");
+      g4_rows = b;
+    }
+    grt[3].ensure(b * NOUT, s);
     tb.ensure(b * NOUT, s);
-    db.ensure(NH, s);
-    part.ensure(nblk(b * NGP, 256), s);
+    part.ensure((size_t) splits * count * NPARAM, s);
     ensure_err(s);
-    bcap = B;
+    gemm::TrainArgs t{};
+    t.members = count;
+    t.B = B;
+    t.n_valid = n_valid;
+    t.splits = splits;
+    t.tps = tps;
+    t.p = p.p + (size_t) first * NPARAM;
+    t.pstride = NPARAM;
+    const long ow[4] = {oW1, oW2, oW3, oW4}, ob[4] = {ob1, ob2, ob3, ob4};
+    const size_t wrow[4] = {NH * NINP, NH * NH, NH * NH, NOUT * NH},
+                 wtrow[4] = {0, NH * NH, NH * NH, NH * NGP};
+    for (int l = 0; l < 4; l++) {
+      t.ow[l] = ow[l];
+      t.ob[l] = ob[l];
+      t.h[l] = h[l].p;
+      t.ht[l] = ht[l].p;
+      t.g[l] = gr[l].p;
+      t.gt[l] = grt[l].p;
+      t.w[l] = w[l].p + first * wrow[l];
+      t.wt[l] = l ? wt[l].p + first * wtrow[l] : nullptr;
+      if (l < 3) t.z[l] = z[l].p;
+    }
+    t.tb = tb.p;
+    t.part = part.p;
+    t.err = errflag.p;
+    return t;
   }
 
-  void transpose(const bf16 *in, int rows, int cols, int ldi, bf16 *out, int ldo) {
-    dim3 g(nblk(cols, 32), nblk(rows, 32)), b(32, 8);
-    k_transpose<<<g, b, 0, stream>>>(in, rows, cols, ldi, out, ldo);
-    check(cudaGetLastError(), "transpose");
-  }
-
-  void colsum(const bf16 *g, int rows, int cols, int ld, float *out) {
-    check(cudaMemsetAsync(out, 0, sizeof(float) * cols, stream), "colsum zero");
-    k_colsum<<<dim3(nblk(cols, 32), nblk(rows, 256)), dim3(32, 8), 0, stream>>>(g, rows, cols, ld, out);
-    check(cudaGetLastError(), "colsum");
-  }
-
-  // forward of member k on x0 (B rows), keeping z and h for the backward pass
-  void forward_train(int k, int B) {
-    Member &M = mem[k];
-    int *e = errflag.p;
-    gemm::gemm_tn(x0.p, NINP, M.w1.p, NINP, B, NH, NINP, 2, M.p.p + ob1, z1.p, NH, h1.p, NH, e, stream);
-    gemm::gemm_tn(h1.p, NH, M.w2.p, NH, B, NH, NH, 2, M.p.p + ob2, z2.p, NH, h2.p, NH, e, stream);
-    gemm::gemm_tn(h2.p, NH, M.w3.p, NH, B, NH, NH, 2, M.p.p + ob3, z3.p, NH, h3.p, NH, e, stream);
-    gemm::gemm_tn(h3.p, NH, M.w4.p, NH, B, NOUT, NH, 1, M.p.p + ob4, y.p, NOUT, nullptr, 0, e, stream);
-  }
-
-  // loss against tb (n_valid of B rows) and all gradients of member k into M.g
-  double backward(int k, int B, int n_valid, bool want_loss) {
-    Member &M = mem[k];
-    int *e = errflag.p;
-    cudaStream_t s = stream;
-    const int nb = nblk((long) B * NGP, 256);
-    k_loss_grad<<<nb, 256, 0, s>>>(y.p, tb.p, B, n_valid, g4.p, part.p);
-    check(cudaGetLastError(), "loss");
-    // backward through the layers: g_{l} = (g_{l+1} W_{l+1}) * silu'(z_l)
-    gemm::gemm_tn(g4.p, NGP, M.w4t.p, NGP, B, NH, NGP, 3, nullptr, z3.p, NH, g3.p, NH, e, s);
-    gemm::gemm_tn(g3.p, NH, M.w3t.p, NH, B, NH, NH, 3, nullptr, z2.p, NH, g2.p, NH, e, s);
-    gemm::gemm_tn(g2.p, NH, M.w2t.p, NH, B, NH, NH, 3, nullptr, z1.p, NH, g1.p, NH, e, s);
-    // weight gradients dW_l = g_l^T h_{l-1} (operands transposed to K = batch)
-    transpose(x0.p, B, NINP, NINP, x0t.p, B);
-    transpose(h1.p, B, NH, NH, h1t.p, B);
-    transpose(h2.p, B, NH, NH, h2t.p, B);
-    transpose(h3.p, B, NH, NH, h3t.p, B);
-    transpose(g1.p, B, NH, NH, g1t.p, B);
-    transpose(g2.p, B, NH, NH, g2t.p, B);
-    transpose(g3.p, B, NH, NH, g3t.p, B);
-    transpose(g4.p, B, NOUT, NGP, g4t.p, B);
-    // dW1 lands in a [256][64] scratch (z1 is free now), then compacts to [256][32]
-    gemm::gemm_tn(g1t.p, B, x0t.p, B, NH, NINP, B, 0, nullptr, z1.p, NINP, nullptr, 0, e, s);
-    check(cudaMemcpy2DAsync(M.g.p + oW1, sizeof(float) * NIN, z1.p, sizeof(float) * NINP,
-                            sizeof(float) * NIN, NH, cudaMemcpyDeviceToDevice, s), "dW1");
-    gemm::gemm_tn(g2t.p, B, h1t.p, B, NH, NH, B, 0, nullptr, M.g.p + oW2, NH, nullptr, 0, e, s);
-    gemm::gemm_tn(g3t.p, B, h2t.p, B, NH, NH, B, 0, nullptr, M.g.p + oW3, NH, nullptr, 0, e, s);
-    gemm::gemm_tn(g4t.p, B, h3t.p, B, NOUT, NH, B, 0, nullptr, M.g.p + oW4, NH, nullptr, 0, e, s);
-    colsum(g1.p, B, NH, NH, M.g.p + ob1);
-    colsum(g2.p, B, NH, NH, M.g.p + ob2);
-    colsum(g3.p, B, NH, NH, M.g.p + ob3);
-    colsum(g4.p, B, NOUT, NGP, M.g.p + ob4);
-    if (!want_loss) return 0.0;
-    std::vector<double> h(nb);
-    check(cudaMemcpyAsync(h.data(), part.p, sizeof(double) * nb, cudaMemcpyDeviceToHost, s), "loss");
-    sync();
-    double l = 0.0;
-    for (double v : h) l += v;
-    return l / ((double) n_valid * NOUT);
+  void gather(const gemm::TrainArgs &t, const bf16 *xall, const float *tall, const int *idx,
+              long istride, int n) {
+    k_gather<<<dim3(t.B / 32, t.members), 256, 0, stream>>>(xall, tall, idx, istride, n, t.B, h[0].p,
+                                                           ht[0].p, tb.p);
+    check(cudaGetLastError(), "gather");
   }
 
   void check_err() {
-    int v = 0;
-    check(cudaMemcpyAsync(&v, errflag.p, sizeof(int), cudaMemcpyDeviceToHost, stream), "errflag");
+    int f = 0;
+    check(cudaMemcpyAsync(&f, errflag.p, sizeof(int), cudaMemcpyDeviceToHost, stream), "errflag");
     sync();
-    if (v) throw CudaError{cudaErrorLaunchTimeout, "tensor-core GEMM: a bounded wait ran out"};
+    if (f) throw CudaError{cudaErrorLaunchTimeout, "tensor-core GEMM: a bounded wait ran out"};
   }
 
-  void adam(int k, float lr) {
-    Member &M = mem[k];
-    const float b1 = 0.9f, b2 = 0.999f;
-    const double t = (double) adam_steps + 1;
-    k_adam<<<nblk(NPARAM, 256), 256, 0, stream>>>(M.p.p, M.g.p, M.m.p, M.v.p, NPARAM, lr, b1, b2,
-                                                  1e-8f, (float) (1 - std::pow(b1, t)),
-                                                  (float) (1 - std::pow(b2, t)));
+  // the members' gradients into g
+  void gradients(const gemm::TrainArgs &t, int first) {
+    UpdateArgs a = update_args(first);
+    a.part = part.p;
+    a.splits = t.splits;
+    a.B = t.B;
+    k_update<UPDATE_GRAD><<<dim3(WB + BB, t.members), UB, 0, stream>>>(a);
+    check(cudaGetLastError(), "gradients");
+  }
+
+  void adam(const gemm::TrainArgs &t, float lr) {
+    UpdateArgs a = update_args(0);
+    a.part = part.p;
+    a.splits = t.splits;
+    a.B = t.B;
+    a.lr = lr;
+    a.b1 = 0.9f;
+    a.b2 = 0.999f;
+    a.eps = 1e-8f;
+    const double step = (double) adam_steps + 1;
+    a.bc1 = (float) (1 - std::pow(a.b1, step));
+    a.bc2 = (float) (1 - std::pow(a.b2, step));
+    k_update<UPDATE_ADAM><<<dim3(WB + BB, t.members), UB, 0, stream>>>(a);
     check(cudaGetLastError(), "adam");
-    refresh(k);
   }
-
-  bool stacked = false;  // iw1/iw1b hold the current first layers
 
   // ensemble prediction on normalised bf16 features already on the device:
   // one fused launch over all members and layers (gemm::mlp_ensemble)
-  DBuf<bf16> iw2, iw3, iw4;
-  DBuf<float> ibias;
   void predict_device(const bf16 *xf, long long n, float *mean, float *spread, cudaStream_t s,
                       const int *dcount = nullptr) {
     if (n <= 0) return;
     ensure_err(s);
-    if (!stacked) {
-      const int BS = 3 * NH + NOUT;
-      iw1.ensure((size_t) members * NH * NINP, s);
-      iw2.ensure((size_t) members * NH * NH, s);
-      iw3.ensure((size_t) members * NH * NH, s);
-      iw4.ensure((size_t) members * NOUT * NH, s);
-      ibias.ensure((size_t) members * BS, s);
-      for (int k = 0; k < members; k++) {
-        Member &M = mem[k];
-        check(cudaMemcpyAsync(iw1.p + (size_t) k * NH * NINP, M.w1.p, sizeof(bf16) * NH * NINP, cudaMemcpyDeviceToDevice, s), "w1s");
-        check(cudaMemcpyAsync(iw2.p + (size_t) k * NH * NH, M.w2.p, sizeof(bf16) * NH * NH, cudaMemcpyDeviceToDevice, s), "w2s");
-        check(cudaMemcpyAsync(iw3.p + (size_t) k * NH * NH, M.w3.p, sizeof(bf16) * NH * NH, cudaMemcpyDeviceToDevice, s), "w3s");
-        check(cudaMemcpyAsync(iw4.p + (size_t) k * NOUT * NH, M.w4.p, sizeof(bf16) * NOUT * NH, cudaMemcpyDeviceToDevice, s), "w4s");
-        float *b = ibias.p + (size_t) k * BS;
-        check(cudaMemcpyAsync(b, M.p.p + ob1, sizeof(float) * NH, cudaMemcpyDeviceToDevice, s), "b1s");
-        check(cudaMemcpyAsync(b + NH, M.p.p + ob2, sizeof(float) * NH, cudaMemcpyDeviceToDevice, s), "b2s");
-        check(cudaMemcpyAsync(b + 2 * NH, M.p.p + ob3, sizeof(float) * NH, cudaMemcpyDeviceToDevice, s), "b3s");
-        check(cudaMemcpyAsync(b + 3 * NH, M.p.p + ob4, sizeof(float) * NOUT, cudaMemcpyDeviceToDevice, s), "b4s");
-      }
-      stacked = true;
-    }
-    gemm::mlp_ensemble(xf, (int) n, iw1.p, iw2.p, iw3.p, iw4.p, ibias.p, members, d_norm.p, mean,
+    gemm::mlp_ensemble(xf, (int) n, w[0].p, w[1].p, w[2].p, w[3].p, bias.p, members, d_norm.p, mean,
                        spread, errflag.p, s, dcount);
   }
 };
@@ -452,12 +429,6 @@ void features_bf16(const float *x, long long n, const float *norm, bf16 *out, cu
 void targets(const float *t, long long n, const float *norm, float *out, cudaStream_t s) {
   k_targets<<<nblk(n * NOUT, 256), 256, 0, s>>>(t, n, norm, out);
   check(cudaGetLastError(), "targets");
-}
-
-void gather(const bf16 *xall, const float *tall, const int *idx, int nb, bf16 *x0, float *tb,
-            cudaStream_t s) {
-  k_gather<<<nblk((long) nb * NINP, 256), 256, 0, s>>>(xall, tall, idx, nb, x0, tb);
-  check(cudaGetLastError(), "gather");
 }
 
 }  // namespace mlp
@@ -517,6 +488,34 @@ constexpr long kNParam = (long) MLP_HIDDEN * MLP_IN + MLP_HIDDEN +
                          2L * (MLP_HIDDEN * MLP_HIDDEN + MLP_HIDDEN) + (long) MLP_OUT * MLP_HIDDEN +
                          MLP_OUT;
 
+struct Plan {
+  cacg::gemm::TrainPlan *p;
+  explicit Plan(const cacg::gemm::TrainArgs &t) : p(cacg::gemm::train_plan(t)) {}
+  ~Plan() { cacg::gemm::train_plan_free(p); }
+  Plan(const Plan &) = delete;
+  Plan &operator=(const Plan &) = delete;
+};
+
+// host tasks on threads of their own; a task whose thread cannot be started
+// runs at once.  The destructor waits for all of them.
+struct Workers {
+  std::vector<std::thread> t;
+  template <class F>
+  void run(F f) {
+    try {
+      t.reserve(t.size() + 1);
+      t.emplace_back(f);
+    } catch (const std::exception &) {
+      f();
+    }
+  }
+  void wait() {
+    for (std::thread &x : t) x.join();
+    t.clear();
+  }
+  ~Workers() { wait(); }
+};
+
 // upload normalised features (bf16 [n][64]) and targets (fp32 [n][24])
 void upload_set(Net &N, const float *x, const float *t, long long n, cacg::DBuf<bf16> &xf,
                 cacg::DBuf<float> &tf) {
@@ -561,7 +560,6 @@ int cacg_mlp_create(cacg_mlp *out, int device, int members, unsigned long long s
     for (int i = 0; i < MLP_OUT; i++)
       m->net.norm[2 * MLP_IN + i] = 0.f, m->net.norm[2 * MLP_IN + MLP_OUT + i] = 1.f;
     m->net.upload_norm();
-    m->net.mem.resize(members);
     m->net.init_params(seed);
   } catch (const MlpError &e) {
     rc = e.code;
@@ -581,17 +579,11 @@ int cacg_mlp_destroy(cacg_mlp m) {
   cudaSetDevice(m->net.device);
   if (m->net.stream) cudaStreamSynchronize(m->net.stream);
   Net &N = m->net;
-  for (Member &M : N.mem)
-    for (auto *b : {&M.p, &M.m, &M.v, &M.g}) b->release();
-  for (Member &M : N.mem)
-    for (auto *b : {&M.w1, &M.w2, &M.w3, &M.w4, &M.w2t, &M.w3t, &M.w4t}) b->release();
-  for (auto *b : {&N.x0, &N.h1, &N.h2, &N.h3, &N.g4, &N.g3, &N.g2, &N.g1, &N.x0t, &N.h1t, &N.h2t,
-                  &N.h3t, &N.g1t, &N.g2t, &N.g3t, &N.g4t, &N.ix0, &N.ih1, &N.ih2, &N.ih3, &N.iw1})
-    b->release();
-  for (auto *b : {&N.d_norm, &N.z1, &N.z2, &N.z3, &N.y, &N.tb, &N.db, &N.iy, &N.iw1b, &N.ibias})
-    b->release();
-  for (auto *b : {&N.iw2, &N.iw3, &N.iw4}) b->release();
-  N.part.release();
+  for (auto *b : {&N.p, &N.m, &N.v, &N.g, &N.bias, &N.d_norm, &N.tb, &N.part}) b->release();
+  for (int l = 0; l < 4; l++)
+    for (auto *b : {&N.w[l], &N.wt[l], &N.h[l], &N.ht[l], &N.gr[l], &N.grt[l]}) b->release();
+  for (auto &b : N.z) b.release();
+  N.loss.release();
   N.errflag.release();
   if (N.stream) cudaStreamDestroy(N.stream);
   delete m;
@@ -611,7 +603,7 @@ int cacg_mlp_sizes(cacg_mlp m, long long *sizes, int n) {
 int cacg_mlp_get_params(cacg_mlp m, int member, float *p) {
   MLP_BEGIN
   need(p && member >= 0 && member < m->net.members, "bad member or array");
-  cacg::check(cudaMemcpyAsync(p, m->net.mem[member].p.p, sizeof(float) * kNParam,
+  cacg::check(cudaMemcpyAsync(p, m->net.p.p + (size_t) member * kNParam, sizeof(float) * kNParam,
                               cudaMemcpyDeviceToHost, m->net.stream), "params");
   m->net.sync();
   MLP_END
@@ -620,9 +612,9 @@ int cacg_mlp_get_params(cacg_mlp m, int member, float *p) {
 int cacg_mlp_set_params(cacg_mlp m, int member, const float *p) {
   MLP_BEGIN
   need(p && member >= 0 && member < m->net.members, "bad member or array");
-  cacg::check(cudaMemcpyAsync(m->net.mem[member].p.p, p, sizeof(float) * kNParam,
+  cacg::check(cudaMemcpyAsync(m->net.p.p + (size_t) member * kNParam, p, sizeof(float) * kNParam,
                               cudaMemcpyHostToDevice, m->net.stream), "params");
-  m->net.refresh(member);
+  m->net.refresh(member, 1);
   m->net.sync();
   MLP_END
 }
@@ -667,21 +659,24 @@ int cacg_mlp_loss_grad(cacg_mlp m, int member, const float *x, const float *t, i
   MLP_BEGIN
   Net &N = m->net;
   need(x && t && n > 0 && member >= 0 && member < N.members, "bad arguments");
-  const int B = (n + 127) / 128 * 128;
-  N.ensure_batch(B);
+  const int B = (n + 127) / 128 * 128, tiles = B / 128;
   cacg::DBuf<bf16> xf;
   cacg::DBuf<float> tf;
   upload_set(N, x, t, n, xf, tf);
-  cacg::check(cudaMemsetAsync(N.x0.p, 0, sizeof(bf16) * (size_t) B * 64, N.stream), "x0");
-  cacg::check(cudaMemsetAsync(N.tb.p, 0, sizeof(float) * (size_t) B * MLP_OUT, N.stream), "tb");
-  cacg::check(cudaMemcpyAsync(N.x0.p, xf.p, sizeof(bf16) * (size_t) n * 64, cudaMemcpyDeviceToDevice, N.stream), "x0");
-  cacg::check(cudaMemcpyAsync(N.tb.p, tf.p, sizeof(float) * (size_t) n * MLP_OUT, cudaMemcpyDeviceToDevice, N.stream), "tb");
-  N.forward_train(member, B);
-  double l = N.backward(member, B, n, true);
+  const cacg::gemm::TrainArgs ta = N.batch(member, 1, B, n);
+  N.loss.ensure(tiles, N.stream);
+  Plan plan(ta);
+  N.gather(ta, xf.p, tf.p, nullptr, 0, n);
+  cacg::gemm::train_passes(*plan.p, N.loss.p, N.stream);
+  N.gradients(ta, member);
+  std::vector<double> h(tiles);
+  cacg::check(cudaMemcpyAsync(h.data(), N.loss.p, sizeof(double) * tiles, cudaMemcpyDeviceToHost, N.stream), "loss");
   N.check_err();
-  if (loss) *loss = l;
+  double l = 0.0;
+  for (double q : h) l += q;
+  if (loss) *loss = l / ((double) n * MLP_OUT);
   if (grad) {
-    cacg::check(cudaMemcpyAsync(grad, N.mem[member].g.p, sizeof(float) * kNParam,
+    cacg::check(cudaMemcpyAsync(grad, N.g.p + (size_t) member * kNParam, sizeof(float) * kNParam,
                                 cudaMemcpyDeviceToHost, N.stream), "grad");
     N.sync();
   }
@@ -696,36 +691,63 @@ int cacg_mlp_train(cacg_mlp m, const float *x, const float *t, long long n, int 
   Net &N = m->net;
   need(x && t && epochs > 0 && batch >= 128 && batch % 128 == 0 && n >= batch && lr > 0,
        "bad training arguments (batch a positive multiple of 128, n >= batch)");
-  N.ensure_batch(batch);
   cacg::DBuf<bf16> xf;
   cacg::DBuf<float> tf;
-  upload_set(N, x, t, n, xf, tf);
-  cacg::DBuf<int> didx;
   const long long nbatch = n / batch;  // whole batches only
-  didx.ensure((size_t) batch * std::max<long long>(nbatch, 1), N.stream);
-  cacg::mlp::Rng rng{seed};
-  std::vector<int> perm(n);
+  const int members = N.members, tiles = batch / 128;
+  // the shuffles of an epoch, member by member from one random sequence: each
+  // takes n - 1 numbers, so every shuffle's place in the sequence is known, and
+  // the members' are made side by side, the next epoch's while this one runs
+  std::vector<std::vector<int>> perm[2];
+  for (auto &e : perm) e.assign(members, std::vector<int>(n));
+  auto shuffle = [&](int ep, int k) {
+    std::vector<int> &q = perm[ep & 1][k];
+    cacg::mlp::Rng rng{seed};
+    rng.skip((unsigned long long) ((long long) ep * members + k) * (unsigned long long) (n - 1));
+    for (long long i = 0; i < n; i++) q[i] = (int) i;
+    for (long long i = n - 1; i > 0; i--) std::swap(q[i], q[rng.next() % (unsigned long long) (i + 1)]);
+  };
+  Workers workers;
+  auto start = [&](int ep) {
+    for (int k = 0; k < members; k++) workers.run([&shuffle, ep, k] { shuffle(ep, k); });
+  };
+  start(0);
+  upload_set(N, x, t, n, xf, tf);
+  const cacg::gemm::TrainArgs ta = N.batch(0, members, batch, batch);
+  N.loss.ensure((size_t) nbatch * members * tiles, N.stream);
+  Plan plan(ta);
+  cacg::DBuf<int> didx;
+  const long long istride = batch * nbatch;
+  didx.ensure((size_t) istride * members, N.stream);
   for (int ep = 0; ep < epochs; ep++) {
     // cosine schedule from lr to lr/20
     const float lr_ep = (float) (lr * (0.05 + 0.95 * 0.5 * (1 + std::cos(M_PI * ep / epochs))));
-    double lsum = 0.0;
-    for (int k = 0; k < N.members; k++) {
-      for (long long i = 0; i < n; i++) perm[i] = (int) i;
-      for (long long i = n - 1; i > 0; i--) std::swap(perm[i], perm[rng.next() % (unsigned long long) (i + 1)]);
-      cacg::check(cudaMemcpyAsync(didx.p, perm.data(), sizeof(int) * batch * nbatch,
+    workers.wait();
+    for (int k = 0; k < members; k++)
+      cacg::check(cudaMemcpyAsync(didx.p + k * istride, perm[ep & 1][k].data(), sizeof(int) * istride,
                                   cudaMemcpyHostToDevice, N.stream), "perm");
-      for (long long b = 0; b < nbatch; b++) {
-        cacg::mlp::gather(xf.p, tf.p, didx.p + b * batch, batch, N.x0.p, N.tb.p, N.stream);
-        N.forward_train(k, batch);
-        bool last = ep == epochs - 1 && epoch_loss;
-        double l = N.backward(k, batch, batch, last);
-        lsum += l;
-        N.adam(k, lr_ep);
-      }
-      N.sync();  // perm is reused for the next member
+    if (ep + 1 < epochs) start(ep + 1);  // into the other buffers
+    for (long long b = 0; b < nbatch; b++) {
+      N.gather(ta, xf.p, tf.p, didx.p + b * batch, istride, batch);
+      cacg::gemm::train_passes(*plan.p, N.loss.p + (size_t) b * members * tiles, N.stream);
+      N.adam(ta, lr_ep);
     }
+    N.sync();  // the shuffles' buffers are reused two epochs on
     N.adam_steps += nbatch;
-    if (epoch_loss && ep == epochs - 1) *epoch_loss = lsum / (double) (N.members * nbatch);
+  }
+  if (epoch_loss) {
+    std::vector<double> h((size_t) nbatch * members * tiles);
+    cacg::check(cudaMemcpyAsync(h.data(), N.loss.p, sizeof(double) * h.size(), cudaMemcpyDeviceToHost,
+                                N.stream), "loss");
+    N.sync();
+    double lsum = 0.0;
+    for (int k = 0; k < members; k++)
+      for (long long b = 0; b < nbatch; b++) {
+        double l = 0.0;
+        for (int q = 0; q < tiles; q++) l += h[((size_t) b * members + k) * tiles + q];
+        lsum += l / ((double) batch * MLP_OUT);
+      }
+    *epoch_loss = lsum / (double) (members * nbatch);
   }
   N.check_err();
   xf.release();
@@ -761,8 +783,7 @@ int cacg_gemm_bf16_tn(const void *a, int lda, const void *b, int ldb, float *c, 
                       int n_, int k_, int *err, void *stream) {
   if (!a || !b || !c || !err || m_ <= 0 || n_ <= 0 || k_ <= 0 || ldc < n_) return CACG_EINVAL;
   try {
-    cacg::gemm::gemm_tn(a, lda, b, ldb, m_, n_, k_, 0, nullptr, c, ldc, nullptr, 0, err,
-                        static_cast<cudaStream_t>(stream));
+    cacg::gemm::gemm_tn(a, lda, b, ldb, m_, n_, k_, c, ldc, err, static_cast<cudaStream_t>(stream));
   } catch (const CudaError &e) {
     return e.code == cudaErrorInvalidValue ? CACG_EINVAL : CACG_ECUDA;
   }
