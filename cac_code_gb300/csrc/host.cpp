@@ -235,6 +235,7 @@ struct cacg_context {
   DBuf<unsigned long long> d_line_mask_n, d_line_mask_nf;
   DBuf<unsigned char> d_row_isforce;
   long long elist_builds = 0, epart_of = -1;
+  bool epart_fused = false;  // the last reorder was the fused passes'
   bool ereorders_zeroed = false;  // the reorder counter (d_misc slot 15)
   bool areorders_zeroed = false;  // the atom-list reorder counter (d_misc slot 16)
   // lattice lines that the integration-point lists reference (all rows; force
@@ -2611,8 +2612,8 @@ void cacg_context::pair_compute_mixed(int pass) {
     // slot 12: reordered in this pass
     const bool same = part_of == list_builds && ref_g == g && ref_l0[0] == l0[0] &&
                       ref_l0[1] == l0[1] && ref_l0[2] == l0[2];
-    check(cudaMemsetAsync(d_misc.p + 11, same ? 0 : 0x7F, sizeof(int), s), "dmax");
-    check(cudaMemsetAsync(d_misc.p + 12, 0, sizeof(int), s), "reordered");
+    check(cudaMemsetAsync(d_misc.p + 11, 0, 2 * sizeof(int), s), "dmax, reordered");
+    if (!same) check(cudaMemsetAsync(d_misc.p + 11, 0x7F, sizeof(int), s), "dmax");
     mixed::pack_rel(d_x.p, nall, mixed::make_pack_grid(l0, g, d_misc.p + 9), d_xh.p,
                     same ? d_xq_ref.p : nullptr, nlocal,
                     reinterpret_cast<unsigned *>(d_misc.p + 11), s);
@@ -2718,56 +2719,66 @@ void cacg_context::pair_ecompute_mixed() {
   }
   const mixed::PackGrid pg = mixed::make_pack_grid(l0, g, d_misc.p + 9);
   const long long nmask = (long long) std::max(nall, 1) * std::max(maxlines, 1);
+  const EamTables et = pair_style == 2 ? eamtab() : EamTables{};
+  const bool fused = fused_on && self_contained && fused_types_ok &&
+                     mixed::fused_fits(pair_style == 2 ? et.nr : 0, pair_style == 2 ? et.nrho : 0);
+  fused_used = fused;
   d_node_hl.ensure((size_t) 24 * nall, s);
-  d_line_pos.ensure(3 * (size_t) nmask, s);
   // displacement culling of the integration-point lists: slot 13 holds the
   // largest squared node displacement since the last reorder (set huge after
-  // an element list build, so that this pass reorders), slot 14 flags a
-  // reorder in this pass.  The lists are kept reordered even with "tune cull
-  // no", so that culling changes no bit: it only stops each row early.
+  // an element list build, or when the other kind of passes made the reorder,
+  // so that this pass reorders), slot 14 flags a reorder in this pass.  The
+  // lists are kept reordered even with "tune cull no", so that culling changes
+  // no bit: it only stops each row early.
   const bool cull_e = mixed_cull;
   unsigned *eflags = reinterpret_cast<unsigned *>(d_misc.p + 13);
-  const bool same_e = epart_of == elist_builds;
+  const bool same_e = epart_of == elist_builds && epart_fused == fused;
   d_ent_near.ensure(std::max((size_t) 1, d_ent.cap), s);
   d_nnear_row.ensure(std::max(nrows, 1), s);
   d_node_ref.ensure((size_t) 24 * nall, s);
-  d_line_mask_n.ensure(nmask, s);
-  d_line_mask_nf.ensure(nmask, s);
   if (!ereorders_zeroed) {
     check(cudaMemsetAsync(d_misc.p + 15, 0, sizeof(int), s), "ereorders");
     ereorders_zeroed = true;
   }
-  check(cudaMemsetAsync(d_misc.p + 13, same_e ? 0 : 0x7F, sizeof(int), s), "edmax");
-  check(cudaMemsetAsync(d_misc.p + 14, 0, sizeof(int), s), "ereordered");
-  const EamTables et = pair_style == 2 ? eamtab() : EamTables{};
-  const bool fused = fused_on && self_contained && fused_types_ok &&
-                     mixed::fused_fits(pair_style == 2 ? et.nr : 0, pair_style == 2 ? et.nrho : 0);
-  // the fused passes need the line data and row points only to reorder the lists
-  const unsigned *gate = fused ? eflags : nullptr;
-  fused_used = fused;
+  check(cudaMemsetAsync(d_misc.p + 13, 0, 2 * sizeof(int), s), "edmax, ereordered");
+  if (!same_e) check(cudaMemsetAsync(d_misc.p + 13, 0x7F, sizeof(int), s), "edmax");
   kmark(KT_SITES, 0);
   mixed::node_split(d_nodex.p, nall, d_node_hl.p, same_e ? d_node_ref.p : nullptr, eflags, s);
   const mixed::Lattice lat{d_nae.p, d_frac.p, fstride, code_kb};
-  // the lattice lines that the scanned entries reference (all referenced
-  // lines in a step that reorders)
-  mixed::lines(d_node_hl.p, d_etype.p, lat, max_nax, d_line_mask.p,
-               cull_e ? d_line_mask_n.p : nullptr, eflags, maxlines, pg, nall, d_line_pos.p, s,
-               gate);
-  kmark(KT_SITES, 1);
-  d_ip_q.ensure(std::max(nrows, 1), s);
-  d_ip_h.ensure(std::max(nrows, 1), s);
-  d_ip_l.ensure(std::max(nrows, 1), s);
-  kmark(KT_EPREP, 0);
-  mixed::row_q(d_row_elem.p, d_row_jj.p, d_etype.p, d_int_off.p, d_spa_int_hl.p, d_node_hl.p, nrows,
-               pg, d_ip_q.p, d_ip_h.p, d_ip_l.p, s, gate);
   const double csq_e = pair_style == 1 ? ljtab.cutsq[1 * (MAXT + 1) + 1] : cutforcesq;
-  mixed::ip_reorder(d_row_start.p, d_ent.p, nrows, d_ip_q.p, d_line_pos.p, lat, pg,
-                    (float) std::sqrt(csq_e), d_ent_near.p, d_nnear_row.p, d_node_hl.p, nall,
-                    d_node_ref.p, eflags, s);
-  mixed::line_masks(d_row_start.p, d_ent_near.p, d_nnear_row.p, nrows, lat, d_row_isforce.p,
-                    d_line_mask_n.p, d_line_mask_nf.p, nmask, eflags, s);
-  kmark(KT_EPREP, 1);
-  launches += 6;
+  if (fused) {
+    kmark(KT_SITES, 1);
+    kmark(KT_EPREP, 0);
+    mixed::fused_reorder(d_node_hl.p, d_etype.p, d_row_first.p, d_numint.p, d_int_off.p, d_intp4.p,
+                         d_lat_rec.p, lat, maxlines, pg, d_row_start.p, d_ent.p, enlocal, nall,
+                         (float) std::sqrt(csq_e), d_ent_near.p, d_nnear_row.p, d_node_ref.p, eflags,
+                         s);
+    kmark(KT_EPREP, 1);
+    launches += 2;
+  } else {
+    d_line_pos.ensure(3 * (size_t) nmask, s);
+    d_line_mask_n.ensure(nmask, s);
+    d_line_mask_nf.ensure(nmask, s);
+    // the lattice lines that the scanned entries reference (all referenced
+    // lines in a step that reorders)
+    mixed::lines(d_node_hl.p, d_etype.p, lat, max_nax, d_line_mask.p,
+                 cull_e ? d_line_mask_n.p : nullptr, eflags, maxlines, pg, nall, d_line_pos.p, s);
+    kmark(KT_SITES, 1);
+    d_ip_q.ensure(std::max(nrows, 1), s);
+    d_ip_h.ensure(std::max(nrows, 1), s);
+    d_ip_l.ensure(std::max(nrows, 1), s);
+    kmark(KT_EPREP, 0);
+    mixed::row_q(d_row_elem.p, d_row_jj.p, d_etype.p, d_int_off.p, d_spa_int_hl.p, d_node_hl.p, nrows,
+                 pg, d_ip_q.p, d_ip_h.p, d_ip_l.p, s);
+    mixed::ip_reorder(d_row_start.p, d_ent.p, nrows, d_ip_q.p, d_line_pos.p, lat, pg,
+                      (float) std::sqrt(csq_e), d_ent_near.p, d_nnear_row.p, d_node_hl.p, nall,
+                      d_node_ref.p, eflags, s);
+    mixed::line_masks(d_row_start.p, d_ent_near.p, d_nnear_row.p, nrows, lat, d_row_isforce.p,
+                      d_line_mask_n.p, d_line_mask_nf.p, nmask, eflags, s);
+    kmark(KT_EPREP, 1);
+    launches += 6;
+  }
+  epart_fused = fused;
   epart_of = elist_builds;
   const bool use_sur = sur && nfar > 0;
   const float eps = band_eps;

@@ -396,11 +396,10 @@ void node_split(const double *nodex, int n, float2 *hl, const float2 *ref, unsig
                 cudaStream_t s);
 // Lattice lines: U, D (double-single, relative to l0) of every line that
 // mask (mask_near while culling holds) marks; FP32 nodal-density lines
-// (with gate: only in a step whose node displacement calls for a list reorder)
 void lines(const float2 *node_hl, const int *etype, const Lattice &lat, int max_nax,
            const unsigned long long *mask, const unsigned long long *mask_near,
            const unsigned *eflags, int maxlines, const PackGrid &pg, int nelem, float4 *line_pos,
-           cudaStream_t s, const unsigned *gate = nullptr);
+           cudaStream_t s);
 void line_rho(const double *erho, const int *etype, const Lattice &lat,
               const unsigned long long *mask, const unsigned long long *mask_near,
               const unsigned *eflags, int maxlines, int nelem, float2 *out, cudaStream_t s);
@@ -482,10 +481,16 @@ void eam_force_atoms(const MixedAtoms &m, const float4 *ftab, const EamTables &e
 void lj_atoms(const MixedAtoms &m, const int *type, const float *lj1, const float *lj2,
               const float *cutsq_t, const double *cutsq64, double *f, cudaStream_t s);
 // every row's integration point: packed, and its double-single position
+// ip_reorder for the fused passes, in one launch (nall_e: elements whose nodes
+// become the reference)
+void fused_reorder(const float2 *node_hl, const int *etype, const int *row_first, const int *numint,
+                   const int *int_off, const int4 *intp, const float4 *lat_rec, const Lattice &lat,
+                   int maxlines, const PackGrid &pg, const int *row_start, const int *ent,
+                   int nlocal_e, int nall_e, float cutoff, int *ent_near, int4 *nnear_row,
+                   float2 *node_ref, unsigned *eflags, cudaStream_t s);
 void row_q(const int *row_elem, const int *row_jj, const int *etype, const int *int_off,
            const float2 *spa_int_hl, const float2 *node_hl, int nrows, const PackGrid &pg,
-           float4 *ip_q, float4 *ip_h, float4 *ip_l, cudaStream_t s,
-           const unsigned *gate = nullptr);
+           float4 *ip_q, float4 *ip_h, float4 *ip_l, cudaStream_t s);
 // FP32 F'(rho) at the rows of nonzero weight, rho in FP64 from the nodal densities
 void row_fp(const int *rows, int nforce, const int *row_elem, const int *row_jj,
             const int *etype, const int *int_off, const double *spa_int, const double *erho,
@@ -537,7 +542,6 @@ void gemm_tn(const void *A, int lda, const void *B, int ldb, int M, int N, int K
 // 0..3; B rows per member, a multiple of 128)
 struct TrainArgs {
   int members, B, n_valid;       // n_valid rows of each member count
-  int splits, tps;               // the batch in `splits` parts of `tps` 64-row tiles
   const float *p;                // parameters [members][pstride]
   long pstride, ow[4], ob[4];    // offsets of weights and biases
   const float *tb;               // targets [members * B][24]
@@ -545,7 +549,7 @@ struct TrainArgs {
   float *z[3];                   // pre-activations [members * B][256], tile-transposed
   void *g[4], *gt[4];            // bf16 gradients [members * B][256 | 64], transposed
   void *w[4], *wt[4];            // bf16 weights [members * 256 | 24][64 | 256]; transposed (1..3)
-  float *part;                   // weight-gradient partial sums [splits][members][pstride]
+  float *grad;                   // weight gradients [members][pstride]
   int *err;
 };
 struct TrainPlan;  // the arrays' tensor maps, made once per call

@@ -506,9 +506,8 @@ k_mlp_ensemble(const __grid_constant__ CUtensorMap tma_x, const __grid_constant_
 // for the next layer, and transposed, K-major for the weight gradients, so that
 // no transpose runs by itself; Z transposed within the tile, so that a warp's
 // loads and stores are whole lines.  The weight gradients of all layers are one
-// launch, the batch split over blocks that leave partial sums, which the
-// update kernel adds in order (no atomics: the same result at every run), with
-// the bias gradients, Adam and the new BF16 weights.
+// launch; the update kernel adds up the bias gradients in a fixed order (no
+// atomics: the same result at every run) and does Adam and the new BF16 weights.
 //
 // What bounded it: launches and idle SMs.  One member's 2,048-row step was 45
 // launches, GEMMs on 2 to 16 blocks whose epilogues stored one float a line,
@@ -730,17 +729,17 @@ k_train_layer(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CU
 }
 
 // weight gradients dW_l = G_l^T H_{l-1} of layers 0..3, both operands transposed
-// (K = the batch): blocks of a layer's 128-row tiles x `splits` parts of the
-// batch of `tps` k-tiles; partial sums to part[split][member][nparam]
+// (K = the batch, in one accumulator): 128 x 128 tiles, 12 per member
 struct TrainDwMaps {
   CUtensorMap a[4], b[4];
 };
 struct TrainDw {
-  int B, splits, tps;
-  float *part;
+  int B;
+  float *g;
   long nparam, off[4];
   int *err;
 };
+constexpr int TR_DW_TILES = 12;
 
 __global__ void __launch_bounds__(TR_NT, 1)
 k_train_dw(const __grid_constant__ TrainDwMaps maps, TrainDw d) {
@@ -748,31 +747,22 @@ k_train_dw(const __grid_constant__ TrainDwMaps maps, TrainDw d) {
   __shared__ int s_fail;
   const TrainSmem sm = train_smem_of(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = warp & 3, cg = warp >> 2;
-  const int member = blockIdx.y, S = d.splits;
-  // layers 1, 2 (256 x 256), 0 (256 x 32), 3 (24 x 256)
-  int b = blockIdx.x, l = 1;
-  if (b >= 6 * S) {
-    l = 3;
-    b -= 6 * S;
-  } else if (b >= 4 * S) {
-    l = 0;
-    b -= 4 * S;
-  } else if (b >= 2 * S) {
-    l = 2;
-    b -= 2 * S;
-  }
-  const int tile = b / S, split = b % S;
+  const int member = blockIdx.y, b = blockIdx.x;
+  // layers 1, 2 (256 x 256: 4 tiles each), 0 (256 x 64: 2), 3 (24 x 256: 2)
+  const int l = b < 4 ? 1 : b < 8 ? 2 : b < 10 ? 0 : 3;
+  const int rt = b < 8 ? (b & 2) >> 1 : b < 10 ? b - 8 : 0;   // row tile
+  const int ct = b < 8 ? b & 1 : b < 10 ? 0 : b - 10;         // column tile
   const int arows = l == 3 ? TR_OUT : TR_H, brows = l == 0 ? TR_IN : TR_H, ldw = l == 0 ? 32 : TR_H;
-  const int k0 = split * d.tps, nk = min(d.tps, d.B / BK - k0);
+  const int bn = l == 0 ? TR_IN : 128;
   const unsigned tmem = train_begin(sm, &s_fail);
-  const bool ok = train_mma(sm, tmem, &maps.a[l], &maps.b[l], k0, nk, member * arows + tile * BM,
-                            member * brows, brows, d.err, &s_fail);
-  const int row = tile * BM + q * 32 + lane;
+  const bool ok = train_mma(sm, tmem, &maps.a[l], &maps.b[l], 0, d.B / BK, member * arows + rt * BM,
+                            member * brows + ct * 128, bn, d.err, &s_fail);
+  const int row = rt * BM + q * 32 + lane;
   if (ok) {
     const unsigned tl = tmem + ((unsigned) (q * 32) << 16);
-    float *out = d.part + ((size_t) split * gridDim.y + member) * d.nparam + d.off[l] + (size_t) row * ldw;
+    float *out = d.g + (size_t) member * d.nparam + d.off[l] + (size_t) row * ldw + ct * 128;
 #pragma unroll 1
-    for (int c = cg * 64; c < min(cg * 64 + 64, ldw); c += 16) {
+    for (int c = cg * 32; c < min(cg * 32 + 32, min(ldw, 128)); c += 16) {
       float v[16];
       tmem_ld16(tl + c, v);
       if (row < arows)
@@ -885,7 +875,7 @@ TrainPlan *train_plan(const TrainArgs &t) {
       pl->act[l] = act(t.h[l], kc);
       pl->wts[l] = make_map(t.w[l], M * rows, kc, kc, l == 3 ? 32 : TR_H);
       pl->dw.a[l] = make_map(t.gt[l], M * rows, B, B, BM);
-      pl->dw.b[l] = make_map(t.ht[l], M * kc, B, B, kc);
+      pl->dw.b[l] = make_map(t.ht[l], M * kc, B, B, l == 0 ? TR_IN : 128);
     }
     for (int l = 2; l >= 0; l--) {
       const int kc = l == 2 ? TR_OUTP : TR_H;
@@ -901,8 +891,8 @@ TrainPlan *train_plan(const TrainArgs &t) {
 
 void train_plan_free(TrainPlan *p) { delete p; }
 
-// One step's forward and backward passes and weight-gradient partial sums; the
-// squared errors go to `loss` ([members][B / 128])
+// One step's forward and backward passes and weight gradients; the squared
+// errors go to `loss` ([members][B / 128])
 void train_passes(const TrainPlan &pl, double *loss, cudaStream_t s) {
   const TrainArgs &t = pl.t;
   const size_t smem = train_smem();
@@ -944,13 +934,11 @@ void train_passes(const TrainPlan &pl, double *loss, cudaStream_t s) {
   }
   TrainDw d{};
   d.B = t.B;
-  d.splits = t.splits;
-  d.tps = t.tps;
-  d.part = t.part;
+  d.g = t.grad;
   d.nparam = t.pstride;
   d.err = t.err;
   for (int l = 0; l < 4; l++) d.off[l] = t.ow[l];
-  k_train_dw<<<dim3(7 * t.splits, t.members), TR_NT, smem, s>>>(pl.dw, d);
+  k_train_dw<<<dim3(TR_DW_TILES, t.members), TR_NT, smem, s>>>(pl.dw, d);
   check(cudaGetLastError(), "train_passes");
 }
 

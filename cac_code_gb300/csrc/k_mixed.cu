@@ -176,6 +176,17 @@ __device__ __forceinline__ bool inside64(const double4 &a, const double4 &b, dou
   return dx * dx + dy * dy + dz * dz < cutsq;
 }
 
+// The guard-band lanes of a warp decided one after another (i, j: the pair of
+// this lane).  A loop over the lanes that are in the band, rarely one: as a
+// plain branch the compiler predicates it, and FP64 instructions without an
+// active lane hold the FP64 unit all the same (77 % of the time of a pass).
+__device__ __forceinline__ bool band_decide(bool band, bool in, const double4 *__restrict__ x, int i,
+                                            int j, double cutsq) {
+  for (unsigned todo = __ballot_sync(0xffffffffu, band); todo; todo &= todo - 1)
+    if ((threadIdx.x & 31) == (unsigned) (__ffs(todo) - 1)) in = inside64(x[i], x[j], cutsq);
+  return in;
+}
+
 // The cell fields as floats without a conversion instruction: a field k below
 // 2^23 OR-ed into the bits of 2^23 reads as the float 2^23 + k, so the
 // difference of two such floats is the exact integer difference of the
@@ -336,10 +347,10 @@ k_eam_rho_atoms(AtomArgs a, const float4 *__restrict__ rhor_val, int nr, float r
       rel_vec(qi, cx, cy, cz, qj, a.qg, dx, dy, dz);
       float rsq = dx * dx + dy * dy + dz * dz;
       if (rsq > a.band_hi) continue;
-      a.slist[(size_t) ns++ * a.stride + i] = j;
       bool in = rsq < a.cutsq_f;
       if (rsq >= a.band_lo) in = inside64(a.x[i], a.x[j], a.cutsq);
-      if (in) {
+      if (in) {  // decided before it is listed: the force pass tests nothing
+        a.slist[(size_t) ns++ * a.stride + i] = j;
         float p;
         int m = findex(sqrtf(rsq), rdr, nr, p);
         float4 c = s_val[m];
@@ -355,6 +366,80 @@ k_eam_rho_atoms(AtomArgs a, const float4 *__restrict__ rhor_val, int nr, float r
     rho[i] = acc.value();
     fp[i] = a.frho_ds ? fprime_ds(ds_renorm(acc.h, acc.l), a.frho_ds, nrho, a.rdrho_ds)
                        : fprime32(__fadd_rn(acc.h, acc.l), fp4, nrho, rdrho);
+  }
+}
+
+// Small systems: G lanes per atom (group_lanes), the same sums bit for bit.  A
+// lane takes whole chunks of 8 pairs, and the chunk sums are added in the
+// chunks' order, which every lane of the atom follows by shuffles.  The density
+// pass numbers the entries in range by a ballot into the short list first.
+template <int G>
+__device__ __forceinline__ void add_chunks(dsacc &acc, float part, int first) {
+#pragma unroll
+  for (int l = 0; l < G; l++) acc.add(__shfl_sync(0xffffffffu, part, first + l));
+}
+
+template <int G>
+__global__ void __launch_bounds__(512, 2)
+k_eam_rho_lanes(AtomArgs a, const float4 *__restrict__ rhor_val, int nr, float rdr,
+                const float4 *__restrict__ fp4, int nrho, float rdrho,
+                double *__restrict__ rho, float *__restrict__ fp) {
+  extern __shared__ float4 s_val[];
+  for (int m = threadIdx.x; m <= nr; m += blockDim.x) s_val[m] = rhor_val[m];
+  __syncthreads();
+  const int level = a.nnear ? cull_level(a.dmax2) : 4;
+  const int lane = threadIdx.x & 31, g = lane & (G - 1), first = lane & ~(G - 1);
+  const unsigned below = (1u << g) - 1u;
+  const int step = (int) (gridDim.x * blockDim.x) / G;
+  // each warp's first atom; every lane of a warp makes the same rounds
+  for (int ib = (int) ((blockIdx.x * blockDim.x + threadIdx.x) & ~31u) / G; ib < a.nlocal; ib += step) {
+    const int i = ib + lane / G;
+    const bool live = i < a.nlocal;
+    const float4 qi = a.xq[live ? i : 0];
+    float cx, cy, cz;
+    cell_of(qi, cx, cy, cz);
+    const int n = !live ? 0 : level < 4 ? culled_count(level, a.nnear[i], 0) : a.num[i];
+    const int nw = (int) __reduce_max_sync(0xffffffffu, (unsigned) n);
+    int ns = 0, jn = 0;
+    if (g < n) jn = __ldg(a.list + (size_t) g * a.stride + i);
+    for (int k = g; k < nw + g; k += G) {
+      const int j = jn;
+      if (k + G < n) jn = __ldg(a.list + (size_t) (k + G) * a.stride + i);
+      float dx, dy, dz;
+      rel_vec(qi, cx, cy, cz, __ldg(a.xq + j), a.qg, dx, dy, dz);
+      const float rsq = dx * dx + dy * dy + dz * dz;
+      const bool band = k < n && rsq >= a.band_lo && rsq <= a.band_hi;
+      const bool in = band_decide(band, k < n && rsq < a.cutsq_f, a.x, i, j, a.cutsq);
+      const unsigned m = (__ballot_sync(0xffffffffu, in) >> first) & ((1u << G) - 1u);
+      if (in) a.slist[(size_t) (ns + __popc(m & below)) * a.stride + i] = j;
+      ns += __popc(m);
+    }
+    __syncwarp();  // the short list, as all lanes of the atom left it
+    const int sw = (int) __reduce_max_sync(0xffffffffu, (unsigned) ns);
+    dsacc acc;
+    for (int c = 0; c * CHUNK < sw; c += G) {
+      float part = 0.f;
+      const int k0 = (c + g) * CHUNK;
+#pragma unroll
+      for (int t = 0; t < CHUNK; t++)
+        if (k0 + t < ns) {
+          const int j = a.slist[(size_t) (k0 + t) * a.stride + i];
+          float dx, dy, dz;
+          rel_vec(qi, cx, cy, cz, __ldg(a.xq + j), a.qg, dx, dy, dz);
+          const float rsq = dx * dx + dy * dy + dz * dz;
+          float p;
+          const int m = findex(sqrtf(rsq), rdr, nr, p);
+          const float4 v = s_val[m];
+          part += ((v.x * p + v.y) * p + v.z) * p + v.w;
+        }
+      add_chunks<G>(acc, part, first);
+    }
+    if (live && g == 0) {
+      a.snum[i] = ns;
+      rho[i] = acc.value();
+      fp[i] = a.frho_ds ? fprime_ds(ds_renorm(acc.h, acc.l), a.frho_ds, nrho, a.rdrho_ds)
+                         : fprime32(__fadd_rn(acc.h, acc.l), fp4, nrho, rdrho);
+    }
   }
 }
 
@@ -634,7 +719,7 @@ constexpr int FORCE_BLOCK = 1024;
 __global__ void __launch_bounds__(FORCE_BLOCK, 1)
 k_eam_force_atoms(AtomArgs a, const float4 *__restrict__ ftab, int nr, float rdr,
                   const float *__restrict__ fp, double *__restrict__ f) {
-  extern __shared__ float4 s_tab[];  // 3 float4 per knot
+  extern __shared__ float4 s_tab[];  // FTAB_W float4 per knot
   for (int m = threadIdx.x; m < FTAB_W * (nr + 1); m += blockDim.x) s_tab[m] = ftab[m];
   __syncthreads();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.nlocal; i += gridDim.x * blockDim.x) {
@@ -659,7 +744,6 @@ k_eam_force_atoms(AtomArgs a, const float4 *__restrict__ ftab, int nr, float rdr
     }
     if (n > 1) jnn = __ldg(a.slist + (size_t) a.stride + i);
     for (int k = 0; k < n; k++) {
-      const int j = jn;
       const float4 qj = qn;
       const float fpj = fpn;
       jn = jnn;
@@ -671,28 +755,24 @@ k_eam_force_atoms(AtomArgs a, const float4 *__restrict__ ftab, int nr, float rdr
       float dx, dy, dz;
       rel_vec(qi, cx, cy, cz, qj, a.qg, dx, dy, dz);
       float rsq = dx * dx + dy * dy + dz * dz;
-      bool in = rsq < a.cutsq_f;
-      if (rsq >= a.band_lo && rsq <= a.band_hi) in = inside64(a.x[i], a.x[j], a.cutsq);
-      if (in) {
-        float recip = rsqrtf(rsq);
-        float r = rsq * recip;
-        float p;
-        int m = findex(r, rdr, nr, p);
-        float rhoip, z2, z2p;
-        force_spline(s_tab, m, p, rdr, rhoip, z2, z2p);
-        float phi = z2 * recip;
-        float phip = z2p * recip - phi * recip;
-        float psip = (fpi + fpj) * rhoip + phip;
-        float fpair = -psip * recip;
-        px += dx * fpair;
-        py += dy * fpair;
-        pz += dz * fpair;
-        if ((++cnt & (CHUNK - 1)) == 0) {
-          fx.add(px);
-          fy.add(py);
-          fz.add(pz);
-          px = py = pz = 0.f;
-        }
+      float recip = rsqrtf(rsq);
+      float r = rsq * recip;
+      float p;
+      int m = findex(r, rdr, nr, p);
+      float rhoip, z2, z2p;
+      force_spline(s_tab, m, p, rdr, rhoip, z2, z2p);
+      float phi = z2 * recip;
+      float phip = z2p * recip - phi * recip;
+      float psip = (fpi + fpj) * rhoip + phip;
+      float fpair = -psip * recip;
+      px += dx * fpair;
+      py += dy * fpair;
+      pz += dz * fpair;
+      if ((++cnt & (CHUNK - 1)) == 0) {
+        fx.add(px);
+        fy.add(py);
+        fz.add(pz);
+        px = py = pz = 0.f;
       }
     }
     fx.add(px);
@@ -701,6 +781,66 @@ k_eam_force_atoms(AtomArgs a, const float4 *__restrict__ ftab, int nr, float rdr
     f[3 * i + 1] = fy.value();
     fz.add(pz);
     f[3 * i + 2] = fz.value();
+  }
+}
+
+// G lanes per atom, a chunk of 8 pairs each (see k_eam_rho_lanes)
+template <int G>
+__global__ void __launch_bounds__(512, 1)
+k_eam_force_lanes(AtomArgs a, const float4 *__restrict__ ftab, int nr, float rdr,
+                  const float *__restrict__ fp, double *__restrict__ f) {
+  extern __shared__ float4 s_tab[];  // FTAB_W float4 per knot
+  for (int m = threadIdx.x; m < FTAB_W * (nr + 1); m += blockDim.x) s_tab[m] = ftab[m];
+  __syncthreads();
+  const int lane = threadIdx.x & 31, g = lane & (G - 1), first = lane & ~(G - 1);
+  const int step = (int) (gridDim.x * blockDim.x) / G;
+  for (int ib = (int) ((blockIdx.x * blockDim.x + threadIdx.x) & ~31u) / G; ib < a.nlocal; ib += step) {
+    const int i = ib + lane / G;
+    const bool live = i < a.nlocal;
+    const float4 qi = a.xq[live ? i : 0];
+    float cx, cy, cz;
+    cell_of(qi, cx, cy, cz);
+    const float fpi = live ? fp[i] : 0.f;
+    const int n = live ? a.snum[i] : 0;
+    const int nw = (int) __reduce_max_sync(0xffffffffu, (unsigned) n);
+    dsacc fx, fy, fz;
+    for (int c = 0; c * CHUNK < nw; c += G) {
+      float px = 0.f, py = 0.f, pz = 0.f;
+      const int k0 = (c + g) * CHUNK;
+      int jn[CHUNK];
+#pragma unroll
+      for (int t = 0; t < CHUNK; t++)
+        jn[t] = k0 + t < n ? __ldg(a.slist + (size_t) (k0 + t) * a.stride + i) : 0;
+#pragma unroll
+      for (int t = 0; t < CHUNK; t++)
+        if (k0 + t < n) {
+          float dx, dy, dz;
+          rel_vec(qi, cx, cy, cz, __ldg(a.xq + jn[t]), a.qg, dx, dy, dz);
+          const float fpj = __ldg(fp + jn[t]);
+          float rsq = dx * dx + dy * dy + dz * dz;
+          float recip = rsqrtf(rsq);
+          float r = rsq * recip;
+          float p;
+          int m = findex(r, rdr, nr, p);
+          float rhoip, z2, z2p;
+          force_spline(s_tab, m, p, rdr, rhoip, z2, z2p);
+          float phi = z2 * recip;
+          float phip = z2p * recip - phi * recip;
+          float psip = (fpi + fpj) * rhoip + phip;
+          float fpair = -psip * recip;
+          px += dx * fpair;
+          py += dy * fpair;
+          pz += dz * fpair;
+        }
+      add_chunks<G>(fx, px, first);
+      add_chunks<G>(fy, py, first);
+      add_chunks<G>(fz, pz, first);
+    }
+    if (live && g == 0) {
+      f[3 * i] = fx.value();
+      f[3 * i + 1] = fy.value();
+      f[3 * i + 2] = fz.value();
+    }
   }
 }
 
@@ -760,6 +900,62 @@ k_lj_atoms(AtomArgs a, const int *__restrict__ type, const float *__restrict__ l
     f[3 * i + 1] = fy.value();
     fz.add(pz);
     f[3 * i + 2] = fz.value();
+  }
+}
+
+// G lanes per atom, a chunk of 8 list entries each (see k_eam_rho_lanes)
+template <int G>
+__global__ void __launch_bounds__(512, 2)
+k_lj_lanes(AtomArgs a, const int *__restrict__ type, const float *__restrict__ lj1,
+           const float *__restrict__ lj2, const float *__restrict__ cutsq_t,
+           const double *__restrict__ cutsq64, double *__restrict__ f) {
+  const int lane = threadIdx.x & 31, g = lane & (G - 1), first = lane & ~(G - 1);
+  const int step = (int) (gridDim.x * blockDim.x) / G;
+  for (int ib = (int) ((blockIdx.x * blockDim.x + threadIdx.x) & ~31u) / G; ib < a.nlocal; ib += step) {
+    const int i = ib + lane / G;
+    const bool live = i < a.nlocal;
+    const float4 qi = a.xq[live ? i : 0];
+    float cx, cy, cz;
+    cell_of(qi, cx, cy, cz);
+    const int it = live ? type[i] : 0;
+    const int n = live ? a.num[i] : 0;
+    const int nw = (int) __reduce_max_sync(0xffffffffu, (unsigned) n);
+    dsacc fx, fy, fz;
+    for (int c = 0; c * CHUNK < nw; c += G) {
+      float px = 0.f, py = 0.f, pz = 0.f;
+      const int k0 = (c + g) * CHUNK;
+      int jn[CHUNK];
+#pragma unroll
+      for (int t = 0; t < CHUNK; t++)
+        jn[t] = k0 + t < n ? __ldg(a.list + (size_t) (k0 + t) * a.stride + i) : 0;
+#pragma unroll
+      for (int t = 0; t < CHUNK; t++) {
+        const bool valid = k0 + t < n;
+        const int j = jn[t];
+        float dx, dy, dz;
+        rel_vec(qi, cx, cy, cz, __ldg(a.xq + j), a.qg, dx, dy, dz);
+        const float rsq = dx * dx + dy * dy + dz * dz;
+        const int ij = it * (MAXT + 1) + type[j];
+        const float cs = cutsq_t[ij];
+        const bool band = valid && rsq >= a.band_lo * cs && rsq <= a.band_hi * cs;
+        if (band_decide(band, valid && rsq < cs, a.x, i, j, cutsq64[ij])) {
+          float r2inv = __frcp_rn(rsq);
+          float r6inv = r2inv * r2inv * r2inv;
+          float fpair = r6inv * (lj1[ij] * r6inv - lj2[ij]) * r2inv;
+          px += dx * fpair;
+          py += dy * fpair;
+          pz += dz * fpair;
+        }
+      }
+      add_chunks<G>(fx, px, first);
+      add_chunks<G>(fy, py, first);
+      add_chunks<G>(fz, pz, first);
+    }
+    if (live && g == 0) {
+      f[3 * i] = fx.value();
+      f[3 * i + 1] = fy.value();
+      f[3 * i + 2] = fz.value();
+    }
   }
 }
 
@@ -921,16 +1117,13 @@ __global__ void __launch_bounds__(LCH)
 k_lines(const float2 *__restrict__ node_hl, const int *__restrict__ etype, Lattice lat,
         const unsigned long long *__restrict__ line_mask,
         const unsigned long long *__restrict__ line_mask_near, const unsigned *__restrict__ eflags,
-        int maxlines, PackGrid pg, int nelem, int max_nax, float4 *__restrict__ line_pos,
-        const unsigned *__restrict__ gate) {
+        int maxlines, PackGrid pg, int nelem, int max_nax, float4 *__restrict__ line_pos) {
   // one warp per element: [nax][3][4] P, Q, R, S of the warp's element
   extern __shared__ ds s_cols[];
   __shared__ float2 s_nodes[LCH / 32][24];
-  if (gate && moved_little(gate)) return;  // no list reorder in this step
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ds *s_col = s_cols + (size_t) w * 12 * max_nax;
   float2 *s_nx = s_nodes[w];
-  // a persistent grid (a gated step then costs one short launch)
   for (int e = blockIdx.x * (LCH / 32) + w; e < nelem; e += gridDim.x * (LCH / 32)) {
   const int ty = etype[e];
   const int *nae = lat.nae;
@@ -1135,9 +1328,7 @@ __global__ void k_row_q(const int *__restrict__ row_elem, const int *__restrict_
                         const int *__restrict__ etype, const int *__restrict__ int_off,
                         const float2 *__restrict__ spa_int_hl, const float2 *__restrict__ node_hl,
                         int nrows, PackGrid pg, float4 *__restrict__ ip_q,
-                        float4 *__restrict__ ip_h, float4 *__restrict__ ip_l,
-                        const unsigned *__restrict__ gate) {
-  if (gate && moved_little(gate)) return;  // no list reorder in this step
+                        float4 *__restrict__ ip_h, float4 *__restrict__ ip_l) {
   const ds l0[3] = {{pg.l0h[0], pg.l0l[0]}, {pg.l0h[1], pg.l0l[1]}, {pg.l0h[2], pg.l0l[2]}};
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += gridDim.x * blockDim.x) {
     const int e = row_elem[r], ty = etype[e];
@@ -1757,17 +1948,20 @@ __device__ __forceinline__ void band_done(int *band, int ne) {
 
 // EAM nodal densities: the element's 8 node rows, one row per FG lanes
 // (FIX: the listed elements, guard-band pairs decided in FP64)
-template <int V, bool FIX>
+// STAGE: the spline tables in shared memory; otherwise read where they are
+// (few elements: their blocks would each copy 32 to 96 KB first)
+template <int V, bool FIX, bool STAGE>
 __global__ void __launch_bounds__(fused_block(V), 1)
 k_elem_rho_fused(FusedArgs a, const float4 *__restrict__ tab, int nr, float rdr,
                  double *__restrict__ erho) {
   const int ne = FIX ? min(a.band[0], a.nlocal_e) : a.e_end - a.e_begin;
   if (FIX && ne == 0) return;  // the whole grid (the count is the same for every block)
   extern __shared__ float4 smem[];
-  float4 *s_tab = smem;
-  for (int m = threadIdx.x; m <= nr; m += blockDim.x) s_tab[m] = tab[m];
+  const float4 *s_tab = STAGE ? smem : tab;
+  if (STAGE)
+    for (int m = threadIdx.x; m <= nr; m += blockDim.x) smem[m] = tab[m];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float *s_k = reinterpret_cast<float *>(smem + nr + 1) + (size_t) w * FUSED_WARP_FLOATS;
+  float *s_k = reinterpret_cast<float *>(smem + (STAGE ? nr + 1 : 0)) + (size_t) w * FUSED_WARP_FLOATS;
   __syncthreads();
   const int gw = (int) (((long long) blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int nw = (int) (((long long) gridDim.x * blockDim.x) >> 5);
@@ -1825,19 +2019,18 @@ k_elem_rho_fused(FusedArgs a, const float4 *__restrict__ tab, int nr, float rdr,
 // Forces of the element's rows of nonzero weight and their gather onto the
 // nodes (EAM with the nodal densities and row F'(rho), or LJ)
 // (FIX: the listed elements, guard-band pairs decided in FP64)
-template <bool EAM, int V, bool FIX>
+template <bool EAM, int V, bool FIX, bool STAGE>
 __global__ void __launch_bounds__(fused_block(V), 1)
 k_elem_force_fused(FusedArgs a, const float4 *__restrict__ tab, int nr, float rdr, float lj1,
                    float lj2, const double *__restrict__ erho, double *__restrict__ nodef) {
   const int ne = FIX ? min(a.band[0], a.nlocal_e) : a.e_end - a.e_begin;
   if (FIX && ne == 0) return;  // the whole grid (the count is the same for every block)
   extern __shared__ float4 smem[];
-  float4 *s_tab = smem;
-  const int ntab = EAM ? FTAB_W * (nr + 1) : 0;
-  const int nfp = EAM ? a.nrho + 1 : 0;
-  float4 *s_fp = smem + ntab;
-  for (int m = threadIdx.x; m < ntab; m += blockDim.x) s_tab[m] = tab[m];
-  for (int m = threadIdx.x; m < nfp; m += blockDim.x) s_fp[m] = a.fp4[m];
+  const int ntab = EAM && STAGE ? FTAB_W * (nr + 1) : 0;
+  const int nfp = EAM && STAGE ? a.nrho + 1 : 0;
+  const float4 *s_tab = STAGE ? smem : tab, *s_fp = STAGE ? smem + ntab : a.fp4;
+  for (int m = threadIdx.x; m < ntab; m += blockDim.x) smem[m] = tab[m];
+  for (int m = threadIdx.x; m < nfp; m += blockDim.x) smem[ntab + m] = a.fp4[m];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float *s_k = reinterpret_cast<float *>(smem + ntab + nfp) + (size_t) w * FUSED_WARP_FLOATS;
   float *s_r = s_k + 24;
@@ -1953,6 +2146,90 @@ k_elem_force_fused(FusedArgs a, const float4 *__restrict__ tab, int nr, float rd
   if (FIX) band_done(a.band, ne);
 }
 
+// Displacement culling of the fused passes' lists (k_ip_reorder's parts and
+// gate) in one launch: half a warp per element, a lane per row, distances from
+// the element's trilinear coefficients like the passes themselves (rows and
+// lines of packed points, and the line masks that the unfused passes keep, are
+// not needed: five launches a step less, 6 us of a small system's element
+// chain).  Keeps the nodes as the new reference and counts nodes outside the
+// packed-coordinate range (*oob), as the unfused passes do.
+constexpr int FR_BLOCK = 256, FR_STRIDE = 24 * 2 + 22;  // floats per half warp: nodes, coefficients
+
+__global__ void __launch_bounds__(FR_BLOCK)
+k_fused_reorder(const float2 *__restrict__ node_hl, const int *__restrict__ etype,
+                const int *__restrict__ row_first, const int *__restrict__ numint,
+                const int *__restrict__ int_off, const int4 *__restrict__ intp,
+                const float4 *__restrict__ lat_rec, Lattice lat, int maxlines, PackGrid pg,
+                const int *__restrict__ row_start, const int *__restrict__ ent, int nlocal_e,
+                int nall_e, float4 lim, int *__restrict__ ent_near, int4 *__restrict__ nnear_row,
+                float2 *__restrict__ node_ref, unsigned *__restrict__ eflags) {
+  if (moved_little(eflags)) return;  // reads eflags[0] only, which no block writes
+  __shared__ float2 s_mem[FR_BLOCK / 16][FR_STRIDE / 2];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    eflags[1] = 1u;
+    eflags[2] += 1u;  // reorders so far
+  }
+  const int half = threadIdx.x >> 4, hl = threadIdx.x & 15;
+  const unsigned hmask = 0xFFFFu << (threadIdx.x & 16);
+  float2 *s_nx = s_mem[half];
+  float *s_k = reinterpret_cast<float *>(s_nx + 24);
+  const int stride = gridDim.x * (FR_BLOCK / 16);
+  for (int e = blockIdx.x * (FR_BLOCK / 16) + half; e < nlocal_e; e += stride) {
+    const int ty = etype[e], rf = row_first[e], nint = numint[ty];
+    const FusedLat g = fused_lat(lat, lat_rec, ty);
+    for (int k = hl; k < 24; k += 16) {
+      const float2 v = node_hl[24 * (size_t) e + k];
+      s_nx[k] = v;
+      int cell;
+      bool bad = false;
+      const int d = k % 3;
+      rel_of(ds_sub(ds{v.x, v.y}, ds{pg.l0h[d], pg.l0l[d]}), pg.g, pg.ig, d == 0 ? 4095 : 1023, cell, bad);
+      if (bad && pg.oob) atomicAdd(pg.oob, 1);
+    }
+    __syncwarp(hmask);
+    for (int q = hl; q < 21; q += 16) fused_coeffs(s_nx, q, s_k, false);
+    __syncwarp(hmask);
+    for (int jj = hl; jj < nint; jj += 16) {
+      const int r = rf + jj, s0 = row_start[r];
+      const int4 p = intp[int_off[ty] + jj];
+      const float ap = (float) p.x * g.ia, bp = (float) p.y * g.ib, cp = (float) p.z * g.ic;
+      const float abp = ap * bp;
+      const int lbase = e * maxlines;
+      auto index = [&](int k) { return __ldg(ent + s0 + k); };
+      auto fetch = [&](int code) { return code; };
+      auto rsq = [&](int code) {
+        const int L = code_line(lat, code) - lbase, kk = code_kk(lat, code);
+        const int ii = (int) (((float) L + 0.5f) * g.inay), js = L - ii * g.nay;
+        const float da = (float) (p.x - ii) * g.ia, db = (float) (p.y - js) * g.ib,
+                    dc = (float) (p.z - kk) * g.ic;
+        const float dab = fmaf(ap, db, fmaf(bp, da, -da * db));
+        const float dac = fmaf(ap, dc, fmaf(cp, da, -da * dc));
+        const float dbc = fmaf(bp, dc, fmaf(cp, db, -db * dc));
+        const float dabc = fmaf(abp, dc, fmaf(cp, dab, -dab * dc));
+        float q = 0.f;
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          float w = s_k[d] * da;
+          w = fmaf(s_k[3 + d], db, w);
+          w = fmaf(s_k[6 + d], dc, w);
+          w = fmaf(s_k[9 + d], dab, w);
+          w = fmaf(s_k[12 + d], dac, w);
+          w = fmaf(s_k[15 + d], dbc, w);
+          w = fmaf(s_k[18 + d], dabc, w);
+          q = fmaf(w, w, q);
+        }
+        return q;
+      };
+      auto put = [&](int at, int code) { ent_near[s0 + at] = code; };
+      nnear_row[r] = reorder_parts(row_start[r + 1] - s0, lim, index, fetch, rsq, put);
+    }
+    __syncwarp(hmask);  // the half's shared memory is rewritten for its next element
+  }
+  for (long long t = blockIdx.x * (long long) FR_BLOCK + threadIdx.x; t < 24LL * nall_e;
+       t += (long long) gridDim.x * FR_BLOCK)
+    node_ref[t] = node_hl[t];
+}
+
 // every entry of every row references a site of the row's own element:
 // count the entries that do not
 __global__ void k_self_check(const int *__restrict__ row_start, const int *__restrict__ ent,
@@ -2007,6 +2284,18 @@ int persistent_grid(const void *kernel, int threads, size_t smem, long long work
   return (int) (need < g ? (need > 0 ? need : 1) : g);
 }
 
+// Lanes per atom: as many, up to 8, as leave all atoms in one round of the
+// threads that the GPU holds.  Measured, density / force pass: 9,677 atoms with 8
+// lanes 8 / 10 us against 25 / 25 with one; 266,200 atoms with 4 lanes 97 / 91 us
+// against 103 / 87, 1,982,464 with 2 lanes 604 us against 457 (more lanes take
+// the neighbors of fewer atoms together, which lie less close in memory).
+int group_lanes(const void *kernel, int threads, size_t smem, int n) {
+  const long long slots = (long long) threads * persistent_grid(kernel, threads, smem, 1LL << 60);
+  int g = 1;
+  while (g < 8 && 2LL * g * n <= slots) g *= 2;
+  return g;
+}
+
 }  // namespace
 
 PackGrid make_pack_grid(const double l0[3], double g, int *oob) {
@@ -2039,9 +2328,11 @@ void eam_rho_atoms(const MixedAtoms &m, const float4 *rhor_val, const EamTables 
     a.rdrho_ds = make_float2(h, (float) (e.rdrho - (double) h));
   }
   size_t smem = sizeof(float4) * (e.nr + 1);
-  int g = persistent_grid((const void *) k_eam_rho_atoms, m.block, smem, m.nlocal);
-  k_eam_rho_atoms<<<g, m.block, smem, s>>>(a, rhor_val, e.nr, (float) e.rdr, fp4, e.nrho,
-                                           (float) e.rdrho, rho, fp);
+  const int lanes = group_lanes((const void *) k_eam_rho_atoms, m.block, smem, m.nlocal);
+  auto k = lanes == 8 ? k_eam_rho_lanes<8> : lanes == 4 ? k_eam_rho_lanes<4>
+           : lanes == 2 ? k_eam_rho_lanes<2> : k_eam_rho_atoms;
+  int g = persistent_grid((const void *) k, m.block, smem, (long long) m.nlocal * lanes);
+  k<<<g, m.block, smem, s>>>(a, rhor_val, e.nr, (float) e.rdr, fp4, e.nrho, (float) e.rdrho, rho, fp);
   check(cudaGetLastError(), "eam_rho_atoms_mixed");
 }
 
@@ -2121,8 +2412,11 @@ void eam_force_atoms(const MixedAtoms &m, const float4 *ftab, const EamTables &e
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const int block = m.nlocal >= 4LL * nsm * FORCE_BLOCK ? FORCE_BLOCK : m.block;
-  int g = persistent_grid((const void *) k_eam_force_atoms, block, smem, m.nlocal);
-  k_eam_force_atoms<<<g, block, smem, s>>>(a, ftab, e.nr, (float) e.rdr, fp, f);
+  const int lanes = group_lanes((const void *) k_eam_force_atoms, block, smem, m.nlocal);
+  auto k = lanes == 8 ? k_eam_force_lanes<8> : lanes == 4 ? k_eam_force_lanes<4>
+           : lanes == 2 ? k_eam_force_lanes<2> : k_eam_force_atoms;
+  int g = persistent_grid((const void *) k, block, smem, (long long) m.nlocal * lanes);
+  k<<<g, block, smem, s>>>(a, ftab, e.nr, (float) e.rdr, fp, f);
   check(cudaGetLastError(), "eam_force_atoms_mixed");
 }
 
@@ -2131,8 +2425,11 @@ void lj_atoms(const MixedAtoms &m, const int *type, const float *lj1, const floa
   if (m.nlocal <= 0) return;
   AtomArgs a{m.x, m.xq, m.qg, m.num, m.list, m.stride, m.nlocal, m.cutsq_f, m.band_lo,
              m.band_hi, m.cutsq, m.snum, m.slist, nullptr, nullptr};
-  int g = persistent_grid((const void *) k_lj_atoms, m.block, 0, m.nlocal);
-  k_lj_atoms<<<g, m.block, 0, s>>>(a, type, lj1, lj2, cutsq_t, cutsq64, f);
+  const int lanes = group_lanes((const void *) k_lj_atoms, m.block, 0, m.nlocal);
+  auto k = lanes == 8 ? k_lj_lanes<8> : lanes == 4 ? k_lj_lanes<4>
+           : lanes == 2 ? k_lj_lanes<2> : k_lj_atoms;
+  int g = persistent_grid((const void *) k, m.block, 0, (long long) m.nlocal * lanes);
+  k<<<g, m.block, 0, s>>>(a, type, lj1, lj2, cutsq_t, cutsq64, f);
   check(cudaGetLastError(), "lj_atoms_mixed");
 }
 
@@ -2147,12 +2444,12 @@ void node_split(const double *nodex, int n, float2 *hl, const float2 *ref, unsig
 void lines(const float2 *node_hl, const int *etype, const Lattice &lat, int max_nax,
            const unsigned long long *mask, const unsigned long long *mask_near,
            const unsigned *eflags, int maxlines, const PackGrid &pg, int nelem, float4 *line_pos,
-           cudaStream_t s, const unsigned *gate) {
+           cudaStream_t s) {
   if (nelem <= 0) return;
   const size_t smem = sizeof(ds) * 12 * (size_t) max_nax * (LCH / 32);
   const int grid = persistent_grid((const void *) k_lines, LCH, smem, (long long) nelem * 32);
   k_lines<<<grid, LCH, smem, s>>>(node_hl, etype, lat, mask, mask_near, eflags, maxlines, pg,
-                                  nelem, max_nax, line_pos, gate);
+                                  nelem, max_nax, line_pos);
   check(cudaGetLastError(), "lines");
 }
 
@@ -2207,13 +2504,27 @@ void ip_reorder(const int *row_start, const int *ent, int nrows, const float4 *i
   check(cudaGetLastError(), "ip_reorder");
 }
 
+void fused_reorder(const float2 *node_hl, const int *etype, const int *row_first, const int *numint,
+                   const int *int_off, const int4 *intp, const float4 *lat_rec, const Lattice &lat,
+                   int maxlines, const PackGrid &pg, const int *row_start, const int *ent,
+                   int nlocal_e, int nall_e, float cutoff, int *ent_near, int4 *nnear_row,
+                   float2 *node_ref, unsigned *eflags, cudaStream_t s) {
+  if (nlocal_e <= 0) return;
+  const int grid = persistent_grid((const void *) k_fused_reorder, FR_BLOCK, 0, 16LL * nlocal_e);
+  k_fused_reorder<<<grid, FR_BLOCK, 0, s>>>(node_hl, etype, row_first, numint, int_off, intp, lat_rec,
+                                            lat, maxlines, pg, row_start, ent, nlocal_e, nall_e,
+                                            part_limits(cutoff * cutoff, cutoff), ent_near, nnear_row,
+                                            node_ref, eflags);
+  check(cudaGetLastError(), "fused_reorder");
+}
+
 void row_q(const int *row_elem, const int *row_jj, const int *etype, const int *int_off,
            const float2 *spa_int_hl, const float2 *node_hl, int nrows, const PackGrid &pg,
-           float4 *ip_q, float4 *ip_h, float4 *ip_l, cudaStream_t s, const unsigned *gate) {
+           float4 *ip_q, float4 *ip_h, float4 *ip_l, cudaStream_t s) {
   if (nrows <= 0) return;
   const int grid = persistent_grid((const void *) k_row_q, 128, 0, nrows);
   k_row_q<<<grid, 128, 0, s>>>(row_elem, row_jj, etype, int_off, spa_int_hl, node_hl, nrows, pg,
-                               ip_q, ip_h, ip_l, gate);
+                               ip_q, ip_h, ip_l);
   check(cudaGetLastError(), "row_q");
 }
 
@@ -2268,37 +2579,34 @@ void ip_pass(const MixedElems &m, int pass, const float4 *tab, const EamTables &
   check(cudaGetLastError(), "ip_pass_mixed");
 }
 
-template <int V>
+// Blocks of as many warps as spread the elements over all SMs, up to the
+// variant's block (one warp takes one element at a time): 64 elements on 3
+// blocks of 24 warps took 10 us a pass and 23 us a guard-band pass, on 64 one
+// warp blocks half of that.  Below 8 warps a block reads the EAM tables where
+// they are instead of copying them to shared memory.
+template <int V, bool STAGE>
 static void launch_fused(const FusedArgs &a, int pass, const float4 *tab, const EamTables &e,
-                         size_t table, float lj1, float lj2, const double *erho_in,
+                         size_t table, int B, float lj1, float lj2, const double *erho_in,
                          double *erho_out, double *nodef, cudaStream_t s) {
-  constexpr int B = fused_block(V);
-  const size_t smem = table + sizeof(float) * FUSED_WARP_FLOATS * (B / 32);
+  const size_t smem = (STAGE ? table : 0) + sizeof(float) * FUSED_WARP_FLOATS * (B / 32);
   const long long items = (long long) (a.e_end - a.e_begin) * 32;
   // the pass, then the exact pass over the elements it listed (a grid of the
   // same shape; it returns at once when the list is empty)
-  if (pass == 1) {
-    const int g = persistent_grid((const void *) k_elem_rho_fused<V, false>, B, smem, items);
-    k_elem_rho_fused<V, false><<<g, B, smem, s>>>(a, tab, e.nr, (float) e.rdr, erho_out);
-    persistent_grid((const void *) k_elem_rho_fused<V, true>, B, smem, items);
-    k_elem_rho_fused<V, true><<<g, B, smem, s>>>(a, tab, e.nr, (float) e.rdr, erho_out);
-  } else if (pass == 2) {
-    const int g =
-        persistent_grid((const void *) k_elem_force_fused<true, V, false>, B, smem, items);
-    k_elem_force_fused<true, V, false><<<g, B, smem, s>>>(a, tab, e.nr, (float) e.rdr, 0.f, 0.f,
-                                                          erho_in, nodef);
-    persistent_grid((const void *) k_elem_force_fused<true, V, true>, B, smem, items);
-    k_elem_force_fused<true, V, true><<<g, B, smem, s>>>(a, tab, e.nr, (float) e.rdr, 0.f, 0.f,
-                                                         erho_in, nodef);
-  } else {
-    const int g =
-        persistent_grid((const void *) k_elem_force_fused<false, V, false>, B, smem, items);
-    k_elem_force_fused<false, V, false><<<g, B, smem, s>>>(a, nullptr, 0, 0.f, lj1, lj2, nullptr,
-                                                           nodef);
-    persistent_grid((const void *) k_elem_force_fused<false, V, true>, B, smem, items);
-    k_elem_force_fused<false, V, true><<<g, B, smem, s>>>(a, nullptr, 0, 0.f, lj1, lj2, nullptr,
-                                                          nodef);
-  }
+  auto run = [&](auto k, auto fix, auto... args) {
+    const int g = persistent_grid((const void *) k, B, smem, items);
+    k<<<g, B, smem, s>>>(a, args...);
+    persistent_grid((const void *) fix, B, smem, items);
+    fix<<<g, B, smem, s>>>(a, args...);
+  };
+  if (pass == 1)
+    run(k_elem_rho_fused<V, false, STAGE>, k_elem_rho_fused<V, true, STAGE>, tab, e.nr, (float) e.rdr,
+        erho_out);
+  else if (pass == 2)
+    run(k_elem_force_fused<true, V, false, STAGE>, k_elem_force_fused<true, V, true, STAGE>, tab, e.nr,
+        (float) e.rdr, 0.f, 0.f, erho_in, nodef);
+  else
+    run(k_elem_force_fused<false, V, false, true>, k_elem_force_fused<false, V, true, true>,
+        (const float4 *) nullptr, 0, 0.f, lj1, lj2, (const double *) nullptr, nodef);
 }
 
 bool fused_fits(int nr, int nrho) {
@@ -2362,10 +2670,20 @@ void elem_fused(const MixedElems &m, const FusedTables &t, int pass, const float
   const size_t table =
       eam ? sizeof(float4) * ((force ? FTAB_W : 1) * (size_t) (e.nr + 1) + (force ? e.nrho + 1 : 0))
           : 0;
-  if (t.variant == 1) launch_fused<1>(a, pass, tab, e, table, lj1, lj2, erho_in, erho_out, nodef, s);
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int full = t.variant == 0 ? fused_block(0) : fused_block(1);
+  const long long warps = ((long long) (e_end - e_begin) + nsm - 1) / std::max(nsm, 1);
+  const int B = (int) std::min<long long>(full, 32 * std::max(1LL, warps));
+  if (eam && B < 256)  // few elements: one arrangement, tables unstaged
+    launch_fused<1, false>(a, pass, tab, e, table, B, lj1, lj2, erho_in, erho_out, nodef, s);
+  else if (t.variant == 1)
+    launch_fused<1, true>(a, pass, tab, e, table, B, lj1, lj2, erho_in, erho_out, nodef, s);
   else if (t.variant == 2)
-    launch_fused<2>(a, pass, tab, e, table, lj1, lj2, erho_in, erho_out, nodef, s);
-  else launch_fused<0>(a, pass, tab, e, table, lj1, lj2, erho_in, erho_out, nodef, s);
+    launch_fused<2, true>(a, pass, tab, e, table, B, lj1, lj2, erho_in, erho_out, nodef, s);
+  else
+    launch_fused<0, true>(a, pass, tab, e, table, B, lj1, lj2, erho_in, erho_out, nodef, s);
   check(cudaGetLastError(), "elem_fused");
 }
 

@@ -68,17 +68,16 @@ __device__ __forceinline__ void put_copy(const Copies &c, int member, int layer,
 enum { UPDATE_COPY = 0, UPDATE_GRAD = 1, UPDATE_ADAM = 2 };
 
 struct UpdateArgs {
-  float *p, *m, *v, *g;   // [members][NPARAM] (GRAD writes g, ADAM p, m, v)
-  const float *part;      // weight-gradient partial sums [splits][members][NPARAM]
+  float *p, *m, *v, *g;   // [members][NPARAM]; g holds the weight gradients
   const bf16 *gt[4];      // gradients at the layers' outputs, transposed [members * rows][B]
-  int splits, B, first;   // first: member of blockIdx.y == 0
+  int B, first;           // first: member of blockIdx.y == 0
   float lr, b1, b2, eps, bc1, bc2;
   Copies c;
 };
 
-// blockIdx.y: member; the first WB blocks take the weights (a thread each, the
-// partial sums added in order), the others the biases (a warp each, the column
-// sum of the gradient: rows of the transposed array)
+// blockIdx.y: member; the first WB blocks take the weights (a thread each), the
+// others the biases (a warp each: the column sum of the gradient, by 256 rows,
+// of these by eights, in order)
 constexpr int UB = 256;
 constexpr int WB = (int) ((WEIGHTS + UB - 1) / UB), BB = (BIASES + UB / 32 - 1) / (UB / 32);
 
@@ -102,9 +101,7 @@ __global__ void __launch_bounds__(UB) k_update(UpdateArgs a) {
     r = (int) (i / cols);
     col = (int) (i % cols);
     off = (layer == 0 ? oW1 : layer == 1 ? oW2 : layer == 2 ? oW3 : oW4) + i;
-    if (MODE != UPDATE_COPY)
-      for (int s = 0; s < a.splits; s++)
-        g += a.part[((size_t) s * gridDim.y + blockIdx.y) * NPARAM + off];
+    if (MODE != UPDATE_COPY) g = a.g[(size_t) member * NPARAM + off];
   } else {
     const int j = ((int) blockIdx.x - WB) * (UB / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (j >= BIASES) return;
@@ -114,15 +111,19 @@ __global__ void __launch_bounds__(UB) k_update(UpdateArgs a) {
     off = (layer == 0 ? ob1 : layer == 1 ? ob2 : layer == 2 ? ob3 : ob4) + r;
     if (MODE != UPDATE_COPY) {
       const int rows = layer == 3 ? NOUT : NH;
-      const uint4 *q = reinterpret_cast<const uint4 *>(a.gt[layer] +
-                                                       ((size_t) blockIdx.y * rows + r) * a.B);
-      for (int k = lane; k < a.B / 8; k += 32) {
-        const uint4 u = __ldg(q + k);
-        for (unsigned w : {u.x, u.y, u.z, u.w})
-          g += __uint_as_float(w << 16) + __uint_as_float(w & 0xFFFF0000u);
+      const bf16 *q = a.gt[layer] + ((size_t) blockIdx.y * rows + r) * a.B;
+      // four groups of 256 rows at a time, a lane per group and row modulo 8
+      for (int r0 = 0; r0 < a.B; r0 += 1024) {
+        const int first = r0 + (lane >> 3) * 256;
+        float t = 0.f, s = 0.f;
+        for (int k = first + (lane & 7); k < min(first + 256, a.B); k += 8)
+          s += __bfloat162float(q[k]);
+        for (int w = 0; w < 4; w++) {
+          t = 0.f;
+          for (int y = 0; y < 8; y++) t += __shfl_sync(0xffffffffu, s, 8 * w + y);
+          if (r0 + 256 * w < a.B) g += t;
+        }
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
     }
     if (lane != 0) return;
   }
@@ -133,8 +134,8 @@ __global__ void __launch_bounds__(UB) k_update(UpdateArgs a) {
   }
   float p = a.p[at];
   if (MODE == UPDATE_ADAM) {
-    const float mi = a.b1 * a.m[at] + (1.f - a.b1) * g;
-    const float vi = a.b2 * a.v[at] + (1.f - a.b2) * g * g;
+    const float mi = __fmaf_rn(1.f - a.b1, g, __fmul_rn(a.b1, a.m[at]));
+    const float vi = __fmaf_rn(__fmul_rn(1.f - a.b2, g), g, __fmul_rn(a.b2, a.v[at]));
     a.m[at] = mi;
     a.v[at] = vi;
     p -= a.lr * (mi / a.bc1) / (sqrtf(vi / a.bc2) + a.eps);
@@ -218,7 +219,7 @@ struct Net {
   DBuf<bf16> w[4], wt[4];
   // one step's arrays (see gemm::TrainArgs)
   DBuf<bf16> h[4], ht[4], gr[4], grt[4];
-  DBuf<float> z[3], tb, part;
+  DBuf<float> z[3], tb;
   DBuf<double> loss;
   DBuf<int> errflag;
   size_t g4_rows = 0;  // rows of gr[3] whose padding is zero
@@ -292,21 +293,10 @@ struct Net {
     check(cudaGetLastError(), "mlp refresh");
   }
 
-  // the batch in parts of at least 8 k-tiles (512 rows), at most 16 parts: the
-  // weight-gradient blocks of 4 members x 2,048 rows then fill one wave (112
-  // blocks), and a part's sums cost 0.6 MB a member
-  static void split(int B, int &splits, int &tps) {
-    const int nkt = B / 64;
-    tps = std::max(8, (nkt + 15) / 16);
-    splits = (nkt + tps - 1) / tps;
-  }
-
   // `count` members from `first` with B rows each
   gemm::TrainArgs batch(int first, int count, int B, int n_valid) {
     cudaStream_t s = stream;
     const size_t b = (size_t) count * B;
-    int splits, tps;
-    split(B, splits, tps);
     h[0].ensure(b * NINP, s);
     ht[0].ensure(b * NINP, s);
     for (int l = 1; l < 4; l++) {
@@ -324,14 +314,11 @@ struct Net {
     }
     grt[3].ensure(b * NOUT, s);
     tb.ensure(b * NOUT, s);
-    part.ensure((size_t) splits * count * NPARAM, s);
     ensure_err(s);
     gemm::TrainArgs t{};
     t.members = count;
     t.B = B;
     t.n_valid = n_valid;
-    t.splits = splits;
-    t.tps = tps;
     t.p = p.p + (size_t) first * NPARAM;
     t.pstride = NPARAM;
     const long ow[4] = {oW1, oW2, oW3, oW4}, ob[4] = {ob1, ob2, ob3, ob4};
@@ -349,7 +336,7 @@ struct Net {
       if (l < 3) t.z[l] = z[l].p;
     }
     t.tb = tb.p;
-    t.part = part.p;
+    t.grad = g.p + (size_t) first * NPARAM;
     t.err = errflag.p;
     return t;
   }
@@ -371,8 +358,6 @@ struct Net {
   // the members' gradients into g
   void gradients(const gemm::TrainArgs &t, int first) {
     UpdateArgs a = update_args(first);
-    a.part = part.p;
-    a.splits = t.splits;
     a.B = t.B;
     k_update<UPDATE_GRAD><<<dim3(WB + BB, t.members), UB, 0, stream>>>(a);
     check(cudaGetLastError(), "gradients");
@@ -380,8 +365,6 @@ struct Net {
 
   void adam(const gemm::TrainArgs &t, float lr) {
     UpdateArgs a = update_args(0);
-    a.part = part.p;
-    a.splits = t.splits;
     a.B = t.B;
     a.lr = lr;
     a.b1 = 0.9f;
@@ -579,7 +562,7 @@ int cacg_mlp_destroy(cacg_mlp m) {
   cudaSetDevice(m->net.device);
   if (m->net.stream) cudaStreamSynchronize(m->net.stream);
   Net &N = m->net;
-  for (auto *b : {&N.p, &N.m, &N.v, &N.g, &N.bias, &N.d_norm, &N.tb, &N.part}) b->release();
+  for (auto *b : {&N.p, &N.m, &N.v, &N.g, &N.bias, &N.d_norm, &N.tb}) b->release();
   for (int l = 0; l < 4; l++)
     for (auto *b : {&N.w[l], &N.wt[l], &N.h[l], &N.ht[l], &N.gr[l], &N.grt[l]}) b->release();
   for (auto &b : N.z) b.release();
