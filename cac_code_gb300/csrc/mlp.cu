@@ -223,6 +223,17 @@ struct Net {
   DBuf<double> loss;
   DBuf<int> errflag;
   size_t g4_rows = 0;  // rows of gr[3] whose padding is zero
+  // a call's data set and results: kept for the next call (cudaMalloc and
+  // cudaFree of a prediction's buffers cost more than its kernel), unless larger
+  // than KEEP_BYTES
+  DBuf<float> raw, rt, tf, dm, ds;
+  DBuf<bf16> xf;
+  static constexpr size_t KEEP_BYTES = 64u << 20;
+  void trim() {
+    for (DBuf<float> *b : {&raw, &rt, &tf, &dm, &ds})
+      if (b->cap * sizeof(float) > KEEP_BYTES) b->release();
+    if (xf.cap * sizeof(bf16) > KEEP_BYTES) xf.release();
+  }
 
   void sync() { check(cudaStreamSynchronize(stream), "mlp sync"); }
 
@@ -499,26 +510,20 @@ struct Workers {
   ~Workers() { wait(); }
 };
 
-// upload normalised features (bf16 [n][64]) and targets (fp32 [n][24])
-void upload_set(Net &N, const float *x, const float *t, long long n, cacg::DBuf<bf16> &xf,
-                cacg::DBuf<float> &tf) {
+// upload normalised features (bf16 [n][64]) and targets (fp32 [n][24]) into the
+// net's data buffers
+void upload_set(Net &N, const float *x, const float *t, long long n) {
   cudaStream_t s = N.stream;
-  cacg::DBuf<float> raw;
-  raw.ensure((size_t) n * MLP_IN + 1, s);
-  cacg::check(cudaMemcpyAsync(raw.p, x, sizeof(float) * n * MLP_IN, cudaMemcpyHostToDevice, s), "x");
-  xf.ensure((size_t) n * 64 + 64, s);
-  cacg::mlp::features_bf16(raw.p, n, N.d_norm.p, xf.p, s);
+  N.raw.ensure((size_t) n * MLP_IN + 1, s);
+  cacg::check(cudaMemcpyAsync(N.raw.p, x, sizeof(float) * n * MLP_IN, cudaMemcpyHostToDevice, s), "x");
+  N.xf.ensure((size_t) n * 64 + 64, s);
+  cacg::mlp::features_bf16(N.raw.p, n, N.d_norm.p, N.xf.p, s);
   if (t) {
-    cacg::DBuf<float> rt;
-    rt.ensure((size_t) n * MLP_OUT + 1, s);
-    cacg::check(cudaMemcpyAsync(rt.p, t, sizeof(float) * n * MLP_OUT, cudaMemcpyHostToDevice, s), "t");
-    tf.ensure((size_t) n * MLP_OUT + 1, s);
-    cacg::mlp::targets(rt.p, n, N.d_norm.p, tf.p, s);
-    N.sync();
-    rt.release();
+    N.rt.ensure((size_t) n * MLP_OUT + 1, s);
+    cacg::check(cudaMemcpyAsync(N.rt.p, t, sizeof(float) * n * MLP_OUT, cudaMemcpyHostToDevice, s), "t");
+    N.tf.ensure((size_t) n * MLP_OUT + 1, s);
+    cacg::mlp::targets(N.rt.p, n, N.d_norm.p, N.tf.p, s);
   }
-  N.sync();
-  raw.release();
 }
 
 }  // namespace
@@ -562,11 +567,12 @@ int cacg_mlp_destroy(cacg_mlp m) {
   cudaSetDevice(m->net.device);
   if (m->net.stream) cudaStreamSynchronize(m->net.stream);
   Net &N = m->net;
-  for (auto *b : {&N.p, &N.m, &N.v, &N.g, &N.bias, &N.d_norm, &N.tb}) b->release();
+  for (auto *b : {&N.p, &N.m, &N.v, &N.g, &N.bias, &N.d_norm, &N.tb, &N.raw, &N.rt, &N.tf, &N.dm, &N.ds}) b->release();
   for (int l = 0; l < 4; l++)
     for (auto *b : {&N.w[l], &N.wt[l], &N.h[l], &N.ht[l], &N.gr[l], &N.grt[l]}) b->release();
   for (auto &b : N.z) b.release();
   N.loss.release();
+  N.xf.release();
   N.errflag.release();
   if (N.stream) cudaStreamDestroy(N.stream);
   delete m;
@@ -643,13 +649,11 @@ int cacg_mlp_loss_grad(cacg_mlp m, int member, const float *x, const float *t, i
   Net &N = m->net;
   need(x && t && n > 0 && member >= 0 && member < N.members, "bad arguments");
   const int B = (n + 127) / 128 * 128, tiles = B / 128;
-  cacg::DBuf<bf16> xf;
-  cacg::DBuf<float> tf;
-  upload_set(N, x, t, n, xf, tf);
+  upload_set(N, x, t, n);
   const cacg::gemm::TrainArgs ta = N.batch(member, 1, B, n);
   N.loss.ensure(tiles, N.stream);
   Plan plan(ta);
-  N.gather(ta, xf.p, tf.p, nullptr, 0, n);
+  N.gather(ta, N.xf.p, N.tf.p, nullptr, 0, n);
   cacg::gemm::train_passes(*plan.p, N.loss.p, N.stream);
   N.gradients(ta, member);
   std::vector<double> h(tiles);
@@ -663,8 +667,7 @@ int cacg_mlp_loss_grad(cacg_mlp m, int member, const float *x, const float *t, i
                                 cudaMemcpyDeviceToHost, N.stream), "grad");
     N.sync();
   }
-  xf.release();
-  tf.release();
+  N.trim();
   MLP_END
 }
 
@@ -674,8 +677,6 @@ int cacg_mlp_train(cacg_mlp m, const float *x, const float *t, long long n, int 
   Net &N = m->net;
   need(x && t && epochs > 0 && batch >= 128 && batch % 128 == 0 && n >= batch && lr > 0,
        "bad training arguments (batch a positive multiple of 128, n >= batch)");
-  cacg::DBuf<bf16> xf;
-  cacg::DBuf<float> tf;
   const long long nbatch = n / batch;  // whole batches only
   const int members = N.members, tiles = batch / 128;
   // the shuffles of an epoch, member by member from one random sequence: each
@@ -695,7 +696,7 @@ int cacg_mlp_train(cacg_mlp m, const float *x, const float *t, long long n, int 
     for (int k = 0; k < members; k++) workers.run([&shuffle, ep, k] { shuffle(ep, k); });
   };
   start(0);
-  upload_set(N, x, t, n, xf, tf);
+  upload_set(N, x, t, n);
   const cacg::gemm::TrainArgs ta = N.batch(0, members, batch, batch);
   N.loss.ensure((size_t) nbatch * members * tiles, N.stream);
   Plan plan(ta);
@@ -711,7 +712,7 @@ int cacg_mlp_train(cacg_mlp m, const float *x, const float *t, long long n, int 
                                   cudaMemcpyHostToDevice, N.stream), "perm");
     if (ep + 1 < epochs) start(ep + 1);  // into the other buffers
     for (long long b = 0; b < nbatch; b++) {
-      N.gather(ta, xf.p, tf.p, didx.p + b * batch, istride, batch);
+      N.gather(ta, N.xf.p, N.tf.p, didx.p + b * batch, istride, batch);
       cacg::gemm::train_passes(*plan.p, N.loss.p + (size_t) b * members * tiles, N.stream);
       N.adam(ta, lr_ep);
     }
@@ -733,8 +734,7 @@ int cacg_mlp_train(cacg_mlp m, const float *x, const float *t, long long n, int 
     *epoch_loss = lsum / (double) (members * nbatch);
   }
   N.check_err();
-  xf.release();
-  tf.release();
+  N.trim();
   didx.release();
   MLP_END
 }
@@ -743,22 +743,17 @@ int cacg_mlp_predict(cacg_mlp m, const float *x, long long n, float *mean, float
   MLP_BEGIN
   Net &N = m->net;
   need(x && n > 0 && (mean || spread), "bad arguments");
-  cacg::DBuf<bf16> xf;
-  cacg::DBuf<float> tf, dm, ds;
-  upload_set(N, x, nullptr, n, xf, tf);
-  dm.ensure((size_t) n * MLP_OUT, N.stream);
-  ds.ensure((size_t) n, N.stream);
+  upload_set(N, x, nullptr, n);
+  N.dm.ensure((size_t) n * MLP_OUT, N.stream);
+  N.ds.ensure((size_t) n, N.stream);
   N.ensure_err(N.stream);
-  N.predict_device(xf.p, n, dm.p, ds.p, N.stream);
-  N.check_err();
+  N.predict_device(N.xf.p, n, N.dm.p, N.ds.p, N.stream);
   if (mean)
-    cacg::check(cudaMemcpyAsync(mean, dm.p, sizeof(float) * n * MLP_OUT, cudaMemcpyDeviceToHost, N.stream), "mean");
+    cacg::check(cudaMemcpyAsync(mean, N.dm.p, sizeof(float) * n * MLP_OUT, cudaMemcpyDeviceToHost, N.stream), "mean");
   if (spread)
-    cacg::check(cudaMemcpyAsync(spread, ds.p, sizeof(float) * n, cudaMemcpyDeviceToHost, N.stream), "spread");
-  N.sync();
-  xf.release();
-  dm.release();
-  ds.release();
+    cacg::check(cudaMemcpyAsync(spread, N.ds.p, sizeof(float) * n, cudaMemcpyDeviceToHost, N.stream), "spread");
+  N.check_err();  // waits for the copies too
+  N.trim();
   MLP_END
 }
 
