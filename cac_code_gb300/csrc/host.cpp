@@ -418,10 +418,12 @@ struct cacg_context {
   DBuf<unsigned short> d_slot, d_sslot;
   bool ran = false;  // steps taken since init (positions may have left the box)
   bool oob_zeroed = false;  // d_misc[9] (packed-range counter) initialised
-  bool use_graphs = true, graph_ok = true, graph_valid = false;
-  cudaGraphExec_t gexec = nullptr;
-  unsigned long long graph_epoch = 0;
-  long long graph_launches = 0, graph_steps = 0;
+  // captured plain steps: [2 first half-step with the previous step's second,
+  // 1 second half-step left to the next step]
+  bool use_graphs = true, graph_ok = true, graph_valid[4] = {};
+  cudaGraphExec_t gexec[4] = {};
+  unsigned long long graph_epoch[4] = {};
+  long long graph_launches[4] = {}, graph_steps = 0;
   int eager_since = 0;
   // device step loop ("tune loop device|host"): one graph launch runs steps
   // back to back, the rebuild decision taken on the device (a WHILE node
@@ -436,12 +438,12 @@ struct cacg_context {
   long long lgraph_pre = 0, lgraph_post = 0;  // kernels per iteration before / after the decision
   long long loop_launches = 0, host_decisions = 0;
   void invalidate_graph() {
-    graph_valid = false;
+    for (bool &g : graph_valid) g = false;
     hgraph_valid = false;
     lgraph_valid = false;
     eager_since = 0;
   }
-  bool capture_plain_step();
+  bool capture_plain_step(int key);
   void loop_prepare();
   bool add_loop(cudaGraph_t top, long long &pre, long long &post, bool *destroyable);
   bool capture_loop();
@@ -582,6 +584,21 @@ struct cacg_context {
   void setup_bins();
   void borders();
   void forward_comm(int which = 3);  // 1 atoms, 2 elements, 3 both
+  // forward_comm inside a step: the atoms' ghosts take their positions where the
+  // float copies are made (fwd_pending), and ghost elements that no pass reads wait for
+  // the end of the run (eghost_stale)
+  void step_comm(int which = 3);
+  void refresh_eghosts();
+  bool fused_now() const;
+  bool lazy_eghosts() const;
+  bool fwd_pending = false, eghost_stale = false;
+  bool split_done = false;  // the split nodes and their displacement are this step's
+  // the second half-step of a step whose successor in the same run follows at
+  // once is left to that step's first (one kernel for both)
+  bool defer_kick = false, kick_a = false, kick_n = false;
+  void step_final(int which = 3);
+  void flush_kicks();
+  SwapChain swap_chain(bool elems) const;
   void pbc();
   void neighbor_build();
   void neighbor_ebuild();
@@ -635,7 +652,7 @@ struct cacg_context {
   void force_passes(long long b);  // b: phase-mark base of the step, < 0 for none
   void run_host(int n, double *x, double *v, double *nodex, double *nodev);
   bool fork_ok() const {
-    return two_streams && mode == CACG_MIXED && !timing && nlocal > 0 && enlocal > 0;
+    return two_streams && !timing && nlocal > 0 && enlocal > 0;
   }
   template <class A, class E>
   void forked(A atoms, E elems, bool elems_first = false);
@@ -727,7 +744,8 @@ cacg_context::~cacg_context() {
     if (e) cudaEventDestroy(e);
   for (auto &e : pev) cudaEventDestroy(e);
   for (auto &e : kev) cudaEventDestroy(e);
-  if (gexec) cudaGraphExecDestroy(gexec);
+  for (cudaGraphExec_t g : gexec)
+    if (g) cudaGraphExecDestroy(g);
   if (lexec) cudaGraphExecDestroy(lexec);
   if (h_pin) cudaFreeHost(h_pin);
   if (fork_ev) cudaEventDestroy(fork_ev);
@@ -2285,6 +2303,7 @@ void cacg_context::borders_elems() {
     send_total += cnt;
     enghost += cnt;
   }
+  eghost_stale = false;
   // per-element site offsets (types of ghosts from their roots)
   int nall_e = enlocal + enghost;
   if (enlocal) {
@@ -2305,23 +2324,71 @@ void cacg_context::borders_elems() {
   }
 }
 
+SwapChain cacg_context::swap_chain(bool elems) const {
+  SwapChain c{};
+  c.n = (int) swaps.size();
+  for (size_t k = 0; k < swaps.size(); k++) {
+    c.first[k] = elems ? swaps[k].efirstrecv : swaps[k].firstrecv;
+    for (int d = 0; d < 3; d++) c.d[k][d] = swaps[k].d[d];
+  }
+  return c;
+}
+
+// the mixed element pass runs fused (one warp per element)
+bool cacg_context::fused_now() const {
+  return fused_on && self_contained && fused_types_ok &&
+         mixed::fused_fits(pair_style == 2 ? nr : 0, pair_style == 2 ? nrho : 0);
+}
+
+// no pass of a step reads ghost elements: every pair lies inside an element (and
+// mixed passes run fused)
+bool cacg_context::lazy_eghosts() const {
+  return enlocal > 0 && elists_built && codes_ok && self_contained &&
+         (mode != CACG_MIXED || fused_now());
+}
+
+void cacg_context::step_comm(int which) {
+  if (which & 1) {
+    if (nlocal && !swaps.empty() && swaps.size() <= (size_t) MAX_SWAPS) fwd_pending = nghost > 0;
+    else forward_comm(1);
+  }
+  if (which & 2) {
+    if (lazy_eghosts()) eghost_stale = true;
+    else forward_comm(2);
+  }
+}
+
+void cacg_context::refresh_eghosts() {
+  if (eghost_stale) forward_comm(2);
+}
+
+void cacg_context::step_final(int which) {
+  if (!defer_kick) {
+    nve_final(which);
+    return;
+  }
+  if (which & 1) kick_a = true;
+  if (which & 2) kick_n = true;
+}
+
+void cacg_context::flush_kicks() {
+  const int which = (kick_a ? 1 : 0) | (kick_n ? 2 : 0);
+  kick_a = kick_n = false;
+  if (which) nve_final(which);
+}
+
 // CommBrick::forward_comm / eforward_comm: ghost positions from their sources,
 // swap by swap (comm_brick.cpp:1017-1112)
 void cacg_context::forward_comm(int which) {
+  if (which & 1) fwd_pending = false;
+  if (which & 2) eghost_stale = false;
   if (!swaps.empty() && swaps.size() <= (size_t) MAX_SWAPS) {
-    SwapChain ca{}, ce{};
-    ca.n = ce.n = (int) swaps.size();
-    for (size_t k = 0; k < swaps.size(); k++) {
-      ca.first[k] = swaps[k].firstrecv;
-      ce.first[k] = swaps[k].efirstrecv;
-      for (int d = 0; d < 3; d++) ca.d[k][d] = ce.d[k][d] = swaps[k].d[d];
-    }
     if ((which & 1) && nlocal && nghost) {
-      launch_forward_atoms_all(d_x.p, d_send.p, nlocal, nghost, ca, stream);
+      launch_forward_atoms_all(d_x.p, d_send.p, nlocal, nghost, swap_chain(false), stream);
       launches++;
     }
     if ((which & 2) && enlocal && enghost) {
-      launch_forward_elems_all(d_nodex.p, d_esend.p, enlocal, enghost, ce, stream);
+      launch_forward_elems_all(d_nodex.p, d_esend.p, enlocal, enghost, swap_chain(true), stream);
       launches++;
     }
     return;
@@ -2547,7 +2614,9 @@ void cacg_context::pair_compute_pass(int pass) {
   q.f = d_f.p;
   if (pass == 1) {
     d_xh.ensure(nall, s);
-    launch_split_hi(d_x.p, d_xh.p, nall, s);
+    if (fwd_pending) launch_forward_split(d_x.p, d_send.p, nlocal, nghost, swap_chain(false), d_xh.p, s);
+    else launch_split_hi(d_x.p, d_xh.p, nall, s);
+    fwd_pending = false;
     launches++;
   }
   q.xh = d_xh.p;
@@ -2614,9 +2683,15 @@ void cacg_context::pair_compute_mixed(int pass) {
                       ref_l0[1] == l0[1] && ref_l0[2] == l0[2];
     check(cudaMemsetAsync(d_misc.p + 11, 0, 2 * sizeof(int), s), "dmax, reordered");
     if (!same) check(cudaMemsetAsync(d_misc.p + 11, 0x7F, sizeof(int), s), "dmax");
-    mixed::pack_rel(d_x.p, nall, mixed::make_pack_grid(l0, g, d_misc.p + 9), d_xh.p,
-                    same ? d_xq_ref.p : nullptr, nlocal,
-                    reinterpret_cast<unsigned *>(d_misc.p + 11), s);
+    const mixed::PackGrid pg = mixed::make_pack_grid(l0, g, d_misc.p + 9);
+    const float4 *ref = same ? d_xq_ref.p : nullptr;
+    unsigned *dmax = reinterpret_cast<unsigned *>(d_misc.p + 11);
+    if (fwd_pending) {
+      mixed::forward_pack(d_x.p, d_send.p, nlocal, nghost, swap_chain(false), pg, d_xh.p, ref, dmax, s);
+      fwd_pending = false;
+    } else {
+      mixed::pack_rel(d_x.p, nall, pg, d_xh.p, ref, nlocal, dmax, s);
+    }
     launches++;
   }
   m.xq = d_xh.p;
@@ -2720,9 +2795,9 @@ void cacg_context::pair_ecompute_mixed() {
   const mixed::PackGrid pg = mixed::make_pack_grid(l0, g, d_misc.p + 9);
   const long long nmask = (long long) std::max(nall, 1) * std::max(maxlines, 1);
   const EamTables et = pair_style == 2 ? eamtab() : EamTables{};
-  const bool fused = fused_on && self_contained && fused_types_ok &&
-                     mixed::fused_fits(pair_style == 2 ? et.nr : 0, pair_style == 2 ? et.nrho : 0);
+  const bool fused = fused_now();
   fused_used = fused;
+  if (!fused) refresh_eghosts();
   d_node_hl.ensure((size_t) 24 * nall, s);
   // displacement culling of the integration-point lists: slot 13 holds the
   // largest squared node displacement since the last reorder (set huge after
@@ -2740,21 +2815,26 @@ void cacg_context::pair_ecompute_mixed() {
     check(cudaMemsetAsync(d_misc.p + 15, 0, sizeof(int), s), "ereorders");
     ereorders_zeroed = true;
   }
-  check(cudaMemsetAsync(d_misc.p + 13, 0, 2 * sizeof(int), s), "edmax, ereordered");
-  if (!same_e) check(cudaMemsetAsync(d_misc.p + 13, 0x7F, sizeof(int), s), "edmax");
   kmark(KT_SITES, 0);
-  mixed::node_split(d_nodex.p, nall, d_node_hl.p, same_e ? d_node_ref.p : nullptr, eflags, s);
+  if (!(split_done && fused && same_e)) {  // else the first half-step split the nodes
+    check(cudaMemsetAsync(d_misc.p + 13, 0, 2 * sizeof(int), s), "edmax, ereordered");
+    if (!same_e) check(cudaMemsetAsync(d_misc.p + 13, 0x7F, sizeof(int), s), "edmax");
+    mixed::node_split(d_nodex.p, fused ? enlocal : nall, d_node_hl.p, same_e ? d_node_ref.p : nullptr,
+                      eflags, s);
+    launches++;
+  }
+  split_done = false;
   const mixed::Lattice lat{d_nae.p, d_frac.p, fstride, code_kb};
   const double csq_e = pair_style == 1 ? ljtab.cutsq[1 * (MAXT + 1) + 1] : cutforcesq;
   if (fused) {
     kmark(KT_SITES, 1);
     kmark(KT_EPREP, 0);
     mixed::fused_reorder(d_node_hl.p, d_etype.p, d_row_first.p, d_numint.p, d_int_off.p, d_intp4.p,
-                         d_lat_rec.p, lat, maxlines, pg, d_row_start.p, d_ent.p, enlocal, nall,
+                         d_lat_rec.p, lat, maxlines, pg, d_row_start.p, d_ent.p, enlocal, enlocal,
                          (float) std::sqrt(csq_e), d_ent_near.p, d_nnear_row.p, d_node_ref.p, eflags,
                          s);
     kmark(KT_EPREP, 1);
-    launches += 2;
+    launches++;
   } else {
     d_line_pos.ensure(3 * (size_t) nmask, s);
     d_line_mask_n.ensure(nmask, s);
@@ -2776,7 +2856,7 @@ void cacg_context::pair_ecompute_mixed() {
     mixed::line_masks(d_row_start.p, d_ent_near.p, d_nnear_row.p, nrows, lat, d_row_isforce.p,
                       d_line_mask_n.p, d_line_mask_nf.p, nmask, eflags, s);
     kmark(KT_EPREP, 1);
-    launches += 6;
+    launches += 5;
   }
   epart_fused = fused;
   epart_of = elist_builds;
@@ -3050,6 +3130,7 @@ void cacg_context::surrogate_samples(float *x, float *t) {
   sur = nullptr;
   try {
     forward_comm();  // ghosts follow nodes put since the last step
+    split_done = false;
     pair_ecompute();
   } catch (...) {
     sur = keep;
@@ -3333,6 +3414,7 @@ void cacg_context::pair_ecompute() {
 void cacg_context::compute_thermo(double *out) {
   if (!setup_done || (nlocal && !list_built) || (enlocal && !elists_built))
     fail(CACG_ESTATE, "thermo before the neighbor lists are built");
+  refresh_eghosts();
   cudaStream_t s = stream;
   for (int k = 0; k < 17; k++) out[k] = 0.0;
   auto reduce = [&](int nblocks, double *acc) {
@@ -3428,13 +3510,25 @@ void cacg_context::nve_initial(int which) {
   TypeScale a, e;
   nve_scales(a, e);
   if (which & 1) {
-    launch_nve_atoms_initial(d_x.p, d_v.p, d_f.p, d_type.p, a, nlocal, dt, fast(), stream);
+    launch_nve_atoms_initial(d_x.p, d_v.p, d_f.p, d_type.p, a, nlocal, dt, fast(), kick_a ? 2 : 1,
+                             stream);
+    kick_a = false;
     launches++;
   }
   if (which & 2) {
-    launch_nve_nodes_initial(d_ex.p, d_nodex.p, d_nodev.p, d_nodef.p, d_etype.p, e, enlocal, dt, fast(),
-                             stream);
+    const int kicks = kick_n ? 2 : 1;
+    kick_n = false;
     launches++;
+    split_done = mode == CACG_MIXED && lazy_eghosts() && epart_of == elist_builds && epart_fused && ereorders_zeroed;
+    if (split_done) {
+      unsigned *eflags = reinterpret_cast<unsigned *>(d_misc.p + 13);
+      check(cudaMemsetAsync(eflags, 0, 2 * sizeof(int), stream), "edmax, ereordered");
+      mixed::nve_nodes_split(d_ex.p, d_nodex.p, d_nodev.p, d_nodef.p, d_etype.p, e, enlocal, dt, kicks,
+                             d_node_hl.p, d_node_ref.p, eflags, stream);
+    } else {
+      launch_nve_nodes_initial(d_ex.p, d_nodex.p, d_nodev.p, d_nodef.p, d_etype.p, e, enlocal, dt,
+                               fast(), kicks, stream);
+    }
   }
 }
 
@@ -3506,6 +3600,7 @@ void cacg_context::rebuild(int flags) {
   check_packed_range();
   nrebuild++;
   invalidate_graph();
+  split_done = fwd_pending = false;
   if (!rb_ev[0]) {
     check(cudaEventCreate(&rb_ev[0]), "event");
     check(cudaEventCreate(&rb_ev[1]), "event");
@@ -3572,7 +3667,10 @@ void cacg_context::run(int n) {
   const size_t P = 6;  // phase marks per step
   std::fill(kev_used.begin(), kev_used.end(), 0);
   cur_step = 0;
+  try {
   for (int step = 0; step < n; step++) {
+    // (nothing between two steps of this loop reads the velocities)
+    defer_kick = step + 1 < n && !timing && !deform_on && !(loop_device && use_graphs && graph_ok);
     // the device loop runs the steps it can; it hands back a step that must
     // run here first (after set-up or a rebuild: first-call allocations and
     // read-backs stay outside the capture), and all steps once its capture
@@ -3592,16 +3690,14 @@ void cacg_context::run(int n) {
     const bool plain = !(ago + 1 >= delay && (ago + 1) % every == 0);
     if (plain && use_graphs && graph_ok && !deform_on) {
       ago++;
-      if (graph_valid && graph_epoch == dbuf_epoch()) {
-        check(cudaGraphLaunch(gexec, stream), "graph launch");
-        launches += graph_launches;
+      const int key = (kick_a || kick_n ? 2 : 0) | (defer_kick ? 1 : 0);
+      if ((graph_valid[key] && graph_epoch[key] == dbuf_epoch()) ||
+          (eager_since >= 1 && capture_plain_step(key))) {
+        check(cudaGraphLaunch(gexec[key], stream), "graph launch");
+        launches += graph_launches[key];
         graph_steps++;
-        continue;
-      }
-      if (eager_since >= 1 && capture_plain_step()) {
-        check(cudaGraphLaunch(gexec, stream), "graph launch");
-        launches += graph_launches;
-        graph_steps++;
+        kick_a = kick_n = defer_kick;
+        eghost_stale = eghost_stale || lazy_eghosts();
         continue;
       }
       mark(b);
@@ -3610,26 +3706,26 @@ void cacg_context::run(int n) {
         forked(
             [&] {
               nve_initial(1);
-              forward_comm(1);
+              step_comm(1);
               pair_compute_pass(1);
               pair_compute_pass(2);
             },
             [&] {
               nve_initial(2);
-              forward_comm(2);
+              step_comm(2);
               pair_ecompute();
-              if (nodes_done) nve_final(2);  // no fix acts on the forces in between
+              if (nodes_done) step_final(2);  // no fix acts on the forces in between
             });
         post_force();
-        nve_final(nodes_done ? 1 : 3);
+        step_final(nodes_done ? 1 : 3);
       } else {
         nve_initial();
-        forward_comm();
+        step_comm();
         mark(b + 1);
         force_passes((long long) b);
         post_force();
         mark(b + 4);
-        nve_final();
+        step_final();
         mark(b + 5);
       }
       eager_since++;
@@ -3638,17 +3734,28 @@ void cacg_context::run(int n) {
     mark(b);
     nve_initial();
     int nflag = decide();
-    if (nflag == 0) forward_comm();
+    if (nflag == 0) step_comm();
     else rebuild(nflag);
     mark(b + 1);
     force_passes((long long) b);
     post_force();  // verlet.cpp:206
     mark(b + 4);
-    nve_final();
+    step_final();
     deform_step();
     mark(b + 5);
     if (nflag == 0) eager_since++;  // every pass of a plain step has run eagerly
   }
+  } catch (...) {  // the state as the steps done leave it
+    defer_kick = false;
+    try {
+      flush_kicks();
+    } catch (...) {
+    }
+    throw;
+  }
+  defer_kick = false;
+  flush_kicks();
+  refresh_eghosts();
   // the packed-range counter is read back behind the last step, so that one
   // synchronisation serves both
   const bool oob_read = mode == CACG_MIXED && d_misc.p && oob_zeroed;
@@ -3788,7 +3895,7 @@ void cacg_context::run_host(int n, double *x, double *v, double *nodex, double *
   d_stage.ensure(3 * (size_t) std::max(nlocal, 1), stream);
   const long long ago_last = (long long) ago + n - 1;
   const bool last_plain = !(ago_last + 1 >= delay && (ago_last + 1) % every == 0);
-  const bool overlap = fork_ok() && setup_done && list_built && elists_built && !deform_on;
+  const bool overlap = mode == CACG_MIXED && fork_ok() && setup_done && list_built && elists_built && !deform_on;
   const size_t xb = sizeof(double) * 3 * (size_t) nlocal, nb = sizeof(double) * 24 * (size_t) enlocal;
   if (!overlap) {
     cudaStream_t s = stream;
@@ -3895,7 +4002,7 @@ void cacg_context::run_host(int n, double *x, double *v, double *nodex, double *
         launch_check_distance(d_x.p, d_xhold.p, nlocal, nullptr, nullptr, 0, nullptr, box,
                               triggersq, d_misc.p + 6, stream);
         check(cudaEventRecord(ev_acheck, stream), "atom check");
-        forward_comm(1);
+        step_comm(1);
         pair_compute_pass(1);
         pair_compute_pass(2);
         check(cudaEventRecord(ev_apass, stream), "atom passes");
@@ -3919,7 +4026,7 @@ void cacg_context::run_host(int n, double *x, double *v, double *nodex, double *
       check(cudaEventRecord(ev_nxout, stream), "nodex final");
       if (nflag == 0) {
         early = true;
-        forward_comm(2);
+        step_comm(2);
         out_split = true;
         parts_done = 1;
         try {
@@ -3964,7 +4071,7 @@ void cacg_context::run_host(int n, double *x, double *v, double *nodex, double *
       }
       nve_initial();
       const int nflag = decide();
-      if (nflag == 0) forward_comm();
+      if (nflag == 0) step_comm();
       else rebuild(nflag);
       check(cudaEventRecord(ev_xout, stream), "x final");
       check(cudaEventRecord(ev_nxout, stream), "nodex final");
@@ -3982,7 +4089,7 @@ void cacg_context::run_host(int n, double *x, double *v, double *nodex, double *
             }
             nve_initial(1);
             check(cudaEventRecord(ev_xout, stream), "x final");
-            forward_comm(1);
+            step_comm(1);
             pair_compute_pass(1);
             pair_compute_pass(2);
             if (early_nodes) {  // the atoms' velocities go out while the elements run
@@ -3994,7 +4101,7 @@ void cacg_context::run_host(int n, double *x, double *v, double *nodex, double *
             check(cudaStreamWaitEvent(stream, ev_nin, 0), "wait nodes in");
             nve_initial(2);
             check(cudaEventRecord(ev_nxout, stream), "nodex final");
-            forward_comm(2);
+            step_comm(2);
             out_split = early_nodes;
             parts_done = 1;
             try {
@@ -4057,6 +4164,7 @@ void cacg_context::run_host(int n, double *x, double *v, double *nodex, double *
     check(cudaStreamWaitEvent(stream, ev_hdone, 0), "copy-out join");
   };
   auto finish = [&] {
+    refresh_eghosts();
     check(cudaStreamSynchronize(stream), "host step");
     if (oob_read && h_pin[9]) {
       const int nout = h_pin[9];
@@ -4090,6 +4198,7 @@ void cacg_context::run_host(int n, double *x, double *v, double *nodex, double *
     launches += hgraph_launches;
     check(cudaGraphLaunch(hexec, stream), "host step graph");
     graph_steps++;
+    eghost_stale = eghost_stale || lazy_eghosts();
     finish();
     return;
   }
@@ -4251,19 +4360,19 @@ bool cacg_context::add_loop(cudaGraph_t top, long long &pre, long long &post, bo
         const bool nodes_done = post_fixes.empty();
         forked(
             [&] {
-              forward_comm(1);
+              step_comm(1);
               pair_compute_pass(1);
               pair_compute_pass(2);
             },
             [&] {
-              forward_comm(2);
+              step_comm(2);
               pair_ecompute();
               if (nodes_done) nve_final(2);
             });
         post_force();
         nve_final(nodes_done ? 1 : 3);
       } else {
-        forward_comm();
+        step_comm();
         force_passes(-1);
         post_force();
         nve_final();
@@ -4278,6 +4387,7 @@ bool cacg_context::add_loop(cudaGraph_t top, long long &pre, long long &post, bo
     ok = false;
   }
   capturing = false;
+  split_done = fwd_pending = false;
   launches = l0;
   cudaGetLastError();  // a failed capture leaves its error behind
   return ok;
@@ -4340,6 +4450,7 @@ int cacg_context::loop_finish(int want, long long pre, long long post) {
   ntimestep += steps;
   graph_steps += steps;
   launches += pre * iters + post * steps;
+  eghost_stale = eghost_stale || lazy_eghosts();
   if (flags) {  // the step after those: initial integration and decision done
     ntimestep++;
     cur_step = (size_t) steps;
@@ -4380,7 +4491,7 @@ int cacg_context::run_loop(int n) {
 // The body of a step without a rebuild decision, captured into a CUDA graph.
 // Anything that would allocate or synchronise ends the capture with an error;
 // the step then runs eagerly and graphs stay off for this handle.
-bool cacg_context::capture_plain_step() {
+bool cacg_context::capture_plain_step(int key) {
   cudaStream_t s = stream;
   upload_masks();  // host-to-device copies stay outside the capture
   if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
@@ -4391,6 +4502,7 @@ bool cacg_context::capture_plain_step() {
   const long long l0 = launches;
   const unsigned long long e0 = dbuf_epoch();
   bool ok = true;
+  const bool ka = kick_a, kn = kick_n;
   capturing = true;
   try {
     if (fork_ok()) {
@@ -4398,24 +4510,24 @@ bool cacg_context::capture_plain_step() {
       forked(
           [&] {
             nve_initial(1);
-            forward_comm(1);
+            step_comm(1);
             pair_compute_pass(1);
             pair_compute_pass(2);
           },
           [&] {
             nve_initial(2);
-            forward_comm(2);
+            step_comm(2);
             pair_ecompute();
-            if (nodes_done) nve_final(2);  // no fix acts on the forces in between
+            if (nodes_done) step_final(2);  // no fix acts on the forces in between
           });
       post_force();
-      nve_final(nodes_done ? 1 : 3);
+      step_final(nodes_done ? 1 : 3);
     } else {
       nve_initial();
-      forward_comm();
+      step_comm();
       force_passes(-1);
       post_force();
-      nve_final();
+      step_final();
     }
   } catch (...) {
     ok = false;
@@ -4432,14 +4544,17 @@ bool cacg_context::capture_plain_step() {
     if (ex) cudaGraphExecDestroy(ex);
     graph_ok = false;
     launches = l0;
+    kick_a = ka;
+    kick_n = kn;
+    split_done = fwd_pending = false;
     return false;
   }
-  if (gexec) cudaGraphExecDestroy(gexec);
-  gexec = ex;
-  graph_launches = launches - l0;
+  if (gexec[key]) cudaGraphExecDestroy(gexec[key]);
+  gexec[key] = ex;
+  graph_launches[key] = launches - l0;
   launches = l0;
-  graph_epoch = dbuf_epoch();
-  graph_valid = true;
+  graph_epoch[key] = dbuf_epoch();
+  graph_valid[key] = true;
   return true;
 }
 
@@ -4706,6 +4821,7 @@ int cacg_pair_compute(cacg_handle h, int eflag, int vflag) {
 
 int cacg_pair_ecompute(cacg_handle h) {
   API_BEGIN
+  h->split_done = false;
   h->pair_ecompute();
   h->sync();
   API_END
@@ -4823,6 +4939,12 @@ int cacg_run_batch(cacg_handle *hs, int nh, int nsteps) {
         EpochScope es(&cur->epoch);
         left[k] -= cur->loop_finish(left[k], pre[k], post[k]);
       }
+    }
+    for (int k = 0; k < nh; k++) {
+      cur = hs[k];
+      EpochScope es(&cur->epoch);
+      cur->refresh_eghosts();
+      cur->sync();
     }
     return CACG_OK;
   } catch (const ApiError &e) {
@@ -4956,6 +5078,7 @@ int cacg_get_elements(cacg_handle h, int all, double *centre, double *nodex, dou
                       double *nodef, int *tag) {
   API_BEGIN
   if (!h->inited) fail(CACG_ESTATE, "no device state yet (cacg_init)");
+  if (all) h->refresh_eghosts();
   int n = all ? h->enlocal + h->enghost : h->enlocal;
   cudaStream_t s = h->stream;
   if (centre && n) check(cudaMemcpyAsync(centre, h->d_ex.p, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, s), "ex");

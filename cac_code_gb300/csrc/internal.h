@@ -144,6 +144,10 @@ void launch_border_scatter_elems(double *ex, double *nodex, int *etype, int *eta
                                  int *sendlist, const int *flags, const int *pos, int nfirst,
                                  int nlast, int n0, double dx, double dy, double dz,
                                  cudaStream_t s);
+// dt/(2m) by type
+struct TypeScale {
+  double v[MAXT + 1];
+};
 // the swaps of a forward communication: first ghost index and shift of each
 constexpr int MAX_SWAPS = 8;
 struct SwapChain {
@@ -192,6 +196,8 @@ void launch_elem_list(const double *ex, const int *bin, const int *bstart, const
                       int *overflow, cudaStream_t s);
 // site_h (may be null): float copy of each site for the FP32 pre-tests
 void launch_split_hi(const double4 *x, float4 *xh, int n, cudaStream_t s);
+void launch_forward_split(double4 *x, const int *send, int nlocal, int nghost, const SwapChain &c,
+                          float4 *xh, cudaStream_t s);
 void launch_sub_centres(const double *nodex, int nelem, ElemTables t, double4 *subc,
                         cudaStream_t s);
 void launch_ip_list(const double *nodex, const double *ex, const int *etype,
@@ -394,6 +400,13 @@ void pack_rel(const double4 *x, int n, const PackGrid &pg, float4 *xq, const flo
 // with ref: the largest squared node displacement against ref -> *dmax2 (atomic max)
 void node_split(const double *nodex, int n, float2 *hl, const float2 *ref, unsigned *dmax2,
                 cudaStream_t s);
+// the nodes' first half-step with node_split of the moved nodes
+void nve_nodes_split(double *ex, double *nodex, double *nodev, const double *nodef, const int *etype,
+                     const TypeScale &dtfm, int n, double dtv, int kicks, float2 *hl,
+                     const float2 *ref, unsigned *dmax2, cudaStream_t s);
+// the ghosts' positions (as launch_forward_atoms_all) and pack_rel of all atoms
+void forward_pack(double4 *x, const int *send, int nlocal, int nghost, const SwapChain &c,
+                  const PackGrid &pg, float4 *xq, const float4 *ref, unsigned *dmax2, cudaStream_t s);
 // Lattice lines: U, D (double-single, relative to l0) of every line that
 // mask (mask_near while culling holds) marks; FP32 nodal-density lines
 void lines(const float2 *node_hl, const int *etype, const Lattice &lat, int max_nax,
@@ -601,19 +614,17 @@ void to_float(const double *src, long long n, float *dst, cudaStream_t s);
 // ---- integration and reductions (k_nve.cu) ----
 // dtf / m per type (FixNVE's dtfm, fix_nve.cpp:54-99), the same IEEE quotient
 // the host forms: no FP64 division per atom on the device
-struct TypeScale {
-  double v[MAXT + 1];
-};
 // fused: one FMA per update (FP64 FMA and mixed modes); else the exact mode's
-// multiply-then-add
+// multiply-then-add.  kicks: half-steps before the positions move (2: the
+// previous step's second half-step was left to this one)
 void launch_nve_atoms_initial(double4 *x, double *v, const double *f, const int *type,
-                              const TypeScale &dtfm, int n, double dtv, bool fused,
+                              const TypeScale &dtfm, int n, double dtv, bool fused, int kicks,
                               cudaStream_t s);
 void launch_nve_atoms_final(double *v, const double *f, const int *type, const TypeScale &dtfm,
                             int n, bool fused, cudaStream_t s);
 void launch_nve_nodes_initial(double *ex, double *nodex, double *nodev, const double *nodef,
                               const int *etype, const TypeScale &dtfm, int n, double dtv,
-                              bool fused, cudaStream_t s);
+                              bool fused, int kicks, cudaStream_t s);
 // fix setforce / fix viscous on the items (atoms, or elements x 8 nodes) whose
 // group mask has `bit` (fix_setforce.cpp:107-161, fix_viscous.cpp:73-123)
 void launch_setforce(double *f, const int *mask, int n, int per_item, int bit, const int *set,

@@ -8,6 +8,7 @@
 // the reference's x + pbc*prd arithmetic.  Bins are a counting sort whose
 // members are re-sorted by index, reproducing the forward-linked bin lists of
 // Neighbor::bin_atoms (neighbor.cpp:656-674).
+#include "ghosts.cuh"
 #include "internal.h"
 
 namespace cacg {
@@ -198,35 +199,12 @@ __global__ void k_forward_elems(double *__restrict__ nodex, const int *__restric
   nodex[24 * (first + m) + r] = nodex[24 * send[m] + r] + d;
 }
 
-// All swaps of a forward communication in one launch: each ghost follows its
-// chain of sources back to the owned item (ghost g was sent from
-// send[g - nfirst], an owned item or an earlier swap's ghost) and applies the
-// swaps' shifts in the order the swaps ran, so every ghost value is the same
-// sum of the same doubles as swap-by-swap communication.
-__device__ __forceinline__ int swap_of(const SwapChain &c, int g) {
-  int w = 0;
-  for (int k = 1; k < c.n; k++)
-    if (g >= c.first[k]) w = k;
-  return w;
-}
-
+// All swaps of a forward communication in one launch (ghosts.cuh).
 __global__ void k_forward_atoms_all(double4 *__restrict__ x, const int *__restrict__ send,
                                     int nlocal, int nghost, SwapChain c) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nghost) return;
-  int chain[MAX_SWAPS], depth = 0, src = nlocal + t;
-  while (src >= nlocal && depth < MAX_SWAPS) {
-    chain[depth++] = swap_of(c, src);
-    src = send[src - nlocal];
-  }
-  double4 p = x[src];
-  for (int k = depth - 1; k >= 0; k--) {
-    const int w = chain[k];
-    p.x = p.x + c.d[w][0];
-    p.y = p.y + c.d[w][1];
-    p.z = p.z + c.d[w][2];
-  }
-  x[nlocal + t] = p;
+  x[nlocal + t] = ghost_position(x, c, send, nlocal, nlocal + t);
 }
 
 __global__ void k_forward_elems_all(double *__restrict__ nodex, const int *__restrict__ send,
@@ -234,11 +212,8 @@ __global__ void k_forward_elems_all(double *__restrict__ nodex, const int *__res
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nghost * 24) return;
   const int m = t / 24, r = t % 24, dim = r % 3;
-  int chain[MAX_SWAPS], depth = 0, src = nlocal + m;
-  while (src >= nlocal && depth < MAX_SWAPS) {
-    chain[depth++] = swap_of(c, src);
-    src = send[src - nlocal];
-  }
+  int chain[MAX_SWAPS], depth;
+  const int src = ghost_chain(c, send, nlocal, nlocal + m, chain, depth);
   double v = nodex[24 * (size_t) src + r];
   for (int k = depth - 1; k >= 0; k--) v = v + c.d[chain[k]][dim];
   nodex[24 * (size_t) (nlocal + m) + r] = v;

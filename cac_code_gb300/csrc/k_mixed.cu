@@ -18,7 +18,9 @@
 #include <algorithm>
 #include <vector>
 
+#include "ghosts.cuh"
 #include "internal.h"
+#include "nve.cuh"
 
 namespace cacg {
 namespace mixed {
@@ -372,7 +374,10 @@ k_eam_rho_atoms(AtomArgs a, const float4 *__restrict__ rhor_val, int nr, float r
 // Small systems: G lanes per atom (group_lanes), the same sums bit for bit.  A
 // lane takes whole chunks of 8 pairs, and the chunk sums are added in the
 // chunks' order, which every lane of the atom follows by shuffles.  The density
-// pass numbers the entries in range by a ballot into the short list first.
+// pass numbers the entries in range by a ballot into the short list first.  The
+// tables are read in place: copying 32 to 64 KB per block is most of such a pass.
+constexpr int LANES_BLOCK = 128;
+
 template <int G>
 __device__ __forceinline__ void add_chunks(dsacc &acc, float part, int first) {
 #pragma unroll
@@ -380,13 +385,10 @@ __device__ __forceinline__ void add_chunks(dsacc &acc, float part, int first) {
 }
 
 template <int G>
-__global__ void __launch_bounds__(512, 2)
+__global__ void __launch_bounds__(LANES_BLOCK)
 k_eam_rho_lanes(AtomArgs a, const float4 *__restrict__ rhor_val, int nr, float rdr,
                 const float4 *__restrict__ fp4, int nrho, float rdrho,
                 double *__restrict__ rho, float *__restrict__ fp) {
-  extern __shared__ float4 s_val[];
-  for (int m = threadIdx.x; m <= nr; m += blockDim.x) s_val[m] = rhor_val[m];
-  __syncthreads();
   const int level = a.nnear ? cull_level(a.dmax2) : 4;
   const int lane = threadIdx.x & 31, g = lane & (G - 1), first = lane & ~(G - 1);
   const unsigned below = (1u << g) - 1u;
@@ -429,7 +431,7 @@ k_eam_rho_lanes(AtomArgs a, const float4 *__restrict__ rhor_val, int nr, float r
           const float rsq = dx * dx + dy * dy + dz * dz;
           float p;
           const int m = findex(sqrtf(rsq), rdr, nr, p);
-          const float4 v = s_val[m];
+          const float4 v = __ldg(rhor_val + m);
           part += ((v.x * p + v.y) * p + v.z) * p + v.w;
         }
       add_chunks<G>(acc, part, first);
@@ -786,12 +788,9 @@ k_eam_force_atoms(AtomArgs a, const float4 *__restrict__ ftab, int nr, float rdr
 
 // G lanes per atom, a chunk of 8 pairs each (see k_eam_rho_lanes)
 template <int G>
-__global__ void __launch_bounds__(512, 1)
+__global__ void __launch_bounds__(LANES_BLOCK)
 k_eam_force_lanes(AtomArgs a, const float4 *__restrict__ ftab, int nr, float rdr,
                   const float *__restrict__ fp, double *__restrict__ f) {
-  extern __shared__ float4 s_tab[];  // FTAB_W float4 per knot
-  for (int m = threadIdx.x; m < FTAB_W * (nr + 1); m += blockDim.x) s_tab[m] = ftab[m];
-  __syncthreads();
   const int lane = threadIdx.x & 31, g = lane & (G - 1), first = lane & ~(G - 1);
   const int step = (int) (gridDim.x * blockDim.x) / G;
   for (int ib = (int) ((blockIdx.x * blockDim.x + threadIdx.x) & ~31u) / G; ib < a.nlocal; ib += step) {
@@ -823,7 +822,7 @@ k_eam_force_lanes(AtomArgs a, const float4 *__restrict__ ftab, int nr, float rdr
           float p;
           int m = findex(r, rdr, nr, p);
           float rhoip, z2, z2p;
-          force_spline(s_tab, m, p, rdr, rhoip, z2, z2p);
+          force_spline(ftab, m, p, rdr, rhoip, z2, z2p);
           float phi = z2 * recip;
           float phip = z2p * recip - phi * recip;
           float psip = (fpi + fpj) * rhoip + phip;
@@ -905,7 +904,7 @@ k_lj_atoms(AtomArgs a, const int *__restrict__ type, const float *__restrict__ l
 
 // G lanes per atom, a chunk of 8 list entries each (see k_eam_rho_lanes)
 template <int G>
-__global__ void __launch_bounds__(512, 2)
+__global__ void __launch_bounds__(LANES_BLOCK)
 k_lj_lanes(AtomArgs a, const int *__restrict__ type, const float *__restrict__ lj1,
            const float *__restrict__ lj2, const float *__restrict__ cutsq_t,
            const double *__restrict__ cutsq64, double *__restrict__ f) {
@@ -1045,17 +1044,26 @@ __device__ __forceinline__ float4 pack_u(ds ux, ds uy, ds uz, const PackGrid &pg
 
 // packed coordinates; with a reference (the packed coordinates of the list
 // reorder, same grid) the largest squared displacement of the first nref
-// atoms is folded into *dmax2 (float bits, one atomic max per block)
+// atoms is folded into *dmax2 (float bits, one atomic max per block).
+// FORWARD: the ghosts (from nref on) take their owners' positions first
 constexpr int PACK_BLOCK = 256;
 
+template <bool FORWARD>
 __global__ void __launch_bounds__(PACK_BLOCK)
-k_pack_rel(const double4 *__restrict__ x, int n, PackGrid pg, float4 *__restrict__ xq,
-           const float4 *__restrict__ ref, int nref, unsigned *__restrict__ dmax2) {
+k_pack_rel(double4 *__restrict__ x, int n, PackGrid pg, float4 *__restrict__ xq,
+           const float4 *__restrict__ ref, int nref, unsigned *__restrict__ dmax2,
+           const int *__restrict__ send, SwapChain chain) {
   __shared__ unsigned s_max[PACK_BLOCK / 32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned m = 0u;
   if (i < n) {
-    const double4 p = x[i];
+    double4 p;
+    if (FORWARD && i >= nref) {
+      p = ghost_position(x, chain, send, nref, i);
+      x[i] = p;
+    } else {
+      p = x[i];
+    }
     const float4 q = pack_u(ds_sub(ds_of_double(p.x), ds{pg.l0h[0], pg.l0l[0]}),
                             ds_sub(ds_of_double(p.y), ds{pg.l0h[1], pg.l0l[1]}),
                             ds_sub(ds_of_double(p.z), ds{pg.l0h[2], pg.l0l[2]}), pg);
@@ -1076,6 +1084,58 @@ k_pack_rel(const double4 *__restrict__ x, int n, PackGrid pg, float4 *__restrict
       m = __reduce_max_sync(0xffffffffu, m);
       if (threadIdx.x == 0 && m) atomicMax(dmax2, m);
     }
+  }
+}
+
+// The nodes' first half-step (k_nve_nodes_initial with fused multiply-adds)
+// with the split of the moved nodes and their largest displacement
+// (k_node_split): the fused passes read the split nodes of owned elements only,
+// so the positions need not be read again.
+template <int KICKS>
+__global__ void __launch_bounds__(SPLIT_BLOCK)
+k_nve_nodes_split(double *__restrict__ ex, double *__restrict__ nodex, double *__restrict__ nodev,
+                  const double *__restrict__ nodef, const int *__restrict__ etype, TypeScale dtfm_t,
+                  int n, double dtv, float2 *__restrict__ hl, const float2 *__restrict__ ref,
+                  unsigned *__restrict__ dmax2) {
+  constexpr int ELEMS = SPLIT_BLOCK / NPE;
+  __shared__ double sx[ELEMS][3 * NPE + 1];
+  __shared__ unsigned s_max[SPLIT_BLOCK / 32];
+  const long long t = blockIdx.x * (long long) SPLIT_BLOCK + threadIdx.x;
+  const long long i = t >> 3;
+  const int q = (int) (t & 7), le = threadIdx.x >> 3;
+  float d2 = 0.f;
+  if (i < n) {
+    const double dtfm = type_scale(dtfm_t, etype[i]);
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const size_t k = 24 * (size_t) i + 3 * q + d;
+      const double vv = kick<true, KICKS>(nodev[k], dtfm, nodef[k]);
+      nodev[k] = vv;
+      const double xn = madd<true>(nodex[k], dtv, vv);
+      nodex[k] = xn;
+      sx[le][3 * q + d] = xn;
+      const ds v = ds_of_double(xn);
+      hl[k] = make_float2(v.h, v.l);
+      const float2 r = ref[k];
+      const float dd = __fsub_rn(v.h, r.x) + __fsub_rn(v.l, r.y);
+      d2 += dd * dd;
+    }
+  }
+  const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(d2));
+  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = m;
+  __syncthreads();
+  const long long e = blockIdx.x * (long long) ELEMS + threadIdx.x;
+  if (threadIdx.x < ELEMS && e < n) {
+    for (int d = 0; d < 3; d++) {
+      double c = 0.0;
+      for (int r = 0; r < NPE; r++) c += sx[threadIdx.x][3 * r + d];
+      ex[3 * e + d] = c / NPE;
+    }
+  }
+  if (threadIdx.x < 32) {
+    unsigned w = threadIdx.x < SPLIT_BLOCK / 32 ? s_max[threadIdx.x] : 0u;
+    w = __reduce_max_sync(0xffffffffu, w);
+    if (threadIdx.x == 0 && w) atomicMax(dmax2, w);
   }
 }
 
@@ -2313,8 +2373,27 @@ PackGrid make_pack_grid(const double l0[3], double g, int *oob) {
 void pack_rel(const double4 *x, int n, const PackGrid &pg, float4 *xq, const float4 *ref, int nref,
               unsigned *dmax2, cudaStream_t s) {
   if (n <= 0) return;
-  k_pack_rel<<<nblk(n, PACK_BLOCK), PACK_BLOCK, 0, s>>>(x, n, pg, xq, ref, nref, dmax2);
+  k_pack_rel<false><<<nblk(n, PACK_BLOCK), PACK_BLOCK, 0, s>>>(
+      const_cast<double4 *>(x), n, pg, xq, ref, nref, dmax2, nullptr, SwapChain{});
   check(cudaGetLastError(), "pack_rel");
+}
+
+void forward_pack(double4 *x, const int *send, int nlocal, int nghost, const SwapChain &c,
+                  const PackGrid &pg, float4 *xq, const float4 *ref, unsigned *dmax2, cudaStream_t s) {
+  const int n = nlocal + nghost;
+  if (n <= 0) return;
+  k_pack_rel<true><<<nblk(n, PACK_BLOCK), PACK_BLOCK, 0, s>>>(x, n, pg, xq, ref, nlocal, dmax2, send, c);
+  check(cudaGetLastError(), "forward_pack");
+}
+
+void nve_nodes_split(double *ex, double *nodex, double *nodev, const double *nodef, const int *etype,
+                     const TypeScale &dtfm, int n, double dtv, int kicks, float2 *hl,
+                     const float2 *ref, unsigned *dmax2, cudaStream_t s) {
+  if (n <= 0) return;
+  auto k = kicks == 2 ? k_nve_nodes_split<2> : k_nve_nodes_split<1>;
+  k<<<nblk((long long) n * NPE, SPLIT_BLOCK), SPLIT_BLOCK, 0, s>>>(ex, nodex, nodev, nodef, etype, dtfm,
+                                                                  n, dtv, hl, ref, dmax2);
+  check(cudaGetLastError(), "nve_nodes_split");
 }
 
 void eam_rho_atoms(const MixedAtoms &m, const float4 *rhor_val, const EamTables &e,
@@ -2331,8 +2410,10 @@ void eam_rho_atoms(const MixedAtoms &m, const float4 *rhor_val, const EamTables 
   const int lanes = group_lanes((const void *) k_eam_rho_atoms, m.block, smem, m.nlocal);
   auto k = lanes == 8 ? k_eam_rho_lanes<8> : lanes == 4 ? k_eam_rho_lanes<4>
            : lanes == 2 ? k_eam_rho_lanes<2> : k_eam_rho_atoms;
-  int g = persistent_grid((const void *) k, m.block, smem, (long long) m.nlocal * lanes);
-  k<<<g, m.block, smem, s>>>(a, rhor_val, e.nr, (float) e.rdr, fp4, e.nrho, (float) e.rdrho, rho, fp);
+  const int block = lanes > 1 ? LANES_BLOCK : m.block;
+  if (lanes > 1) smem = 0;
+  int g = persistent_grid((const void *) k, block, smem, (long long) m.nlocal * lanes);
+  k<<<g, block, smem, s>>>(a, rhor_val, e.nr, (float) e.rdr, fp4, e.nrho, (float) e.rdrho, rho, fp);
   check(cudaGetLastError(), "eam_rho_atoms_mixed");
 }
 
@@ -2411,10 +2492,14 @@ void eam_force_atoms(const MixedAtoms &m, const float4 *ftab, const EamTables &e
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const int block = m.nlocal >= 4LL * nsm * FORCE_BLOCK ? FORCE_BLOCK : m.block;
+  int block = m.nlocal >= 4LL * nsm * FORCE_BLOCK ? FORCE_BLOCK : m.block;
   const int lanes = group_lanes((const void *) k_eam_force_atoms, block, smem, m.nlocal);
   auto k = lanes == 8 ? k_eam_force_lanes<8> : lanes == 4 ? k_eam_force_lanes<4>
            : lanes == 2 ? k_eam_force_lanes<2> : k_eam_force_atoms;
+  if (lanes > 1) {
+    block = LANES_BLOCK;
+    smem = 0;
+  }
   int g = persistent_grid((const void *) k, block, smem, (long long) m.nlocal * lanes);
   k<<<g, block, smem, s>>>(a, ftab, e.nr, (float) e.rdr, fp, f);
   check(cudaGetLastError(), "eam_force_atoms_mixed");
@@ -2428,8 +2513,9 @@ void lj_atoms(const MixedAtoms &m, const int *type, const float *lj1, const floa
   const int lanes = group_lanes((const void *) k_lj_atoms, m.block, 0, m.nlocal);
   auto k = lanes == 8 ? k_lj_lanes<8> : lanes == 4 ? k_lj_lanes<4>
            : lanes == 2 ? k_lj_lanes<2> : k_lj_atoms;
-  int g = persistent_grid((const void *) k, m.block, 0, (long long) m.nlocal * lanes);
-  k<<<g, m.block, 0, s>>>(a, type, lj1, lj2, cutsq_t, cutsq64, f);
+  const int block = lanes > 1 ? LANES_BLOCK : m.block;
+  int g = persistent_grid((const void *) k, block, 0, (long long) m.nlocal * lanes);
+  k<<<g, block, 0, s>>>(a, type, lj1, lj2, cutsq_t, cutsq64, f);
   check(cudaGetLastError(), "lj_atoms_mixed");
 }
 

@@ -10,6 +10,7 @@
 //     at once and a ballot compacts the hits in the reference's site order.
 // Lists are column-major (entry k of row i at k*stride + i) so that the force
 // kernels, one thread per row, read them coalesced.
+#include "ghosts.cuh"
 #include "internal.h"
 
 namespace cacg {
@@ -121,6 +122,21 @@ __global__ void k_split_hi(const double4 *__restrict__ x, float4 *__restrict__ x
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double4 p = x[i];
+  xh[i] = make_float4((float) p.x, (float) p.y, (float) p.z, 0.f);
+}
+
+// the ghosts' positions (ghosts.cuh) with the float copies of all atoms
+__global__ void k_forward_split(double4 *__restrict__ x, const int *__restrict__ send, int nlocal,
+                                int nall, SwapChain c, float4 *__restrict__ xh) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nall) return;
+  double4 p;
+  if (i >= nlocal) {
+    p = ghost_position(x, c, send, nlocal, i);
+    x[i] = p;
+  } else {
+    p = x[i];
+  }
   xh[i] = make_float4((float) p.x, (float) p.y, (float) p.z, 0.f);
 }
 
@@ -307,6 +323,14 @@ void launch_split_hi(const double4 *x, float4 *xh, int n, cudaStream_t s) {
   if (n <= 0) return;
   k_split_hi<<<nblk(n, 256), 256, 0, s>>>(x, xh, n);
   check(cudaGetLastError(), "split_hi");
+}
+
+void launch_forward_split(double4 *x, const int *send, int nlocal, int nghost, const SwapChain &c,
+                          float4 *xh, cudaStream_t s) {
+  const int n = nlocal + nghost;
+  if (n <= 0) return;
+  k_forward_split<<<nblk(n, 256), 256, 0, s>>>(x, send, nlocal, n, c, xh);
+  check(cudaGetLastError(), "forward_split");
 }
 
 void launch_sub_centres(const double *nodex, int nelem, ElemTables t, double4 *subc,

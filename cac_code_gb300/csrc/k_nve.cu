@@ -3,6 +3,7 @@
 // updates are the reference's own multiply-then-add sequences (FixNVE,
 // fix_nve.cpp:54-242); the other modes fuse them explicitly.
 #include "internal.h"
+#include "nve.cuh"
 
 namespace cacg {
 
@@ -10,28 +11,10 @@ namespace {
 
 inline int nblk(long long n, int t) { return (int) ((n + t - 1) / t); }
 
-// dt/(2m) of a type: a select over constant indices, so that the table stays
-// in the parameter space (a runtime index into a by-value parameter array
-// would copy it to each thread's local memory)
-__device__ __forceinline__ double type_scale(const TypeScale &t, int ty) {
-  double d = t.v[0];
-#pragma unroll
-  for (int k = 1; k <= MAXT; k++) d = ty == k ? t.v[k] : d;
-  return d;
-}
-
-// a + b * c: the reference's multiply-then-add, or one fused multiply-add in
-// the FP64 (FMA) and mixed modes (FP64 instructions are scarce on this GPU:
-// the integrators are bound by their FP64 issue, not by HBM)
-template <bool FUSED>
-__device__ __forceinline__ double madd(double a, double b, double c) {
-  return FUSED ? fma(b, c, a) : a + b * c;
-}
-
 // FixNVE::initial_integrate, fix_nve.cpp:54-98 (per-type mass branch).  One
 // thread per component, so the v and f loads of a warp are 256 contiguous
 // bytes; x is the padded double4 array.
-template <bool FUSED>
+template <bool FUSED, int KICKS>
 __global__ void k_nve_atoms_initial(double4 *__restrict__ x, double *__restrict__ v,
                                     const double *__restrict__ f, const int *__restrict__ type,
                                     TypeScale dtfm_t, int n, double dtv) {
@@ -39,7 +22,7 @@ __global__ void k_nve_atoms_initial(double4 *__restrict__ x, double *__restrict_
   if (t >= 3LL * n) return;
   const long long i = t / 3;
   const int d = (int) (t - 3 * i);
-  const double vv = madd<FUSED>(v[t], type_scale(dtfm_t, type[i]), f[t]);
+  const double vv = kick<FUSED, KICKS>(v[t], type_scale(dtfm_t, type[i]), f[t]);
   v[t] = vv;
   double *xp = reinterpret_cast<double *>(x) + 4 * i + d;
   *xp = madd<FUSED>(*xp, dtv, vv);
@@ -63,7 +46,7 @@ __global__ void k_nve_atoms_final(double *__restrict__ v, const double *__restri
 // keeps the FP64 additions at 24 per element).
 static_assert(NPE == 8, "eight nodes per element");
 constexpr int NODE_BLOCK = 256, NODE_ELEMS = NODE_BLOCK / NPE;
-template <bool FUSED>
+template <bool FUSED, int KICKS>
 __global__ void __launch_bounds__(NODE_BLOCK)
 k_nve_nodes_initial(double *__restrict__ ex, double *__restrict__ nodex,
                     double *__restrict__ nodev, const double *__restrict__ nodef,
@@ -76,7 +59,7 @@ k_nve_nodes_initial(double *__restrict__ ex, double *__restrict__ nodex,
     const double dtfm = type_scale(dtfm_t, etype[i]);
     for (int d = 0; d < 3; d++) {
       const size_t k = 24 * (size_t) i + 3 * q + d;
-      const double vv = madd<FUSED>(nodev[k], dtfm, nodef[k]);
+      const double vv = kick<FUSED, KICKS>(nodev[k], dtfm, nodef[k]);
       nodev[k] = vv;
       const double xn = madd<FUSED>(nodex[k], dtv, vv);
       nodex[k] = xn;
@@ -212,9 +195,10 @@ __global__ void k_fma_loop(double *out, int iters) {
 
 void launch_nve_atoms_initial(double4 *x, double *v, const double *f, const int *type,
                               const TypeScale &dtfm, int n, double dtv, bool fused,
-                              cudaStream_t s) {
+                              int kicks, cudaStream_t s) {
   if (n <= 0) return;
-  auto k = fused ? k_nve_atoms_initial<true> : k_nve_atoms_initial<false>;
+  auto k = kicks == 2 ? (fused ? k_nve_atoms_initial<true, 2> : k_nve_atoms_initial<false, 2>)
+                      : (fused ? k_nve_atoms_initial<true, 1> : k_nve_atoms_initial<false, 1>);
   k<<<nblk(3LL * n, 256), 256, 0, s>>>(x, v, f, type, dtfm, n, dtv);
   check(cudaGetLastError(), "nve_atoms_initial");
 }
@@ -229,9 +213,10 @@ void launch_nve_atoms_final(double *v, const double *f, const int *type, const T
 
 void launch_nve_nodes_initial(double *ex, double *nodex, double *nodev, const double *nodef,
                               const int *etype, const TypeScale &dtfm, int n, double dtv,
-                              bool fused, cudaStream_t s) {
+                              bool fused, int kicks, cudaStream_t s) {
   if (n <= 0) return;
-  auto k = fused ? k_nve_nodes_initial<true> : k_nve_nodes_initial<false>;
+  auto k = kicks == 2 ? (fused ? k_nve_nodes_initial<true, 2> : k_nve_nodes_initial<false, 2>)
+                      : (fused ? k_nve_nodes_initial<true, 1> : k_nve_nodes_initial<false, 1>);
   k<<<nblk((long long) n * NPE, NODE_BLOCK), NODE_BLOCK, 0, s>>>(ex, nodex, nodev, nodef, etype,
                                                                   dtfm, n, dtv);
   check(cudaGetLastError(), "nve_nodes_initial");
