@@ -216,6 +216,12 @@ struct cacg_context {
   DBuf<float> d_wn;             // weight x shape function per type row and node (FP32)
   DBuf<float> d_wnf;            // the same for the rows of nonzero weight, per type in order
   DBuf<int> d_band;             // elements with a guard-band pair: count, blocks done, list
+  // the shared stencil of the mixed EAM element passes: its rows and slots (ints),
+  // entries, least distances, counts, state
+  DBuf<int> d_sten_rows, d_sten_num, d_sten_state;
+  DBuf<float4> d_sten_mono;
+  DBuf<unsigned> d_sten_min;
+  int sten_slots = 0, sten_force = 0;
   DBuf<float4> d_lat_rec;       // per type 1/(n_a-1), 1/(n_b-1), 1/(n_c-1), 1/n_b
   int fstride = 1;
   // mixed precision, per row: packed and double-single integration points,
@@ -250,7 +256,8 @@ struct cacg_context {
   // element's coefficients in registers (0, 512 threads a block), read from
   // shared memory at every entry (1, 768 threads: more warps per SM; at C5
   // 2.48 against 3.18 ms for the force pass), or as 1 with two entries in
-  // flight per lane (2)
+  // flight per lane (2).  With 1, EAM passes over many elements take the shared
+  // stencil (elem_stencil.cuh; sums in another order)
   int fused_variant = 1;
   // half-width of the guard band of the mixed cutoff decisions ("tune band")
   float band_eps = 1.0e-4f;
@@ -689,6 +696,11 @@ cacg_context::~cacg_context() {
   d_fipf.release();
   d_wn.release();
   d_wnf.release();
+  d_sten_rows.release();
+  d_sten_num.release();
+  d_sten_state.release();
+  d_sten_mono.release();
+  d_sten_min.release();
   d_band.release();
   d_lat_rec.release();
   d_ip_q.release();
@@ -1820,6 +1832,28 @@ void cacg_context::element_tables() {
     for (int j = fjj_off[t]; j < fjj_off[t + 1]; j++)
       for (int q = 0; q < NPE; q++) wnf[(size_t) j * NPE + q] = wn[((size_t) int_off[t] + fjj[j]) * NPE + q];
   upload(d_wnf, wnf, s);
+  // the shared stencil's slots: the distinct rows of nonzero weight and of the nodes
+  sten_slots = 0;
+  if (netypes == 1 && fused_types_ok && pair_style == 2 && inter_num[1] <= 4096) {
+    std::vector<int> rows, slot;
+    auto add = [&](int jj) {
+      size_t q = std::find(rows.begin(), rows.end(), jj) - rows.begin();
+      if (q == rows.size()) rows.push_back(jj);
+      slot.push_back((int) q);
+    };
+    for (int j = fjj_off[1]; j < fjj_off[2]; j++) add(fjj[j]);
+    sten_force = (int) slot.size();
+    for (int q = 0; q < NPE; q++) add(node_list[NPE + q]);
+    sten_slots = (int) rows.size();
+    rows.insert(rows.end(), slot.begin(), slot.end());
+    upload(d_sten_rows, rows, s);
+    d_sten_num.ensure(sten_slots, s);
+    d_sten_mono.ensure(2 * (size_t) sten_slots * mixed::STENCIL_CAP, s);
+    d_sten_min.ensure((size_t) sten_slots * mixed::STENCIL_CAP, s);
+    d_sten_state.ensure(mixed::STENCIL_STATE, s);
+    check(cudaMemsetAsync(d_sten_state.p, 0, 6 * sizeof(int), s), "stencil state");
+    check(cudaMemsetAsync(d_sten_state.p + 6, 0x80, 42 * sizeof(int), s), "stencil ranges");
+  }
   if (fjj.empty()) fjj.push_back(0);
   upload(d_fjj, fjj, s);
   upload(d_fjj_off, fjj_off, s);
@@ -2826,15 +2860,22 @@ void cacg_context::pair_ecompute_mixed() {
   split_done = false;
   const mixed::Lattice lat{d_nae.p, d_frac.p, fstride, code_kb};
   const double csq_e = pair_style == 1 ? ljtab.cutsq[1 * (MAXT + 1) + 1] : cutforcesq;
+  mixed::Stencil stencil{};
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (fused && sten_slots && pair_style == 2 && enlocal > mixed::STENCIL_PER_SM * nsm)
+    stencil = mixed::Stencil{d_sten_rows.p, d_sten_rows.p + sten_slots, sten_slots, sten_force,
+                             inter_num[1], d_sten_mono.p, d_sten_min.p, d_sten_num.p, d_sten_state.p};
   if (fused) {
     kmark(KT_SITES, 1);
     kmark(KT_EPREP, 0);
     mixed::fused_reorder(d_node_hl.p, d_etype.p, d_row_first.p, d_numint.p, d_int_off.p, d_intp4.p,
                          d_lat_rec.p, lat, maxlines, pg, d_row_start.p, d_ent.p, enlocal, enlocal,
                          (float) std::sqrt(csq_e), d_ent_near.p, d_nnear_row.p, d_node_ref.p, eflags,
-                         s);
+                         stencil, s);
     kmark(KT_EPREP, 1);
-    launches++;
+    launches += stencil.state ? 2 : 1;
   } else {
     d_line_pos.ensure(3 * (size_t) nmask, s);
     d_line_mask_n.ensure(nmask, s);
@@ -2867,9 +2908,6 @@ void cacg_context::pair_ecompute_mixed() {
   if (mixed_ip_group) {
     m.group = mixed_ip_group;
   } else {
-    int dev = 0, nsm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const long long want = (long long) nsm * 2048;
     m.group = (long long) nforce * 4 >= want ? 4 : (long long) nforce * 8 >= want ? 8 : 16;
   }
@@ -2899,7 +2937,7 @@ void cacg_context::pair_ecompute_mixed() {
     mixed::FusedTables ft{d_node_hl.p, d_nodex.p, d_int_off.p, d_inter_off.p, d_intp4.p,
                           d_spa_int.p, d_spa_inter.p, d_fjj.p, d_fjj_off.p, d_wn.p, maxlines,
                           fused_variant, d_spa_int_hl.p, d_frho_ds.p, d_wnf.p, d_band.p,
-                          d_lat_rec.p};
+                          d_lat_rec.p, use_sur ? mixed::Stencil{} : stencil};
     // the surrogate's nodal forces go in before the force pass, which skips
     // (writes nothing for) the elements the surrogate evaluates
     auto sur_write = [&] {

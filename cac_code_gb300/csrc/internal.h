@@ -430,6 +430,22 @@ void line_masks(const int *row_start, const int *ent, const int4 *nnear_row, int
 // densities) or the rows of nonzero weight with the nodal gather (pass 2: EAM
 // forces; pass 0: LJ), pair vectors from the element's trilinear coefficient
 // vectors and lattice-index differences; guard-band pairs are decided in FP64
+// The shared stencil of the mixed EAM element passes (elem_stencil.cuh), for the
+// distinct rows of nonzero weight and of the nodes (slots).  state null: not in use.
+// From more than 24 elements an SM on: up to there the passes from the lists take one
+// round of their warps (3,072 elements: 7.1 and 17.9 us for densities and forces
+// against 9.0 and 23.3 from the stencil), beyond it two (4,096: 11.4 and 32.3 against
+// 9.6 and 23.3; 64,000: 89.8 and 277 against 34.9 and 137).
+constexpr int STENCIL_CAP = 256, STENCIL_STATE = 48, STENCIL_PER_SM = 24;
+struct Stencil {
+  const int *rows;    // the row of each slot
+  const int *slot;    // slots of the nf rows of nonzero weight, then of the 8 node rows
+  int ns, nf, nsites;
+  float4 *mono;       // [slot][STENCIL_CAP][2]: monomial differences a, b, c, ab | ac, bc, abc
+  unsigned *minsq;    // [slot][STENCIL_CAP]: least squared distance at the reorder (float bits)
+  int *num;           // [slot]: entries
+  int *state;         // valid, counters, the coefficients' ranges (ST_*)
+};
 struct FusedTables {
   const float2 *node_hl;      // split nodes of this step
   const double *nodex;        // FP64 nodes
@@ -447,6 +463,7 @@ struct FusedTables {
   int *band;                  // guard-band list: count, blocks done, elements re-run so
                               // far, then the listed elements (3 + nlocal_e ints, zeroed once)
   const float4 *lat_rec;      // per type 1/(n_a-1), 1/(n_b-1), 1/(n_c-1), 1/n_b
+  Stencil stencil;
 };
 bool fused_fits(int nr, int nrho);
 // elements [e_begin, e_end) (e_end < 0: all local elements); the guard-band
@@ -500,7 +517,7 @@ void fused_reorder(const float2 *node_hl, const int *etype, const int *row_first
                    const int *int_off, const int4 *intp, const float4 *lat_rec, const Lattice &lat,
                    int maxlines, const PackGrid &pg, const int *row_start, const int *ent,
                    int nlocal_e, int nall_e, float cutoff, int *ent_near, int4 *nnear_row,
-                   float2 *node_ref, unsigned *eflags, cudaStream_t s);
+                   float2 *node_ref, unsigned *eflags, const Stencil &st, cudaStream_t s);
 void row_q(const int *row_elem, const int *row_jj, const int *etype, const int *int_off,
            const float2 *spa_int_hl, const float2 *node_hl, int nrows, const PackGrid &pg,
            float4 *ip_q, float4 *ip_h, float4 *ip_l, cudaStream_t s);

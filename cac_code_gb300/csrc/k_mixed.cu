@@ -1748,6 +1748,7 @@ __device__ __forceinline__ float4 lds_v4(const float4 *p) {
 // the double-single shape functions, nodal densities (erds) and spline
 // coefficients: the FP32 value of the FP64 result, without an FP64
 // instruction (also *rho32, rho rounded to FP32)
+template <int STRIDE = 1>
 __device__ __forceinline__ float row_fprime_ds(const float2 *__restrict__ N,
                                                const float2 *__restrict__ erds,
                                                const float2 *__restrict__ c3, int nrho,
@@ -1755,7 +1756,7 @@ __device__ __forceinline__ float row_fprime_ds(const float2 *__restrict__ N,
   ds rho = ds{0.f, 0.f};
 #pragma unroll
   for (int k = 0; k < NPE; k++)
-    rho = ds_madd(ds{N[k].x, N[k].y}, ds{erds[k].x, erds[k].y}, rho);
+    rho = ds_madd(ds{N[k].x, N[k].y}, ds{erds[STRIDE * k].x, erds[STRIDE * k].y}, rho);
   rho32 = rho.h + rho.l;
   return fprime_ds(rho, c3, nrho, rdrho);
 }
@@ -2011,9 +2012,8 @@ __device__ __forceinline__ void band_done(int *band, int ne) {
 // STAGE: the spline tables in shared memory; otherwise read where they are
 // (few elements: their blocks would each copy 32 to 96 KB first)
 template <int V, bool FIX, bool STAGE>
-__global__ void __launch_bounds__(fused_block(V), 1)
-k_elem_rho_fused(FusedArgs a, const float4 *__restrict__ tab, int nr, float rdr,
-                 double *__restrict__ erho) {
+__device__ __forceinline__ void elem_rho_body(const FusedArgs &a, const float4 *__restrict__ tab, int nr,
+                                              float rdr, double *__restrict__ erho) {
   const int ne = FIX ? min(a.band[0], a.nlocal_e) : a.e_end - a.e_begin;
   if (FIX && ne == 0) return;  // the whole grid (the count is the same for every block)
   extern __shared__ float4 smem[];
@@ -2075,14 +2075,21 @@ k_elem_rho_fused(FusedArgs a, const float4 *__restrict__ tab, int nr, float rdr,
   }
   if (FIX) band_done(a.band, ne);
 }
+template <int V, bool FIX, bool STAGE>
+__global__ void __launch_bounds__(fused_block(V), 1)
+k_elem_rho_fused(FusedArgs a, const float4 *__restrict__ tab, int nr, float rdr,
+                 double *__restrict__ erho) {
+  elem_rho_body<V, FIX, STAGE>(a, tab, nr, rdr, erho);
+}
 
 // Forces of the element's rows of nonzero weight and their gather onto the
 // nodes (EAM with the nodal densities and row F'(rho), or LJ)
 // (FIX: the listed elements, guard-band pairs decided in FP64)
 template <bool EAM, int V, bool FIX, bool STAGE>
-__global__ void __launch_bounds__(fused_block(V), 1)
-k_elem_force_fused(FusedArgs a, const float4 *__restrict__ tab, int nr, float rdr, float lj1,
-                   float lj2, const double *__restrict__ erho, double *__restrict__ nodef) {
+__device__ __forceinline__ void elem_force_body(const FusedArgs &a, const float4 *__restrict__ tab, int nr,
+                                                float rdr, float lj1, float lj2,
+                                                const double *__restrict__ erho,
+                                                double *__restrict__ nodef) {
   const int ne = FIX ? min(a.band[0], a.nlocal_e) : a.e_end - a.e_begin;
   if (FIX && ne == 0) return;  // the whole grid (the count is the same for every block)
   extern __shared__ float4 smem[];
@@ -2205,6 +2212,14 @@ k_elem_force_fused(FusedArgs a, const float4 *__restrict__ tab, int nr, float rd
   }
   if (FIX) band_done(a.band, ne);
 }
+template <bool EAM, int V, bool FIX, bool STAGE>
+__global__ void __launch_bounds__(fused_block(V), 1)
+k_elem_force_fused(FusedArgs a, const float4 *__restrict__ tab, int nr, float rdr, float lj1,
+                   float lj2, const double *__restrict__ erho, double *__restrict__ nodef) {
+  elem_force_body<EAM, V, FIX, STAGE>(a, tab, nr, rdr, lj1, lj2, erho, nodef);
+}
+
+#include "elem_stencil.cuh"
 
 // Displacement culling of the fused passes' lists (k_ip_reorder's parts and
 // gate) in one launch: half a warp per element, a lane per row, distances from
@@ -2222,9 +2237,14 @@ k_fused_reorder(const float2 *__restrict__ node_hl, const int *__restrict__ etyp
                 const float4 *__restrict__ lat_rec, Lattice lat, int maxlines, PackGrid pg,
                 const int *__restrict__ row_start, const int *__restrict__ ent, int nlocal_e,
                 int nall_e, float4 lim, int *__restrict__ ent_near, int4 *__restrict__ nnear_row,
-                float2 *__restrict__ node_ref, unsigned *__restrict__ eflags) {
+                float2 *__restrict__ node_ref, unsigned *__restrict__ eflags, Stencil st) {
   if (moved_little(eflags)) return;  // reads eflags[0] only, which no block writes
   __shared__ float2 s_mem[FR_BLOCK / 16][FR_STRIDE / 2];
+  // the range of every coefficient over the elements, for the stencil
+  __shared__ int s_range[42], s_last;
+  float kmin[2] = {INFINITY, INFINITY}, kmax[2] = {-INFINITY, -INFINITY};
+  for (int q = threadIdx.x; q < 42; q += FR_BLOCK) s_range[q] = INT_MIN;
+  __syncthreads();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     eflags[1] = 1u;
     eflags[2] += 1u;  // reorders so far
@@ -2249,6 +2269,12 @@ k_fused_reorder(const float2 *__restrict__ node_hl, const int *__restrict__ etyp
     __syncwarp(hmask);
     for (int q = hl; q < 21; q += 16) fused_coeffs(s_nx, q, s_k, false);
     __syncwarp(hmask);
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+      if (hl + 16 * h < 21) {
+        kmin[h] = fminf(kmin[h], s_k[hl + 16 * h]);
+        kmax[h] = fmaxf(kmax[h], s_k[hl + 16 * h]);
+      }
     for (int jj = hl; jj < nint; jj += 16) {
       const int r = rf + jj, s0 = row_start[r];
       const int4 p = intp[int_off[ty] + jj];
@@ -2288,6 +2314,23 @@ k_fused_reorder(const float2 *__restrict__ node_hl, const int *__restrict__ etyp
   for (long long t = blockIdx.x * (long long) FR_BLOCK + threadIdx.x; t < 24LL * nall_e;
        t += (long long) gridDim.x * FR_BLOCK)
     node_ref[t] = node_hl[t];
+  if (!st.state) return;
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+    if (hl + 16 * h < 21) {
+      atomicMax(s_range + hl + 16 * h, ordered_int(kmax[h]));
+      atomicMax(s_range + 21 + hl + 16 * h, ordered_int(-kmin[h]));
+    }
+  __syncthreads();
+  if (threadIdx.x < 42) atomicMax(st.state + ST_RANGE + threadIdx.x, s_range[threadIdx.x]);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(st.state + ST_BUILT, 1) == (int) gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  float *s_k0 = reinterpret_cast<float *>(s_mem);
+  stencil_build(st, fused_lat(lat, lat_rec, 1), intp + int_off[1], lim, s_k0, s_k0 + 32);
 }
 
 // every entry of every row references a site of the row's own element:
@@ -2333,8 +2376,16 @@ int persistent_grid(const void *kernel, int threads, size_t smem, long long work
     }
   if (!hit) {
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    if (smem > 48 * 1024) {
+      // as much as the device allows: a limit set to this launch's size would refuse
+      // a larger launch of the kernel that is in the cache already
+      int optin = 0;
+      cudaFuncAttributes at;
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+      cudaFuncGetAttributes(&at, kernel);
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           optin - (int) at.sharedSizeBytes);
+    }
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem);
     cache.push_back(Key{kernel, threads, smem, dev, nsm, occ});
   }
@@ -2594,13 +2645,18 @@ void fused_reorder(const float2 *node_hl, const int *etype, const int *row_first
                    const int *int_off, const int4 *intp, const float4 *lat_rec, const Lattice &lat,
                    int maxlines, const PackGrid &pg, const int *row_start, const int *ent,
                    int nlocal_e, int nall_e, float cutoff, int *ent_near, int4 *nnear_row,
-                   float2 *node_ref, unsigned *eflags, cudaStream_t s) {
+                   float2 *node_ref, unsigned *eflags, const Stencil &st, cudaStream_t s) {
   if (nlocal_e <= 0) return;
   const int grid = persistent_grid((const void *) k_fused_reorder, FR_BLOCK, 0, 16LL * nlocal_e);
   k_fused_reorder<<<grid, FR_BLOCK, 0, s>>>(node_hl, etype, row_first, numint, int_off, intp, lat_rec,
                                             lat, maxlines, pg, row_start, ent, nlocal_e, nall_e,
                                             part_limits(cutoff * cutoff, cutoff), ent_near, nnear_row,
-                                            node_ref, eflags);
+                                            node_ref, eflags, st);
+  if (st.state) {
+    const int g2 = persistent_grid((const void *) k_stencil_check, 256, 0, nlocal_e);
+    k_stencil_check<<<g2, 256, 0, s>>>(st, node_hl, row_first, nnear_row, nlocal_e,
+                                       part_limits(cutoff * cutoff, cutoff), eflags);
+  }
   check(cudaGetLastError(), "fused_reorder");
 }
 
@@ -2665,17 +2721,67 @@ void ip_pass(const MixedElems &m, int pass, const float4 *tab, const EamTables &
   check(cudaGetLastError(), "ip_pass_mixed");
 }
 
+// entries staged, for a mean of at most 128 a row, and shared memory of a stencil pass
+static int stencil_cap(const Stencil &st, int pass) { return 128 * (pass == 1 ? NPE : st.nf); }
+
+static size_t stencil_smem(const Stencil &st, int pass, int teams) {
+  return sizeof(float) * STENCIL_ENT * (size_t) stencil_cap(st, pass) +
+         sizeof(float2) * (size_t) teams * team_float2(pass == 1 ? 0 : st.nf);
+}
+
+static bool stencil_fits(const Stencil &st, int pass) {
+  int dev = 0, optin = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  return stencil_smem(st, pass, STENCIL_TEAMS) + 1024 <= (size_t) optin;  // and the static part
+}
+
+// teams as many as spread the elements over all SMs, at most three a block
+static void launch_stencil(const FusedArgs &a, const Stencil &st, int pass, const float4 *tab,
+                           const EamTables &e, size_t lists_smem, const double *erho_in,
+                           double *erho_out, double *nodef, cudaStream_t s) {
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int ntask = (a.e_end - a.e_begin + 31) / 32, cap = stencil_cap(st, pass);
+  const int teams = std::max(1, std::min(STENCIL_TEAMS, (ntask + nsm - 1) / std::max(nsm, 1)));
+  const size_t smem = std::max(lists_smem, stencil_smem(st, pass, teams));
+  const int B = STENCIL_TEAM * teams;
+  auto run = [&](auto k, const double *in, double *out) {
+    // (blocks for the passes from the lists, which the stencil's absence falls back to)
+    const int g = persistent_grid((const void *) k, B, smem, 32LL * (a.e_end - a.e_begin));
+    k<<<g, B, smem, s>>>(a, st, cap, tab, e.nr, (float) e.rdr, in, out);
+  };
+  if (pass == 1) run(k_elem_stencil<true>, nullptr, erho_out);
+  else run(k_elem_stencil<false>, erho_in, nodef);
+}
+
 // Blocks of as many warps as spread the elements over all SMs, up to the
 // variant's block (one warp takes one element at a time): 64 elements on 3
 // blocks of 24 warps took 10 us a pass and 23 us a guard-band pass, on 64 one
 // warp blocks half of that.  Below 8 warps a block reads the EAM tables where
-// they are instead of copying them to shared memory.
+// they are instead of copying them to shared memory; from there on the EAM passes
+// take full blocks, which leave SMs to the atom passes on the other stream (1,680
+// elements beside 203,000 atoms: 201 us a step, spread 235; LJ, 2,240 elements
+// beside 129,000 atoms: 111, spread 106).
 template <int V, bool STAGE>
 static void launch_fused(const FusedArgs &a, int pass, const float4 *tab, const EamTables &e,
                          size_t table, int B, float lj1, float lj2, const double *erho_in,
-                         double *erho_out, double *nodef, cudaStream_t s) {
+                         double *erho_out, double *nodef, const Stencil *st, cudaStream_t s) {
   const size_t smem = (STAGE ? table : 0) + sizeof(float) * FUSED_WARP_FLOATS * (B / 32);
   const long long items = (long long) (a.e_end - a.e_begin) * 32;
+  if (st && pass != 0) {
+    launch_stencil(a, *st, pass, tab, e, smem, erho_in, erho_out, nodef, s);
+    const void *fix = pass == 1 ? (const void *) k_elem_rho_fused<V, true, STAGE>
+                                : (const void *) k_elem_force_fused<true, V, true, STAGE>;
+    const int g = persistent_grid(fix, B, smem, items);
+    if (pass == 1)
+      k_elem_rho_fused<V, true, STAGE><<<g, B, smem, s>>>(a, tab, e.nr, (float) e.rdr, erho_out);
+    else
+      k_elem_force_fused<true, V, true, STAGE><<<g, B, smem, s>>>(a, tab, e.nr, (float) e.rdr, 0.f, 0.f,
+                                                                  erho_in, nodef);
+    return;
+  }
   // the pass, then the exact pass over the elements it listed (a grid of the
   // same shape; it returns at once when the list is empty)
   auto run = [&](auto k, auto fix, auto... args) {
@@ -2761,15 +2867,16 @@ void elem_fused(const MixedElems &m, const FusedTables &t, int pass, const float
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const int full = t.variant == 0 ? fused_block(0) : fused_block(1);
   const long long warps = ((long long) (e_end - e_begin) + nsm - 1) / std::max(nsm, 1);
-  const int B = (int) std::min<long long>(full, 32 * std::max(1LL, warps));
+  const int B = eam && warps >= 8 ? full : (int) std::min<long long>(full, 32 * std::max(1LL, warps));
   if (eam && B < 256)  // few elements: one arrangement, tables unstaged
-    launch_fused<1, false>(a, pass, tab, e, table, B, lj1, lj2, erho_in, erho_out, nodef, s);
+    launch_fused<1, false>(a, pass, tab, e, table, B, lj1, lj2, erho_in, erho_out, nodef, nullptr, s);
   else if (t.variant == 1)
-    launch_fused<1, true>(a, pass, tab, e, table, B, lj1, lj2, erho_in, erho_out, nodef, s);
+    launch_fused<1, true>(a, pass, tab, e, table, B, lj1, lj2, erho_in, erho_out, nodef,
+                          t.stencil.state && stencil_fits(t.stencil, pass) ? &t.stencil : nullptr, s);
   else if (t.variant == 2)
-    launch_fused<2, true>(a, pass, tab, e, table, B, lj1, lj2, erho_in, erho_out, nodef, s);
+    launch_fused<2, true>(a, pass, tab, e, table, B, lj1, lj2, erho_in, erho_out, nodef, nullptr, s);
   else
-    launch_fused<0, true>(a, pass, tab, e, table, B, lj1, lj2, erho_in, erho_out, nodef, s);
+    launch_fused<0, true>(a, pass, tab, e, table, B, lj1, lj2, erho_in, erho_out, nodef, nullptr, s);
   check(cudaGetLastError(), "elem_fused");
 }
 
