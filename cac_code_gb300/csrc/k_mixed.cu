@@ -46,12 +46,16 @@ __device__ __forceinline__ int findex(float r, float rdr, int nr, float &p) {
 // then r*phi c4..c6.  The derivative of r*phi comes from its value
 // coefficients, as array2spline forms it (c0 = 3 c3 / dr, c1 = 2 c4 / dr,
 // c2 = c5 / dr, pair_eam.cpp:565-571): one 16-byte shared load less per pair.
-__device__ __forceinline__ void force_spline(const float4 *__restrict__ tab, int m, float p,
-                                             float rdr, float &rhoip, float &z2, float &z2p) {
-  const float4 t0 = tab[FTAB_W * m], t1 = tab[FTAB_W * m + 1];
+__device__ __forceinline__ void force_spline(const float4 t0, const float4 t1, float p, float rdr,
+                                             float &rhoip, float &z2, float &z2p) {
   rhoip = (t0.x * p + t0.y) * p + t0.z;
   z2 = ((t0.w * p + t1.x) * p + t1.y) * p + t1.z;
   z2p = ((3.0f * t0.w * p + 2.0f * t1.x) * p + t1.y) * rdr;
+}
+
+__device__ __forceinline__ void force_spline(const float4 *__restrict__ tab, int m, float p,
+                                             float rdr, float &rhoip, float &z2, float &z2p) {
+  force_spline(tab[FTAB_W * m], tab[FTAB_W * m + 1], p, rdr, rhoip, z2, z2p);
 }
 
 __device__ __forceinline__ double fprime64(double rho, const double *__restrict__ frho,
@@ -312,8 +316,14 @@ __device__ __forceinline__ int4 reorder_parts(int n, const float4 &lim, Index in
   return nn;
 }
 
-// 40 registers at three 512-thread blocks per SM (48 warps): more gathers in flight
-__global__ void __launch_bounds__(512, 3)
+// The atom passes take their list entries in batches: a batch's gathers are issued
+// together and the next batch's list indices with them, so that a warp has several
+// gathers in flight (with one in flight a warp waited on it at every entry: 10 of 16
+// cycles between two issues).  Batches of 4 and 32 warps an SM, 1,982,464 atoms: 439 us;
+// one entry at a time and 48 warps 507, batches of 2, 3 and 6 497, 453 and 447, of 2 on
+// 48 warps 447.  266,200 atoms, no longer a short second round: 90 -> 71 us.
+constexpr int RHO_BATCH = 4;
+__global__ void __launch_bounds__(512, 2)
 k_eam_rho_atoms(AtomArgs a, const float4 *__restrict__ rhor_val, int nr, float rdr,
                 const float4 *__restrict__ fp4, int nrho, float rdrho,
                 double *__restrict__ rho, float *__restrict__ fp) {
@@ -329,39 +339,45 @@ k_eam_rho_atoms(AtomArgs a, const float4 *__restrict__ rhor_val, int nr, float r
     dsacc acc;
     float part = 0.f;
     int ns = 0, cnt = 0;
-    // software pipeline: the list index two entries ahead and the coordinates
-    // one entry ahead are in flight while this entry is evaluated, so the
-    // gather never waits on a list load issued in the same iteration
-    int jn = 0, jnn = 0;
-    float4 qn = qi;
-    if (n > 0) {
-      jn = __ldg(a.list + i);
-      qn = __ldg(a.xq + jn);
-    }
-    if (n > 1) jnn = __ldg(a.list + (size_t) a.stride + i);
-    for (int k = 0; k < n; k++) {
-      const int j = jn;
-      const float4 qj = qn;
-      jn = jnn;
-      if (k + 2 < n) jnn = __ldg(a.list + (size_t) (k + 2) * a.stride + i);
-      if (k + 1 < n) qn = __ldg(a.xq + jn);
+    auto take = [&](int j, const float4 &qj) {
       float dx, dy, dz;
       rel_vec(qi, cx, cy, cz, qj, a.qg, dx, dy, dz);
-      float rsq = dx * dx + dy * dy + dz * dz;
-      if (rsq > a.band_hi) continue;
+      const float rsq = dx * dx + dy * dy + dz * dz;
+      if (rsq > a.band_hi) return;
       bool in = rsq < a.cutsq_f;
       if (rsq >= a.band_lo) in = inside64(a.x[i], a.x[j], a.cutsq);
       if (in) {  // decided before it is listed: the force pass tests nothing
         a.slist[(size_t) ns++ * a.stride + i] = j;
         float p;
-        int m = findex(sqrtf(rsq), rdr, nr, p);
-        float4 c = s_val[m];
+        const int m = findex(sqrtf(rsq), rdr, nr, p);
+        const float4 c = s_val[m];
         part += ((c.x * p + c.y) * p + c.z) * p + c.w;
         if ((++cnt & (CHUNK - 1)) == 0) {
           acc.add(part);
           part = 0.f;
         }
       }
+    };
+    const int *lp = a.list + i;
+    const size_t st = a.stride;
+    int jn[RHO_BATCH];
+#pragma unroll
+    for (int u = 0; u < RHO_BATCH; u++) jn[u] = u < n ? __ldg(lp + u * st) : i;
+    for (int k = 0; k < n; k += RHO_BATCH) {
+      int j[RHO_BATCH];
+      float4 q[RHO_BATCH];
+      lp += RHO_BATCH * st;
+#pragma unroll
+      for (int u = 0; u < RHO_BATCH; u++) {
+        j[u] = jn[u];
+        q[u] = __ldg(a.xq + j[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < RHO_BATCH; u++)
+        jn[u] = k + RHO_BATCH + u < n ? __ldg(lp + u * st) : i;
+#pragma unroll
+      for (int u = 0; u < RHO_BATCH; u++)
+        if (k + u < n) take(j[u], q[u]);
     }
     a.snum[i] = ns;
     acc.add(part);
@@ -713,18 +729,33 @@ k_eam_force_union(AtomArgs a, UnionArgs u, const float4 *__restrict__ ftab, int 
   }
 }
 
+// This thread's first atom and the end of its block's: every block an equal run of
+// whole warps.  A stride of the whole grid leaves SMs idle in the last round (247,808
+// atoms are 1.6 rounds of the force pass's threads: 84 us, in runs 74).
+__device__ __forceinline__ int block_atoms(int n, int &hi) {
+  const int run = (n + 32 * (int) gridDim.x - 1) / (32 * (int) gridDim.x) * 32;
+  hi = min(n, ((int) blockIdx.x + 1) * run);
+  return (int) blockIdx.x * run + (int) threadIdx.x;
+}
+
 // force table per knot: FTAB_W float4 (force_spline).  For large systems one
 // 1024-thread block per SM: the 64 KB table is held once per SM, which leaves
 // the unified L1/shared memory's rest to the neighbor gathers (smaller systems
-// keep the tuned block size, for more blocks than SMs).
-constexpr int FORCE_BLOCK = 1024;
+// keep the tuned block size, for more blocks than SMs).  Batches as in the density
+// pass: 1,982,464 atoms 606 us one entry at a time, 555 with the table's halves apart,
+// 472 in batches of 2 (of 3 and 4: 477 and 486).
+constexpr int FORCE_BLOCK = 1024, FORCE_BATCH = 2;
 __global__ void __launch_bounds__(FORCE_BLOCK, 1)
 k_eam_force_atoms(AtomArgs a, const float4 *__restrict__ ftab, int nr, float rdr,
                   const float *__restrict__ fp, double *__restrict__ f) {
-  extern __shared__ float4 s_tab[];  // FTAB_W float4 per knot
-  for (int m = threadIdx.x; m < FTAB_W * (nr + 1); m += blockDim.x) s_tab[m] = ftab[m];
+  // the knots' first and second float4 apart: 16-byte words at a stride of 32 bytes
+  // meet twice the bank conflicts
+  extern __shared__ float4 s_tab[];
+  for (int m = threadIdx.x; m < FTAB_W * (nr + 1); m += blockDim.x)
+    s_tab[m % FTAB_W * (nr + 1) + m / FTAB_W] = ftab[m];
   __syncthreads();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.nlocal; i += gridDim.x * blockDim.x) {
+  int hi;
+  for (int i = block_atoms(a.nlocal, hi); i < hi; i += blockDim.x) {
     const float4 qi = a.xq[i];
     float cx, cy, cz;
     cell_of(qi, cx, cy, cz);
@@ -733,27 +764,7 @@ k_eam_force_atoms(AtomArgs a, const float4 *__restrict__ ftab, int nr, float rdr
     dsacc fx, fy, fz;
     float px = 0.f, py = 0.f, pz = 0.f;
     int cnt = 0;
-    // software pipeline: the list index two entries ahead and the next
-    // entry's coordinates and F' in flight while this entry is evaluated, so
-    // that no gather waits on a list load issued in the same iteration
-    int jn = 0, jnn = 0;
-    float4 qn = qi;
-    float fpn = 0.f;
-    if (n > 0) {
-      jn = __ldg(a.slist + i);
-      qn = __ldg(a.xq + jn);
-      fpn = __ldg(fp + jn);
-    }
-    if (n > 1) jnn = __ldg(a.slist + (size_t) a.stride + i);
-    for (int k = 0; k < n; k++) {
-      const float4 qj = qn;
-      const float fpj = fpn;
-      jn = jnn;
-      if (k + 2 < n) jnn = __ldg(a.slist + (size_t) (k + 2) * a.stride + i);
-      if (k + 1 < n) {
-        qn = __ldg(a.xq + jn);
-        fpn = __ldg(fp + jn);
-      }
+    auto take = [&](const float4 &qj, float fpj) {
       float dx, dy, dz;
       rel_vec(qi, cx, cy, cz, qj, a.qg, dx, dy, dz);
       float rsq = dx * dx + dy * dy + dz * dz;
@@ -762,7 +773,7 @@ k_eam_force_atoms(AtomArgs a, const float4 *__restrict__ ftab, int nr, float rdr
       float p;
       int m = findex(r, rdr, nr, p);
       float rhoip, z2, z2p;
-      force_spline(s_tab, m, p, rdr, rhoip, z2, z2p);
+      force_spline(s_tab[m], s_tab[nr + 1 + m], p, rdr, rhoip, z2, z2p);
       float phi = z2 * recip;
       float phip = z2p * recip - phi * recip;
       float psip = (fpi + fpj) * rhoip + phip;
@@ -776,6 +787,27 @@ k_eam_force_atoms(AtomArgs a, const float4 *__restrict__ ftab, int nr, float rdr
         fz.add(pz);
         px = py = pz = 0.f;
       }
+    };
+    const int *lp = a.slist + i;
+    const size_t st = a.stride;
+    int jn[FORCE_BATCH];
+#pragma unroll
+    for (int u = 0; u < FORCE_BATCH; u++) jn[u] = u < n ? __ldg(lp + u * st) : i;
+    for (int k = 0; k < n; k += FORCE_BATCH) {
+      float4 q[FORCE_BATCH];
+      float fj[FORCE_BATCH];
+      lp += FORCE_BATCH * st;
+#pragma unroll
+      for (int u = 0; u < FORCE_BATCH; u++) {
+        q[u] = __ldg(a.xq + jn[u]);
+        fj[u] = __ldg(fp + jn[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < FORCE_BATCH; u++)
+        jn[u] = k + FORCE_BATCH + u < n ? __ldg(lp + u * st) : i;
+#pragma unroll
+      for (int u = 0; u < FORCE_BATCH; u++)
+        if (k + u < n) take(q[u], fj[u]);
     }
     fx.add(px);
     f[3 * i] = fx.value();
@@ -845,6 +877,9 @@ k_eam_force_lanes(AtomArgs a, const float4 *__restrict__ ftab, int nr, float rdr
 
 // band_lo/band_hi are relative factors here: a pair with rsq in
 // [band_lo, band_hi] * cutsq(type pair) is decided in FP64
+// (batches as in the EAM density pass, with the neighbors' types and cutoffs: 324,000
+// atoms 165 -> 124 us)
+constexpr int LJ_BATCH = 4;
 __global__ void __launch_bounds__(512, 2)
 k_lj_atoms(AtomArgs a, const int *__restrict__ type, const float *__restrict__ lj1,
            const float *__restrict__ lj2, const float *__restrict__ cutsq_t,
@@ -857,25 +892,10 @@ k_lj_atoms(AtomArgs a, const int *__restrict__ type, const float *__restrict__ l
     const int n = a.num[i];
     dsacc fx, fy, fz;
     float px = 0.f, py = 0.f, pz = 0.f;
-    // the list index two entries ahead, the next coordinates one ahead
-    int jn = 0, jnn = 0;
-    float4 qn = qi;
-    if (n > 0) {
-      jn = __ldg(a.list + i);
-      qn = __ldg(a.xq + jn);
-    }
-    if (n > 1) jnn = __ldg(a.list + (size_t) a.stride + i);
-    for (int k = 0; k < n; k++) {
-      const int j = jn;
-      const float4 qj = qn;
-      jn = jnn;
-      if (k + 2 < n) jnn = __ldg(a.list + (size_t) (k + 2) * a.stride + i);
-      if (k + 1 < n) qn = __ldg(a.xq + jn);
+    auto take = [&](int k, int j, const float4 &qj, int ij, float cs) {
       float dx, dy, dz;
       rel_vec(qi, cx, cy, cz, qj, a.qg, dx, dy, dz);
       float rsq = dx * dx + dy * dy + dz * dz;
-      int ij = it * (MAXT + 1) + type[j];
-      float cs = cutsq_t[ij];
       bool in = rsq < cs;
       if (rsq >= a.band_lo * cs && rsq <= a.band_hi * cs) in = inside64(a.x[i], a.x[j], cutsq64[ij]);
       if (in) {
@@ -892,6 +912,31 @@ k_lj_atoms(AtomArgs a, const int *__restrict__ type, const float *__restrict__ l
         fz.add(pz);
         px = py = pz = 0.f;
       }
+    };
+    const int *lp = a.list + i;
+    const size_t st = a.stride;
+    int jn[LJ_BATCH];
+#pragma unroll
+    for (int u = 0; u < LJ_BATCH; u++) jn[u] = u < n ? __ldg(lp + u * st) : i;
+    for (int k = 0; k < n; k += LJ_BATCH) {
+      int j[LJ_BATCH], ij[LJ_BATCH];
+      float4 q[LJ_BATCH];
+      float cs[LJ_BATCH];
+      lp += LJ_BATCH * st;
+#pragma unroll
+      for (int u = 0; u < LJ_BATCH; u++) {
+        j[u] = jn[u];
+        q[u] = __ldg(a.xq + j[u]);
+        ij[u] = it * (MAXT + 1) + __ldg(type + j[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < LJ_BATCH; u++) {
+        cs[u] = __ldg(cutsq_t + ij[u]);
+        jn[u] = k + LJ_BATCH + u < n ? __ldg(lp + u * st) : i;
+      }
+#pragma unroll
+      for (int u = 0; u < LJ_BATCH; u++)
+        if (k + u < n) take(k + u, j[u], q[u], ij[u], cs[u]);
     }
     fx.add(px);
     f[3 * i] = fx.value();
@@ -2396,10 +2441,9 @@ int persistent_grid(const void *kernel, int threads, size_t smem, long long work
 }
 
 // Lanes per atom: as many, up to 8, as leave all atoms in one round of the
-// threads that the GPU holds.  Measured, density / force pass: 9,677 atoms with 8
-// lanes 8 / 10 us against 25 / 25 with one; 266,200 atoms with 4 lanes 97 / 91 us
-// against 103 / 87, 1,982,464 with 2 lanes 604 us against 457 (more lanes take
-// the neighbors of fewer atoms together, which lie less close in memory).
+// threads that the GPU holds.  Measured, force pass: 9,677 atoms with 8 lanes 10 us
+// against 25 with one; 46,464 with 2 lanes 19 against 22, 72,600 24 against 22 (more
+// lanes take the neighbors of fewer atoms together, which lie less close in memory).
 int group_lanes(const void *kernel, int threads, size_t smem, int n) {
   const long long slots = (long long) threads * persistent_grid(kernel, threads, smem, 1LL << 60);
   int g = 1;
@@ -2458,9 +2502,13 @@ void eam_rho_atoms(const MixedAtoms &m, const float4 *rhor_val, const EamTables 
     a.rdrho_ds = make_float2(h, (float) (e.rdrho - (double) h));
   }
   size_t smem = sizeof(float4) * (e.nr + 1);
-  const int lanes = group_lanes((const void *) k_eam_rho_atoms, m.block, smem, m.nlocal);
-  auto k = lanes == 8 ? k_eam_rho_lanes<8> : lanes == 4 ? k_eam_rho_lanes<4>
-           : lanes == 2 ? k_eam_rho_lanes<2> : k_eam_rho_atoms;
+  // lanes per atom, for 152 SMs: 8 up to 29,184 atoms, 4 up to 48,640 (26,136 atoms: 14.0
+  // us with 8, 15.3 with 4, 22.5 with one; 46,464: 23.8, 20.2, 22.0; 61,952: 32, 28, 22.6;
+  // with 2 lanes 26 to 31 us)
+  const long long slots =
+      (long long) m.block * persistent_grid((const void *) k_eam_rho_atoms, m.block, smem, 1LL << 60);
+  const int lanes = 16LL * m.nlocal <= 3 * slots ? 8 : 16LL * m.nlocal <= 5 * slots ? 4 : 1;
+  auto k = lanes == 8 ? k_eam_rho_lanes<8> : lanes == 4 ? k_eam_rho_lanes<4> : k_eam_rho_atoms;
   const int block = lanes > 1 ? LANES_BLOCK : m.block;
   if (lanes > 1) smem = 0;
   int g = persistent_grid((const void *) k, block, smem, (long long) m.nlocal * lanes);
