@@ -14,7 +14,11 @@
 // per atom and component adds the terms in list order.  The density pass
 // leaves the short list and each pair's r (and 1/r with contraction) for the
 // force pass, which then has no distance, cutoff or square root to form: 17
-// of its 65 FP64 instructions per pair.
+// of its 65 FP64 instructions per pair.  Without contraction, the squared distance
+// and the splines are formed by the integer units (soft_fp64.cuh; the FP64 unit does
+// 20 of 31 instructions a pair in the density pass, 30 of 44 in the force pass):
+// 266,200 atoms 854 -> 594 and 1,199 -> 819 us, the FP64 unit still busy 84 %; LJ, 16,384
+// atoms, 86 -> 68 us.
 #pragma once
 #include "internal.h"
 
@@ -25,7 +29,16 @@ namespace {
 
 constexpr int AB = 8;           // atoms per block
 constexpr int ATOM_CAP = 96;    // buffered entries per atom and round
-constexpr int ATOM_NT = 128;    // threads per block
+// Threads per block of a pass.  (The force pass with contraction waits on its loads,
+// 70 % FP64 unit: 247,808 atoms 743 us with 128 threads, 628 with 64; the others, 84 %
+// FP64 unit, get slower, 664 -> 683 and 819 -> 869 us.)
+__host__ __device__ constexpr int atom_nt(int pass) {
+#ifdef FP64_EXACT_TU
+  return 128;
+#else
+  return pass == 2 ? 64 : 128;
+#endif
+}
 
 #ifdef FP64_EXACT_TU
 using PairR = double;           // r; negative: outside the cutoff
@@ -38,11 +51,46 @@ __device__ __forceinline__ float rsq_f32(float4 a, float4 b) {
   return dx * dx + dy * dy + dz * dz;
 }
 
+#ifdef FP64_EXACT_TU
+// a spline's cubic, or its derivative's quadratic, by the integer units
+// (spline_value, spline_deriv: N = 3, 2 Horner steps)
+template <int N>
+__device__ __forceinline__ double soft_spline(const double *__restrict__ c, const soft::Op &p) {
+  auto op = [&](int k) {
+    const double v = c[k];
+    return soft::op_of((unsigned) __double2hiint(v), (unsigned) __double2loint(v));
+  };
+  constexpr int first = N == 3 ? 3 : 0;
+  soft::Acc s = soft::add(soft::mul(op(first), p), soft::acc_of(op(first + 1)));
+#pragma unroll
+  for (int k = 2; k <= N; k++)
+    s = soft::add(soft::mul(soft::op_of(s), p), soft::acc_of(op(first + k)));
+  return __longlong_as_double((long long) soft::bits(s));
+}
+
+// dx^2 + dy^2 + dz^2 by the integer units
+__device__ __forceinline__ double soft_rsq(double dx, double dy, double dz) {
+  const unsigned hx = (unsigned) __double2hiint(dx), lx = (unsigned) __double2loint(dx);
+  const unsigned hy = (unsigned) __double2hiint(dy), ly = (unsigned) __double2loint(dy);
+  const unsigned hz = (unsigned) __double2hiint(dz), lz = (unsigned) __double2loint(dz);
+  if (!soft::dot_ready(hx, lx) || !soft::dot_ready(hy, ly) || !soft::dot_ready(hz, lz))
+    return dx * dx + dy * dy + dz * dz;
+  soft::Op o = soft::op_of(hx, lx);
+  soft::Acc s = soft::mul(o, o);
+  o = soft::op_of(hy, ly);
+  s = soft::add(s, soft::mul(o, o));
+  o = soft::op_of(hz, lz);
+  s = soft::add(s, soft::mul(o, o));
+  return __longlong_as_double((long long) soft::bits(s));
+}
+#endif
+
 // PASS 0: LJ forces; 1: EAM densities and F'(rho); 2: EAM forces from the
 // short lists and distances of pass 1
 template <int PASS>
-__global__ void __launch_bounds__(ATOM_NT)
+__global__ void __launch_bounds__(atom_nt(PASS))
 k_atoms64(Atoms64Args a, EamTables e, const LJTab *__restrict__ tab) {
+  constexpr int ATOM_NT = atom_nt(PASS);
   constexpr int NC = PASS == 1 ? 1 : NT3;   // buffered values per pair
   constexpr int NS = PASS == 1 ? 1 : 3;     // sums per atom
   __shared__ double s_t[AB][NC][ATOM_CAP + 1];
@@ -123,13 +171,24 @@ k_atoms64(Atoms64Args a, EamTables e, const LJTab *__restrict__ tab) {
             double p;
             const int m = split_index(r * e.rdr + 1.0, e.nr - 1, p);
             const double *c = e.rhor + 7 * (size_t) m;
-            const double rhoip = spline_deriv(c, p);
             const double *z = e.z2r + 7 * (size_t) m;
-            const double z2p = spline_deriv(z, p);
-            const double z2 = spline_value(z, p);
 #ifdef FP64_EXACT_TU
+            double rhoip, z2p, z2;
+            if (e.soft) {
+              const soft::Op q = soft::op_of((unsigned) __double2hiint(p), (unsigned) __double2loint(p));
+              rhoip = soft_spline<2>(c, q);
+              z2p = soft_spline<2>(z, q);
+              z2 = soft_spline<3>(z, q);
+            } else {
+              rhoip = spline_deriv(c, p);
+              z2p = spline_deriv(z, p);
+              z2 = spline_value(z, p);
+            }
             const double recip = 1.0 / r;
 #else
+            const double rhoip = spline_deriv(c, p);
+            const double z2p = spline_deriv(z, p);
+            const double z2 = spline_value(z, p);
             const double recip = pr.y;
 #endif
             const double phi = z2 * recip;
@@ -139,7 +198,11 @@ k_atoms64(Atoms64Args a, EamTables e, const LJTab *__restrict__ tab) {
             fpair = -psip * recip;
           }
         } else {
+#ifdef FP64_EXACT_TU
+          const double rsq = soft_rsq(dx, dy, dz);
+#else
           const double rsq = dx * dx + dy * dy + dz * dz;
+#endif
           const int ij = PASS == 0 ? ti + a.type[j] : 0;
           in = rsq < (PASS == 0 ? tab->cutsq[ij] : e.cutforcesq);
           if (PASS == 0) {
@@ -172,7 +235,13 @@ k_atoms64(Atoms64Args a, EamTables e, const LJTab *__restrict__ tab) {
 #endif
               double p;
               const int m = split_index(r * e.rdr + 1.0, e.nr - 1, p);
-              t = spline_value(e.rhor + 7 * (size_t) m, p);
+#ifdef FP64_EXACT_TU
+              if (e.soft)
+                t = soft_spline<3>(e.rhor + 7 * (size_t) m,
+                                   soft::op_of((unsigned) __double2hiint(p), (unsigned) __double2loint(p)));
+              else
+#endif
+                t = spline_value(e.rhor + 7 * (size_t) m, p);
             }
             s_t[my][0][k] = t;
             a.slist[at] = j;
@@ -233,7 +302,7 @@ k_atoms64(Atoms64Args a, EamTables e, const LJTab *__restrict__ tab) {
 void atom_pass(const Atoms64Args &a, int pass, const EamTables &e, const void *ljtab, cudaStream_t s) {
   if (a.nlocal <= 0) return;
   auto k = pass == 0 ? k_atoms64<0> : pass == 1 ? k_atoms64<1> : k_atoms64<2>;
-  k<<<(a.nlocal + AB - 1) / AB, ATOM_NT, 0, s>>>(a, e, (const LJTab *) ljtab);
+  k<<<(a.nlocal + AB - 1) / AB, atom_nt(pass), 0, s>>>(a, e, (const LJTab *) ljtab);
   check(cudaGetLastError(), "atom_pass");
 }
 

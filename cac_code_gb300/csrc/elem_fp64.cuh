@@ -16,7 +16,12 @@
 // relative to the element's node 0 with a bound derived from their size
 // (pass_limit), and only the entries that pass get an FP64 position, formed
 // where the pair is evaluated: no site array, no list of the step in memory,
-// no F'(rho) of sites that nothing reaches.
+// no F'(rho) of sites that nothing reaches.  And the positions, with the densities of
+// the sites where they are not contracted, come from the integer units
+// (soft_fp64.cuh), which are idle otherwise: the FP64 unit is left 53 of 98
+// instructions a pair.  64,000 elements with contraction: forces 5,084 -> 3,230 us, the
+// FP64 unit busy 74 % of it and the ALU 67 %, densities 1,122 -> 925 us (ALU 77 %); 7,200
+// without: forces 1,113 -> 690 us.
 //
 // A block takes RB rows at a time.  Its warps scan the rows' lists 32 entries
 // at a time and append what passes, in list order, to the rows' buffers in
@@ -26,6 +31,7 @@
 // buffer fills up go on where they stopped in a further round.
 #pragma once
 #include "internal.h"
+#include "soft_fp64.cuh"
 
 namespace cacg {
 namespace FP64NS {
@@ -38,8 +44,10 @@ constexpr int ELEM_NT = 128;    // threads per block
 
 #ifdef FP64_EXACT_TU
 constexpr int NT3 = 3;          // buffered per pair: the three terms
+constexpr bool SOFT_RHO = true; // a site's density by the integer units as well
 #else
 constexpr int NT3 = 4;          // the vector and the pair factor (summed with one FMA)
+constexpr bool SOFT_RHO = false;  // (contracted here)
 #endif
 
 // m = min((int) q, n1) and p = min(q - m, 1): for 1 <= q < 2^20 from the bits
@@ -106,11 +114,37 @@ __device__ __forceinline__ double eam_slope(const EamTables &e, double rho) {
   return (c[0] * p + c[1]) * p + c[2];
 }
 
+// the sums of the weights times N groups of 8 operands (x, y, z, then the densities)
+template <int N>
+__device__ __forceinline__ void soft_dots(const double (&w)[NPE], const soft::Op *s_op, double &x,
+                                          double &y, double &z, double &rho) {
+  soft::Op o[NPE];
+  x = y = z = rho = 0.0;
+#pragma unroll
+  for (int k = 0; k < NPE; k++)
+    o[k] = soft::op_of((unsigned) __double2hiint(w[k]), (unsigned) __double2loint(w[k]));
+#pragma unroll 1
+  for (int d = 0; d < N; d++) {
+    soft::Acc s = soft::mul(o[0], s_op[8 * d]);
+#pragma unroll
+    for (int k = 1; k < NPE; k++) s = soft::add(s, soft::mul(o[k], s_op[8 * d + k]));
+    const double v = __longlong_as_double((long long) soft::bits(s));
+    x = y;
+    y = z;
+    if (N == 4) {
+      z = rho;
+      rho = v;
+    } else {
+      z = v;
+    }
+  }
+}
+
 // DENSITY: the 8 node rows of each element -> erho; otherwise the force rows
 // (row list fjj of the type; all rows when it is null) -> nodef.
 // SELF: every list entry is a site of the row's own element.
 template <bool EAM, bool DENSITY, bool SELF>
-__global__ void __launch_bounds__(ELEM_NT)
+__global__ void __launch_bounds__(ELEM_NT, 7)  // (five blocks an SM, as it comes: 3,630 us, six 3,388)
 k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
          double *__restrict__ out) {
   constexpr int NC = DENSITY ? 1 : NT3, NS = DENSITY ? 1 : 3;  // buffered values, sums
@@ -121,6 +155,11 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
   __shared__ float4 s_nf4[6];
   __shared__ float s_pf[RB][3];
   __shared__ float s_lim;
+  // by the integer units (soft_fp64.cuh): the nodes' coordinates by axis, then their
+  // densities; whether all of them can be
+  constexpr int NDOT = SOFT_RHO && EAM && !DENSITY ? 4 : 3;
+  __shared__ soft::Op s_op[SELF ? 8 * NDOT : 1];
+  __shared__ int s_hard;
   float *s_nf = reinterpret_cast<float *>(s_nf4);
   const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ty = a.etype[e], ioff = a.int_off[ty];
@@ -128,11 +167,20 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
   const double *__restrict__ S0 = a.spa_inter + (size_t) a.inter_off[ty] * NPE;
   const float4 *__restrict__ F0 = a.spa_inter_f + (size_t) a.inter_off[ty] * 2;
   const int kb = a.kb, kmask = (1 << kb) - 1;
+  if (SELF) {
+    if (tid == 0) s_hard = !a.soft;
+    __syncthreads();
+  }
   if (warp == 0) {
     float r = 0.f, x = 0.f;
     if (lane < 24) {
       const double v = a.nodex[24 * (size_t) e + lane];
       s_nx[lane] = v;
+      if (SELF) {
+        const unsigned h = (unsigned) __double2hiint(v), l = (unsigned) __double2loint(v);
+        s_op[lane % 3 * 8 + lane / 3] = soft::op_of(h, l);
+        if (!soft::dot_ready(h, l)) s_hard = 1;
+      }
       const double v0 = __shfl_sync(0x00FFFFFFu, v, lane % 3);
       const float f = SELF ? (float) (v - v0) : (float) v;
       s_nf[lane] = f;
@@ -146,7 +194,15 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
     }
     if (lane == 0) s_lim = SELF ? pass_limit((float) cutsq, r, x) : a.cut_pass;
   } else if (warp == 1 && EAM && !DENSITY) {
-    if (lane < NPE) s_er[lane] = a.erho[NPE * (size_t) e + lane];
+    if (lane < NPE) {
+      const double v = a.erho[NPE * (size_t) e + lane];
+      s_er[lane] = v;
+      if (SELF && NDOT == 4) {
+        const unsigned h = (unsigned) __double2hiint(v), l = (unsigned) __double2loint(v);
+        s_op[SELF ? 8 * (NDOT - 1) + lane : 0] = soft::op_of(h, l);
+        if (!soft::dot_ready(h, l)) s_hard = 1;
+      }
+    }
   }
   const int nr_rows = DENSITY ? NPE : (a.fjj ? a.fjj_off[ty + 1] - a.fjj_off[ty] : a.numint[ty]);
   double nf = 0.0;  // threads 0..23: the nodal force component
@@ -265,10 +321,17 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
         const int nj = line * naz + (code & kmask);
         double S[NPE];
         load8(S0 + (size_t) nj * NPE, S);
-        const double *x = SELF || j == e ? s_nx : a.nodex + 24 * (size_t) j;
-        const double dx = s_p[r][0] - node_sum(S, x, 3);
-        const double dy = s_p[r][1] - node_sum(S, x + 1, 3);
-        const double dz = s_p[r][2] - node_sum(S, x + 2, 3);
+        double sx, sy, sz, srho = 0.0;
+        const bool hard = !SELF || s_hard;
+        if (hard) {
+          const double *x = SELF || j == e ? s_nx : a.nodex + 24 * (size_t) j;
+          sx = node_sum(S, x, 3);
+          sy = node_sum(S, x + 1, 3);
+          sz = node_sum(S, x + 2, 3);
+        } else {
+          soft_dots<NDOT>(S, s_op, sx, sy, sz, srho);
+        }
+        const double dx = s_p[r][0] - sx, dy = s_p[r][1] - sy, dz = s_p[r][2] - sz;
         const double rsq = dx * dx + dy * dy + dz * dz;
         double t0 = 0.0, fpair = 0.0;
         const bool in = rsq < cutsq;
@@ -287,9 +350,12 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
               t0 = ((c[3] * p + c[4]) * p + c[5]) * p + c[6];
             } else {
               const double *er = SELF || j == e ? s_er : a.erho + NPE * (size_t) j;
-              double rho = 0.0;
+              double rho = srho;
+              if (hard || NDOT == 3) {
+                rho = 0.0;
 #pragma unroll
-              for (int q = 0; q < NPE; q++) rho += S[q] * er[q];
+                for (int q = 0; q < NPE; q++) rho += S[q] * er[q];
+              }
               const double fpj = eam_slope(eam, rho);
               const double rhoip = (c[0] * p + c[1]) * p + c[2];
               const double *z = eam.z2r + 7 * (size_t) m;

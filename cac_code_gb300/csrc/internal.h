@@ -125,6 +125,7 @@ struct EamTables {
   const double *z2r;   // [(nr+1)*7]
   int nr, nrho;
   double rdr, rdrho, cutforcesq;
+  int soft = 0;        // rhor and z2r suit soft::dot_ready
 };
 
 // ---- scan / compaction (k_comm.cu) ----
@@ -233,6 +234,7 @@ struct Elem64Args {
   const int *nae;               // lattice sizes per type
   int kb;                       // bits of the site index in a line code
   float cut_pass;               // FP32 limit for absolute coordinates
+  int soft;                     // the site shape functions suit soft::dot_ready
 };
 
 // ---- forces: same kernels in two translation units (force_fp64.cuh) ----
