@@ -145,6 +145,85 @@ __global__ void __launch_bounds__(UB) k_update(UpdateArgs a) {
   else a.c.bias[(size_t) member * BIASES + layer * NH + r] = p;
 }
 
+// Column means and standard deviations of two [n][cols] arrays, a block each: FP32
+// sums down the rows in order, as an array library forms them (so that a data set is
+// normalised to the same bits), the quotients by n in FP64 where wide is set.  Bound by
+// the chain of additions, 4 cycles a row: the rows come through shared memory, MO_STAGES
+// chunks ahead.  65,536 rows of 32 and 24: 1.2 ms with the copies, by the host 7.3.
+constexpr int MO_NT = 256, MO_ROWS = 64, MO_STAGES = 4;
+struct Moments {
+  const float *a[2];
+  int cols[2];
+  float *mean[2], *std[2];
+};
+
+__global__ void __launch_bounds__(MO_NT) k_moments(Moments q, long n, int wide) {
+  __shared__ __align__(16) float s_buf[MO_STAGES][MO_ROWS * NIN];
+  const int cols = q.cols[blockIdx.x], tid = threadIdx.x;
+  const float *a = q.a[blockIdx.x];
+  const long total = n * cols, chunk = (long) MO_ROWS * cols, chunks = (n + MO_ROWS - 1) / MO_ROWS;
+  auto fetch = [&](long c) {
+    if (c < chunks) {
+      const float *src = a + c * chunk;
+      const long len = min(chunk, total - c * chunk);  // a multiple of 4 floats
+      const unsigned dst = (unsigned) __cvta_generic_to_shared(s_buf[c % MO_STAGES]);
+      for (int i = 4 * tid; i < len; i += 4 * MO_NT)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 4 * i), "l"(src + i));
+    }
+    asm volatile("cp.async.commit_group;");
+  };
+  auto quotient = [&](float v) {
+    return wide ? (float) ((double) v / (double) n) : __fdiv_rn(v, (float) n);
+  };
+  float mean = 0.f;
+  for (int pass = 0; pass < 2; pass++) {
+    float s = 0.f;
+    for (int c = 0; c < MO_STAGES - 1; c++) fetch(c);
+    for (long c = 0; c < chunks; c++) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(MO_STAGES - 2));
+      __syncthreads();
+      fetch(c + MO_STAGES - 1);
+      if (tid < cols) {
+        const float *b = s_buf[c % MO_STAGES] + tid;
+        const int rows = (int) min((long) MO_ROWS, n - c * MO_ROWS);
+        auto take = [&](float v) {
+          if (pass) {
+            v = __fsub_rn(v, mean);
+            v = __fmul_rn(v, v);
+          }
+          s = __fadd_rn(s, v);
+        };
+        if (rows == MO_ROWS) {
+#pragma unroll 16
+          for (int r = 0; r < MO_ROWS; r++) take(b[r * cols]);
+        } else {
+          for (int r = 0; r < rows; r++) take(b[r * cols]);
+        }
+      }
+    }
+    __syncthreads();
+    if (pass == 0) mean = quotient(s);
+    else if (tid < cols) {
+      q.mean[blockIdx.x][tid] = mean;
+      q.std[blockIdx.x][tid] = __fsqrt_rn(quotient(s));
+    }
+  }
+}
+
+// sums of the squares of the rows' 24 values in FP64, by eight strands added in pairs
+__global__ void k_row_squares(const float *__restrict__ t, long n, double *__restrict__ out) {
+  const long i = blockIdx.x * (long) blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double r[8];
+#pragma unroll
+  for (int k = 0; k < NOUT; k++) {
+    const double v = t[i * NOUT + k], w = __dmul_rn(v, v);
+    r[k % 8] = k < 8 ? w : __dadd_rn(r[k % 8], w);
+  }
+  out[i] = __dadd_rn(__dadd_rn(__dadd_rn(r[0], r[1]), __dadd_rn(r[2], r[3])),
+                     __dadd_rn(__dadd_rn(r[4], r[5]), __dadd_rn(r[6], r[7])));
+}
+
 // normalised features as bf16 [n][64]: (x - mean) * inv_std, zero padded
 __global__ void k_features(const float *__restrict__ x, long n, const float *__restrict__ norm,
                            bf16 *__restrict__ out) {
@@ -364,6 +443,31 @@ struct Net {
     check(cudaMemcpyAsync(&f, errflag.p, sizeof(int), cudaMemcpyDeviceToHost, stream), "errflag");
     sync();
     if (f) throw CudaError{cudaErrorLaunchTimeout, "tensor-core GEMM: a bounded wait ran out"};
+  }
+
+  // means and deviations of a data set (in, then out), sums of its targets' squares
+  void moments(const float *x, const float *t, long long n, int wide, float *const out[4],
+               double *row_squares) {
+    cudaStream_t s = stream;
+    constexpr int C = NIN + NOUT;
+    raw.ensure((size_t) n * NIN, s);
+    rt.ensure((size_t) n * NOUT, s);
+    tf.ensure((size_t) n * 2, s);
+    dm.ensure(2 * C, s);
+    double *rows = reinterpret_cast<double *>(tf.p);
+    check(cudaMemcpyAsync(raw.p, x, sizeof(float) * n * NIN, cudaMemcpyHostToDevice, s), "x");
+    check(cudaMemcpyAsync(rt.p, t, sizeof(float) * n * NOUT, cudaMemcpyHostToDevice, s), "t");
+    const Moments q{{raw.p, rt.p}, {NIN, NOUT}, {dm.p, dm.p + 2 * NIN}, {dm.p + NIN, dm.p + 2 * NIN + NOUT}};
+    k_moments<<<2, MO_NT, 0, s>>>(q, (long) n, wide);
+    k_row_squares<<<nblk(n, 256), 256, 0, s>>>(rt.p, (long) n, rows);
+    check(cudaGetLastError(), "moments");
+    float h[2 * C];
+    check(cudaMemcpyAsync(h, dm.p, sizeof h, cudaMemcpyDeviceToHost, s), "moments");
+    check(cudaMemcpyAsync(row_squares, rows, sizeof(double) * n, cudaMemcpyDeviceToHost, s), "rows");
+    sync();
+    const int off[4] = {0, NIN, 2 * NIN, 2 * NIN + NOUT}, len[4] = {NIN, NIN, NOUT, NOUT};
+    for (int k = 0; k < 4; k++) std::memcpy(out[k], h + off[k], sizeof(float) * len[k]);
+    trim();
   }
 
   // the members' gradients into g
@@ -605,6 +709,15 @@ int cacg_mlp_set_params(cacg_mlp m, int member, const float *p) {
                               cudaMemcpyHostToDevice, m->net.stream), "params");
   m->net.refresh(member, 1);
   m->net.sync();
+  MLP_END
+}
+
+int cacg_mlp_moments(cacg_mlp m, const float *x, const float *t, long long n, int wide, float *in_mean,
+                     float *in_std, float *out_mean, float *out_std, double *row_squares) {
+  MLP_BEGIN
+  need(x && t && in_mean && in_std && out_mean && out_std && row_squares && n > 0, "bad arrays");
+  float *out[4] = {in_mean, in_std, out_mean, out_std};
+  m->net.moments(x, t, n, wide, out, row_squares);
   MLP_END
 }
 

@@ -248,6 +248,11 @@ int cacg_mlp_set_normalization(cacg_mlp m, const float *in_mean, const float *in
                                const float *out_mean, const float *out_std, double force_scale);
 int cacg_mlp_get_normalization(cacg_mlp m, float *in_mean, float *in_std, float *out_mean,
                                float *out_std, double *force_scale);
+/* column means and standard deviations of x[n][32] and t[n][24], FP32 sums in row
+   order, divided by n in FP64 if wide; row_squares[n]: each t row's sum of squares */
+int cacg_mlp_moments(cacg_mlp m, const float *x, const float *t, long long n, int wide,
+                     float *in_mean, float *in_std, float *out_mean, float *out_std,
+                     double *row_squares);
 /* mean-squared error of member's normalised outputs on n samples x[n][32],
    t[n][24] and its gradient with respect to every parameter (no update) */
 int cacg_mlp_loss_grad(cacg_mlp m, int member, const float *x, const float *t, int n,
