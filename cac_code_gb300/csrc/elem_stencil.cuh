@@ -328,9 +328,9 @@ k_elem_stencil(FusedArgs a, Stencil st, int cap, const float4 *__restrict__ tab,
       !stencil_stage(st, st.slot + (DENSITY ? st.nf : 0), nrow, a.eflags, a.nnear_row != nullptr, a.cutsq_f, cap,
                      s_ent, s_off)) {
     if (DENSITY)
-      elem_rho_body<1, false, true>(a, tab, nr, rdr, out);
+      elem_rho_body<1, PASS, true>(a, tab, nr, rdr, out);
     else
-      elem_force_body<true, 1, false, true>(a, tab, nr, rdr, 0.f, 0.f, erho, out);
+      elem_force_body<true, 1, PASS, true>(a, tab, nr, rdr, 0.f, 0.f, erho, out);
     return;
   }
   const int ntask = (a.e_end - a.e_begin + 31) / 32, nteam = blockDim.x / STENCIL_TEAM;

@@ -2967,8 +2967,7 @@ void cacg_context::pair_ecompute_mixed() {
       part_bounds.assign(parts + 1, enlocal);
       for (int p = 0; p < parts; p++) part_bounds[p] = (int) ((long long) enlocal * p / parts);
       for (int p = 0; p < parts; p++) {
-        pass(part_bounds[p], part_bounds[p + 1]);
-        launches += 2;  // the pass and its guard-band exact pass
+        launches += pass(part_bounds[p], part_bounds[p + 1]);
         if (p + 1 < parts) {
           nve_nodes_final_range(part_bounds[p], part_bounds[p + 1]);
           check(cudaEventRecord(ev_nvpart[p], s), "nodev part final");
@@ -2990,7 +2989,7 @@ void cacg_context::pair_ecompute_mixed() {
       }
       kmark(KT_ELEM_FORCE, 0);
       force_parts([&](int b0, int b1) {
-        mixed::elem_fused(m, ft, 0, nullptr, et, (float) ljtab.lj1[a], (float) ljtab.lj2[a],
+        return mixed::elem_fused(m, ft, 0, nullptr, et, (float) ljtab.lj1[a], (float) ljtab.lj2[a],
                           nullptr, nullptr, d_nodef.p, s, b0, b1);
       });
       kmark(KT_ELEM_FORCE, 1);
@@ -3004,9 +3003,8 @@ void cacg_context::pair_ecompute_mixed() {
       m.rdrho = (float) rdrho;
       d_erho.ensure((size_t) NPE * nall, s);
       kmark(KT_ELEM_RHO, 0);
-      mixed::elem_fused(m, ft, 1, d_rhor_val4.p, et, 0.f, 0.f, nullptr, d_erho.p, nullptr, s);
+      launches += mixed::elem_fused(m, ft, 1, d_rhor_val4.p, et, 0.f, 0.f, nullptr, d_erho.p, nullptr, s);
       kmark(KT_ELEM_RHO, 1);
-      launches += 2;  // the pass and its guard-band exact pass
       if (use_sur) {
         kmark(KT_SUR, 0);
         surrogate_predict(et);
@@ -3015,7 +3013,7 @@ void cacg_context::pair_ecompute_mixed() {
       }
       kmark(KT_ELEM_FORCE, 0);
       force_parts([&](int b0, int b1) {
-        mixed::elem_fused(m, ft, 2, d_ftab.p, et, 0.f, 0.f, d_erho.p, nullptr, d_nodef.p, s, b0,
+        return mixed::elem_fused(m, ft, 2, d_ftab.p, et, 0.f, 0.f, d_erho.p, nullptr, d_nodef.p, s, b0,
                           b1);
       });
       kmark(KT_ELEM_FORCE, 1);

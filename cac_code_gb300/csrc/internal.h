@@ -469,8 +469,8 @@ struct FusedTables {
 };
 bool fused_fits(int nr, int nrho);
 // elements [e_begin, e_end) (e_end < 0: all local elements); the guard-band
-// exact pass runs after each launch
-void elem_fused(const MixedElems &m, const FusedTables &t, int pass, const float4 *tab,
+// exact pass runs after each launch, or with it (few elements); the number of launches
+int elem_fused(const MixedElems &m, const FusedTables &t, int pass, const float4 *tab,
                 const EamTables &e, float lj1, float lj2, const double *erho_in,
                 double *erho_out, double *nodef, cudaStream_t s, int e_begin = 0,
                 int e_end = -1);

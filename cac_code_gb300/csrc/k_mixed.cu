@@ -1806,22 +1806,31 @@ __device__ __forceinline__ float row_fprime_ds(const float2 *__restrict__ N,
   return fprime_ds(rho, c3, nrho, rdrho);
 }
 
-// FP64 cutoff decision of a guard-band pair: the row's point and the site from
-// the FP64 nodes and shape functions
-__device__ __noinline__ bool fused_band64(const double *N, const double *M, const double *x,
-                                          double cutsq) {
-  double rsq = 0.0;
+// FP64 cutoff decisions of a warp's guard-band pairs (band: this lane has one; row,
+// site: its shape functions' rows in N and M; x: the element's FP64 nodes), one pair
+// after another: six lanes interpolate a coordinate each of the row's point and the
+// site.  By the lane that has the pair the decision is 54 FP64 instructions, which
+// cost a warp the same for one lane as for all; so it is 12.
+__device__ __noinline__ bool fused_band64(bool band, bool in, const double *__restrict__ N, int row,
+                                          const double *__restrict__ M, int site,
+                                          const double *__restrict__ x, double cutsq) {
+  const int lane = threadIdx.x & 31;
+  for (unsigned todo = __ballot_sync(0xffffffffu, band); todo; todo &= todo - 1) {
+    const int src = __ffs(todo) - 1;
+    const int r = __shfl_sync(0xffffffffu, row, src), m = __shfl_sync(0xffffffffu, site, src);
+    double p = 0.0;
+    if (lane < 6) {
+      const double *w = (lane < 3 ? N + (size_t) r * NPE : M + (size_t) m * NPE), *y = x + lane % 3;
 #pragma unroll
-  for (int d = 0; d < 3; d++) {
-    double p = 0.0, q = 0.0;
-#pragma unroll
-    for (int k = 0; k < NPE; k++) {
-      p += N[k] * x[3 * k + d];
-      q += M[k] * x[3 * k + d];
+      for (int k = 0; k < NPE; k++) p = fma(w[k], y[3 * k], p);
     }
-    rsq += (p - q) * (p - q);
+    const double d = p - __shfl_down_sync(0xffffffffu, p, 3);
+    const double dx = __shfl_sync(0xffffffffu, d, 0), dy = __shfl_sync(0xffffffffu, d, 1),
+                 dz = __shfl_sync(0xffffffffu, d, 2);
+    const bool inside = fma(dz, dz, fma(dy, dy, dx * dx)) < cutsq;
+    if (lane == src) in = inside;
   }
-  return rsq < cutsq;
+  return in;
 }
 
 // lattice geometry of a type as the kernels use it
@@ -1849,9 +1858,9 @@ __device__ __forceinline__ float fprime32_s(float rho, const float4 *s_fp, int n
 // two float4 per axis, then the density coefficients) at every entry, fewer
 // registers; V = 2: as 1, two entries in flight per lane.
 // EXACT: a pair in the guard band is decided in FP64 (fused_band64) in the
-// loop; otherwise the loop only reports that it met one (the return value):
-// the caller lists the element for the exact pass, and the call with its
-// register saves stays out of the common case's loop
+// loop, whose rounds all lanes then make together; otherwise the loop only reports
+// that it met one (the return value): the caller lists the element for the exact
+// pass, and the call with its register saves stays out of the common case's loop
 template <bool EAM, bool DENSITY, int V, bool EXACT>
 __device__ __forceinline__ bool fused_row(const FusedArgs &a, const FusedLat &g, int e, int rfirst,
                                           int ty, int jj, int level, int glane, const float (&k)[21],
@@ -1877,8 +1886,9 @@ __device__ __forceinline__ bool fused_row(const FusedArgs &a, const FusedLat &g,
   int cn = 0, cnt = 0;
   bool band = false;
   if (glane < n) cn = __ldg(a.ent + s0 + glane);
+  const int nw = EXACT ? (int) __reduce_max_sync(0xffffffffu, (unsigned) n) + glane : n;
 #pragma unroll(V == 2 ? 2 : 1)
-  for (int t = glane; t < n; t += FG) {
+  for (int t = glane; t < nw; t += FG) {
     const int code = cn;
     if (t + FG < n) cn = __ldg(a.ent + s0 + t + FG);
     const int L = code_line(a.lat, code) - lbase, kk = code_kk(a.lat, code);
@@ -1919,14 +1929,12 @@ __device__ __forceinline__ bool fused_row(const FusedArgs &a, const FusedLat &g,
     const float dx = v[0], dy = v[1], dz = v[2];
     const float rsq = dx * dx + dy * dy + dz * dz;
     bool in = rsq < a.cutsq_f;
-    if (rsq >= a.band_lo && rsq <= a.band_hi) {
-      if (EXACT)
-        in = fused_band64(a.spa_int + ((size_t) a.int_off[ty] + jj) * NPE,
-                          a.spa_inter + ((size_t) a.inter_off[ty] + L * g.naz + kk) * NPE,
-                          a.nodex + 24 * (size_t) e, a.cutsq);
-      else
-        band = true;
-    }
+    const bool near = (!EXACT || t < n) && rsq >= a.band_lo && rsq <= a.band_hi;
+    band |= near;
+    if (EXACT)
+      in = fused_band64(near, in, a.spa_int, a.int_off[ty] + jj, a.spa_inter,
+                        a.inter_off[ty] + L * g.naz + kk, a.nodex + 24 * (size_t) e, a.cutsq) &&
+           t < n;
     if (in) {
       if (EAM) {
         const float recip = rsqrtf(rsq);
@@ -2027,12 +2035,19 @@ static_assert(FUSED_NX_AT % 2 == 0 && FUSED_ER_AT % 2 == 0 && FUSED_WARP_FLOATS 
 
 // threads per block of each variant (V = 0: coefficients in registers)
 __host__ __device__ constexpr int fused_block(int V) { return V == 0 ? FUSED_BLOCK : 768; }
+constexpr int FEW_BLOCK = 256;  // at most, of the passes over few elements (DIRECT)
 
 // The guard-band list (a.band: count, blocks done, elements re-run so far,
 // then the element indices).  A fused pass lists every element in which some
-// pair fell in the guard band; the exact pass (FIX) runs the listed elements
+// pair fell in the guard band; the exact pass (LISTED) runs the listed elements
 // again with the FP64 decisions, overwriting their outputs, and its last block
 // to finish resets the list for the next pass.
+// DIRECT, for few elements (one round of the SMs: their time is a single element's):
+// one pass over all of them that takes the FP64 decisions itself.  64 elements, LJ: 7.3
+// and 17.1 us in two passes (15.7 in one with a pair's decision by its own lane), 11.2
+// in one; 160, EAM: 5.5 and 1.5, 13.4 and 1.8 us in two, 5.9 and 13.9 in one.  With more
+// rounds the decisions' registers cost every element.
+enum { PASS = 0, LISTED = 1, DIRECT = 2 };
 constexpr int BAND_LIST = 3;
 
 __device__ __forceinline__ void band_list(int *band, int e, int cap) {
@@ -2053,12 +2068,13 @@ __device__ __forceinline__ void band_done(int *band, int ne) {
 }
 
 // EAM nodal densities: the element's 8 node rows, one row per FG lanes
-// (FIX: the listed elements, guard-band pairs decided in FP64)
+// (LISTED: the listed elements, guard-band pairs decided in FP64)
 // STAGE: the spline tables in shared memory; otherwise read where they are
 // (few elements: their blocks would each copy 32 to 96 KB first)
-template <int V, bool FIX, bool STAGE>
+template <int V, int MODE, bool STAGE>
 __device__ __forceinline__ void elem_rho_body(const FusedArgs &a, const float4 *__restrict__ tab, int nr,
                                               float rdr, double *__restrict__ erho) {
+  constexpr bool FIX = MODE == LISTED;
   const int ne = FIX ? min(a.band[0], a.nlocal_e) : a.e_end - a.e_begin;
   if (FIX && ne == 0) return;  // the whole grid (the count is the same for every block)
   extern __shared__ float4 smem[];
@@ -2110,31 +2126,35 @@ __device__ __forceinline__ void elem_rho_body(const FusedArgs &a, const float4 *
       const bool live = q < NPE;
       const int jj = live ? a.node_list[ty * NPE + q] : 0;
       dsacc acc, fx, fy, fz;
-      band |= fused_row<true, true, V, FIX>(a, g, e, rfirst, ty, jj, level, glane, k, rk,
+      band |= fused_row<true, true, V, MODE != PASS>(a, g, e, rfirst, ty, jj, level, glane, k, rk,
                                             reinterpret_cast<const float4 *>(s_k), s_tab, nullptr,
                                             nr, rdr, 0.f, 0.f, 0.f, live, acc, fx, fy, fz);
       if (live && glane == 0) erho[NPE * (size_t) e + q] = acc.value();
     }
-    if (!FIX && __any_sync(0xffffffffu, band) && lane == 0) band_list(a.band, e, a.nlocal_e);
+    if (!FIX && __any_sync(0xffffffffu, band) && lane == 0) {
+      if (MODE == PASS) band_list(a.band, e, a.nlocal_e);
+      else atomicAdd(a.band + 2, 1);
+    }
     __syncwarp();
   }
   if (FIX) band_done(a.band, ne);
 }
-template <int V, bool FIX, bool STAGE>
-__global__ void __launch_bounds__(fused_block(V), 1)
+template <int V, int MODE, bool STAGE>
+__global__ void __launch_bounds__(MODE == DIRECT ? FEW_BLOCK : fused_block(V), 1)
 k_elem_rho_fused(FusedArgs a, const float4 *__restrict__ tab, int nr, float rdr,
                  double *__restrict__ erho) {
-  elem_rho_body<V, FIX, STAGE>(a, tab, nr, rdr, erho);
+  elem_rho_body<V, MODE, STAGE>(a, tab, nr, rdr, erho);
 }
 
 // Forces of the element's rows of nonzero weight and their gather onto the
 // nodes (EAM with the nodal densities and row F'(rho), or LJ)
-// (FIX: the listed elements, guard-band pairs decided in FP64)
-template <bool EAM, int V, bool FIX, bool STAGE>
+// (LISTED: the listed elements, guard-band pairs decided in FP64)
+template <bool EAM, int V, int MODE, bool STAGE>
 __device__ __forceinline__ void elem_force_body(const FusedArgs &a, const float4 *__restrict__ tab, int nr,
                                                 float rdr, float lj1, float lj2,
                                                 const double *__restrict__ erho,
                                                 double *__restrict__ nodef) {
+  constexpr bool FIX = MODE == LISTED;
   const int ne = FIX ? min(a.band[0], a.nlocal_e) : a.e_end - a.e_begin;
   if (FIX && ne == 0) return;  // the whole grid (the count is the same for every block)
   extern __shared__ float4 smem[];
@@ -2229,7 +2249,7 @@ __device__ __forceinline__ void elem_force_body(const FusedArgs &a, const float4
         }
       }
       dsacc acc, fx, fy, fz;
-      band |= fused_row<EAM, false, V, FIX>(a, g, e, rfirst, ty, jj, level, glane, k, rk,
+      band |= fused_row<EAM, false, V, MODE != PASS>(a, g, e, rfirst, ty, jj, level, glane, k, rk,
                                             reinterpret_cast<const float4 *>(s_k), s_tab, s_fp,
                                             nr, rdr, fpi, lj1, lj2, live, acc, fx, fy, fz);
       if (live && glane == 0) {
@@ -2252,16 +2272,19 @@ __device__ __forceinline__ void elem_force_body(const FusedArgs &a, const float4
       }
       nodef[24 * (size_t) e + lane] = acc.value();
     }
-    if (!FIX && __any_sync(0xffffffffu, band) && lane == 0) band_list(a.band, e, a.nlocal_e);
+    if (!FIX && __any_sync(0xffffffffu, band) && lane == 0) {
+      if (MODE == PASS) band_list(a.band, e, a.nlocal_e);
+      else atomicAdd(a.band + 2, 1);
+    }
     __syncwarp();
   }
   if (FIX) band_done(a.band, ne);
 }
-template <bool EAM, int V, bool FIX, bool STAGE>
-__global__ void __launch_bounds__(fused_block(V), 1)
+template <bool EAM, int V, int MODE, bool STAGE>
+__global__ void __launch_bounds__(MODE == DIRECT ? FEW_BLOCK : fused_block(V), 1)
 k_elem_force_fused(FusedArgs a, const float4 *__restrict__ tab, int nr, float rdr, float lj1,
                    float lj2, const double *__restrict__ erho, double *__restrict__ nodef) {
-  elem_force_body<EAM, V, FIX, STAGE>(a, tab, nr, rdr, lj1, lj2, erho, nodef);
+  elem_force_body<EAM, V, MODE, STAGE>(a, tab, nr, rdr, lj1, lj2, erho, nodef);
 }
 
 #include "elem_stencil.cuh"
@@ -2813,40 +2836,48 @@ static void launch_stencil(const FusedArgs &a, const Stencil &st, int pass, cons
 // elements beside 203,000 atoms: 201 us a step, spread 235; LJ, 2,240 elements
 // beside 129,000 atoms: 111, spread 106).
 template <int V, bool STAGE>
-static void launch_fused(const FusedArgs &a, int pass, const float4 *tab, const EamTables &e,
-                         size_t table, int B, float lj1, float lj2, const double *erho_in,
-                         double *erho_out, double *nodef, const Stencil *st, cudaStream_t s) {
+static int launch_fused(const FusedArgs &a, int pass, const float4 *tab, const EamTables &e,
+                        size_t table, int B, bool few, float lj1, float lj2, const double *erho_in,
+                        double *erho_out, double *nodef, const Stencil *st, cudaStream_t s) {
   const size_t smem = (STAGE ? table : 0) + sizeof(float) * FUSED_WARP_FLOATS * (B / 32);
   const long long items = (long long) (a.e_end - a.e_begin) * 32;
   if (st && pass != 0) {
     launch_stencil(a, *st, pass, tab, e, smem, erho_in, erho_out, nodef, s);
-    const void *fix = pass == 1 ? (const void *) k_elem_rho_fused<V, true, STAGE>
-                                : (const void *) k_elem_force_fused<true, V, true, STAGE>;
+    const void *fix = pass == 1 ? (const void *) k_elem_rho_fused<V, LISTED, STAGE>
+                                : (const void *) k_elem_force_fused<true, V, LISTED, STAGE>;
     const int g = persistent_grid(fix, B, smem, items);
     if (pass == 1)
-      k_elem_rho_fused<V, true, STAGE><<<g, B, smem, s>>>(a, tab, e.nr, (float) e.rdr, erho_out);
+      k_elem_rho_fused<V, LISTED, STAGE><<<g, B, smem, s>>>(a, tab, e.nr, (float) e.rdr, erho_out);
     else
-      k_elem_force_fused<true, V, true, STAGE><<<g, B, smem, s>>>(a, tab, e.nr, (float) e.rdr, 0.f, 0.f,
-                                                                  erho_in, nodef);
-    return;
+      k_elem_force_fused<true, V, LISTED, STAGE><<<g, B, smem, s>>>(a, tab, e.nr, (float) e.rdr, 0.f,
+                                                                    0.f, erho_in, nodef);
+    return 2;
   }
   // the pass, then the exact pass over the elements it listed (a grid of the
-  // same shape; it returns at once when the list is empty)
-  auto run = [&](auto k, auto fix, auto... args) {
+  // same shape; it returns at once when the list is empty); or both in one
+  auto run = [&](auto k, auto fix, auto direct, auto... args) {
+    if constexpr (V == 1)
+      if (few) {
+        const int g = persistent_grid((const void *) direct, B, smem, items);
+        direct<<<g, B, smem, s>>>(a, args...);
+        return 1;
+      }
     const int g = persistent_grid((const void *) k, B, smem, items);
     k<<<g, B, smem, s>>>(a, args...);
     persistent_grid((const void *) fix, B, smem, items);
     fix<<<g, B, smem, s>>>(a, args...);
+    return 2;
   };
   if (pass == 1)
-    run(k_elem_rho_fused<V, false, STAGE>, k_elem_rho_fused<V, true, STAGE>, tab, e.nr, (float) e.rdr,
-        erho_out);
-  else if (pass == 2)
-    run(k_elem_force_fused<true, V, false, STAGE>, k_elem_force_fused<true, V, true, STAGE>, tab, e.nr,
-        (float) e.rdr, 0.f, 0.f, erho_in, nodef);
-  else
-    run(k_elem_force_fused<false, V, false, true>, k_elem_force_fused<false, V, true, true>,
-        (const float4 *) nullptr, 0, 0.f, lj1, lj2, (const double *) nullptr, nodef);
+    return run(k_elem_rho_fused<V, PASS, STAGE>, k_elem_rho_fused<V, LISTED, STAGE>,
+               k_elem_rho_fused<1, DIRECT, STAGE>, tab, e.nr, (float) e.rdr, erho_out);
+  if (pass == 2)
+    return run(k_elem_force_fused<true, V, PASS, STAGE>, k_elem_force_fused<true, V, LISTED, STAGE>,
+               k_elem_force_fused<true, 1, DIRECT, STAGE>, tab, e.nr, (float) e.rdr, 0.f, 0.f, erho_in,
+               nodef);
+  return run(k_elem_force_fused<false, V, PASS, true>, k_elem_force_fused<false, V, LISTED, true>,
+             k_elem_force_fused<false, 1, DIRECT, true>, (const float4 *) nullptr, 0, 0.f, lj1, lj2,
+             (const double *) nullptr, nodef);
 }
 
 bool fused_fits(int nr, int nrho) {
@@ -2858,11 +2889,11 @@ bool fused_fits(int nr, int nrho) {
   return need <= (size_t) optin;
 }
 
-void elem_fused(const MixedElems &m, const FusedTables &t, int pass, const float4 *tab,
+int elem_fused(const MixedElems &m, const FusedTables &t, int pass, const float4 *tab,
                 const EamTables &e, float lj1, float lj2, const double *erho_in, double *erho_out,
                 double *nodef, cudaStream_t s, int e_begin, int e_end) {
   if (e_end < 0) e_end = m.nlocal_e;
-  if (m.nlocal_e <= 0 || e_begin >= e_end) return;
+  if (m.nlocal_e <= 0 || e_begin >= e_end) return 0;
   FusedArgs a{};
   a.e_begin = e_begin;
   a.e_end = e_end;
@@ -2916,16 +2947,19 @@ void elem_fused(const MixedElems &m, const FusedTables &t, int pass, const float
   const int full = t.variant == 0 ? fused_block(0) : fused_block(1);
   const long long warps = ((long long) (e_end - e_begin) + nsm - 1) / std::max(nsm, 1);
   const int B = eam && warps >= 8 ? full : (int) std::min<long long>(full, 32 * std::max(1LL, warps));
+  const bool few = warps < 8 && t.variant == 1;
+  const Stencil *st = t.stencil.state && stencil_fits(t.stencil, pass) ? &t.stencil : nullptr;
+  int n;
   if (eam && B < 256)  // few elements: one arrangement, tables unstaged
-    launch_fused<1, false>(a, pass, tab, e, table, B, lj1, lj2, erho_in, erho_out, nodef, nullptr, s);
+    n = launch_fused<1, false>(a, pass, tab, e, table, B, few, lj1, lj2, erho_in, erho_out, nodef, nullptr, s);
   else if (t.variant == 1)
-    launch_fused<1, true>(a, pass, tab, e, table, B, lj1, lj2, erho_in, erho_out, nodef,
-                          t.stencil.state && stencil_fits(t.stencil, pass) ? &t.stencil : nullptr, s);
+    n = launch_fused<1, true>(a, pass, tab, e, table, B, few, lj1, lj2, erho_in, erho_out, nodef, st, s);
   else if (t.variant == 2)
-    launch_fused<2, true>(a, pass, tab, e, table, B, lj1, lj2, erho_in, erho_out, nodef, nullptr, s);
+    n = launch_fused<2, true>(a, pass, tab, e, table, B, false, lj1, lj2, erho_in, erho_out, nodef, nullptr, s);
   else
-    launch_fused<0, true>(a, pass, tab, e, table, B, lj1, lj2, erho_in, erho_out, nodef, nullptr, s);
+    n = launch_fused<0, true>(a, pass, tab, e, table, B, false, lj1, lj2, erho_in, erho_out, nodef, nullptr, s);
   check(cudaGetLastError(), "elem_fused");
+  return n;
 }
 
 long long self_check(const int *row_start, const int *ent, const int *row_elem, int nrows,
