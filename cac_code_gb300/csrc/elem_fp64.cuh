@@ -32,6 +32,7 @@
 #pragma once
 #include "internal.h"
 #include "soft_fp64.cuh"
+#include <type_traits>
 
 namespace cacg {
 namespace FP64NS {
@@ -41,6 +42,7 @@ namespace {
 constexpr int RB = 8;           // rows of an element per round
 constexpr int ROW_CAP = 96;     // buffered entries per row
 constexpr int ELEM_NT = 128;    // threads per block
+constexpr int FEW_NT = 256, FEW_CL = 4;  // with few elements: threads, or blocks an element
 
 #ifdef FP64_EXACT_TU
 constexpr int NT3 = 3;          // buffered per pair: the three terms
@@ -114,6 +116,17 @@ __device__ __forceinline__ double eam_slope(const EamTables &e, double rho) {
   return (c[0] * p + c[1]) * p + c[2];
 }
 
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// *p of the cluster's first block
+__device__ __forceinline__ void store_first(double *p, double v) {
+  unsigned a = (unsigned) __cvta_generic_to_shared(p);
+  asm volatile("{\n .reg .u32 r;\n mapa.shared::cluster.u32 r, %0, 0;\n st.shared::cluster.f64 [r], %1;\n}"
+               ::"r"(a), "d"(v) : "memory");
+}
+
 // the sums of the weights times N groups of 8 operands (x, y, z, then the densities)
 template <int N>
 __device__ __forceinline__ void soft_dots(const double (&w)[NPE], const soft::Op *s_op, double &x,
@@ -143,11 +156,22 @@ __device__ __forceinline__ void soft_dots(const double (&w)[NPE], const soft::Op
 // DENSITY: the 8 node rows of each element -> erho; otherwise the force rows
 // (row list fjj of the type; all rows when it is null) -> nodef.
 // SELF: every list entry is a site of the row's own element.
-template <bool EAM, bool DENSITY, bool SELF>
-__global__ void __launch_bounds__(ELEM_NT, 7)  // (five blocks an SM, as it comes: 3,630 us, six 3,388)
+// FEW: with few elements a block has an SM's FP64 unit to itself or SMs are idle.  2:
+// twice the threads and no integer arithmetic; 1: a cluster of FEW_CL blocks per element
+// instead, two rows of a round each, whose forces the first block gathers from its shared
+// memory.  EAM forces in the exact mode alone, us, with FEW 1 / 2 / 0: 64 elements 31 / 37 /
+// 51, 128 45 / 37 / 52, 256 84 / 56 / 63, 512 164 / 106 / 78; LJ 12 / 16 / 21, 16 / 16 / 21, 30
+// / 23 / 24, 57 / 42 / 32.  Beside the atom passes, which share the FP64 units, a run: 32
+// elements and 1,024 atoms 706 / 877 / 912, 64 and 16,384 1,885 / 1,719 / 1,838, 128 and 23,232
+// 3,994 / 3,746 / 3,695, 256 and 23,232 4,839 / 4,219 / 3,872: 1 where the atoms' blocks leave
+// SMs idle, 2 up to an element an SM.
+template <bool EAM, bool DENSITY, bool SELF, int FEW>
+__global__ void __launch_bounds__(FEW == 2 ? FEW_NT : ELEM_NT, FEW == 2 ? 2 : FEW ? 4 : 7)
 k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
          double *__restrict__ out) {
   constexpr int NC = DENSITY ? 1 : NT3, NS = DENSITY ? 1 : 3;  // buffered values, sums
+  constexpr int ELEM_NT = FEW == 2 ? FEW_NT : FP64NS::ELEM_NT;
+  constexpr bool SOFT = SELF && FEW == 0, CL = FEW == 1;
   __shared__ double s_nx[24], s_er[NPE], s_p[RB][3], s_N[RB][NPE], s_fpi[RB], s_f[RB][3];
   __shared__ double s_t[RB][NC][ROW_CAP + 1];
   __shared__ int s_ent[RB][ROW_CAP];
@@ -158,16 +182,22 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
   // by the integer units (soft_fp64.cuh): the nodes' coordinates by axis, then their
   // densities; whether all of them can be
   constexpr int NDOT = SOFT_RHO && EAM && !DENSITY ? 4 : 3;
-  __shared__ soft::Op s_op[SELF ? 8 * NDOT : 1];
+  __shared__ soft::Op s_op[SOFT ? 8 * NDOT : 1];
   __shared__ int s_hard;
   float *s_nf = reinterpret_cast<float *>(s_nf4);
-  const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (CL && !DENSITY) cluster_sync();  // the first block runs before others store to it
+  // (a cluster: the gather's rows, of all blocks)
+  __shared__ double s_gN[CL && !DENSITY ? RB : 1][NPE];
+  __shared__ int s_gj[CL && !DENSITY ? RB : 1];
+  const int rank = CL ? (int) blockIdx.x % FEW_CL : 0;
+  const int e = CL ? (int) blockIdx.x / FEW_CL : (int) blockIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ty = a.etype[e], ioff = a.int_off[ty];
   const int naz = a.nae[3 * ty + 2];
   const double *__restrict__ S0 = a.spa_inter + (size_t) a.inter_off[ty] * NPE;
   const float4 *__restrict__ F0 = a.spa_inter_f + (size_t) a.inter_off[ty] * 2;
   const int kb = a.kb, kmask = (1 << kb) - 1;
-  if (SELF) {
+  if (SOFT) {
     if (tid == 0) s_hard = !a.soft;
     __syncthreads();
   }
@@ -176,7 +206,7 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
     if (lane < 24) {
       const double v = a.nodex[24 * (size_t) e + lane];
       s_nx[lane] = v;
-      if (SELF) {
+      if (SOFT) {
         const unsigned h = (unsigned) __double2hiint(v), l = (unsigned) __double2loint(v);
         s_op[lane % 3 * 8 + lane / 3] = soft::op_of(h, l);
         if (!soft::dot_ready(h, l)) s_hard = 1;
@@ -197,9 +227,9 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
     if (lane < NPE) {
       const double v = a.erho[NPE * (size_t) e + lane];
       s_er[lane] = v;
-      if (SELF && NDOT == 4) {
+      if (SOFT && NDOT == 4) {
         const unsigned h = (unsigned) __double2hiint(v), l = (unsigned) __double2loint(v);
-        s_op[SELF ? 8 * (NDOT - 1) + lane : 0] = soft::op_of(h, l);
+        s_op[SOFT ? 8 * (NDOT - 1) + lane : 0] = soft::op_of(h, l);
         if (!soft::dot_ready(h, l)) s_hard = 1;
       }
     }
@@ -207,10 +237,17 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
   const int nr_rows = DENSITY ? NPE : (a.fjj ? a.fjj_off[ty + 1] - a.fjj_off[ty] : a.numint[ty]);
   double nf = 0.0;  // threads 0..23: the nodal force component
   for (int rb = 0; rb < nr_rows; rb += RB) {
-    const int nb = min(RB, nr_rows - rb);
+    const int all = min(RB, nr_rows - rb), lo = CL ? rank * (RB / FEW_CL) : 0;
+    const int nb = CL ? max(0, min(RB / FEW_CL, all - lo)) : all;
     __syncthreads();
+    if (CL && !DENSITY && rank == 0)
+      for (int t = tid; t < all * NPE; t += ELEM_NT) {
+        const int q = rb + t / NPE, jj = a.fjj ? a.fjj[a.fjj_off[ty] + q] : q;
+        s_gN[CL && !DENSITY ? t / NPE : 0][t % NPE] = a.spa_int[((size_t) ioff + jj) * NPE + t % NPE];
+        if (t % NPE == 0) s_gj[CL && !DENSITY ? t / NPE : 0] = jj;
+      }
     if (tid < nb) {
-      const int q = rb + tid;
+      const int q = rb + lo + tid;
       const int jj = DENSITY ? a.node_list[ty * NPE + q] : (a.fjj ? a.fjj[a.fjj_off[ty] + q] : q);
       const int r = a.row_first[e] + jj;
       s_jj[tid] = jj;
@@ -223,8 +260,8 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
     for (int t = tid; t < nb * 3; t += ELEM_NT) {
       const int r = t / 3, d = t % 3;
       if (DENSITY) {
-        s_p[r][d] = s_nx[3 * (rb + r) + d];
-        s_pf[r][d] = s_nf[3 * (rb + r) + d];
+        s_p[r][d] = s_nx[3 * (rb + lo + r) + d];
+        s_pf[r][d] = s_nf[3 * (rb + lo + r) + d];
         continue;
       }
       double w[NPE];
@@ -322,7 +359,7 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
         double S[NPE];
         load8(S0 + (size_t) nj * NPE, S);
         double sx, sy, sz, srho = 0.0;
-        const bool hard = !SELF || s_hard;
+        const bool hard = !SOFT || s_hard;
         if (hard) {
           const double *x = SELF || j == e ? s_nx : a.nodex + 24 * (size_t) j;
           sx = node_sum(S, x, 3);
@@ -413,17 +450,29 @@ k_elem64(Elem64Args a, EamTables eam, double lj1, double lj2, double cutsq,
       __syncthreads();
     }
     if (DENSITY) {
-      if (tid < nb) out[NPE * (size_t) e + rb + tid] = acc;
+      if (tid < nb) out[NPE * (size_t) e + rb + lo + tid] = acc;
     } else {
-      if (tid < 3 * nb) s_f[tid / 3][tid % 3] = acc;
-      __syncthreads();
+      if (tid < 3 * nb) {
+        if (CL) store_first(&s_f[lo + tid / 3][tid % 3], acc);
+        else s_f[tid / 3][tid % 3] = acc;
+      }
+      if (CL) cluster_sync();
+      else __syncthreads();
       // the nodal gather in row order (rows of weight 0 add nothing)
-      if (tid < 24)
-        for (int r = 0; r < nb; r++)
-          nf += a.weight[ioff + s_jj[r]] * s_N[r][tid / 3] * s_f[r][tid % 3];
+      if (rank == 0 && tid < 24) {
+        if (CL) {
+          for (int r = 0; r < all; r++)
+            nf += a.weight[ioff + s_gj[CL && !DENSITY ? r : 0]] *
+                  s_gN[CL && !DENSITY ? r : 0][tid / 3] * s_f[r][tid % 3];
+        } else {
+          for (int r = 0; r < nb; r++)
+            nf += a.weight[ioff + s_jj[r]] * s_N[r][tid / 3] * s_f[r][tid % 3];
+        }
+      }
+      if (CL && rb + RB < nr_rows) cluster_sync();  // s_f is written again
     }
   }
-  if (!DENSITY && tid < 24) out[24 * (size_t) e + tid] = nf;
+  if (!DENSITY && rank == 0 && tid < 24) out[24 * (size_t) e + tid] = nf;
 }
 
 }  // namespace
@@ -448,10 +497,33 @@ void node_floats(const double *nodex, int nelem, float4 *out, cudaStream_t s) {
 void elem_pass(const Elem64Args &a, int pass, bool self, const EamTables &e, double lj1, double lj2,
                double cutsq, double *out, cudaStream_t s) {
   if (a.nlocal_e <= 0) return;
-  auto k = pass == 0 ? (self ? k_elem64<false, false, true> : k_elem64<false, false, false>)
-           : pass == 1 ? (self ? k_elem64<true, true, true> : k_elem64<true, true, false>)
-                       : (self ? k_elem64<true, false, true> : k_elem64<true, false, false>);
-  k<<<a.nlocal_e, ELEM_NT, 0, s>>>(a, e, lj1, lj2, cutsq, out);
+  auto pick = [&](auto few) {
+    constexpr int FEW = decltype(few)::value;
+    return pass == 0 ? (self ? k_elem64<false, false, true, FEW> : k_elem64<false, false, false, FEW>)
+           : pass == 1 ? (self ? k_elem64<true, true, true, FEW> : k_elem64<true, true, false, FEW>)
+                       : (self ? k_elem64<true, false, true, FEW> : k_elem64<true, false, false, FEW>);
+  };
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (3LL * a.nlocal_e <= 2LL * nsm && a.natoms <= 8 * nsm) {
+    cudaLaunchConfig_t c{};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = FEW_CL;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    c.gridDim = dim3(FEW_CL * a.nlocal_e);
+    c.blockDim = dim3(ELEM_NT);
+    c.stream = s;
+    c.attrs = at;
+    c.numAttrs = 1;
+    check(cudaLaunchKernelEx(&c, pick(std::integral_constant<int, 1>{}), a, e, lj1, lj2, cutsq, out),
+          "elem_pass");
+  } else if (a.nlocal_e <= nsm) {
+    pick(std::integral_constant<int, 2>{})<<<a.nlocal_e, FEW_NT, 0, s>>>(a, e, lj1, lj2, cutsq, out);
+  } else {
+    pick(std::integral_constant<int, 0>{})<<<a.nlocal_e, ELEM_NT, 0, s>>>(a, e, lj1, lj2, cutsq, out);
+  }
   check(cudaGetLastError(), "elem_pass");
 }
 

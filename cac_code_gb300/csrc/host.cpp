@@ -3349,12 +3349,8 @@ void cacg_context::pair_ecompute() {
     q.spa_inter_f = d_spa_inter_f.p;
     q.weight = d_weight.p;
     q.maxlines = maxlines;
-    // by the integer units where there are blocks enough to keep the FP64 unit busy
-    // (64 elements, EAM forces: 44 us without, 51 with; 512: 101 and 78)
-    int dev = 0, nsm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    q.soft = spa_soft && enlocal >= 2 * nsm;
+    q.soft = spa_soft;
+    q.natoms = nlocal;
     q.nlocal_e = enlocal;
     q.nae = d_nae.p;
     q.kb = code_kb;

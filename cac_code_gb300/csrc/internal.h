@@ -235,6 +235,7 @@ struct Elem64Args {
   int kb;                       // bits of the site index in a line code
   float cut_pass;               // FP32 limit for absolute coordinates
   int soft;                     // the site shape functions suit soft::dot_ready
+  int natoms;                   // local atoms, whose passes run beside
 };
 
 // ---- forces: same kernels in two translation units (force_fp64.cuh) ----

@@ -78,13 +78,17 @@ def test_soft_sums_are_the_hosts(harness, mode):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("tiny", [False, True])
-def test_exact_forces_of_many_elements(cacg_lib, oracle_lib, tiny):
-    """320 elements, from which on the positions come from the integer units; with
-    ``tiny`` some nodes have coordinates outside their range, and those elements'
-    positions come from the FP64 unit."""
+@pytest.mark.parametrize("layers,tiny", [(4, False), (8, False), (20, False), (20, True)])
+def test_exact_forces(cacg_lib, oracle_lib, layers, tiny):
+    """64 elements and at most 1,216 atoms (a cluster of blocks each), 128 (a block of 256
+    threads) and 320 (positions from the integer units); with ``tiny`` some nodes have
+    coordinates outside their range, and those elements' positions come from the FP64
+    unit."""
     rng = np.random.default_rng(8)
-    m = L.make_slab_model(C.A_CU, L.AnalyticEAM().mass, (2, 22, 22), 11, 20, L.gauss_intp(11, True))
+    m = L.make_slab_model(C.A_CU, L.AnalyticEAM().mass, (2, 22, 22), 11, layers,
+                          L.gauss_intp(11, True))
+    if layers == 4:  # a few atoms of the slab
+        m.atom_x, m.atom_v = m.atom_x[:1200], m.atom_v[:1200]
     m.atom_x = m.atom_x + rng.normal(0.0, 0.05, m.atom_x.shape)
     m.nodex = m.nodex + rng.normal(0.0, 0.05, m.nodex.shape)
     L.remap_into_box(m)
@@ -123,6 +127,6 @@ def test_exact_forces_of_many_elements(cacg_lib, oracle_lib, tiny):
         f, nf = s.atoms()["f"], s.elements()["nodef"]
     finally:
         s.close()
-    assert m.nelements == 320
+    assert m.nelements == 16 * layers
     for got, ref in ((f, fr), (nf, nr)):
         assert np.array_equal(got.view(np.int64), np.ascontiguousarray(ref).view(np.int64))
