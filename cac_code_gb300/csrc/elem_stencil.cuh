@@ -347,6 +347,10 @@ k_elem_stencil(FusedArgs a, Stencil st, int cap, const float4 *__restrict__ tab,
   const float knots = 8388608.f + (float) (nr - 1), fknots = 8388608.f + (float) (a.nrho - 1);
   for (int task = blockIdx.x * nteam + team; task < ntask; task += gridDim.x * nteam) {
     const int e0 = a.e_begin + 32 * task, ne = min(32, a.e_end - e0);
+    // elements whose forces come from the surrogate: computed with the others of their
+    // 32, unless it has all of these, and not written
+    const bool skip = !DENSITY && a.skip && (lane >= ne || a.skip[e0 + lane]);
+    if (__all_sync(0xffffffffu, skip)) continue;
     for (int i = tt; i < 32 * 24; i += STENCIL_TEAM)
       if (i < 24 * ne) s_nx[i / 24 * 25 + i % 24] = __ldg(a.node_hl + 24 * (size_t) e0 + i);
     if (!DENSITY) {
@@ -460,11 +464,12 @@ k_elem_stencil(FusedArgs a, Stencil st, int cap, const float4 *__restrict__ tab,
       }
     }
     // an element with a pair in the guard band is run again from the lists
-    if (far >= a.band_lo && lane < ne) s_mark[lane] = 1;
+    if (far >= a.band_lo && lane < ne && !skip) s_mark[lane] = 1;
     team_sync(team);
     if (!DENSITY)
       for (int i = tt; i < 24 * ne; i += STENCIL_TEAM) {  // the nodal gather, rows ascending
         const int el = i / 24, q = i % 24 / 3, c = i % 3;
+        if (a.skip && a.skip[e0 + el]) continue;
         const float *wt = a.wnf + (size_t) f0 * NPE + q;
         dsacc acc;
         for (int j = 0; j < nrow; j++) {

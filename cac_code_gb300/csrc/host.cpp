@@ -2951,7 +2951,7 @@ void cacg_context::pair_ecompute_mixed() {
     mixed::FusedTables ft{d_node_hl.p, d_nodex.p, d_int_off.p, d_inter_off.p, d_intp4.p,
                           d_spa_int.p, d_spa_inter.p, d_fjj.p, d_fjj_off.p, d_wn.p, maxlines,
                           fused_variant, d_spa_int_hl.p, d_frho_ds.p, d_wnf.p, d_band.p,
-                          d_lat_rec.p, use_sur ? mixed::Stencil{} : stencil};
+                          d_lat_rec.p, stencil};
     // the surrogate's nodal forces go in before the force pass, which skips
     // (writes nothing for) the elements the surrogate evaluates
     auto sur_write = [&] {

@@ -86,3 +86,40 @@ def test_stencil_run_follows_the_lists(cacg_lib, eam_file, vscale):
     assert np.abs(e1["nodex"] - e0["nodex"]).max() < 1e-6
     if vscale > 1.0:
         assert c1["ip_reorders"] >= 2, c1["ip_reorders"]
+
+
+def test_stencil_with_the_surrogate(cacg_lib, eam_file):
+    """Elements that the surrogate evaluates are left as it wrote them, the others get the
+    same bits as without it (an untrained net: every far element, then none)."""
+    m, cfg = _model("alike")
+    net = cacg_lib.Mlp(0, members=2, seed=3)
+    s = cacg.System(0)
+    try:
+        net.set_normalization(np.zeros(32), np.ones(32), np.zeros(24), np.ones(24), 1.0)
+        W.configure_system(s, m, cfg, eam_file)
+        s.set_precision(cacg.MIXED)
+        s.init()
+        s.setup()
+        s.neighbor_build()
+        s.neighbor_ebuild()
+        s.neighbor_nbuild()
+        s.surrogate_reference(m.nodex)
+        s.pair_ecompute()
+        plain = s.elements()["nodef"].copy()
+        s.surrogate_attach(net, tol=1e30, dist=11.0)
+        s.pair_ecompute()
+        far = s.counts()["surrogate_elements"]
+        some = s.elements()["nodef"].copy()
+        changed = np.any(some != plain, axis=(1, 2))
+        assert 0 < far < m.nelements and changed.sum() == far
+        assert np.array_equal(some[~changed], plain[~changed])
+        s.command("tune fused_variant 0")  # from the lists
+        s.pair_ecompute()
+        assert np.array_equal(s.elements()["nodef"][changed], some[changed])
+        s.command("tune fused_variant 1")
+        s.surrogate_attach(net, tol=0.0, dist=11.0)
+        s.pair_ecompute()
+        assert np.array_equal(s.elements()["nodef"], plain)
+    finally:
+        s.close()
+        net.close()
