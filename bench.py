@@ -251,6 +251,10 @@ def cpu_leg(sample, cores, steps, warm, eam):
 # read once per pass; neighbor gathers count as cache hits).  c: counts after
 # the timed steps; L: lattice lines the lists reference (all rows, force rows).
 
+# elements (24 an SM of 152) beyond which the EAM passes share one stencil
+STENCIL_ELEMENTS = 24 * 152
+
+
 def kernel_bytes(name, c, mode, lines_all, lines_force, nae_lines):
     n = c["nlocal"]
     ne = c["enlocal"]
@@ -260,19 +264,18 @@ def kernel_bytes(name, c, mode, lines_all, lines_force, nae_lines):
     scan_e = c["ip_scan_entries"] / max(c["ip_rows"], 1)   # entries scanned per row
     n_s = c["short_entries"] / max(n, 1)
     if mode == "mixed" and c.get("elem_fused"):
-        # the fused element passes (one warp per element): per element the split
-        # nodes 192 (read in both passes), the nodal densities 64 (written by
-        # the density pass, read by the force pass) and the nodal forces 192;
-        # per row the row start pair 8, culling counts 16, lattice indices 16
-        # and the list codes 4 n.  No line or site data reaches memory.
+        # the fused element passes: per element the split nodes 192 (read in both
+        # passes), the nodal densities 64 (written by the density pass, read by
+        # the force pass) and the nodal forces 192; from the lists also, per row,
+        # the row start pair 8, culling counts 16, lattice indices 16 and the list
+        # codes 4 n.  No line or site data reaches memory.
         n_scan = c["density_scan_entries"] / max(n, 1)
+        row = 0 if ne > STENCIL_ELEMENTS else 8 + 16 + 16 + 4 * scan_e
         return {
             "atom1": n * (16 + 4 + 4 * n_scan + 4 + 4 * n_s + 8 + 4),
             "atom2": n * (16 + 4 + 4 * n_s + 4 + 24),
-            "elem_rho": ne * (192 + 64) + rows_n * (8 + 16 + 16 + 4 * scan_e),
-            "elem_force": ne * (192 + 64 + 192) + rows_f * (8 + 16 + 16 + 4 * scan_e),
-            # node split only (the lines are formed on list-reorder steps alone)
-            "sites": ne_all * (192 + 192),
+            "elem_rho": ne * (192 + 64) + rows_n * row,
+            "elem_force": ne * (192 + 64 + 192) + rows_f * row,
         }
     if mode == "mixed":
         n_scan = c["density_scan_entries"] / max(n, 1)
@@ -306,18 +309,18 @@ def kernel_bytes(name, c, mode, lines_all, lines_force, nae_lines):
 
 
 # FP64 operations per launch of the plain FP64 path's kernels (a multiply and
-# an add count two; the site kernels run without contraction, so each is one
-# FP64 instruction).  Sites: 8 nodes x 3 coordinates, a multiply and an add
-# each; site F': 8 density products and sums plus the spline derivative (8);
-# atom density pass: difference, squared distance, root, index and cubic per
-# short-list entry (20); atom force pass: 45 per entry (two splines, the
-# derivative terms and the force components).
+# an add count two, whichever unit carries them out).  Atom density pass:
+# difference, squared distance, root, index and cubic per short-list entry (20);
+# atom force pass: 45 per entry (two splines, the derivative terms and the force
+# components); element force pass, per pair of a Gauss row, with as many pairs in
+# reach as an atom has: the site's position 45, difference and squared distance 8,
+# root and index 14, density and F' 24, splines 14, derivative terms and force 15.
 
 def fp64_flops(name, c):
     n = max(c["nlocal"], 1)
     n_s = c["short_entries"] / n
-    return {"sites": 48.0 * c["sites_needed"], "site_fp": 24.0 * c["sites_needed"],
-            "atom1": 20.0 * c["nlocal"] * n_s, "atom2": 45.0 * c["nlocal"] * n_s}.get(name)
+    return {"atom1": 20.0 * c["nlocal"] * n_s, "atom2": 45.0 * c["nlocal"] * n_s,
+            "elem_force": 120.0 * c["force_rows"] * n_s}.get(name)
 
 
 # ----------------------------------------------------------------------------- arms
@@ -533,11 +536,11 @@ def run_ours(a, ws, rank, local):
     kernel_names = {
         "atom1": "k_eam_rho_atoms (EAM density pass over the atom list)",
         "atom2": "k_eam_force_atoms (EAM force pass over the atom list)",
-        "elem_rho": ("k_elem_rho_fused (nodal densities, one warp per element)"
+        "elem_rho": ("k_elem_stencil / k_elem_rho_fused (nodal densities)"
                      if c1.get("elem_fused") else
                      "k_ipg<EAM, density> (nodal densities over the node rows)"),
-        "elem_force": ("k_elem_force_fused (integration-point forces and nodal gather, one "
-                       "warp per element)" if c1.get("elem_fused") else
+        "elem_force": ("k_elem_stencil / k_elem_force_fused (integration-point forces and "
+                       "nodal gather)" if c1.get("elem_fused") else
                        "k_ipg<EAM, force> (integration-point forces over the Gauss rows)"),
         "sur": "surrogate (features, k_mlp_ensemble, acceptance)",
         "sites": "k_node_split + k_lines (lattice lines)",

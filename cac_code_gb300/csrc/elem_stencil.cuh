@@ -311,6 +311,23 @@ __device__ __forceinline__ void team_sync(int team) {
   asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(STENCIL_TEAM) : "memory");
 }
 
+// the elements of [begin, end) that the surrogate leaves: todo[0] of them (zeroed
+// before), in any order
+__global__ void k_unskipped(const unsigned char *__restrict__ skip, int begin, int end,
+                            int *__restrict__ todo) {
+  const int lane = threadIdx.x & 31;
+  for (int e0 = begin + (int) ((blockIdx.x * blockDim.x + threadIdx.x) & ~31u); e0 < end;
+       e0 += gridDim.x * blockDim.x) {
+    const int e = e0 + lane;
+    const bool left = e < end && !skip[e];
+    const unsigned b = __ballot_sync(0xffffffffu, left);
+    int at = 0;
+    if (lane == 0 && b) at = atomicAdd(todo, __popc(b));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (left) todo[1 + at + __popc(b & ((1u << lane) - 1u))] = e;
+  }
+}
+
 // DENSITY: EAM nodal densities (rows: the element's 8 nodes) into out = erho; else
 // the forces of the rows of nonzero weight gathered onto the nodes, out = nodef.
 // Bound by instruction issue (66 to 75 % of the slots).  C5 (499,712 elements):
@@ -333,7 +350,10 @@ k_elem_stencil(FusedArgs a, Stencil st, int cap, const float4 *__restrict__ tab,
       elem_force_body<true, 1, PASS, true>(a, tab, nr, rdr, 0.f, 0.f, erho, out);
     return;
   }
-  const int ntask = (a.e_end - a.e_begin + 31) / 32, nteam = blockDim.x / STENCIL_TEAM;
+  // with a surrogate: the listed elements (k_unskipped), any 32 of them a task
+  const int *todo = !DENSITY && a.skip ? st.todo + 1 : nullptr;
+  const int count = todo ? st.todo[0] : a.e_end - a.e_begin;
+  const int ntask = (count + 31) / 32, nteam = blockDim.x / STENCIL_TEAM;
   if ((int) blockIdx.x * nteam >= ntask) return;
   const int team = threadIdx.x / STENCIL_TEAM, tt = threadIdx.x % STENCIL_TEAM;
   const int w = tt >> 5, lane = tt & 31;
@@ -346,16 +366,14 @@ k_elem_stencil(FusedArgs a, Stencil st, int cap, const float4 *__restrict__ tab,
   const float band_hi = a.band_hi;
   const float knots = 8388608.f + (float) (nr - 1), fknots = 8388608.f + (float) (a.nrho - 1);
   for (int task = blockIdx.x * nteam + team; task < ntask; task += gridDim.x * nteam) {
-    const int e0 = a.e_begin + 32 * task, ne = min(32, a.e_end - e0);
-    // elements whose forces come from the surrogate: computed with the others of their
-    // 32, unless it has all of these, and not written
-    const bool skip = !DENSITY && a.skip && (lane >= ne || a.skip[e0 + lane]);
-    if (__all_sync(0xffffffffu, skip)) continue;
-    for (int i = tt; i < 32 * 24; i += STENCIL_TEAM)
-      if (i < 24 * ne) s_nx[i / 24 * 25 + i % 24] = __ldg(a.node_hl + 24 * (size_t) e0 + i);
+    const int t0 = 32 * task, ne = min(32, count - t0);
+    auto element = [&](int k) { return todo ? todo[t0 + k] : a.e_begin + t0 + k; };
+    for (int i = tt; i < 24 * ne; i += STENCIL_TEAM)
+      s_nx[i / 24 * 25 + i % 24] = __ldg(a.node_hl + 24 * (size_t) element(i / 24) + i % 24);
     if (!DENSITY) {
       const int el = tt >> 3;
-      const ds v = el < ne ? ds_of_double(__ldg(erho + NPE * (size_t) e0 + tt)) : ds{0.f, 0.f};
+      const ds v = el < ne ? ds_of_double(__ldg(erho + NPE * (size_t) element(el) + (tt & 7)))
+                           : ds{0.f, 0.f};
       s_er[32 * (tt & 7) + el] = make_float2(v.h, v.l);
     }
     if (tt < 32) s_mark[tt] = 0;
@@ -456,7 +474,7 @@ k_elem_stencil(FusedArgs a, Stencil st, int cap, const float4 *__restrict__ tab,
         }
       }
       if (DENSITY) {
-        if (lane < ne) out[NPE * (size_t) (e0 + lane) + r] = fx.value();
+        if (lane < ne) out[NPE * (size_t) element(lane) + r] = fx.value();
       } else {
         s_f[32 * (3 * r) + lane] = make_float2(fx.h, fx.l);
         s_f[32 * (3 * r + 1) + lane] = make_float2(fy.h, fy.l);
@@ -464,12 +482,11 @@ k_elem_stencil(FusedArgs a, Stencil st, int cap, const float4 *__restrict__ tab,
       }
     }
     // an element with a pair in the guard band is run again from the lists
-    if (far >= a.band_lo && lane < ne && !skip) s_mark[lane] = 1;
+    if (far >= a.band_lo && lane < ne) s_mark[lane] = 1;
     team_sync(team);
     if (!DENSITY)
       for (int i = tt; i < 24 * ne; i += STENCIL_TEAM) {  // the nodal gather, rows ascending
         const int el = i / 24, q = i % 24 / 3, c = i % 3;
-        if (a.skip && a.skip[e0 + el]) continue;
         const float *wt = a.wnf + (size_t) f0 * NPE + q;
         dsacc acc;
         for (int j = 0; j < nrow; j++) {
@@ -478,9 +495,9 @@ k_elem_stencil(FusedArgs a, Stencil st, int cap, const float4 *__restrict__ tab,
           acc.add(__fmul_rn(wq, f.x));
           acc.add(__fmul_rn(wq, f.y));
         }
-        out[24 * (size_t) e0 + i] = acc.value();
+        out[24 * (size_t) element(el) + i % 24] = acc.value();
       }
-    if (tt < ne && s_mark[tt]) band_list(a.band, e0 + tt, a.nlocal_e);
+    if (tt < ne && s_mark[tt]) band_list(a.band, element(tt), a.nlocal_e);
     team_sync(team);
   }
 }

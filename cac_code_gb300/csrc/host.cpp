@@ -219,7 +219,7 @@ struct cacg_context {
   DBuf<int> d_band;             // elements with a guard-band pair: count, blocks done, list
   // the shared stencil of the mixed EAM element passes: its rows and slots (ints),
   // entries, least distances, counts, state
-  DBuf<int> d_sten_rows, d_sten_num, d_sten_state;
+  DBuf<int> d_sten_rows, d_sten_num, d_sten_state, d_sten_todo;
   DBuf<float4> d_sten_mono;
   DBuf<unsigned> d_sten_min;
   int sten_slots = 0, sten_force = 0;
@@ -711,6 +711,7 @@ cacg_context::~cacg_context() {
   d_sten_rows.release();
   d_sten_num.release();
   d_sten_state.release();
+  d_sten_todo.release();
   d_sten_mono.release();
   d_sten_min.release();
   d_band.release();
@@ -2880,7 +2881,8 @@ void cacg_context::pair_ecompute_mixed() {
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (fused && sten_slots && pair_style == 2 && enlocal > mixed::STENCIL_PER_SM * nsm)
     stencil = mixed::Stencil{d_sten_rows.p, d_sten_rows.p + sten_slots, sten_slots, sten_force,
-                             inter_num[1], d_sten_mono.p, d_sten_min.p, d_sten_num.p, d_sten_state.p};
+                             inter_num[1], d_sten_mono.p, d_sten_min.p, d_sten_num.p, d_sten_state.p,
+                             nullptr};
   if (fused) {
     kmark(KT_SITES, 1);
     kmark(KT_EPREP, 0);
@@ -2916,6 +2918,10 @@ void cacg_context::pair_ecompute_mixed() {
   epart_fused = fused;
   epart_of = elist_builds;
   const bool use_sur = sur && nfar > 0;
+  if (use_sur && stencil.state) {
+    d_sten_todo.ensure(1 + (size_t) enlocal, s);  // outside captures: the eager step allocates
+    stencil.todo = d_sten_todo.p;
+  }
   const float eps = band_eps;
   mixed::MixedElems m{};
   m.block = mixed_block;

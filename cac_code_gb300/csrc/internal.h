@@ -448,6 +448,7 @@ struct Stencil {
   unsigned *minsq;    // [slot][STENCIL_CAP]: least squared distance at the reorder (float bits)
   int *num;           // [slot]: entries
   int *state;         // valid, counters, the coefficients' ranges (ST_*)
+  int *todo;          // with a surrogate: elements that it leaves, their count first
 };
 struct FusedTables {
   const float2 *node_hl;      // split nodes of this step

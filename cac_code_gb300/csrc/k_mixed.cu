@@ -2823,6 +2823,12 @@ static void launch_stencil(const FusedArgs &a, const Stencil &st, int pass, cons
     const int g = persistent_grid((const void *) k, B, smem, 32LL * (a.e_end - a.e_begin));
     k<<<g, B, smem, s>>>(a, st, cap, tab, e.nr, (float) e.rdr, in, out);
   };
+  if (pass == 2 && a.skip) {
+    check(cudaMemsetAsync(st.todo, 0, sizeof(int), s), "unskipped");
+    const int n = a.e_end - a.e_begin;
+    k_unskipped<<<persistent_grid((const void *) k_unskipped, 256, 0, n), 256, 0, s>>>(a.skip, a.e_begin,
+                                                                                     a.e_end, st.todo);
+  }
   if (pass == 1) run(k_elem_stencil<true>, nullptr, erho_out);
   else run(k_elem_stencil<false>, erho_in, nodef);
 }
@@ -2851,7 +2857,7 @@ static int launch_fused(const FusedArgs &a, int pass, const float4 *tab, const E
     else
       k_elem_force_fused<true, V, LISTED, STAGE><<<g, B, smem, s>>>(a, tab, e.nr, (float) e.rdr, 0.f,
                                                                     0.f, erho_in, nodef);
-    return 2;
+    return pass == 2 && a.skip ? 3 : 2;
   }
   // the pass, then the exact pass over the elements it listed (a grid of the
   // same shape; it returns at once when the list is empty); or both in one
