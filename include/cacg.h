@@ -144,7 +144,7 @@ int cacg_run_host(cacg_handle h, int nsteps, double *x, double *v, double *nodex
    trigger; "tune elists lazy", FP64 and mixed modes) 24 reorders of the mixed
    atom lists so far 25 lattice lines (element, line) with a site in some
    integration-point list 26 of these, lines with a site in a list of a row of
-   nonzero weight 27 1 if the last mixed element pass ran fused (one warp per
+   nonzero weight 27 1 if the last mixed element pass ran fused (element by
    element: every list entry references its row's own element) 28 graph
    launches of the device step loop so far ("tune loop device") 29 rebuild
    decisions taken on the host so far (the device loop takes its own)
