@@ -255,6 +255,20 @@ struct cacg_context {
   bool epart_fused = false;  // the last reorder was the fused passes'
   bool ereorders_zeroed = false;  // the reorder counter (d_misc slot 15)
   bool areorders_zeroed = false;  // the atom-list reorder counter (d_misc slot 16)
+  // the nodes' displacement of nve_nodes_split (d_misc slots 18-19) and its mark (20).
+  // The mark has 32 bits and a run's steps 31: they are zeroed at the head of a run, and
+  // after a split that no pass read (split_unread)
+  bool split_unread = false;
+  mixed::SplitMax split_max() {
+    return {reinterpret_cast<unsigned long long *>(d_misc.p + 18),
+            reinterpret_cast<unsigned *>(d_misc.p + 20)};
+  }
+  void split_reset() {
+    if (!ereorders_zeroed || !d_misc.p) return;  // else the first reorder zeroes them
+    check(cudaMemsetAsync(d_misc.p + 18, 0, 3 * sizeof(int), stream), "split mark");
+    split_unread = false;
+  }
+  bool dmax_zeroed = false;  // slots 11 and 12, by the atoms' first half-step
   // lattice lines that the integration-point lists reference (all rows; force
   // rows), counted at each element list build
   DBuf<unsigned long long> d_nlines;
@@ -2728,10 +2742,13 @@ void cacg_context::pair_compute_mixed(int pass) {
     // against the reorder's packed coordinates when the lists and the grid are
     // unchanged, else set huge so that the lists are reordered in this pass;
     // slot 12: reordered in this pass
-    const bool same = part_of == list_builds && ref_g == g && ref_l0[0] == l0[0] &&
+    const bool parts = pair_style == 2 && !mixed_union;  // else nothing reorders or reads them
+    const bool same = parts && part_of == list_builds && ref_g == g && ref_l0[0] == l0[0] &&
                       ref_l0[1] == l0[1] && ref_l0[2] == l0[2];
-    check(cudaMemsetAsync(d_misc.p + 11, 0, 2 * sizeof(int), s), "dmax, reordered");
-    if (!same) check(cudaMemsetAsync(d_misc.p + 11, 0x7F, sizeof(int), s), "dmax");
+    if (parts && !(dmax_zeroed && same))
+      check(cudaMemsetAsync(d_misc.p + 11, 0, 2 * sizeof(int), s), "dmax, reordered");
+    if (parts && !same) check(cudaMemsetAsync(d_misc.p + 11, 0x7F, sizeof(int), s), "dmax");
+    dmax_zeroed = false;
     const mixed::PackGrid pg = mixed::make_pack_grid(l0, g, d_misc.p + 9);
     const float4 *ref = same ? d_xq_ref.p : nullptr;
     unsigned *dmax = reinterpret_cast<unsigned *>(d_misc.p + 11);
@@ -2862,10 +2879,15 @@ void cacg_context::pair_ecompute_mixed() {
   d_node_ref.ensure((size_t) 24 * nall, s);
   if (!ereorders_zeroed) {
     check(cudaMemsetAsync(d_misc.p + 15, 0, sizeof(int), s), "ereorders");
-    ereorders_zeroed = true;
+    ereorders_zeroed = split_unread = true;
   }
   kmark(KT_SITES, 0);
-  if (!(split_done && fused && same_e)) {  // else the first half-step split the nodes
+  mixed::SplitMax sm{};
+  if (split_done && fused && same_e) {  // the first half-step split the nodes
+    sm = split_max();
+    split_unread = false;
+  } else {
+    if (split_unread) split_reset();
     check(cudaMemsetAsync(d_misc.p + 13, 0, 2 * sizeof(int), s), "edmax, ereordered");
     if (!same_e) check(cudaMemsetAsync(d_misc.p + 13, 0x7F, sizeof(int), s), "edmax");
     mixed::node_split(d_nodex.p, fused ? enlocal : nall, d_node_hl.p, same_e ? d_node_ref.p : nullptr,
@@ -2889,7 +2911,7 @@ void cacg_context::pair_ecompute_mixed() {
     mixed::fused_reorder(d_node_hl.p, d_etype.p, d_row_first.p, d_numint.p, d_int_off.p, d_intp4.p,
                          d_lat_rec.p, lat, maxlines, pg, d_row_start.p, d_ent.p, enlocal, enlocal,
                          (float) std::sqrt(csq_e), d_ent_near.p, d_nnear_row.p, d_node_ref.p, eflags,
-                         stencil, s);
+                         sm, stencil, s);
     kmark(KT_EPREP, 1);
     launches += stencil.state ? 2 : 1;
   } else {
@@ -3568,8 +3590,10 @@ void cacg_context::nve_initial(int which) {
   TypeScale a, e;
   nve_scales(a, e);
   if (which & 1) {
+    dmax_zeroed = mode == CACG_MIXED && pair_style == 2 && !mixed_union && nlocal > 0 &&
+                  part_of == list_builds && d_misc.p;
     launch_nve_atoms_initial(d_x.p, d_v.p, d_f.p, d_type.p, a, nlocal, dt, fast(), kick_a ? 2 : 1,
-                             stream);
+                             dmax_zeroed ? d_misc.p + 11 : nullptr, stream);
     kick_a = false;
     launches++;
   }
@@ -3579,10 +3603,9 @@ void cacg_context::nve_initial(int which) {
     launches++;
     split_done = mode == CACG_MIXED && lazy_eghosts() && epart_of == elist_builds && epart_fused && ereorders_zeroed;
     if (split_done) {
-      unsigned *eflags = reinterpret_cast<unsigned *>(d_misc.p + 13);
-      check(cudaMemsetAsync(eflags, 0, 2 * sizeof(int), stream), "edmax, ereordered");
       mixed::nve_nodes_split(d_ex.p, d_nodex.p, d_nodev.p, d_nodef.p, d_etype.p, e, enlocal, dt, kicks,
-                             d_node_hl.p, d_node_ref.p, eflags, stream);
+                             d_node_hl.p, d_node_ref.p, split_max(), stream);
+      split_unread = true;
     } else {
       launch_nve_nodes_initial(d_ex.p, d_nodex.p, d_nodev.p, d_nodef.p, d_etype.p, e, enlocal, dt,
                                fast(), kicks, stream);
@@ -3658,7 +3681,9 @@ void cacg_context::rebuild(int flags) {
   check_packed_range();
   nrebuild++;
   invalidate_graph();
-  split_done = fwd_pending = false;
+  // (a device loop that stops for a rebuild leaves its last split unread)
+  split_unread = split_unread || mode == CACG_MIXED;
+  split_done = fwd_pending = dmax_zeroed = false;
   if (!rb_ev[0]) {
     check(cudaEventCreate(&rb_ev[0]), "event");
     check(cudaEventCreate(&rb_ev[1]), "event");
@@ -3715,6 +3740,7 @@ void cacg_context::run(int n) {
     neighbor_nbuild();
   }
   if (!fix_nve) fail(CACG_ESTATE, "run without fix nve");
+  split_reset();
   ran = ran || n > 0;
   for (int k = 0; k < 8; k++) t_ms[k] = 0.0;
   for (int k = 0; k < KT_N; k++) t_kern[k] = 0.0;
@@ -3979,6 +4005,7 @@ void cacg_context::run_host(int n, double *x, double *v, double *nodex, double *
     sync();
     return;
   }
+  split_reset();
   if (!cin) check(cudaStreamCreateWithFlags(&cin, cudaStreamNonBlocking), "copy-in stream");
   if (!cout_s) check(cudaStreamCreateWithFlags(&cout_s, cudaStreamNonBlocking), "copy-out stream");
   for (cudaEvent_t *e : {&ev_ain, &ev_nin, &ev_xout, &ev_nxout, &ev_nvout, &ev_end, &ev_hstart,
@@ -4445,7 +4472,7 @@ bool cacg_context::add_loop(cudaGraph_t top, long long &pre, long long &post, bo
     ok = false;
   }
   capturing = false;
-  split_done = fwd_pending = false;
+  split_done = fwd_pending = dmax_zeroed = false;
   launches = l0;
   cudaGetLastError();  // a failed capture leaves its error behind
   return ok;
@@ -4604,7 +4631,7 @@ bool cacg_context::capture_plain_step(int key) {
     launches = l0;
     kick_a = ka;
     kick_n = kn;
-    split_done = fwd_pending = false;
+    split_done = fwd_pending = dmax_zeroed = false;
     return false;
   }
   if (gexec[key]) cudaGraphExecDestroy(gexec[key]);

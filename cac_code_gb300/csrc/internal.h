@@ -403,10 +403,15 @@ void pack_rel(const double4 *x, int n, const PackGrid &pg, float4 *xq, const flo
 // with ref: the largest squared node displacement against ref -> *dmax2 (atomic max)
 void node_split(const double *nodex, int n, float2 *hl, const float2 *ref, unsigned *dmax2,
                 cudaStream_t s);
-// the nodes' first half-step with node_split of the moved nodes
+// the nodes' first half-step with node_split of the moved nodes; the displacement goes to
+// *moved, marked with the mark (both of SplitMax) that fused_reorder moves on
+struct SplitMax {
+  unsigned long long *moved;  // mark << 32 | bits of the largest squared displacement
+  unsigned *mark;             // of the split to come
+};
 void nve_nodes_split(double *ex, double *nodex, double *nodev, const double *nodef, const int *etype,
                      const TypeScale &dtfm, int n, double dtv, int kicks, float2 *hl,
-                     const float2 *ref, unsigned *dmax2, cudaStream_t s);
+                     const float2 *ref, const SplitMax &sm, cudaStream_t s);
 // the ghosts' positions (as launch_forward_atoms_all) and pack_rel of all atoms
 void forward_pack(double4 *x, const int *send, int nlocal, int nghost, const SwapChain &c,
                   const PackGrid &pg, float4 *xq, const float4 *ref, unsigned *dmax2, cudaStream_t s);
@@ -516,12 +521,13 @@ void lj_atoms(const MixedAtoms &m, const int *type, const float *lj1, const floa
               const float *cutsq_t, const double *cutsq64, double *f, cudaStream_t s);
 // every row's integration point: packed, and its double-single position
 // ip_reorder for the fused passes, in one launch (nall_e: elements whose nodes
-// become the reference)
+// become the reference); sm: of nve_nodes_split, or null pointers after node_split
 void fused_reorder(const float2 *node_hl, const int *etype, const int *row_first, const int *numint,
                    const int *int_off, const int4 *intp, const float4 *lat_rec, const Lattice &lat,
                    int maxlines, const PackGrid &pg, const int *row_start, const int *ent,
                    int nlocal_e, int nall_e, float cutoff, int *ent_near, int4 *nnear_row,
-                   float2 *node_ref, unsigned *eflags, const Stencil &st, cudaStream_t s);
+                   float2 *node_ref, unsigned *eflags, const SplitMax &sm, const Stencil &st,
+                   cudaStream_t s);
 void row_q(const int *row_elem, const int *row_jj, const int *etype, const int *int_off,
            const float2 *spa_int_hl, const float2 *node_hl, int nrows, const PackGrid &pg,
            float4 *ip_q, float4 *ip_h, float4 *ip_l, cudaStream_t s);
@@ -637,10 +643,10 @@ void to_float(const double *src, long long n, float *dst, cudaStream_t s);
 // the host forms: no FP64 division per atom on the device
 // fused: one FMA per update (FP64 FMA and mixed modes); else the exact mode's
 // multiply-then-add.  kicks: half-steps before the positions move (2: the
-// previous step's second half-step was left to this one)
+// previous step's second half-step was left to this one).  zero: two words set to 0
 void launch_nve_atoms_initial(double4 *x, double *v, const double *f, const int *type,
                               const TypeScale &dtfm, int n, double dtv, bool fused, int kicks,
-                              cudaStream_t s);
+                              int *zero, cudaStream_t s);
 void launch_nve_atoms_final(double *v, const double *f, const int *type, const TypeScale &dtfm,
                             int n, bool fused, cudaStream_t s);
 void launch_nve_nodes_initial(double *ex, double *nodex, double *nodev, const double *nodef,

@@ -1135,13 +1135,15 @@ k_pack_rel(double4 *__restrict__ x, int n, PackGrid pg, float4 *__restrict__ xq,
 // The nodes' first half-step (k_nve_nodes_initial with fused multiply-adds)
 // with the split of the moved nodes and their largest displacement
 // (k_node_split): the fused passes read the split nodes of owned elements only,
-// so the positions need not be read again.
+// so the positions need not be read again.  The displacement is folded under the step's
+// mark, a higher one each step, so that no memset comes before the kernel (1 us and a
+// dependency at the head of the elements' chain).
 template <int KICKS>
 __global__ void __launch_bounds__(SPLIT_BLOCK)
 k_nve_nodes_split(double *__restrict__ ex, double *__restrict__ nodex, double *__restrict__ nodev,
                   const double *__restrict__ nodef, const int *__restrict__ etype, TypeScale dtfm_t,
                   int n, double dtv, float2 *__restrict__ hl, const float2 *__restrict__ ref,
-                  unsigned *__restrict__ dmax2) {
+                  SplitMax sm) {
   constexpr int ELEMS = SPLIT_BLOCK / NPE;
   __shared__ double sx[ELEMS][3 * NPE + 1];
   __shared__ unsigned s_max[SPLIT_BLOCK / 32];
@@ -1180,7 +1182,12 @@ k_nve_nodes_split(double *__restrict__ ex, double *__restrict__ nodex, double *_
   if (threadIdx.x < 32) {
     unsigned w = threadIdx.x < SPLIT_BLOCK / 32 ? s_max[threadIdx.x] : 0u;
     w = __reduce_max_sync(0xffffffffu, w);
-    if (threadIdx.x == 0 && w) atomicMax(dmax2, w);
+    if (threadIdx.x == 0) {
+      // (the plain look spares most blocks the atomic: the word only grows, and an old
+      // value merely costs one)
+      const unsigned long long mine = (unsigned long long) *sm.mark << 32 | w;
+      if (mine > *(volatile unsigned long long *) sm.moved) atomicMax(sm.moved, mine);
+    }
   }
 }
 
@@ -2295,7 +2302,9 @@ k_elem_force_fused(FusedArgs a, const float4 *__restrict__ tab, int nr, float rd
 // lines of packed points, and the line masks that the unfused passes keep, are
 // not needed: five launches a step less, 6 us of a small system's element
 // chain).  Keeps the nodes as the new reference and counts nodes outside the
-// packed-coordinate range (*oob), as the unfused passes do.
+// packed-coordinate range (*oob), as the unfused passes do.  After nve_nodes_split
+// (sm) it also puts the step's displacement and whether it reordered into eflags for
+// the passes that follow, and moves the mark on.
 constexpr int FR_BLOCK = 256, FR_STRIDE = 24 * 2 + 22;  // floats per half warp: nodes, coefficients
 
 __global__ void __launch_bounds__(FR_BLOCK)
@@ -2305,8 +2314,17 @@ k_fused_reorder(const float2 *__restrict__ node_hl, const int *__restrict__ etyp
                 const float4 *__restrict__ lat_rec, Lattice lat, int maxlines, PackGrid pg,
                 const int *__restrict__ row_start, const int *__restrict__ ent, int nlocal_e,
                 int nall_e, float4 lim, int *__restrict__ ent_near, int4 *__restrict__ nnear_row,
-                float2 *__restrict__ node_ref, unsigned *__restrict__ eflags, Stencil st) {
-  if (moved_little(eflags)) return;  // reads eflags[0] only, which no block writes
+                float2 *__restrict__ node_ref, unsigned *__restrict__ eflags, SplitMax sm,
+                Stencil st) {
+  // reads a word that no block writes: of *sm.moved the low half, else eflags[0]
+  const unsigned *bits = sm.moved ? reinterpret_cast<const unsigned *>(sm.moved) : eflags;
+  const bool little = moved_little(bits);
+  if (sm.moved && blockIdx.x == 0 && threadIdx.x == 0) {
+    eflags[0] = *bits;
+    eflags[1] = 0u;
+    *sm.mark += 1u;
+  }
+  if (little) return;
   __shared__ float2 s_mem[FR_BLOCK / 16][FR_STRIDE / 2];
   // the range of every coefficient over the elements, for the stencil
   __shared__ int s_range[42], s_last;
@@ -2506,11 +2524,11 @@ void forward_pack(double4 *x, const int *send, int nlocal, int nghost, const Swa
 
 void nve_nodes_split(double *ex, double *nodex, double *nodev, const double *nodef, const int *etype,
                      const TypeScale &dtfm, int n, double dtv, int kicks, float2 *hl,
-                     const float2 *ref, unsigned *dmax2, cudaStream_t s) {
+                     const float2 *ref, const SplitMax &sm, cudaStream_t s) {
   if (n <= 0) return;
   auto k = kicks == 2 ? k_nve_nodes_split<2> : k_nve_nodes_split<1>;
   k<<<nblk((long long) n * NPE, SPLIT_BLOCK), SPLIT_BLOCK, 0, s>>>(ex, nodex, nodev, nodef, etype, dtfm,
-                                                                  n, dtv, hl, ref, dmax2);
+                                                                  n, dtv, hl, ref, sm);
   check(cudaGetLastError(), "nve_nodes_split");
 }
 
@@ -2716,13 +2734,14 @@ void fused_reorder(const float2 *node_hl, const int *etype, const int *row_first
                    const int *int_off, const int4 *intp, const float4 *lat_rec, const Lattice &lat,
                    int maxlines, const PackGrid &pg, const int *row_start, const int *ent,
                    int nlocal_e, int nall_e, float cutoff, int *ent_near, int4 *nnear_row,
-                   float2 *node_ref, unsigned *eflags, const Stencil &st, cudaStream_t s) {
+                   float2 *node_ref, unsigned *eflags, const SplitMax &sm, const Stencil &st,
+                   cudaStream_t s) {
   if (nlocal_e <= 0) return;
   const int grid = persistent_grid((const void *) k_fused_reorder, FR_BLOCK, 0, 16LL * nlocal_e);
   k_fused_reorder<<<grid, FR_BLOCK, 0, s>>>(node_hl, etype, row_first, numint, int_off, intp, lat_rec,
                                             lat, maxlines, pg, row_start, ent, nlocal_e, nall_e,
                                             part_limits(cutoff * cutoff, cutoff), ent_near, nnear_row,
-                                            node_ref, eflags, st);
+                                            node_ref, eflags, sm, st);
   if (st.state) {
     const int g2 = persistent_grid((const void *) k_stencil_check, 256, 0, nlocal_e);
     k_stencil_check<<<g2, 256, 0, s>>>(st, node_hl, row_first, nnear_row, nlocal_e,

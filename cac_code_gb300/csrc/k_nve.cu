@@ -13,13 +13,16 @@ inline int nblk(long long n, int t) { return (int) ((n + t - 1) / t); }
 
 // FixNVE::initial_integrate, fix_nve.cpp:54-98 (per-type mass branch).  One
 // thread per component, so the v and f loads of a warp are 256 contiguous
-// bytes; x is the padded double4 array.
+// bytes; x is the padded double4 array.  zero (or null): two words that the
+// step's packing then accumulates to (a memset before it is a node of its own in
+// the atoms' chain: 1 us and a dependency).
 template <bool FUSED, int KICKS>
 __global__ void k_nve_atoms_initial(double4 *__restrict__ x, double *__restrict__ v,
                                     const double *__restrict__ f, const int *__restrict__ type,
-                                    TypeScale dtfm_t, int n, double dtv) {
+                                    TypeScale dtfm_t, int n, double dtv, int *__restrict__ zero) {
   const long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x;
   if (t >= 3LL * n) return;
+  if (zero && t < 2) zero[t] = 0;
   const long long i = t / 3;
   const int d = (int) (t - 3 * i);
   const double vv = kick<FUSED, KICKS>(v[t], type_scale(dtfm_t, type[i]), f[t]);
@@ -195,11 +198,11 @@ __global__ void k_fma_loop(double *out, int iters) {
 
 void launch_nve_atoms_initial(double4 *x, double *v, const double *f, const int *type,
                               const TypeScale &dtfm, int n, double dtv, bool fused,
-                              int kicks, cudaStream_t s) {
+                              int kicks, int *zero, cudaStream_t s) {
   if (n <= 0) return;
   auto k = kicks == 2 ? (fused ? k_nve_atoms_initial<true, 2> : k_nve_atoms_initial<false, 2>)
                       : (fused ? k_nve_atoms_initial<true, 1> : k_nve_atoms_initial<false, 1>);
-  k<<<nblk(3LL * n, 256), 256, 0, s>>>(x, v, f, type, dtfm, n, dtv);
+  k<<<nblk(3LL * n, 256), 256, 0, s>>>(x, v, f, type, dtfm, n, dtv, zero);
   check(cudaGetLastError(), "nve_atoms_initial");
 }
 
