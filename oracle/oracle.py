@@ -21,6 +21,9 @@ REF_BIN = os.path.join(HERE, "_ref", "cacref")
 # beside the repository
 REF_TREE = os.environ.get("CAC_REFERENCE_TREE",
                           os.path.normpath(os.path.join(HERE, "..", "..", "reference")))
+if not os.path.exists(os.path.join(REF_TREE, "main.cpp")):
+    # a directory without the sources (an empty mount) counts as absent
+    REF_TREE = os.path.join(REF_TREE, "absent")
 
 _dp = ctypes.POINTER(ctypes.c_double)
 _ip = ctypes.POINTER(ctypes.c_int)
