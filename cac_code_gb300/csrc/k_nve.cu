@@ -15,7 +15,7 @@ inline int nblk(long long n, int t) { return (int) ((n + t - 1) / t); }
 // thread per component, so the v and f loads of a warp are 256 contiguous
 // bytes; x is the padded double4 array.  zero (or null): two words that the
 // step's packing then accumulates to (a memset before it is a node of its own in
-// the atoms' chain: 1 us and a dependency).
+// the atoms' chain: 9,677 atoms with 160 elements 44.6 us a step, 42.0 without it).
 template <bool FUSED, int KICKS>
 __global__ void k_nve_atoms_initial(double4 *__restrict__ x, double *__restrict__ v,
                                     const double *__restrict__ f, const int *__restrict__ type,

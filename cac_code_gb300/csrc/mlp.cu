@@ -77,7 +77,8 @@ struct UpdateArgs {
 
 // blockIdx.y: member; the first WB blocks take the weights (a thread each), the
 // others the biases (a warp each: the column sum of the gradient, by 256 rows,
-// of these by eights, in order)
+// of these by eights, in order: the same bits on every run, where atomics add the
+// parts as blocks arrive)
 constexpr int UB = 256;
 constexpr int WB = (int) ((WEIGHTS + UB - 1) / UB), BB = (BIASES + UB / 32 - 1) / (UB / 32);
 

@@ -305,8 +305,8 @@ int cacg_get_timing(cacg_handle h, double *ms, int n);
    cacg_set_timing(h, 1), summed over the eagerly run steps): [0] atom pass 1
    (LJ forces or EAM densities and F'), [1] atom pass 2 (EAM forces), [2]
    nodal densities (element density pass), [3] integration-point forces, [4]
-   surrogate (features, ensemble, acceptance), [5] element sites (FP64 modes)
-   or lattice lines (mixed), [6] mixed atom-list reorder, [7] mixed
+   surrogate (features, ensemble, acceptance), [5] element sites or lattice
+   lines (where a path forms them as a pass of their own), [6] mixed atom-list reorder, [7] mixed
    integration-point rows, reorder and line masks, [8] site F'(rho); then [9]
    the device milliseconds of every rebuild since the handle was created
    (Neighbor::decide -> reneighbor branch of verlet.cpp:184-198, timing on or
