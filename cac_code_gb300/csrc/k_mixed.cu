@@ -2971,9 +2971,12 @@ int elem_fused(const MixedElems &m, const FusedTables &t, int pass, const float4
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const int full = t.variant == 0 ? fused_block(0) : fused_block(1);
   const long long warps = ((long long) (e_end - e_begin) + nsm - 1) / std::max(nsm, 1);
-  const int B = eam && warps >= 8 ? full : (int) std::min<long long>(full, 32 * std::max(1LL, warps));
-  const bool few = warps < 8 && t.variant == 1;
-  const Stencil *st = t.stencil.state && stencil_fits(t.stencil, pass) ? &t.stencil : nullptr;
+  // the stencil: by the whole number of elements (the caller's choice), never by this
+  // launch's part of them, so that a step in parts sums in the same order as one in one
+  const Stencil *st =
+      eam && t.variant == 1 && t.stencil.state && stencil_fits(t.stencil, pass) ? &t.stencil : nullptr;
+  const int B = st || (eam && warps >= 8) ? full : (int) std::min<long long>(full, 32 * std::max(1LL, warps));
+  const bool few = warps < 8 && t.variant == 1 && !st;
   int n;
   if (eam && B < 256)  // few elements: one arrangement, tables unstaged
     n = launch_fused<1, false>(a, pass, tab, e, table, B, few, lj1, lj2, erho_in, erho_out, nodef, nullptr, s);
