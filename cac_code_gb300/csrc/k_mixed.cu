@@ -2743,8 +2743,8 @@ void fused_reorder(const float2 *node_hl, const int *etype, const int *row_first
                                             part_limits(cutoff * cutoff, cutoff), ent_near, nnear_row,
                                             node_ref, eflags, sm, st);
   if (st.state) {
-    const int g2 = persistent_grid((const void *) k_stencil_check, 256, 0, nlocal_e);
-    k_stencil_check<<<g2, 256, 0, s>>>(st, node_hl, row_first, nnear_row, nlocal_e,
+    const int g2 = persistent_grid((const void *) k_stencil_check, CHECK_NT, 0, 8LL * nlocal_e);
+    k_stencil_check<<<g2, CHECK_NT, 0, s>>>(st, node_hl, row_first, nnear_row, nlocal_e,
                                        part_limits(cutoff * cutoff, cutoff), eflags);
   }
   check(cudaGetLastError(), "fused_reorder");

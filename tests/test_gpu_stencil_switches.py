@@ -47,3 +47,33 @@ def test_run_host_in_small_parts_follows_run(cacg_lib, alike, eam_file, parts): 
     finally:
         a.close()
         b.close()
+
+
+def _reorder_us(eam, layers, jitter):
+    """Device time of a step's element list reorder, the least of six."""
+    m, cfg = W.c2_eam(cells=(4, 22, 22), layers=layers, seed=17)
+    m.nodex = m.nodex + np.random.default_rng(5).normal(0.0, jitter, m.nodex.shape)
+    s = _system(m, cfg, eam)
+    try:
+        s.command("neigh_modify every 100000 delay 0 check yes")
+        s.set_graphs(False)
+        s.run(2)
+        x, t = s.elements()["nodex"].copy(), []
+        before = s.counts()["ip_reorders"]
+        for k in range(6):
+            s.put_nodes(x + (0.6 if k % 2 == 0 else 0.0), np.zeros_like(x))  # 0.6 A to and fro
+            s.set_timing(True)
+            s.run(1)
+            t.append(1e3 * s.kernel_timing()[7])
+        assert s.counts()["ip_reorders"] - before == 6
+        return min(t)
+    finally:
+        s.close()
+
+
+@pytest.mark.parametrize("jitter", [0.05, 1.0])
+def test_reorder_with_the_stencil_costs_little_more(cacg_lib, eam_file, jitter):  # noqa: F811
+    """A reorder of 3,664 elements builds and checks a stencil, whether it stands (alike) or
+    not; one of 3,632 does not.  Both work on the same lists, so at most three times."""
+    few, many = (_reorder_us(eam_file, n, jitter) for n in (227, 229))
+    assert many <= 3.0 * few, (few, many)
