@@ -99,7 +99,7 @@ __device__ void stencil_build(const Stencil &st, const FusedLat &g, const int4 *
       if (keep && at < STENCIL_CAP) {
         const size_t o = (size_t) q * STENCIL_CAP + at;
         st.mono[2 * o] = make_float4(m.a, m.b, m.c, m.ab);
-        st.mono[2 * o + 1] = make_float4(m.ac, m.bc, m.abc, 0.f);
+        st.mono[2 * o + 1] = make_float4(m.ac, m.bc, m.abc, __int_as_float(s));
         st.minsq[o] = 0x7F800000u;
       }
       n += __popc(b);
@@ -278,20 +278,23 @@ __host__ __device__ constexpr int team_float2(int nf) {
 }
 constexpr int STENCIL_ENT = 16;  // floats of a staged entry
 
+// The rows' entries, all of them (the choice between stencil and lists does not depend on
+// the culling), fit in cap?
+__device__ __forceinline__ bool stencil_room(const Stencil &st, const int *slot, int nrow, int cap) {
+  int all = 0;
+  for (int r = 0; r < nrow; r++) all += st.num[slot[r]];
+  return all <= cap;
+}
+
 // The stencil's entries in reach (all of them without culling), for the pass's rows,
 // into s_ent (every monomial twice: a packed operand for both halves; then whether the
-// FP32 sums end here); s_off[r] the first of row r.  False (for every thread) if the
-// rows have more than cap.
-__device__ __forceinline__ bool stencil_stage(const Stencil &st, const int *slot, int nrow,
-                                              const unsigned *eflags, bool cull, float cutsq, int cap,
+// FP32 sums end here, and the site); s_off[r] the first of row r.
+__device__ __forceinline__ void stencil_stage(const Stencil &st, const int *slot, int nrow,
+                                              const unsigned *eflags, bool cull, float cutsq,
                                               float *s_ent, int *s_off) {
   const float d = (eflags[1] ? 0.f : 2.0f * sqrtf(__uint_as_float(eflags[0]))) + CULL_MARGIN;
   const float rl = sqrtf(cutsq) + d, lim = cull ? rl * rl * 1.00001f : INFINITY;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  // (all of them count: the choice does not depend on the culling)
-  int all = 0;
-  for (int r = 0; r < nrow; r++) all += st.num[slot[r]];
-  if (all > cap) return false;
   for (int r = w; r < nrow; r += nw) {
     const int q = slot[r], n = st.num[q];
     int c = 0;
@@ -323,13 +326,12 @@ __device__ __forceinline__ bool stencil_stage(const Stencil &st, const int *slot
         p[0] = make_float4(ma.x, ma.x, ma.y, ma.y);
         p[1] = make_float4(ma.z, ma.z, ma.w, ma.w);
         p[2] = make_float4(mb.x, mb.x, mb.y, mb.y);
-        p[3] = make_float4(mb.z, mb.z, last ? 1.f : 0.f, 0.f);
+        p[3] = make_float4(mb.z, mb.z, last ? 1.f : 0.f, mb.w);
       }
       at += __popc(b);
     }
   }
   __syncthreads();
-  return true;
 }
 
 __device__ __forceinline__ void team_sync(int team) {
@@ -358,28 +360,37 @@ __global__ void k_unskipped(const unsigned char *__restrict__ skip, int begin, i
 // Bound by instruction issue (66 to 75 % of the slots).  C5 (499,712 elements):
 // densities 550 -> 225 us, forces 1,917 -> 940 us; 64,000 elements: 90 -> 35 and 277 ->
 // 138 us.
-template <bool DENSITY>
+// LISTED: the listed elements again, any 32 of them a task, with the guard band's pairs
+// decided in FP64 and the sums as in the pass itself, so that neither the band's width nor
+// a pair that enters it changes a bit beyond the decisions.
+template <bool DENSITY, int MODE>
 __global__ void __launch_bounds__(STENCIL_TEAM *STENCIL_TEAMS, 1)
 k_elem_stencil(FusedArgs a, Stencil st, int cap, const float4 *__restrict__ tab, int nr, float rdr,
                const double *__restrict__ erho, double *__restrict__ out) {
   extern __shared__ float4 smem[];
   __shared__ int s_off[FUSED_MAXF + 1];
+  constexpr bool FIX = MODE == LISTED;
+  const int nfix = FIX ? min(a.band[0], a.nlocal_e) : 0;
+  if (FIX && nfix == 0) return;  // the whole grid (the count is the same for every block)
   const int nrow = DENSITY ? NPE : st.nf;
   float *s_ent = reinterpret_cast<float *>(smem);
-  if (st.state[ST_VALID] == 0 ||
-      !stencil_stage(st, st.slot + (DENSITY ? st.nf : 0), nrow, a.eflags, a.nnear_row != nullptr, a.cutsq_f, cap,
-                     s_ent, s_off)) {
+  // with a surrogate: the listed elements (k_unskipped), any 32 of them a task
+  const int *todo = FIX ? a.band + BAND_LIST : !DENSITY && a.skip ? st.todo + 1 : nullptr;
+  const int count = FIX ? nfix : todo ? st.todo[0] : a.e_end - a.e_begin;
+  const int ntask = (count + 31) / 32, nteam = blockDim.x / STENCIL_TEAM;
+  const int *slot = st.slot + (DENSITY ? st.nf : 0);
+  if (st.state[ST_VALID] == 0 || !stencil_room(st, slot, nrow, cap)) {
     if (DENSITY)
-      elem_rho_body<1, PASS, true>(a, tab, nr, rdr, out);
+      elem_rho_body<1, MODE, true>(a, tab, nr, rdr, out);
     else
-      elem_force_body<true, 1, PASS, true>(a, tab, nr, rdr, 0.f, 0.f, erho, out);
+      elem_force_body<true, 1, MODE, true>(a, tab, nr, rdr, 0.f, 0.f, erho, out);
     return;
   }
-  // with a surrogate: the listed elements (k_unskipped), any 32 of them a task
-  const int *todo = !DENSITY && a.skip ? st.todo + 1 : nullptr;
-  const int count = todo ? st.todo[0] : a.e_end - a.e_begin;
-  const int ntask = (count + 31) / 32, nteam = blockDim.x / STENCIL_TEAM;
-  if ((int) blockIdx.x * nteam >= ntask) return;
+  if ((int) blockIdx.x * nteam >= ntask) {
+    if (FIX) band_done(a.band, nfix);
+    return;
+  }
+  stencil_stage(st, slot, nrow, a.eflags, a.nnear_row != nullptr, a.cutsq_f, s_ent, s_off);
   const int team = threadIdx.x / STENCIL_TEAM, tt = threadIdx.x % STENCIL_TEAM;
   const int w = tt >> 5, lane = tt & 31;
   float2 *s_kx = reinterpret_cast<float2 *>(s_ent + (size_t) STENCIL_ENT * cap) +
@@ -388,7 +399,7 @@ k_elem_stencil(FusedArgs a, Stencil st, int cap, const float4 *__restrict__ tab,
   float2 *s_f = s_nx;
   int *s_mark = reinterpret_cast<int *>(s_kx + TEAM_MARK);
   const int f0 = a.fjj_off[1], ioff = a.int_off[1];  // (one element type)
-  const float band_hi = a.band_hi;
+  const float band_lo = a.band_lo, band_hi = a.band_hi;
   const float knots = 8388608.f + (float) (nr - 1), fknots = 8388608.f + (float) (a.nrho - 1);
   for (int task = blockIdx.x * nteam + team; task < ntask; task += gridDim.x * nteam) {
     const int t0 = 32 * task, ne = min(32, count - t0);
@@ -431,7 +442,9 @@ k_elem_stencil(FusedArgs a, Stencil st, int cap, const float4 *__restrict__ tab,
       kz[m] = f2_of(v.x, v.y);
     }
     float far = 0.f;  // the largest squared distance up to the guard band's end
+    const int mine = FIX ? element(min(lane, ne - 1)) : 0;
     for (int r = w; r < nrow; r += STENCIL_TEAM / 32) {
+      const int jj = FIX ? (DENSITY ? a.node_list[NPE + r] : a.fjj[f0 + r]) : 0;
       float fpi = 0.f, rho_p = 0.f;
       if (!DENSITY)
         fpi = row_fprime_ds<32>(a.spa_int_hl + ((size_t) ioff + a.fjj[f0 + r]) * NPE, s_er + lane,
@@ -462,8 +475,14 @@ k_elem_stencil(FusedArgs a, Stencil st, int cap, const float4 *__restrict__ tab,
         v = f2_fma(kz[6], m6, v);
         const float dx = f2_lo(u), dy = f2_hi(u), dz = f2_lo(v);
         const float rsq = fmaf(dz, dz, fmaf(dx, dx, dy * dy));
-        if (rsq <= band_hi) {
-          far = fmaxf(far, rsq);
+        bool in = rsq <= band_hi;
+        if (FIX)
+          in = stencil_band64(in && rsq >= band_lo && lane < ne, rsq < a.cutsq_f,
+                              a.spa_int + ((size_t) ioff + jj) * NPE,
+                              a.spa_inter + ((size_t) a.inter_off[1] + __float_as_int(f2_hi(fl))) * NPE,
+                              a.nodex, mine, a.cutsq);
+        if (in) {
+          if (!FIX) far = fmaxf(far, rsq);
           const float recip = rsqrt_normal(rsq);
           int m;
           const float p = knot_of<false>(fmaf(rsq * recip, rdr, 1.0f), knots, m);
@@ -506,8 +525,8 @@ k_elem_stencil(FusedArgs a, Stencil st, int cap, const float4 *__restrict__ tab,
         s_f[32 * (3 * r + 2) + lane] = make_float2(fz.h, fz.l);
       }
     }
-    // an element with a pair in the guard band is run again from the lists
-    if (far >= a.band_lo && lane < ne) s_mark[lane] = 1;
+    // an element with a pair in the guard band is run again
+    if (!FIX && far >= band_lo && lane < ne) s_mark[lane] = 1;
     team_sync(team);
     if (!DENSITY)
       for (int i = tt; i < 24 * ne; i += STENCIL_TEAM) {  // the nodal gather, rows ascending
@@ -522,7 +541,8 @@ k_elem_stencil(FusedArgs a, Stencil st, int cap, const float4 *__restrict__ tab,
         }
         out[24 * (size_t) element(el) + i % 24] = acc.value();
       }
-    if (tt < ne && s_mark[tt]) band_list(a.band, element(tt), a.nlocal_e);
+    if (!FIX && tt < ne && s_mark[tt]) band_list(a.band, element(tt), a.nlocal_e);
     team_sync(team);
   }
+  if (FIX) band_done(a.band, nfix);
 }

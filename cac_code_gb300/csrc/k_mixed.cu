@@ -1813,29 +1813,51 @@ __device__ __forceinline__ float row_fprime_ds(const float2 *__restrict__ N,
   return fprime_ds(rho, c3, nrho, rdrho);
 }
 
-// FP64 cutoff decisions of a warp's guard-band pairs (band: this lane has one; row,
-// site: its shape functions' rows in N and M; x: the element's FP64 nodes), one pair
-// after another: six lanes interpolate a coordinate each of the row's point and the
-// site.  By the lane that has the pair the decision is 54 FP64 instructions, which
-// cost a warp the same for one lane as for all; so it is 12.
+// FP64 cutoff decisions of a warp's guard-band pairs, one pair after another: six lanes
+// interpolate a coordinate each of the row's point and the site.  By the lane that has the
+// pair the decision is 54 FP64 instructions, which cost a warp the same for one lane as for
+// all; so it is 12.
+
+// One pair (the same for all lanes): w, m the shape functions of its row and site, x the
+// element's FP64 nodes
+__device__ __forceinline__ bool pair_inside64(const double *__restrict__ w, const double *__restrict__ m,
+                                              const double *__restrict__ x, double cutsq) {
+  const int lane = threadIdx.x & 31;
+  double p = 0.0;
+  if (lane < 6) {
+    const double *v = lane < 3 ? w : m, *y = x + lane % 3;
+#pragma unroll
+    for (int k = 0; k < NPE; k++) p = fma(v[k], y[3 * k], p);
+  }
+  const double d = p - __shfl_down_sync(0xffffffffu, p, 3);
+  const double dx = __shfl_sync(0xffffffffu, d, 0), dy = __shfl_sync(0xffffffffu, d, 1),
+               dz = __shfl_sync(0xffffffffu, d, 2);
+  return fma(dz, dz, fma(dy, dy, dx * dx)) < cutsq;
+}
+
+// band: this lane has one; row, site: its shape functions' rows in N and M; x: the
+// warp's element
 __device__ __noinline__ bool fused_band64(bool band, bool in, const double *__restrict__ N, int row,
                                           const double *__restrict__ M, int site,
                                           const double *__restrict__ x, double cutsq) {
-  const int lane = threadIdx.x & 31;
   for (unsigned todo = __ballot_sync(0xffffffffu, band); todo; todo &= todo - 1) {
     const int src = __ffs(todo) - 1;
     const int r = __shfl_sync(0xffffffffu, row, src), m = __shfl_sync(0xffffffffu, site, src);
-    double p = 0.0;
-    if (lane < 6) {
-      const double *w = (lane < 3 ? N + (size_t) r * NPE : M + (size_t) m * NPE), *y = x + lane % 3;
-#pragma unroll
-      for (int k = 0; k < NPE; k++) p = fma(w[k], y[3 * k], p);
-    }
-    const double d = p - __shfl_down_sync(0xffffffffu, p, 3);
-    const double dx = __shfl_sync(0xffffffffu, d, 0), dy = __shfl_sync(0xffffffffu, d, 1),
-                 dz = __shfl_sync(0xffffffffu, d, 2);
-    const bool inside = fma(dz, dz, fma(dy, dy, dx * dx)) < cutsq;
-    if (lane == src) in = inside;
+    const bool inside = pair_inside64(N + (size_t) r * NPE, M + (size_t) m * NPE, x, cutsq);
+    if ((threadIdx.x & 31) == src) in = inside;
+  }
+  return in;
+}
+
+// the same for an element e (nodes in nodex) a lane and one row w and site m
+__device__ __noinline__ bool stencil_band64(bool band, bool in, const double *__restrict__ w,
+                                            const double *__restrict__ m,
+                                            const double *__restrict__ nodex, int e, double cutsq) {
+  for (unsigned todo = __ballot_sync(0xffffffffu, band); todo; todo &= todo - 1) {
+    const int src = __ffs(todo) - 1;
+    const bool inside =
+        pair_inside64(w, m, nodex + 24 * (size_t) __shfl_sync(0xffffffffu, e, src), cutsq);
+    if ((threadIdx.x & 31) == src) in = inside;
   }
   return in;
 }
@@ -2826,18 +2848,19 @@ static bool stencil_fits(const Stencil &st, int pass) {
   return stencil_smem(st, pass, STENCIL_TEAMS) + 1024 <= (size_t) optin;  // and the static part
 }
 
-// teams as many as spread the elements over all SMs, at most three a block
-static void launch_stencil(const FusedArgs &a, const Stencil &st, int pass, const float4 *tab,
-                           const EamTables &e, size_t lists_smem, const double *erho_in,
-                           double *erho_out, double *nodef, cudaStream_t s) {
+// The pass and the exact pass over the elements that it listed, in the same order of
+// summation; the number of launches.  Teams as many as spread the elements over all SMs, at
+// most three a block.
+static int launch_stencil(const FusedArgs &a, const Stencil &st, int pass, const float4 *tab,
+                          const EamTables &e, size_t lists_smem, const double *erho_in,
+                          double *erho_out, double *nodef, cudaStream_t s) {
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const int ntask = (a.e_end - a.e_begin + 31) / 32, cap = stencil_cap(st, pass);
-  const int teams = std::max(1, std::min(STENCIL_TEAMS, (ntask + nsm - 1) / std::max(nsm, 1)));
-  const size_t smem = std::max(lists_smem, stencil_smem(st, pass, teams));
-  const int B = STENCIL_TEAM * teams;
-  auto run = [&](auto k, const double *in, double *out) {
+  auto run = [&](auto k, int teams, const double *in, double *out) {
+    const size_t smem = std::max(lists_smem, stencil_smem(st, pass, teams));
+    const int B = STENCIL_TEAM * teams;
     // (blocks for the passes from the lists, which the stencil's absence falls back to)
     const int g = persistent_grid((const void *) k, B, smem, 32LL * (a.e_end - a.e_begin));
     k<<<g, B, smem, s>>>(a, st, cap, tab, e.nr, (float) e.rdr, in, out);
@@ -2848,8 +2871,15 @@ static void launch_stencil(const FusedArgs &a, const Stencil &st, int pass, cons
     k_unskipped<<<persistent_grid((const void *) k_unskipped, 256, 0, n), 256, 0, s>>>(a.skip, a.e_begin,
                                                                                      a.e_end, st.todo);
   }
-  if (pass == 1) run(k_elem_stencil<true>, nullptr, erho_out);
-  else run(k_elem_stencil<false>, erho_in, nodef);
+  const int teams = std::max(1, std::min(STENCIL_TEAMS, (ntask + nsm - 1) / std::max(nsm, 1)));
+  if (pass == 1) {
+    run(k_elem_stencil<true, PASS>, teams, nullptr, erho_out);
+    run(k_elem_stencil<true, LISTED>, STENCIL_TEAMS, nullptr, erho_out);
+  } else {
+    run(k_elem_stencil<false, PASS>, teams, erho_in, nodef);
+    run(k_elem_stencil<false, LISTED>, STENCIL_TEAMS, erho_in, nodef);
+  }
+  return pass == 2 && a.skip ? 3 : 2;
 }
 
 // Blocks of as many warps as spread the elements over all SMs, up to the
@@ -2866,18 +2896,8 @@ static int launch_fused(const FusedArgs &a, int pass, const float4 *tab, const E
                         double *erho_out, double *nodef, const Stencil *st, cudaStream_t s) {
   const size_t smem = (STAGE ? table : 0) + sizeof(float) * FUSED_WARP_FLOATS * (B / 32);
   const long long items = (long long) (a.e_end - a.e_begin) * 32;
-  if (st && pass != 0) {
-    launch_stencil(a, *st, pass, tab, e, smem, erho_in, erho_out, nodef, s);
-    const void *fix = pass == 1 ? (const void *) k_elem_rho_fused<V, LISTED, STAGE>
-                                : (const void *) k_elem_force_fused<true, V, LISTED, STAGE>;
-    const int g = persistent_grid(fix, B, smem, items);
-    if (pass == 1)
-      k_elem_rho_fused<V, LISTED, STAGE><<<g, B, smem, s>>>(a, tab, e.nr, (float) e.rdr, erho_out);
-    else
-      k_elem_force_fused<true, V, LISTED, STAGE><<<g, B, smem, s>>>(a, tab, e.nr, (float) e.rdr, 0.f,
-                                                                    0.f, erho_in, nodef);
-    return pass == 2 && a.skip ? 3 : 2;
-  }
+  if (st && pass != 0)
+    return launch_stencil(a, *st, pass, tab, e, smem, erho_in, erho_out, nodef, s);
   // the pass, then the exact pass over the elements it listed (a grid of the
   // same shape; it returns at once when the list is empty); or both in one
   auto run = [&](auto k, auto fix, auto direct, auto... args) {

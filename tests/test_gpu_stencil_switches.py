@@ -77,3 +77,29 @@ def test_reorder_with_the_stencil_costs_little_more(cacg_lib, eam_file, jitter):
     not; one of 3,632 does not.  Both work on the same lists, so at most three times."""
     few, many = (_reorder_us(eam_file, n, jitter) for n in (227, 229))
     assert many <= 3.0 * few, (few, many)
+
+
+@pytest.mark.parametrize("shape", ["alike", "shrunk", "crooked"])
+def test_band_width_changes_no_bit(cacg_lib, eam_file, shape):  # noqa: F811
+    """Widened to cutsq (1 +- 0.1), the guard band holds a lattice shell, so that every
+    element is run again with FP64 decisions, at every pass; these are the decisions of the
+    default band, and the sums are taken in the same order: 8 steps to the bit, from the
+    stencil (alike, shrunk) and from the lists (crooked)."""
+    m, cfg = _model(shape)
+    out = []
+    for tune in ((), ("band 0.1",)):
+        s = _system(m, cfg, eam_file, *tune)
+        try:
+            s.pair_compute()
+            s.pair_ecompute()
+            f = s.elements()["nodef"].copy()
+            s.run(8)
+            out.append((f, s.elements(), s.counts()))
+        finally:
+            s.close()
+    (f0, e0, c0), (f1, e1, c1) = out
+    assert c1["elem_fused"] == 1
+    assert c1["band_reruns"] >= 2 * (1 + 8) * c1["enlocal"] > c0["band_reruns"]
+    assert np.array_equal(f0.view(np.int64), f1.view(np.int64))
+    for k in ("nodex", "nodev", "nodef"):
+        assert np.array_equal(e0[k], e1[k]), k
