@@ -804,6 +804,15 @@ CUtensorMap make_map(const void *ptr, int rows, int cols, int ld, int box_rows) 
   return m;
 }
 
+// Raises a kernel's limit of dynamic shared memory before a launch.  The limit belongs to
+// the device's context, so it is set each time: remembered once a process, it would be
+// missing on a second device and after a reset.  Always the same size for a kernel, so that
+// another thread's launch finds it large enough.
+void allow_smem(const void *kernel, size_t smem) {
+  check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem),
+        "shared memory limit");
+}
+
 template <int BN, int STAGES>
 size_t smem_bytes() {
   return 1024 + (size_t) STAGES * (BM * BK * 2 + BN * BK * 2) + (2 * STAGES + 1) * 8 + 16;
@@ -812,14 +821,8 @@ size_t smem_bytes() {
 template <int BN, int STAGES>
 void launch(const CUtensorMap &ta, const CUtensorMap &tb, int M, int N, int K, const Epi &ep,
             int *err, cudaStream_t s) {
-  static bool attr = false;
-  size_t smem = smem_bytes<BN, STAGES>();
-  if (!attr) {
-    check(cudaFuncSetAttribute(k_gemm_tn<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int) smem),
-          "gemm smem attribute");
-    attr = true;
-  }
+  const size_t smem = smem_bytes<BN, STAGES>();
+  allow_smem((const void *) k_gemm_tn<BN, STAGES>, smem);
   dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN);
   k_gemm_tn<BN, STAGES><<<grid, NT, smem, s>>>(ta, tb, M, N, K, ep, err);
   check(cudaGetLastError(), "k_gemm_tn");
@@ -857,14 +860,9 @@ struct TrainPlan {
 };
 
 TrainPlan *train_plan(const TrainArgs &t) {
-  static const bool attr = [] {
-    for (const void *k : {(const void *) k_train_layer<0>, (const void *) k_train_layer<1>,
-                          (const void *) k_train_layer<2>, (const void *) k_train_dw})
-      check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) train_smem()),
-            "training smem attribute");
-    return true;
-  }();
-  (void) attr;
+  for (const void *k : {(const void *) k_train_layer<0>, (const void *) k_train_layer<1>,
+                        (const void *) k_train_layer<2>, (const void *) k_train_dw})
+    allow_smem(k, train_smem());
   const int M = t.members, B = t.B;
   auto act = [&](const void *p, int cols) { return make_map(p, M * B, cols, cols, BM); };
   TrainPlan *pl = new TrainPlan;
@@ -956,14 +954,12 @@ void mlp_ensemble(const void *xf, int n, const void *w1s, const void *w2s, const
   CUtensorMap t2 = make_map(w2s, members * ENS_H, ENS_H, ENS_H, ENS_H);
   CUtensorMap t3 = make_map(w3s, members * ENS_H, ENS_H, ENS_H, ENS_H);
   CUtensorMap t4 = make_map(w4s, members * ENS_OUT, ENS_H, ENS_H, 32);
-  const size_t smem = 1024 + ENS_X_BYTES + ENS_A_BYTES + (size_t) ENS_STAGES * ENS_W_BYTES +
-                      sizeof(float) * members * ENS_BSTRIDE + (2 * ENS_STAGES + 2) * 8 + 16;
-  static size_t attr = 0;
-  if (smem > attr) {
-    check(cudaFuncSetAttribute(k_mlp_ensemble, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem),
-          "ensemble smem attribute");
-    attr = smem;
-  }
+  auto bytes = [](int m) {
+    return 1024 + ENS_X_BYTES + ENS_A_BYTES + (size_t) ENS_STAGES * ENS_W_BYTES +
+           sizeof(float) * m * ENS_BSTRIDE + (2 * ENS_STAGES + 2) * 8 + 16;
+  };
+  const size_t smem = bytes(members);
+  allow_smem((const void *) k_mlp_ensemble, bytes(ENS_MAX_MEMBERS));
   EnsArgs a{bias, norm, mean, spread, n, members, err, count};
   k_mlp_ensemble<<<(n + BM - 1) / BM, ENS_NT, smem, s>>>(tx, t1, t2, t3, t4, a);
   check(cudaGetLastError(), "k_mlp_ensemble");
