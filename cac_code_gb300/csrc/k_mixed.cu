@@ -2841,11 +2841,13 @@ static size_t stencil_smem(const Stencil &st, int pass, int teams) {
          sizeof(float2) * (size_t) teams * team_float2(pass == 1 ? 0 : st.nf);
 }
 
-static bool stencil_fits(const Stencil &st, int pass) {
+// (a launch holds what the pass from the lists needs, which it falls back to; fused_fits
+// allows tables up to the last byte of a block, the stencil's kernels have a static part)
+static bool stencil_fits(const Stencil &st, int pass, size_t lists_smem) {
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  return stencil_smem(st, pass, STENCIL_TEAMS) + 1024 <= (size_t) optin;  // and the static part
+  return std::max(lists_smem, stencil_smem(st, pass, STENCIL_TEAMS)) + 1024 <= (size_t) optin;
 }
 
 // The pass and the exact pass over the elements that it listed, in the same order of
@@ -2864,6 +2866,8 @@ static int launch_stencil(const FusedArgs &a, const Stencil &st, int pass, const
     // (blocks for the passes from the lists, which the stencil's absence falls back to)
     const int g = persistent_grid((const void *) k, B, smem, 32LL * (a.e_end - a.e_begin));
     k<<<g, B, smem, s>>>(a, st, cap, tab, e.nr, (float) e.rdr, in, out);
+    // (at once: this kernel's error was seen to be gone after the next one's first launch)
+    check(cudaGetLastError(), "elem_stencil");
   };
   if (pass == 2 && a.skip) {
     check(cudaMemsetAsync(st.todo, 0, sizeof(int), s), "unskipped");
@@ -2909,6 +2913,7 @@ static int launch_fused(const FusedArgs &a, int pass, const float4 *tab, const E
       }
     const int g = persistent_grid((const void *) k, B, smem, items);
     k<<<g, B, smem, s>>>(a, args...);
+    check(cudaGetLastError(), "elem_fused");
     persistent_grid((const void *) fix, B, smem, items);
     fix<<<g, B, smem, s>>>(a, args...);
     return 2;
@@ -2994,7 +2999,10 @@ int elem_fused(const MixedElems &m, const FusedTables &t, int pass, const float4
   // the stencil: by the whole number of elements (the caller's choice), never by this
   // launch's part of them, so that a step in parts sums in the same order as one in one
   const Stencil *st =
-      eam && t.variant == 1 && t.stencil.state && stencil_fits(t.stencil, pass) ? &t.stencil : nullptr;
+      eam && t.variant == 1 && t.stencil.state &&
+              stencil_fits(t.stencil, pass, table + sizeof(float) * FUSED_WARP_FLOATS * (full / 32))
+          ? &t.stencil
+          : nullptr;
   const int B = st || (eam && warps >= 8) ? full : (int) std::min<long long>(full, 32 * std::max(1LL, warps));
   const bool few = warps < 8 && t.variant == 1 && !st;
   int n;

@@ -5,6 +5,7 @@ import pytest
 
 from cac_code_gb300 import cacg
 from cac_code_gb300 import workloads as W
+from test_gpu_fused import rel_err
 from test_gpu_mixed import _host_array
 from test_gpu_stencil import _model, eam_file  # noqa: F401  (eam_file: a fixture)
 
@@ -104,3 +105,25 @@ def test_band_width_changes_no_bit(cacg_lib, eam_file, shape):  # noqa: F811
     assert np.array_equal(f0.view(np.int64), f1.view(np.int64))
     for k in ("nodex", "nodev", "nodef"):
         assert np.array_equal(e0[k], e1[k]), k
+
+
+def test_tables_that_fill_a_block(cacg_lib, alike, tmp_path):
+    """Splines of 4,266 knots: the force pass from the lists takes all shared memory of a
+    block but 16 bytes, more than the stencil's kernel can have beside its static part."""
+    m, cfg = alike
+    eam = W.write_eam(str(tmp_path / "Cu_4266.eam"), 4266)
+    out = {}
+    for mode in (cacg.MIXED, cacg.FP64_EXACT):
+        s = cacg.System(0)
+        try:
+            W.configure_system(s, m, cfg, eam)
+            s.set_precision(mode)
+            s.init()
+            s.run(0)
+            s.pair_ecompute()
+            out[mode] = s.elements()["nodef"].copy()
+            assert mode != cacg.MIXED or s.counts()["elem_fused"] == 1
+        finally:
+            s.close()
+    rms, mx = rel_err(out[cacg.MIXED], out[cacg.FP64_EXACT])
+    assert rms <= 1e-4 and mx <= 1e-4, (rms, mx)
