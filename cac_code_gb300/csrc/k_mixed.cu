@@ -3003,10 +3003,12 @@ int elem_fused(const MixedElems &m, const FusedTables &t, int pass, const float4
               stencil_fits(t.stencil, pass, table + sizeof(float) * FUSED_WARP_FLOATS * (full / 32))
           ? &t.stencil
           : nullptr;
-  const int B = st || (eam && warps >= 8) ? full : (int) std::min<long long>(full, 32 * std::max(1LL, warps));
+  // EAM in the arrangements 0 and 2 keeps their full blocks with staged tables
+  const bool whole = eam && (st || warps >= 8 || t.variant != 1);
+  const int B = whole ? full : (int) std::min<long long>(full, 32 * std::max(1LL, warps));
   const bool few = warps < 8 && t.variant == 1 && !st;
   int n;
-  if (eam && B < 256)  // few elements: one arrangement, tables unstaged
+  if (eam && few)  // tables unstaged
     n = launch_fused<1, false>(a, pass, tab, e, table, B, few, lj1, lj2, erho_in, erho_out, nodef, nullptr, s);
   else if (t.variant == 1)
     n = launch_fused<1, true>(a, pass, tab, e, table, B, few, lj1, lj2, erho_in, erho_out, nodef, st, s);
