@@ -580,11 +580,16 @@ struct cacg_context {
     float c = (float) (cutsq - cut_guard(cutsq, 1.0));
     return std::nextafter(std::nextafter(c, -3.0e38f), -3.0e38f);
   }
-  double cut_guard(double cutsq, double nu) const {
+  // the coordinates that the bounds hold for
+  double cut_range() const {
     double X = 0.0;
     for (int d = 0; d < 3; d++)
       X = std::max(X, std::max(std::fabs(lo[d]), std::fabs(hi[d])) + cutghost[d] + max_size +
                           10.0 * skin + 1.0);
+    return X;
+  }
+  double cut_guard(double cutsq, double nu) const {
+    const double X = cut_range();
     const double u = std::ldexp(1.0, -24);
     const double rn = std::max(cutneighmax, std::sqrt(cutsq));
     const double delta = 2.0 * nu * u * X * 1.001 + u * (rn + 1.0);
@@ -2493,6 +2498,8 @@ void cacg_context::neighbor_build() {
   launch_gather_bin_x_atoms(d_bmem.p, d_x.p, d_bxf.p, nall, s);
   const float band_hi = cut_pass(cutneighmaxsq);
   const float band_lo = cut_surely(cutneighmaxsq);
+  // an atom within this has its neighbors within cut_range()
+  const float range = (float) ((cut_range() - 1.001 * cutneighmax) * 0.999999);
   launches += 7;
   stride = (nlocal + 31) / 32 * 32;
   d_num.ensure(nlocal, s);
@@ -2500,7 +2507,7 @@ void cacg_context::neighbor_build() {
     d_list.ensure((size_t) maxneigh * stride, s);
     check(cudaMemsetAsync(d_misc.p + 2, 0, sizeof(int), s), "memset");
     launch_atom_list(d_x.p, d_abin.p, d_bstart.p, d_bxf.p, d_runs.p, nruns, bins.mbins, nlocal,
-                     cutneighmaxsq, band_lo, band_hi, maxneigh, stride, d_num.p, d_list.p,
+                     cutneighmaxsq, band_lo, band_hi, range, maxneigh, stride, d_num.p, d_list.p,
                      d_misc.p + 2, s);
     launches++;
     check(cudaMemcpyAsync(h_pin + 1, d_misc.p + 1, sizeof(int) * 2, cudaMemcpyDeviceToHost, s), "ovf");

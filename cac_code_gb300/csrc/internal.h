@@ -186,10 +186,11 @@ void launch_gather_bin_x_elems(const int *members, const double *ex, double4 *bx
 
 // ---- neighbor lists (k_neigh.cu) ----
 // bxf: members in bin order (float xyz, index); runs: first offset and length of
-// the stencil's bins that follow each other; [lo, hi]: decided in FP64
+// the stencil's bins that follow each other; [lo, hi]: decided in FP64, as is every
+// distance of an atom with a coordinate beyond range
 void launch_atom_list(const double4 *x, const int *bin, const int *bstart, const float4 *bxf,
                       const int2 *runs, int nruns, int mbins, int nlocal, double cutsq, float lo,
-                      float hi, int maxneigh, int stride, int *num, int *list, int *overflow,
+                      float hi, float range, int maxneigh, int stride, int *num, int *list, int *overflow,
                       cudaStream_t s);
 void launch_elem_list(const double *ex, const int *bin, const int *bstart, const int *bmem,
                       const double4 *bx, const int *stencil, int nstencil, int mbins, int nlocal,
