@@ -16,6 +16,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <thread>
@@ -432,6 +433,15 @@ struct Net {
     return t;
   }
 
+  // the step's arrays given back
+  void release_batch() {
+    for (int l = 0; l < 4; l++)
+      for (auto *b : {&h[l], &ht[l], &gr[l], &grt[l]}) b->release();
+    for (auto &b : z) b.release();
+    tb.release();
+    g4_rows = 0;
+  }
+
   void gather(const gemm::TrainArgs &t, const bf16 *xall, const float *tall, const int *idx,
               long istride, int n) {
     k_gather<<<dim3(t.B / 32, t.members), 256, 0, stream>>>(xall, tall, idx, istride, n, t.B, h[0].p,
@@ -479,8 +489,9 @@ struct Net {
     check(cudaGetLastError(), "gradients");
   }
 
-  void adam(const gemm::TrainArgs &t, float lr) {
-    UpdateArgs a = update_args(0);
+  // of t's members, the first of which is `first`
+  void adam(const gemm::TrainArgs &t, int first, float lr) {
+    UpdateArgs a = update_args(first);
     a.B = t.B;
     a.lr = lr;
     a.b1 = 0.9f;
@@ -629,6 +640,12 @@ void upload_set(Net &N, const float *x, const float *t, long long n) {
     N.tf.ensure((size_t) n * MLP_OUT + 1, s);
     cacg::mlp::targets(N.rt.p, n, N.d_norm.p, N.tf.p, s);
   }
+  // large ones make room for what the call needs next
+  for (cacg::DBuf<float> *b : {&N.raw, &N.rt})
+    if (b->cap * sizeof(float) > Net::KEEP_BYTES) {
+      N.sync();
+      b->release();
+    }
 }
 
 }  // namespace
@@ -811,9 +828,32 @@ int cacg_mlp_train(cacg_mlp m, const float *x, const float *t, long long n, int 
   };
   start(0);
   upload_set(N, x, t, n);
-  const cacg::gemm::TrainArgs ta = N.batch(0, members, batch, batch);
+  // All members at a time fill the SMs at usual batches; their arrays take 10 KB a row and
+  // member, so with batches of millions of rows as many at a time as the device has room for
+  // (a member's step needs nothing of the others').
+  int at_once = members;
+  while (true) {
+    try {
+      N.batch(0, at_once, batch, batch);
+      break;
+    } catch (const CudaError &e) {
+      if (e.code != cudaErrorMemoryAllocation || at_once == 1) throw;
+      cudaGetLastError();
+      N.release_batch();
+      at_once = (at_once + 1) / 2;
+    }
+  }
   N.loss.ensure((size_t) nbatch * members * tiles, N.stream);
-  Plan plan(ta);
+  struct Group {
+    int first;
+    cacg::gemm::TrainArgs ta;
+    std::unique_ptr<Plan> plan;
+  };
+  std::vector<Group> groups;
+  for (int k = 0; k < members; k += at_once) {
+    const cacg::gemm::TrainArgs ta = N.batch(k, std::min(at_once, members - k), batch, batch);
+    groups.push_back({k, ta, std::unique_ptr<Plan>(new Plan(ta))});
+  }
   cacg::DBuf<int> didx;
   const long long istride = batch * nbatch;
   didx.ensure((size_t) istride * members, N.stream);
@@ -825,11 +865,13 @@ int cacg_mlp_train(cacg_mlp m, const float *x, const float *t, long long n, int 
       cacg::check(cudaMemcpyAsync(didx.p + k * istride, perm[ep & 1][k].data(), sizeof(int) * istride,
                                   cudaMemcpyHostToDevice, N.stream), "perm");
     if (ep + 1 < epochs) start(ep + 1);  // into the other buffers
-    for (long long b = 0; b < nbatch; b++) {
-      N.gather(ta, N.xf.p, N.tf.p, didx.p + b * batch, istride, batch);
-      cacg::gemm::train_passes(*plan.p, N.loss.p + (size_t) b * members * tiles, N.stream);
-      N.adam(ta, lr_ep);
-    }
+    for (long long b = 0; b < nbatch; b++)
+      for (const Group &q : groups) {
+        N.gather(q.ta, N.xf.p, N.tf.p, didx.p + q.first * istride + b * batch, istride, batch);
+        cacg::gemm::train_passes(*q.plan->p, N.loss.p + ((size_t) b * members + q.first) * tiles,
+                                 N.stream);
+        N.adam(q.ta, q.first, lr_ep);
+      }
     N.sync();  // the shuffles' buffers are reused two epochs on
     N.adam_steps += nbatch;
   }
