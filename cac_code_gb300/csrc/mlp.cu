@@ -571,6 +571,8 @@ struct MlpError {
   if (!m) return CACG_EINVAL; \
   try {                       \
     cacg::check(cudaSetDevice(m->net.device), "cudaSetDevice");
+// (an error leaves nothing of the call in flight: a copy from or to the caller's pinned
+// memory may still run)
 #define MLP_END                                                            \
   return CACG_OK;                                                          \
   }                                                                        \
@@ -579,10 +581,12 @@ struct MlpError {
     return e.code;                                                         \
   }                                                                        \
   catch (const CudaError &e) {                                             \
+    cudaStreamSynchronize(m->net.stream);                                  \
     m->net.err = std::string(e.where) + ": " + cudaGetErrorString(e.code); \
     return CACG_ECUDA;                                                     \
   }                                                                        \
   catch (const std::bad_alloc &) {                                         \
+    cudaStreamSynchronize(m->net.stream);                                  \
     m->net.err = "host allocation failed";                                 \
     return CACG_ENOMEM;                                                    \
   }
