@@ -563,10 +563,10 @@ __device__ __forceinline__ void train_end(unsigned tmem) {
   }
 }
 
-// D[128][bn] = sum over nk k-tiles (from tile k0) of A rows ya.. and B rows yb..;
+// D[128][bn] = sum over nk k-tiles of A rows ya.. and B rows yb..;
 // thread 0 streams and issues, all threads wait: true when D is complete
 __device__ __forceinline__ bool train_mma(const TrainSmem &m, unsigned tmem, const CUtensorMap *ta,
-                                          const CUtensorMap *tb, int k0, int nk, int ya, int yb,
+                                          const CUtensorMap *tb, int nk, int ya, int yb,
                                           int bn, int *err, int *s_fail) {
   if (threadIdx.x == 0) {
     const unsigned idesc = idesc_bf16(bn), bytes = TR_A + (unsigned) bn * BK * 2;
@@ -576,8 +576,8 @@ __device__ __forceinline__ bool train_mma(const TrainSmem &m, unsigned tmem, con
       const int st = kt % TR_STAGES;
       const unsigned fb = smem_u32(m.bars + st);
       mbar_expect_tx(fb, bytes);
-      tma_load_2d(smem_u32(m.sa + st * TR_A), ta, (k0 + kt) * BK, ya, fb);
-      tma_load_2d(smem_u32(m.sb + st * TR_B), tb, (k0 + kt) * BK, yb, fb);
+      tma_load_2d(smem_u32(m.sa + st * TR_A), ta, kt * BK, ya, fb);
+      tma_load_2d(smem_u32(m.sb + st * TR_B), tb, kt * BK, yb, fb);
       issued++;
     };
     for (int kt = 0; kt < TR_STAGES && kt < nk; kt++) load(kt);
@@ -650,7 +650,7 @@ k_train_layer(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CU
   const int member = blockIdx.y, r = blockIdx.x * BM + q * 32 + lane;  // row within the member
   const size_t grow = (size_t) member * L.B + r;
   const unsigned tmem = train_begin(sm, &s_fail);
-  const bool ok = train_mma(sm, tmem, &ta, &tb, 0, L.nk, member * L.B + blockIdx.x * BM,
+  const bool ok = train_mma(sm, tmem, &ta, &tb, L.nk, member * L.B + blockIdx.x * BM,
                             member * L.brows, L.bn, L.err, &s_fail);
   const unsigned tl = tmem + ((unsigned) (q * 32) << 16);
   if (ok && KIND != 1) {
@@ -755,7 +755,7 @@ k_train_dw(const __grid_constant__ TrainDwMaps maps, TrainDw d) {
   const int arows = l == 3 ? TR_OUT : TR_H, brows = l == 0 ? TR_IN : TR_H, ldw = l == 0 ? 32 : TR_H;
   const int bn = l == 0 ? TR_IN : 128;
   const unsigned tmem = train_begin(sm, &s_fail);
-  const bool ok = train_mma(sm, tmem, &maps.a[l], &maps.b[l], 0, d.B / BK, member * arows + rt * BM,
+  const bool ok = train_mma(sm, tmem, &maps.a[l], &maps.b[l], d.B / BK, member * arows + rt * BM,
                             member * brows + ct * 128, bn, d.err, &s_fail);
   const int row = rt * BM + q * 32 + lane;
   if (ok) {

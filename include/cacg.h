@@ -257,8 +257,12 @@ int cacg_mlp_moments(cacg_mlp m, const float *x, const float *t, long long n, in
    t[n][24] and its gradient with respect to every parameter (no update) */
 int cacg_mlp_loss_grad(cacg_mlp m, int member, const float *x, const float *t, int n,
                        double *loss, float *grad);
-/* Adam over shuffled whole batches (batch a multiple of 128) for every member;
-   *loss = mean normalised loss of the last epoch */
+/* Adam over shuffled whole batches (batch a multiple of 128) for every member, the
+   learning rate falling from lr to lr / 20 by a cosine over the epochs; *loss = mean
+   normalised loss of the last epoch.  Adam's corrections for the moments' start at zero
+   are those of an epoch's first step throughout the epoch: 1 - b^(s + 1) with s the steps
+   done before the epoch (in a net's first epoch, with a steady gradient, steps of up to
+   2 lr around the tenth, lr at the hundredth and 0.4 lr at the thousandth) */
 int cacg_mlp_train(cacg_mlp m, const float *x, const float *t, long long n, int epochs, int batch,
                    float lr, unsigned long long seed, double *loss);
 /* ensemble mean[n][24] (force units) and spread[n] (largest per-output

@@ -1,4 +1,4 @@
-"""The surrogate's training passes at the edges of their tiles and batch parts,
+"""The surrogate's training passes at the edges of their tiles,
 against the numpy restatement."""
 import numpy as np
 import pytest
@@ -15,8 +15,8 @@ def _data(n, seed):
     return x, np.tanh(x @ w).astype(np.float32)
 
 
-# one row, a full tile, one row more, the first batch split in two parts (nine
-# 64-row tiles of at most eight a part) and one whose last part is shorter
+# one row, a full tile, one row more, a last tile of 65 rows, and one of 8 rows behind 39
+# full ones (the weight gradients run over 2, 2, 4, 10 and 80 k-tiles of 64 rows)
 @pytest.mark.parametrize("n", [1, 128, 129, 577, 5000])
 def test_loss_and_gradient(cacg_lib, n):
     x, t = _data(n, n)
