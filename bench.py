@@ -251,10 +251,6 @@ def cpu_leg(sample, cores, steps, warm, eam):
 # read once per pass; neighbor gathers count as cache hits).  c: counts after
 # the timed steps; L: lattice lines the lists reference (all rows, force rows).
 
-# elements (24 an SM of 152) beyond which the EAM passes share one stencil
-STENCIL_ELEMENTS = 24 * 152
-
-
 def kernel_bytes(name, c, mode, lines_all, lines_force, nae_lines):
     n = c["nlocal"]
     ne = c["enlocal"]
@@ -270,7 +266,7 @@ def kernel_bytes(name, c, mode, lines_all, lines_force, nae_lines):
         # the row start pair 8, culling counts 16, lattice indices 16 and the list
         # codes 4 n.  No line or site data reaches memory.
         n_scan = c["density_scan_entries"] / max(n, 1)
-        row = 0 if ne > STENCIL_ELEMENTS else 8 + 16 + 16 + 4 * scan_e
+        row = 0 if c["elem_stencil"] else 8 + 16 + 16 + 4 * scan_e
         return {
             "atom1": n * (16 + 4 + 4 * n_scan + 4 + 4 * n_s + 8 + 4),
             "atom2": n * (16 + 4 + 4 * n_s + 4 + 24),
@@ -309,18 +305,37 @@ def kernel_bytes(name, c, mode, lines_all, lines_force, nae_lines):
 
 
 # FP64 operations per launch of the plain FP64 path's kernels (a multiply and
-# an add count two, whichever unit carries them out).  Atom density pass:
-# difference, squared distance, root, index and cubic per short-list entry (20);
-# atom force pass: 45 per entry (two splines, the derivative terms and the force
-# components); element force pass, per pair of a Gauss row, with as many pairs in
-# reach as an atom has: the site's position 45, difference and squared distance 8,
-# root and index 14, density and F' 24, splines 14, derivative terms and force 15.
+# an add count two), first those that the FP64 unit carries out, then those that
+# the integer units do.  Atom density pass: difference, squared distance, root,
+# index and cubic per short-list entry (20); atom force pass: 45 per entry (two
+# splines, the derivative terms and the force components); element force pass, per
+# pair of a Gauss row with a site of its element within the cutoff: difference and
+# squared distance 8, root and index 14, density and F' 24, splines 14, derivative
+# terms and force 15; the site's position, 45, by the integer units (with more
+# elements than SMs, else by the FP64 unit as well).
 
-def fp64_flops(name, c):
-    n = max(c["nlocal"], 1)
-    n_s = c["short_entries"] / n
-    return {"atom1": 20.0 * c["nlocal"] * n_s, "atom2": 45.0 * c["nlocal"] * n_s,
-            "elem_force": 120.0 * c["force_rows"] * n_s}.get(name)
+def row_pairs(m, rc):
+    """Pairs of a Gauss row with the sites of its own element within rc, on the
+    undisplaced lattice, the mean over the rows."""
+    import numpy as np
+    from cac_code_gb300 import lattice as L
+    if not m.nelements:
+        return 0.0
+    et = m.etypes[0]
+    r = np.array([[i, j, k] for i in range(et.nae[0]) for j in range(et.nae[1])
+                  for k in range(et.nae[2])]) @ (L.PRIMITIVE * m.lattice_a)
+    rows = et.intp[et.weight > 0] @ (L.PRIMITIVE * m.lattice_a)
+    d2 = ((rows[:, None, :] - r[None, :, :]) ** 2).sum(axis=2)
+    return float(((d2 > 1e-4) & (d2 < rc * rc)).sum() / max(len(rows), 1))
+
+
+def fp64_flops(name, c, pairs, nsm):
+    n_s = c["short_entries"] / max(c["nlocal"], 1)
+    site = 45.0 * c["force_rows"] * pairs
+    soft = c["enlocal"] > nsm
+    return {"atom1": (20.0 * c["nlocal"] * n_s, 0.0), "atom2": (45.0 * c["nlocal"] * n_s, 0.0),
+            "elem_force": (75.0 * c["force_rows"] * pairs + (0.0 if soft else site),
+                           site if soft else 0.0)}.get(name, (None, None))
 
 
 # ----------------------------------------------------------------------------- arms
@@ -328,6 +343,7 @@ def fp64_flops(name, c):
 def run_ours(a, ws, rank, local):
     import numpy as np
     from cac_code_gb300 import build, cacg
+    from cac_code_gb300 import lattice as L
     from cac_code_gb300 import workloads as W
     build.build_library()
     tmp = tempfile.mkdtemp(prefix="cacbench_")
@@ -635,12 +651,17 @@ def run_ours(a, ws, rank, local):
                     (cs1["surrogate_accepted"] - cs0["surrogate_accepted"]) / (far * (nst + 2))
                     if far else 0.0)
             if name == "fp64":
-                # the plain FP64 path against the FP64 roof: its dominant kernel's
-                # FP64 operations per launch over its event time
+                # the plain FP64 path against the FP64 roof: what the FP64 unit does of
+                # its dominant kernel's operations per launch, over its event time
                 k64 = modes[name]["kernel_ms_per_step_eager"]
                 dk64 = max(k64, key=k64.get)
-                fl = fp64_flops(dk64, s.counts())
+                import torch
+                nsm = torch.cuda.get_device_properties(local).multi_processor_count
+                fl = fl_int = None
+                if cfg["pair"] == "eam":
+                    fl, fl_int = fp64_flops(dk64, s.counts(), row_pairs(m, L.AnalyticEAM().cut), nsm)
                 roof64 = {"bound": "fp64", "kernel": dk64, "ms": k64[dk64], "flops_per_launch": fl,
+                          "fp64_operations_by_the_integer_units": fl_int,
                           "achieved": fl / (k64[dk64] * 1e-3) if fl else None,
                           "peak": fp64_peak, "unit": "FLOP/s",
                           "frac": (fl / (k64[dk64] * 1e-3) / fp64_peak) if fl else None,

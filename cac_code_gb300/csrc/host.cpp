@@ -223,6 +223,7 @@ struct cacg_context {
   DBuf<float4> d_sten_mono;
   DBuf<unsigned> d_sten_min;
   int sten_slots = 0, sten_force = 0;
+  bool sten_used = false;  // the last force pass was the stencil's kernel
   // the site shape functions, the pair splines suit soft::dot_ready
   bool spa_soft = false, spline_soft = false;
   static bool soft_ready(const std::vector<double> &v) {
@@ -975,7 +976,7 @@ void cacg_context::command(const std::string &raw) {
     //   passes (0: chosen from the row count)
     // tune cull yes|no: the mixed EAM density pass skips list entries that no
     //   displacement since the list reorder can bring within the cutoff
-    // tune streams yes|no: a mixed step's atom and element chains on two streams
+    // tune streams yes|no: a step's atom and element chains on two streams
     // tune fprime fp64|fp32: F'(rho) of the atoms in the mixed density pass
     // tune fused yes|no: the mixed element passes one warp per element
     //   (when every list entry references its row's own element)
@@ -1867,6 +1868,7 @@ void cacg_context::element_tables() {
   upload(d_wnf, wnf, s);
   // the shared stencil's slots: the distinct rows of nonzero weight and of the nodes
   sten_slots = 0;
+  sten_used = false;
   if (netypes == 1 && fused_types_ok && pair_style == 2 && inter_num[1] <= 4096) {
     std::vector<int> rows, slot;
     auto add = [&](int jj) {
@@ -2912,6 +2914,7 @@ void cacg_context::pair_ecompute_mixed() {
     stencil = mixed::Stencil{d_sten_rows.p, d_sten_rows.p + sten_slots, sten_slots, sten_force,
                              inter_num[1], d_sten_mono.p, d_sten_min.p, d_sten_num.p, d_sten_state.p,
                              nullptr};
+  sten_used = stencil.state && fused_variant == 1 && mixed::stencil_fits(stencil, 2, nr, nrho);
   if (fused) {
     kmark(KT_SITES, 1);
     kmark(KT_EPREP, 0);
@@ -5057,12 +5060,18 @@ int cacg_run_host(cacg_handle h, int nsteps, double *x, double *v, double *nodex
 int cacg_get_counts(cacg_handle h, long long *c, int n) {
   API_BEGIN
   if (h->elists_built && n > 13) h->ensure_need();
-  long long v[31] = {h->nlocal, h->nghost, 0, h->enlocal, h->enghost, 0, h->nrows, 0,
+  long long v[32] = {h->nlocal, h->nghost, 0, h->enlocal, h->enghost, 0, h->nrows, 0,
                      h->nrebuild, (long long) h->stencil.size(), h->ntimestep, h->nsites,
                      h->launches, h->nneed, h->nforce, 0, h->sur ? h->nfar : 0, 0, 0,
                      h->graph_steps, 0, 0, 0, h->nrebuild_atoms, 0,
                      (long long) h->h_nlines[0], (long long) h->h_nlines[1],
-                     h->fused_used ? 1LL : 0LL, h->loop_launches, h->host_decisions, 0};
+                     h->fused_used ? 1LL : 0LL, h->loop_launches, h->host_decisions, 0, 0};
+  if (h->sten_used && n > 31) {
+    int ok = 0;
+    check(cudaMemcpyAsync(&ok, h->d_sten_state.p, sizeof(ok), cudaMemcpyDeviceToHost, h->stream), "stencil");
+    h->sync();
+    v[31] = ok != 0;
+  }
   if (h->d_band.p) {
     int b = 0;
     check(cudaMemcpyAsync(&b, h->d_band.p + 2, sizeof(b), cudaMemcpyDeviceToHost, h->stream), "band");
@@ -5145,7 +5154,7 @@ int cacg_get_counts(cacg_handle h, long long *c, int n) {
       for (const int4 &x : nn) v[21] += level == 1 ? x.x : level == 2 ? x.y : x.z;
     }
   }
-  for (int i = 0; i < n && i < 31; i++) c[i] = v[i];
+  for (int i = 0; i < n && i < 32; i++) c[i] = v[i];
   API_END
 }
 

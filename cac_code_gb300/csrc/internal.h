@@ -196,7 +196,7 @@ void launch_elem_list(const double *ex, const int *bin, const int *bstart, const
                       const double4 *bx, const int *stencil, int nstencil, int mbins, int nlocal,
                       double cutsq, int maxneigh, int stride, int *num, int *list,
                       int *overflow, cudaStream_t s);
-// site_h (may be null): float copy of each site for the FP32 pre-tests
+// float copies of the atoms for the FP32 pre-tests; with the ghosts' positions first
 void launch_split_hi(const double4 *x, float4 *xh, int n, cudaStream_t s);
 void launch_forward_split(double4 *x, const int *send, int nlocal, int nghost, const SwapChain &c,
                           float4 *xh, cudaStream_t s);
@@ -305,7 +305,8 @@ void sites_needed(const double *nodex, const int *etype, const int *site_base, c
 void site_fp_needed(const double *erho, const int *etype, const int *site_base, const int *need,
                     const int *need_elem, int nneed, ElemTables t, EamTables e, double *site_fp,
                     cudaStream_t s);
-// per-step short lists (FP32 guarded cutoff test), used by both FP64 modes
+// per-step short lists of the rows (FP32 guarded cutoff test), of both FP64 modes, for
+// lists that the line codes do not hold
 void filter_rows(const double *nodex, const int *etype, const int *row_elem, const int *row_jj,
                  int nrows, const int *ipnum, const int *ipent, int rowstride,
                  const float4 *site_h, ElemTables t, float cut_pass, int only_needed, int *snum,
@@ -434,11 +435,6 @@ void line_masks(const int *row_start, const int *ent, const int4 *nnear_row, int
                 const Lattice &lat, const unsigned char *isforce, unsigned long long *mask,
                 unsigned long long *mask_f, long long nmask, const unsigned *gate,
                 cudaStream_t s);
-// the fused element passes (every list entry references its row's own
-// element): per element, one warp evaluates the node rows (pass 1: nodal
-// densities) or the rows of nonzero weight with the nodal gather (pass 2: EAM
-// forces; pass 0: LJ), pair vectors from the element's trilinear coefficient
-// vectors and lattice-index differences; guard-band pairs are decided in FP64
 // The shared stencil of the mixed EAM element passes (elem_stencil.cuh), for the
 // distinct rows of nonzero weight and of the nodes (slots).  state null: not in use.
 // From more than 24 elements an SM on: up to there the passes from the lists take one
@@ -456,6 +452,8 @@ struct Stencil {
   int *state;         // valid, counters, the coefficients' ranges (ST_*)
   int *todo;          // with a surrogate: elements that it leaves, their count first
 };
+// the passes' launches (pass 1 or 2) fit a block with tables of nr and nrho knots
+bool stencil_fits(const Stencil &st, int pass, int nr, int nrho);
 struct FusedTables {
   const float2 *node_hl;      // split nodes of this step
   const double *nodex;        // FP64 nodes
@@ -476,6 +474,11 @@ struct FusedTables {
   Stencil stencil;
 };
 bool fused_fits(int nr, int nrho);
+// the fused element passes (every list entry references its row's own
+// element): per element, one warp evaluates the node rows (pass 1: nodal
+// densities) or the rows of nonzero weight with the nodal gather (pass 2: EAM
+// forces; pass 0: LJ), pair vectors from the element's trilinear coefficient
+// vectors and lattice-index differences; guard-band pairs are decided in FP64
 // elements [e_begin, e_end) (e_end < 0: all local elements); the guard-band
 // exact pass runs after each launch, or with it (few elements); the number of launches
 int elem_fused(const MixedElems &m, const FusedTables &t, int pass, const float4 *tab,
@@ -520,7 +523,6 @@ void eam_force_atoms(const MixedAtoms &m, const float4 *ftab, const EamTables &e
                      const float *fp, double *f, cudaStream_t s);
 void lj_atoms(const MixedAtoms &m, const int *type, const float *lj1, const float *lj2,
               const float *cutsq_t, const double *cutsq64, double *f, cudaStream_t s);
-// every row's integration point: packed, and its double-single position
 // ip_reorder for the fused passes, in one launch (nall_e: elements whose nodes
 // become the reference); sm: of nve_nodes_split, or null pointers after node_split
 void fused_reorder(const float2 *node_hl, const int *etype, const int *row_first, const int *numint,
@@ -529,6 +531,7 @@ void fused_reorder(const float2 *node_hl, const int *etype, const int *row_first
                    int nlocal_e, int nall_e, float cutoff, int *ent_near, int4 *nnear_row,
                    float2 *node_ref, unsigned *eflags, const SplitMax &sm, const Stencil &st,
                    cudaStream_t s);
+// every row's integration point: packed, and its double-single position
 void row_q(const int *row_elem, const int *row_jj, const int *etype, const int *int_off,
            const float2 *spa_int_hl, const float2 *node_hl, int nrows, const PackGrid &pg,
            float4 *ip_q, float4 *ip_h, float4 *ip_l, cudaStream_t s);

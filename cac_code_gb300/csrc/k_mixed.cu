@@ -2841,13 +2841,19 @@ static size_t stencil_smem(const Stencil &st, int pass, int teams) {
          sizeof(float2) * (size_t) teams * team_float2(pass == 1 ? 0 : st.nf);
 }
 
+// the spline tables of an EAM pass
+static size_t eam_tables(int pass, int nr, int nrho) {
+  return sizeof(float4) * (pass == 1 ? (size_t) nr + 1 : FTAB_W * ((size_t) nr + 1) + nrho + 1);
+}
+
 // (a launch holds what the pass from the lists needs, which it falls back to; fused_fits
 // allows tables up to the last byte of a block, the stencil's kernels have a static part)
-static bool stencil_fits(const Stencil &st, int pass, size_t lists_smem) {
+bool stencil_fits(const Stencil &st, int pass, int nr, int nrho) {
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  return std::max(lists_smem, stencil_smem(st, pass, STENCIL_TEAMS)) + 1024 <= (size_t) optin;
+  const size_t lists = eam_tables(pass, nr, nrho) + sizeof(float) * FUSED_WARP_FLOATS * (fused_block(1) / 32);
+  return std::max(lists, stencil_smem(st, pass, STENCIL_TEAMS)) + 1024 <= (size_t) optin;
 }
 
 // The pass and the exact pass over the elements that it listed, in the same order of
@@ -2986,11 +2992,8 @@ int elem_fused(const MixedElems &m, const FusedTables &t, int pass, const float4
   a.rdrho = m.rdrho;
   a.frho = e.frho;
   a.rdrho64 = e.rdrho;
-  const bool force = pass != 1;
   const bool eam = pass != 0;
-  const size_t table =
-      eam ? sizeof(float4) * ((force ? FTAB_W : 1) * (size_t) (e.nr + 1) + (force ? e.nrho + 1 : 0))
-          : 0;
+  const size_t table = eam ? eam_tables(pass, e.nr, e.nrho) : 0;
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -2998,11 +3001,10 @@ int elem_fused(const MixedElems &m, const FusedTables &t, int pass, const float4
   const long long warps = ((long long) (e_end - e_begin) + nsm - 1) / std::max(nsm, 1);
   // the stencil: by the whole number of elements (the caller's choice), never by this
   // launch's part of them, so that a step in parts sums in the same order as one in one
-  const Stencil *st =
-      eam && t.variant == 1 && t.stencil.state &&
-              stencil_fits(t.stencil, pass, table + sizeof(float) * FUSED_WARP_FLOATS * (full / 32))
-          ? &t.stencil
-          : nullptr;
+  const Stencil *st = eam && t.variant == 1 && t.stencil.state &&
+                              stencil_fits(t.stencil, pass, e.nr, e.nrho)
+                          ? &t.stencil
+                          : nullptr;
   // EAM in the arrangements 0 and 2 keeps their full blocks with staged tables
   const bool whole = eam && (st || warps >= 8 || t.variant != 1);
   const int B = whole ? full : (int) std::min<long long>(full, 32 * std::max(1LL, warps));

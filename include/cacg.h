@@ -149,7 +149,9 @@ int cacg_run_host(cacg_handle h, int nsteps, double *x, double *v, double *nodex
    launches of the device step loop so far ("tune loop device") 29 rebuild
    decisions taken on the host so far (the device loop takes its own)
    30 element passes re-run so far because a pair of the element fell in the
-   guard band of the FP32 cutoff decision (fused passes; decided in FP64) */
+   guard band of the FP32 cutoff decision (fused passes; decided in FP64) 31 1 if
+   the last mixed EAM element passes took the stencil that all elements share
+   (many elements, alike), 0 if they walked the lists */
 int cacg_get_counts(cacg_handle h, long long *counts, int n);
 /* Atom::x/v/f (atom.h:40); all != 0 includes ghosts for x and tag */
 int cacg_get_atoms(cacg_handle h, int all, double *x, double *v, double *f, int *tag);

@@ -100,7 +100,7 @@ def test_band_width_changes_no_bit(cacg_lib, eam_file, shape):  # noqa: F811
         finally:
             s.close()
     (f0, e0, c0), (f1, e1, c1) = out
-    assert c1["elem_fused"] == 1
+    assert c1["elem_fused"] == 1 and c1["elem_stencil"] == (shape != "crooked")
     assert c1["band_reruns"] >= 2 * (1 + 8) * c1["enlocal"] > c0["band_reruns"]
     assert np.array_equal(f0.view(np.int64), f1.view(np.int64))
     for k in ("nodex", "nodev", "nodef"):
@@ -122,7 +122,8 @@ def test_tables_that_fill_a_block(cacg_lib, alike, tmp_path):
             s.run(0)
             s.pair_ecompute()
             out[mode] = s.elements()["nodef"].copy()
-            assert mode != cacg.MIXED or s.counts()["elem_fused"] == 1
+            c = s.counts()
+            assert mode != cacg.MIXED or (c["elem_fused"], c["elem_stencil"]) == (1, 0)
         finally:
             s.close()
     rms, mx = rel_err(out[cacg.MIXED], out[cacg.FP64_EXACT])
