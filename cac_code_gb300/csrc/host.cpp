@@ -2497,11 +2497,12 @@ void cacg_context::neighbor_build() {
   launch_coord2bin_atoms(d_x.p, nall, bins, d_abin.p, d_misc.p + 1, s);
   build_bins(d_abin.p, nall, bins.mbins, d_bcount, d_bstart, d_bmem, d_scan, s);
   d_bxf.ensure(nall, s);
-  launch_gather_bin_x_atoms(d_bmem.p, d_x.p, d_bxf.p, nall, s);
+  // (an atom beyond cut_range() has its neighbors beyond this, an atom within it none
+  // beyond cut_range() but beyond this)
+  const float range = (float) ((cut_range() - 1.001 * cutneighmax) * 0.999999);
+  launch_gather_bin_x_atoms(d_bmem.p, d_x.p, d_bxf.p, nall, range, s);
   const float band_hi = cut_pass(cutneighmaxsq);
   const float band_lo = cut_surely(cutneighmaxsq);
-  // an atom within this has its neighbors within cut_range()
-  const float range = (float) ((cut_range() - 1.001 * cutneighmax) * 0.999999);
   launches += 7;
   stride = (nlocal + 31) / 32 * 32;
   d_num.ensure(nlocal, s);
@@ -2509,7 +2510,7 @@ void cacg_context::neighbor_build() {
     d_list.ensure((size_t) maxneigh * stride, s);
     check(cudaMemsetAsync(d_misc.p + 2, 0, sizeof(int), s), "memset");
     launch_atom_list(d_x.p, d_abin.p, d_bstart.p, d_bxf.p, d_runs.p, nruns, bins.mbins, nlocal,
-                     cutneighmaxsq, band_lo, band_hi, range, maxneigh, stride, d_num.p, d_list.p,
+                     cutneighmaxsq, band_lo, band_hi, maxneigh, stride, d_num.p, d_list.p,
                      d_misc.p + 2, s);
     launches++;
     check(cudaMemcpyAsync(h_pin + 1, d_misc.p + 1, sizeof(int) * 2, cudaMemcpyDeviceToHost, s), "ovf");

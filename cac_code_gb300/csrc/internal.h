@@ -179,18 +179,18 @@ void launch_coord2bin_elems(const double *ex, int n, const BinGeom &g, int *bin,
 // counting sort by bin, members of a bin in ascending index order
 void build_bins(const int *bin, int n, int mbins, DBuf<int> &count, DBuf<int> &start,
                 DBuf<int> &members, DBuf<int> &scratch, cudaStream_t s);
+// (float x, y, z and the index; NaN for x beyond `range` in a coordinate)
 void launch_gather_bin_x_atoms(const int *members, const double4 *x, float4 *bxf, int n,
-                               cudaStream_t s);
+                               float range, cudaStream_t s);
 void launch_gather_bin_x_elems(const int *members, const double *ex, double4 *bx, int n,
                                cudaStream_t s);
 
 // ---- neighbor lists (k_neigh.cu) ----
 // bxf: members in bin order (float xyz, index); runs: first offset and length of
-// the stencil's bins that follow each other; [lo, hi]: decided in FP64, as is every
-// distance of an atom with a coordinate beyond range
+// the stencil's bins that follow each other; [lo, hi] and a NaN: decided in FP64
 void launch_atom_list(const double4 *x, const int *bin, const int *bstart, const float4 *bxf,
                       const int2 *runs, int nruns, int mbins, int nlocal, double cutsq, float lo,
-                      float hi, float range, int maxneigh, int stride, int *num, int *list, int *overflow,
+                      float hi, int maxneigh, int stride, int *num, int *list, int *overflow,
                       cudaStream_t s);
 void launch_elem_list(const double *ex, const int *bin, const int *bstart, const int *bmem,
                       const double4 *bx, const int *stencil, int nstencil, int mbins, int nlocal,

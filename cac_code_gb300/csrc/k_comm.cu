@@ -343,14 +343,16 @@ __global__ void k_bin_sort(const int *__restrict__ bin, int n, const int *__rest
   members_out[s0 + rank] = i;
 }
 
-// members in bin order: float coordinates and the index
+// members in bin order: float coordinates (NaN beyond the range) and the index
 __global__ void k_gather_bx_atoms(const int *__restrict__ mem, const double4 *__restrict__ x,
-                                  float4 *__restrict__ bxf, int n) {
+                                  float4 *__restrict__ bxf, int n, float range) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
   const int i = mem[p];
   const double4 c = x[i];
-  bxf[p] = make_float4((float) c.x, (float) c.y, (float) c.z, __int_as_float(i));
+  float4 f = make_float4((float) c.x, (float) c.y, (float) c.z, __int_as_float(i));
+  if (fmaxf(fabsf(f.x), fmaxf(fabsf(f.y), fabsf(f.z))) > range) f.x = NAN;
+  bxf[p] = f;
 }
 
 __global__ void k_gather_bx_elems(const int *__restrict__ mem, const double *__restrict__ ex,
@@ -514,9 +516,9 @@ void build_bins(const int *bin, int n, int mbins, DBuf<int> &count, DBuf<int> &s
 }
 
 void launch_gather_bin_x_atoms(const int *members, const double4 *x, float4 *bxf, int n,
-                               cudaStream_t s) {
+                               float range, cudaStream_t s) {
   if (n <= 0) return;
-  k_gather_bx_atoms<<<nblk(n, 256), 256, 0, s>>>(members, x, bxf, n);
+  k_gather_bx_atoms<<<nblk(n, 256), 256, 0, s>>>(members, x, bxf, n, range);
   check(cudaGetLastError(), "gather_bx_atoms");
 }
 

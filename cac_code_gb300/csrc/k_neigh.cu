@@ -26,8 +26,9 @@ inline int nblk(long long n, int t) { return (int) ((n + t - 1) / t); }
 // the float copies outside [lo, hi] (no float rounding moves a pair across the
 // cutoff there) and in the reference's FP64 arithmetic inside: of ~560
 // candidates a pair of FP64 units need not see more than the few in the band.
-// The band is for coordinates up to a range; an atom beyond it (one that left a
-// box with fixed boundaries) has all its candidates decided in FP64.
+// The band is for coordinates up to a range; a member beyond it (an atom that left
+// a box with fixed boundaries, or one near such an atom) has a NaN for a float
+// coordinate (launch_gather_bin_x_atoms), so that neither side of the band takes it.
 // One thread per atom with FP64 throughout took 1,133 us for 72,600 atoms.
 constexpr int AL_BLOCK = 256;
 
@@ -35,17 +36,13 @@ __global__ void __launch_bounds__(AL_BLOCK)
 k_atom_list(const double4 *__restrict__ x, const int *__restrict__ bin,
             const int *__restrict__ bstart, const float4 *__restrict__ bxf,
             const int2 *__restrict__ runs, int nruns, int mbins, int nlocal, double cutsq, float lo,
-            float hi, float range, int maxneigh, int stride, int *__restrict__ num, int *__restrict__ list,
+            float hi, int maxneigh, int stride, int *__restrict__ num, int *__restrict__ list,
             int *__restrict__ overflow) {
   const int i = (int) ((blockIdx.x * (long long) AL_BLOCK + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (i >= nlocal) return;
   const double4 xi = x[i];
   const float fx = (float) xi.x, fy = (float) xi.y, fz = (float) xi.z;
-  if (fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))) > range) {
-    lo = -1.f;
-    hi = INFINITY;
-  }
   const int ib = bin[i];
   int n = 0;
   for (int r0 = 0; r0 < nruns; r0 += 32) {
@@ -305,12 +302,12 @@ k_ip_list(const double *__restrict__ nodex, const double *__restrict__ ex,
 
 void launch_atom_list(const double4 *x, const int *bin, const int *bstart, const float4 *bxf,
                       const int2 *runs, int nruns, int mbins, int nlocal, double cutsq, float lo,
-                      float hi, float range, int maxneigh, int stride, int *num, int *list, int *overflow,
+                      float hi, int maxneigh, int stride, int *num, int *list, int *overflow,
                       cudaStream_t s) {
   if (nlocal <= 0) return;
   k_atom_list<<<nblk((long long) nlocal * 32, AL_BLOCK), AL_BLOCK, 0, s>>>(
-      x, bin, bstart, bxf, runs, nruns, mbins, nlocal, cutsq, lo, hi, range, maxneigh, stride,
-      num, list, overflow);
+      x, bin, bstart, bxf, runs, nruns, mbins, nlocal, cutsq, lo, hi, maxneigh, stride, num, list,
+      overflow);
   check(cudaGetLastError(), "atom_list");
 }
 
