@@ -596,6 +596,9 @@ struct TrainArgs {
   float *grad;                   // weight gradients [members][pstride]
   int *err;
 };
+// the shared memory that a net's kernels need, allowed on the current device: before the
+// first train_passes or mlp_ensemble there
+void allow_net();
 struct TrainPlan;  // the arrays' tensor maps, made once per call
 TrainPlan *train_plan(const TrainArgs &t);
 void train_plan_free(TrainPlan *p);

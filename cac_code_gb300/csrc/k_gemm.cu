@@ -804,10 +804,10 @@ CUtensorMap make_map(const void *ptr, int rows, int cols, int ld, int box_rows) 
   return m;
 }
 
-// Raises a kernel's limit of dynamic shared memory before a launch.  The limit belongs to
-// the device's context, so it is set each time: remembered once a process, it would be
-// missing on a second device and after a reset.  Always the same size for a kernel, so that
-// another thread's launch finds it large enough.
+// Raises a kernel's limit of dynamic shared memory on the current device.  The limit belongs
+// to the device, so nothing remembers it for the process: a net sets its kernels' when it is
+// made, k_gemm_tn its own at each launch.  Always the same size for a kernel, so that another
+// thread's launch finds it large enough.
 void allow_smem(const void *kernel, size_t smem) {
   check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem),
         "shared memory limit");
@@ -860,9 +860,6 @@ struct TrainPlan {
 };
 
 TrainPlan *train_plan(const TrainArgs &t) {
-  for (const void *k : {(const void *) k_train_layer<0>, (const void *) k_train_layer<1>,
-                        (const void *) k_train_layer<2>, (const void *) k_train_dw})
-    allow_smem(k, train_smem());
   const int M = t.members, B = t.B;
   auto act = [&](const void *p, int cols) { return make_map(p, M * B, cols, cols, BM); };
   TrainPlan *pl = new TrainPlan;
@@ -940,6 +937,18 @@ void train_passes(const TrainPlan &pl, double *loss, cudaStream_t s) {
   check(cudaGetLastError(), "train_passes");
 }
 
+static size_t ensemble_smem(int members) {
+  return 1024 + ENS_X_BYTES + ENS_A_BYTES + (size_t) ENS_STAGES * ENS_W_BYTES +
+         sizeof(float) * members * ENS_BSTRIDE + (2 * ENS_STAGES + 2) * 8 + 16;
+}
+
+void allow_net() {
+  for (const void *k : {(const void *) k_train_layer<0>, (const void *) k_train_layer<1>,
+                        (const void *) k_train_layer<2>, (const void *) k_train_dw})
+    allow_smem(k, train_smem());
+  allow_smem((const void *) k_mlp_ensemble, ensemble_smem(ENS_MAX_MEMBERS));
+}
+
 // The fused ensemble on normalised bf16 features xf[n][64]; weights stacked
 // over the members: w1s[m*256][64], w2s/w3s[m*256][256], w4s[m*24][256];
 // bias[m][792] (b1, b2, b3, b4).
@@ -954,12 +963,7 @@ void mlp_ensemble(const void *xf, int n, const void *w1s, const void *w2s, const
   CUtensorMap t2 = make_map(w2s, members * ENS_H, ENS_H, ENS_H, ENS_H);
   CUtensorMap t3 = make_map(w3s, members * ENS_H, ENS_H, ENS_H, ENS_H);
   CUtensorMap t4 = make_map(w4s, members * ENS_OUT, ENS_H, ENS_H, 32);
-  auto bytes = [](int m) {
-    return 1024 + ENS_X_BYTES + ENS_A_BYTES + (size_t) ENS_STAGES * ENS_W_BYTES +
-           sizeof(float) * m * ENS_BSTRIDE + (2 * ENS_STAGES + 2) * 8 + 16;
-  };
-  const size_t smem = bytes(members);
-  allow_smem((const void *) k_mlp_ensemble, bytes(ENS_MAX_MEMBERS));
+  const size_t smem = ensemble_smem(members);
   EnsArgs a{bias, norm, mean, spread, n, members, err, count};
   k_mlp_ensemble<<<(n + BM - 1) / BM, ENS_NT, smem, s>>>(tx, t1, t2, t3, t4, a);
   check(cudaGetLastError(), "k_mlp_ensemble");

@@ -673,6 +673,7 @@ int cacg_mlp_create(cacg_mlp *out, int device, int members, unsigned long long s
     for (int i = 0; i < MLP_IN; i++) m->net.norm[i] = 0.f, m->net.norm[MLP_IN + i] = 1.f;
     for (int i = 0; i < MLP_OUT; i++)
       m->net.norm[2 * MLP_IN + i] = 0.f, m->net.norm[2 * MLP_IN + MLP_OUT + i] = 1.f;
+    cacg::gemm::allow_net();
     m->net.upload_norm();
     m->net.init_params(seed);
   } catch (const MlpError &e) {
