@@ -24,7 +24,9 @@
 // enough (at most 1.5 times a mean list within r_c + CULL_D1).  It also keeps each
 // entry's least distance: a pass leaves out the entries that no displacement since
 // the reorder can have brought within the cutoff.  Otherwise the passes run one
-// warp per element from the lists.
+// warp per element from the lists, in the blocks of this launch (elements not alike,
+// densities and forces without a stencil / now: 3,664 37 + 71 / 27 + 67 us, 14,400 52 +
+// 113 / 40 + 99).
 //
 // Sums: FP32 over the entries of 8 consecutive stencil places, then double-single,
 // whatever was left out, so that leaving entries out changes no bit.
@@ -115,9 +117,9 @@ __device__ void stencil_build(const Stencil &st, const FusedLat &g, const int4 *
 // elements, a lane each, a warp a slot at a time; the distances as k_fused_reorder forms
 // them.  The entries come 32 at a time through shared memory: read one after another from
 // memory by one warp for all slots (which a chain of 2,000 and more loads is) the check
-// took 556 us for 3,664 elements alike, and 2,030 us for elements that are not (a whole
-// reorder of these now: 155 us, of 64,000 1,125, before 9,500).  One element that the
-// stencil does not stand for ends it for all blocks.
+// took 556 us for 3,664 elements alike, and 2,030 us for elements that are not (whole
+// reorders: 652 -> 152 and 1,960 -> 154 us; 64,000 elements 3,250 -> 1,072 and 10,000 ->
+// 1,125).  One element that the stencil does not stand for ends it for all blocks.
 constexpr int CHECK_NT = 256;
 
 __global__ void __launch_bounds__(CHECK_NT)

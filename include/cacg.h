@@ -232,7 +232,10 @@ int cacg_dump_elements(cacg_handle h, const char *path, int append);
    backward passes run on the tensor cores (BF16 operands, FP32 accumulation);
    weights are FP32 masters trained with Adam.  Parameters per member, in
    order: W1[256][32] b1[256] W2[256][256] b2[256] W3[256][256] b3[256]
-   W4[24][256] b4[24].  Arrays are host arrays. */
+   W4[24][256] b4[24].  Arrays are host arrays.  Between calls a net keeps the
+   device arrays of its training steps (10 KB a batch row and member) and of its
+   last data set (six buffers of up to 64 MB each); cacg_mlp_destroy gives them
+   back. */
 typedef struct cacg_mlp_t *cacg_mlp;
 /* members: 1..4 */
 int cacg_mlp_create(cacg_mlp *m, int device, int members, unsigned long long seed);
