@@ -18,7 +18,9 @@
 // and the splines are formed by the integer units (soft_fp64.cuh; the FP64 unit does
 // 20 of 31 instructions a pair in the density pass, 30 of 44 in the force pass):
 // 266,200 atoms 854 -> 594 and 1,199 -> 819 us, the FP64 unit still busy 84 %; LJ, 16,384
-// atoms, 86 -> 68 us.
+// atoms, 86 -> 68 us.  The distances take 8 or 16 bytes a list entry, more than the lists;
+// where the device has no room for them (from some 80 M atoms on) the force pass forms them
+// again, the same bits (STORED false).
 #pragma once
 #include "internal.h"
 
@@ -85,9 +87,26 @@ __device__ __forceinline__ double soft_rsq(double dx, double dy, double dz) {
 }
 #endif
 
+#ifndef FP64_EXACT_TU
+__device__ __forceinline__ double2 pair_r(double rsq) {
+  const double recip = rsqrt_nr(rsq);
+  return make_double2(rsq * recip, recip);
+}
+#else
+__device__ __forceinline__ double pair_r(double rsq) { return sqrt(rsq); }
+#endif
+
+__device__ __forceinline__ double pair_rsq(double dx, double dy, double dz) {
+#ifdef FP64_EXACT_TU
+  return soft_rsq(dx, dy, dz);
+#else
+  return dx * dx + dy * dy + dz * dz;
+#endif
+}
+
 // PASS 0: LJ forces; 1: EAM densities and F'(rho); 2: EAM forces from the
-// short lists and distances of pass 1
-template <int PASS>
+// short lists and distances (STORED) of pass 1
+template <int PASS, bool STORED>
 __global__ void __launch_bounds__(atom_nt(PASS))
 k_atoms64(Atoms64Args a, EamTables e, const LJTab *__restrict__ tab) {
   constexpr int ATOM_NT = atom_nt(PASS);
@@ -160,13 +179,20 @@ k_atoms64(Atoms64Args a, EamTables e, const LJTab *__restrict__ tab) {
         double fpair = 0.0;
         bool in;
         if (PASS == 2) {
-          const PairR pr = reinterpret_cast<const PairR *>(a.sr)[at];
+          PairR pr;
+          if (STORED) {
+            pr = reinterpret_cast<const PairR *>(a.sr)[at];
+          } else {
+            const double rsq = pair_rsq(dx, dy, dz);
+            in = rsq < e.cutforcesq;
+            pr = pair_r(rsq);
+          }
 #ifdef FP64_EXACT_TU
           const double r = pr;
 #else
           const double r = pr.x;
 #endif
-          in = !(r < 0.0);
+          if (STORED) in = !(r < 0.0);
           if (in) {
             double p;
             const int m = split_index(r * e.rdr + 1.0, e.nr - 1, p);
@@ -198,11 +224,7 @@ k_atoms64(Atoms64Args a, EamTables e, const LJTab *__restrict__ tab) {
             fpair = -psip * recip;
           }
         } else {
-#ifdef FP64_EXACT_TU
-          const double rsq = soft_rsq(dx, dy, dz);
-#else
-          const double rsq = dx * dx + dy * dy + dz * dz;
-#endif
+          const double rsq = pair_rsq(dx, dy, dz);
           const int ij = PASS == 0 ? ti + a.type[j] : 0;
           in = rsq < (PASS == 0 ? tab->cutsq[ij] : e.cutforcesq);
           if (PASS == 0) {
@@ -225,13 +247,11 @@ k_atoms64(Atoms64Args a, EamTables e, const LJTab *__restrict__ tab) {
             pr = make_double2(-1.0, 0.0);
 #endif
             if (in) {
+              pr = pair_r(rsq);
 #ifdef FP64_EXACT_TU
-              const double r = sqrt(rsq);
-              pr = r;
+              const double r = pr;
 #else
-              const double recip = rsqrt_nr(rsq);
-              const double r = rsq * recip;
-              pr = make_double2(r, recip);
+              const double r = pr.x;
 #endif
               double p;
               const int m = split_index(r * e.rdr + 1.0, e.nr - 1, p);
@@ -245,7 +265,7 @@ k_atoms64(Atoms64Args a, EamTables e, const LJTab *__restrict__ tab) {
             }
             s_t[my][0][k] = t;
             a.slist[at] = j;
-            reinterpret_cast<PairR *>(a.sr)[at] = pr;
+            if (STORED) reinterpret_cast<PairR *>(a.sr)[at] = pr;
           }
         }
         if (PASS != 1) {
@@ -301,7 +321,9 @@ k_atoms64(Atoms64Args a, EamTables e, const LJTab *__restrict__ tab) {
 // pass 0: LJ forces; 1: EAM densities, F'(rho), short lists; 2: EAM forces
 void atom_pass(const Atoms64Args &a, int pass, const EamTables &e, const void *ljtab, cudaStream_t s) {
   if (a.nlocal <= 0) return;
-  auto k = pass == 0 ? k_atoms64<0> : pass == 1 ? k_atoms64<1> : k_atoms64<2>;
+  auto k = pass == 0   ? k_atoms64<0, false>
+           : pass == 1 ? (a.sr ? k_atoms64<1, true> : k_atoms64<1, false>)
+                       : (a.sr ? k_atoms64<2, true> : k_atoms64<2, false>);
   k<<<(a.nlocal + AB - 1) / AB, atom_nt(pass), 0, s>>>(a, e, (const LJTab *) ljtab);
   check(cudaGetLastError(), "atom_pass");
 }

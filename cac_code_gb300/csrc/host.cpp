@@ -363,7 +363,9 @@ struct cacg_context {
   int nruns = 0;
   DBuf<int> d_num, d_list;
   DBuf<int> d_snum, d_slist;  // per-step short lists (FP32 guarded cutoff test)
-  DBuf<unsigned char> d_sr;   // and their distances (FP64 modes)
+  DBuf<unsigned char> d_sr;   // and their distances (FP64 modes), where they fit:
+  size_t sr_refused = SIZE_MAX;  // a size that the device had no room for
+  bool sr_kept = false;
   int maxneigh = 64, stride = 0;
   // elements
   DBuf<double> d_ex, d_nodex, d_nodev, d_nodef, d_nodexhold, d_erho, d_emass, d_diag, d_fip,
@@ -2704,13 +2706,25 @@ void cacg_context::pair_compute_pass(int pass) {
   const EamTables e = eamtab();
   if (pass == 1) {
     d_slist.ensure((size_t) maxneigh * stride, s);
-    d_sr.ensure((size_t) maxneigh * stride * (exact ? fp64_exact::pair_bytes() : fp64_fma::pair_bytes()),
-                s);
+    // (the distances of the pairs where the device has room for them)
+    const size_t bytes =
+        (size_t) maxneigh * stride * (exact ? fp64_exact::pair_bytes() : fp64_fma::pair_bytes());
+    if (bytes < sr_refused) {
+      try {
+        d_sr.ensure(bytes, s);
+      } catch (const CudaError &e) {
+        if (e.code != cudaErrorMemoryAllocation) throw;
+        cudaGetLastError();
+        d_sr.release();
+        sr_refused = bytes;
+      }
+    }
+    sr_kept = bytes <= d_sr.cap;
     d_rho.ensure(nall, s);
     d_fp.ensure(nall, s);
   }
   q.slist = d_slist.p;
-  q.sr = d_sr.p;
+  q.sr = sr_kept ? d_sr.p : nullptr;
   q.rho = d_rho.p;
   q.fp = d_fp.p;
   const int k = pass == 1 ? KT_ATOM1 : KT_ATOM2;

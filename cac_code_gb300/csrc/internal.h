@@ -218,7 +218,7 @@ struct Atoms64Args {
   int stride, nlocal;
   float cut_pass;
   int *snum, *slist;           // short lists: written by pass 1, read by pass 2
-  void *sr;                    // their distances (pair_bytes() each)
+  void *sr;                    // their distances (pair_bytes() each), or null: not kept
   double *rho, *fp, *f;
 };
 
